@@ -130,7 +130,7 @@ int ctx_panel_map(Ctx *c, void **host, void **dev) {
       c->panel_map = c->panel_map_dev = nullptr;
       return ctx_cuda(c, e, "mapped panel result");
     }
-    *reinterpret_cast<volatile uint32_t *>(static_cast<char *>(c->panel_map) + PANEL_FLAG_OFF) = 0u;
+    memset(c->panel_map, 0, PANEL_MAP_BYTES);  // no sequence number
     c->panel_seq = 0;
   }
   *host = c->panel_map;
@@ -987,6 +987,7 @@ void ctx_trim(Ctx *c) {
     c->buf[i] = nullptr;
     c->buf_bytes[i] = 0;
   }
+  c->inv_p = 0;  // BUF_INV went
   for (int i = 0; i < 4; ++i) {
     if (c->stage[i]) cudaFree(c->stage[i]);
     c->stage[i] = nullptr;

@@ -140,6 +140,11 @@ __device__ __forceinline__ void cp_async8(void *smem, const void *gmem, bool val
                "r"(valid ? 8 : 0)
                : "memory");
 }
+// 16 bytes, both addresses 16-byte aligned, past L1
+__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem)), "l"(gmem)
+               : "memory");
+}
 __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.wait_all;" ::: "memory");
 }

@@ -94,6 +94,9 @@ struct Ctx {
   // search publishes its result and a sequence number; created on first use.
   void *panel_map = nullptr, *panel_map_dev = nullptr;
   uint32_t panel_seq = 0;
+  // Modulus whose inverses BUF_INV holds (0: none).  They are written on the
+  // handle's stream; a change of stream waits for the old one.
+  uint32_t inv_p = 0;
   // Entries of the last Faugere-Lachartre CSR result kept in BUF_FL_CSR_V
   // (SIZE_MAX: none), for lela_cuda_fl_csr_fetch.
   size_t fl_csr_nnz = (size_t)-1;
@@ -155,7 +158,8 @@ enum BufSlot : int {
   BUF_PLUQ = 26,      // PLUQ: kept multipliers, assembled output, column order
   BUF_ELEM = 27,      // uint32 copies of Modular<uint8/uint16/float/double> operands
   BUF_TRANSFORM = 28, // reduced form's transform: kept multipliers, triangles, pivot columns
-  BUF_COUNT = 29,
+  BUF_INV = 29,       // inverses modulo Ctx::inv_p (panel search)
+  BUF_COUNT = 30,
 };
 
 // Grow-only allocation helpers; return ST_OK or ST_NOMEM.
@@ -185,7 +189,10 @@ constexpr size_t PANEL_MAP_BYTES = 4096, PANEL_FLAG_OFF = 4032;
 // next panel's lists only after that panel's search has signalled, which the
 // stream orders after the previous copy.
 constexpr size_t PANEL_PERM_OFF = 1024, PANEL_PERM_INTS = 256;
-static_assert(PANEL_PERM_OFF + PANEL_PERM_INTS * 4 <= PANEL_FLAG_OFF, "staging below the flag");
+// the Z/p search's result: words of a value and the sequence number
+// (echelon.cu)
+constexpr size_t PANEL_WORDS_OFF = 2048;
+static_assert(PANEL_PERM_OFF + PANEL_PERM_INTS * 4 <= PANEL_WORDS_OFF, "staging below the words");
 int ctx_panel_map(Ctx *c, void **host, void **dev);
 // Spin until *flag == seq (the work queued before the publishing kernel
 // included), checking the handle's stream for errors now and then and

@@ -84,6 +84,19 @@ struct PanelOut {
   uint32_t tq[EW];
 };
 
+// The host's copy of a panel's result, in mapped host memory: words of the
+// value (low half) and the search's sequence number (high half).  Each word
+// is written whole, so the host takes a word when its sequence number has
+// arrived and nothing orders the words among themselves.
+enum : int {
+  PANEL_W_T = 0,     // pivots (bits 0-7), U_P^-1 written (bit 8), an inverse failed (bit 9)
+  PANEL_W_LAST = 1,  // last_pos
+  PANEL_W_DET = 2,
+  PANEL_W_PIV = 4,   // per pivot: column, transposition target
+  PANEL_WORDS = PANEL_W_PIV + 2 * EW
+};
+static_assert(PANEL_WORDS_OFF + PANEL_WORDS * 8 <= PANEL_FLAG_OFF, "words below the flag");
+
 // Exact inverse of a unit x modulo p (any p < 2^32): extended Euclid on
 // unsigned remainders with 64-bit signed coefficients.  0 when gcd != 1.
 __device__ __forceinline__ uint32_t inv_exact_u32(uint32_t p, uint32_t x) {
@@ -272,422 +285,895 @@ __global__ void __launch_bounds__(HEADS_THREADS)
   if (threadIdx.x <= EW && s_hist[threadIdx.x]) atomicAdd(&hist[threadIdx.x], s_hist[threadIdx.x]);
 }
 
-// 2. The reference's pivot choice on the panel (see the file comment).
-// The window: the first wcap <= PW_R rows at or below i0, by position, with a nonzero
-// in the panel, kept in shared memory and eliminated eagerly without
-// division: when pivot row P (pivot value y) is chosen, every window row W
-// becomes y W - W[col] P.  So a window row holds S_t times its row reduced
-// by the t pivots so far (S_t = y_0 ... y_{t-1}); pivot rows move to PV,
-// holding S_k U_k.  Rows between window rows are zero in the panel and can
-// never hold a pivot.  The pivot of a column is the first window row, by
-// position, with a nonzero there; rows past the last window position are
-// reached only when no window row has one and the head histogram says one
-// of them may: they are then reduced by the same recurrence, in position
-// order.  At the end the S_k and the pivots x_k = y_k / S_k are inverted in
-// parallel.  Outputs: PanelOut; U (t x EW, row stride EW: the pivot rows'
-// final panel values) and the pivot inverses.  Resets *last_act to -1 and
-// hist[] to zero for the next panel.
+// Field arithmetic of the panel search, in three forms chosen by the host.
 //
-// Bookkeeping: the window is a list of entries sorted by position, entry ->
-// shared-memory slot (perm) and position (ppos), double-buffered and
-// rewritten each column (or, when only its first entry leaves, read from one
-// entry further on); wrow[slot] is the row index in D.  A transposition
-// (i, q) moves the row at position i to q: a window row keeps its entry
-// (with position q); a row outside the window (zero in the panel) is
-// recorded in p2r / stamp.  Rows past the window carry in head[] a lower
-// bound of the first nonzero column of their reduced panel part; cnt[h]
-// counts them by that bound.
-constexpr int PW_R = 80;                   // window rows
-// window rows padded to EW + 1 words: a column read across rows (the pivot
-// test, the multipliers) then touches every bank once
+// SearchSmall, 32 <= p <= 65521 (the largest prime below 2^16): signed
+// residues |v| <= p/2 + 5 and pivots inverted from a table of all inverses
+// (u16, 0: none), which the CTA holds in shared memory, so a row is reduced
+// with its true multiplier l: w - l P (NORM below).  Two products and one more
+// term are below 2 (p/2 + 5)^2 + p/2 + 5 <= 2147123215 < 2^31, and q =
+// (floor(x mu / 2^32) + 2^(s-1)) >> s with mu =
+// round(2^(32+s) / p) in [2^30, 2^31) is x / p rounded up to an error of
+// 1.25 / 2^s (s = 14 for p > 2^15, one less per halving of p), so |x - q p|
+// <= p/2 + 1.25 p / 2^s <= p/2 + 5, and x = 0 mod p gives q = x / p exactly:
+// a zero is stored as 0.  Below 32 s would be 1 or less.
+//
+// SearchMont and SearchWide reduce without division (an inverse costs more
+// than a whole column there): one elimination step is upd(y, w, na, P) = k (y
+// w + na P) and a product mul(a, b) = k a b, with a unit k fixed per form;
+// lin(s, w, a, P) = k (s w + a[0] P[0] + .. + a[3] P[3]); plain(a, b) = a b. A
+// window row then holds S_t times its reduced row with S_{t+1} = k S_t y_t,
+// whatever k is, so the reductions may carry a factor of their own.
+// neg(a) = -a, one() the identity of mul, canon(v) the residue in [0, p).
+struct SearchSmall {
+  using V = int;
+  using V4 = int4;
+  static constexpr bool NORM = true;
+  int p, mu, s, half;
+  const uint16_t *table;  // inverses of 0 .. p - 1
+  __host__ static bool takes(uint32_t p) { return p >= 32 && p <= 65521; }
+  __host__ static SearchSmall make(uint32_t p, const uint16_t *table) {
+    SearchSmall a;
+    a.p = (int)p;
+    a.s = 0;
+    while (((1ull << (33 + a.s)) + p) / (2ull * p) < (1ull << 30)) ++a.s;
+    a.mu = (int)(((1ull << (33 + a.s)) + p) / (2ull * p));
+    a.half = 1 << (a.s - 1);
+    a.table = table;
+    return a;
+  }
+  __device__ __forceinline__ int red(int x) const {
+    return x - ((__mulhi(x, mu) + half) >> s) * p;
+  }
+  __device__ __forceinline__ int load(uint32_t v) const {
+    return (int)v > (p >> 1) ? (int)v - p : (int)v;
+  }
+  // w - l P
+  __device__ __forceinline__ int step(int w, int l, int P) const { return red(w - l * P); }
+  // w - l[0] P[0] - .. - l[3] P[3]
+  __device__ __forceinline__ int lin(int w, const int4 &l, const int (&P)[4]) const {
+    return red(red(w - l.x * P[0] - l.y * P[1]) - l.z * P[2] - l.w * P[3]);
+  }
+  // a b, also for one factor in [0, p)
+  __device__ __forceinline__ int plain(int a, int b) const { return red(a * b); }
+  __device__ __forceinline__ int index(int v) const { return v < 0 ? v + p : v; }
+  __device__ __forceinline__ uint32_t canon(int v) const { return (uint32_t)index(v); }
+};
+
+// The inverses of 0 .. p - 1 modulo p < 2^16, 0 for those that have none.
+__global__ void inverse_table_kernel(uint32_t p, uint16_t *__restrict__ table) {
+  const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x < p) table[x] = (uint16_t)inv_exact_u32(p, x);
+}
+
+// SearchMont, other odd p < 2^31: canonical residues, Montgomery reduction
+// (P. Montgomery, 1985) with k = 2^-32: T = y w + na P < 2 p^2 and m p <
+// 2^32 p sum to less than 2^64, and (T + m p) / 2^32 < 2 p.
+struct SearchMont {
+  using V = uint32_t;
+  using V4 = uint4;
+  static constexpr bool NORM = false;
+  uint32_t p, np, r1, r2;  // -1/p mod 2^32, 2^32 mod p, 2^64 mod p
+  __host__ static bool takes(uint32_t p) { return (p & 1u) && p > 2 && p < 0x80000000u; }
+  __host__ static SearchMont make(uint32_t p) {
+    SearchMont a;
+    a.p = p;
+    uint32_t inv = p;  // Newton: 3 correct bits, doubled four times
+    for (int k = 0; k < 4; ++k) inv *= 2u - p * inv;
+    a.np = 0u - inv;
+    a.r1 = (uint32_t)((1ull << 32) % p);
+    a.r2 = (uint32_t)((uint64_t)a.r1 * a.r1 % p);
+    return a;
+  }
+  __device__ __forceinline__ uint32_t redc(uint64_t T) const {
+    const uint32_t m = (uint32_t)T * np;
+    const uint32_t r = (uint32_t)((T + (uint64_t)m * p) >> 32);
+    return r >= p ? r - p : r;
+  }
+  __device__ __forceinline__ uint32_t load(uint32_t v) const { return v; }
+  __device__ __forceinline__ uint32_t upd(uint32_t y, uint32_t w, uint32_t na, uint32_t P) const {
+    return redc((uint64_t)y * w + (uint64_t)na * P);
+  }
+  __device__ __forceinline__ uint32_t add(uint32_t a, uint32_t b) const {
+    const uint32_t r = a + b;  // below 2 p < 2^32
+    return r >= p ? r - p : r;
+  }
+  __device__ __forceinline__ uint32_t lin(uint32_t s0, uint32_t w, const uint4 &a,
+                                          const uint32_t (&P)[4]) const {
+    return add(add(upd(s0, w, a.x, P[0]), upd(a.y, P[1], a.z, P[2])), mul(a.w, P[3]));
+  }
+  __device__ __forceinline__ uint32_t mul(uint32_t a, uint32_t b) const {
+    return redc((uint64_t)a * b);
+  }
+  __device__ __forceinline__ uint32_t plain(uint32_t a, uint32_t b) const {
+    return mul(mul(a, b), r2);
+  }
+  __device__ __forceinline__ uint32_t neg(uint32_t a) const { return a ? p - a : 0u; }
+  __device__ __forceinline__ uint32_t one() const { return r1; }
+  __device__ __forceinline__ uint32_t canon(uint32_t v) const { return v; }
+};
+// SearchWide, any p < 2^32 (even moduli, p below 3 and p >= 2^31): canonical
+// residues, 64-bit Barrett reduction, k = 1.
+struct SearchWide {
+  using V = uint32_t;
+  using V4 = uint4;
+  static constexpr bool NORM = false;
+  ArithWide w;
+  uint32_t p;
+  __host__ static SearchWide make(uint32_t p) {
+    SearchWide a;
+    a.w = ArithWide::make(p);
+    a.p = p;
+    return a;
+  }
+  __device__ __forceinline__ uint32_t load(uint32_t v) const { return v; }
+  __device__ __forceinline__ uint32_t upd(uint32_t y, uint32_t x, uint32_t na, uint32_t P) const {
+    return w.dot2(y, x, na, P);
+  }
+  __device__ __forceinline__ uint32_t lin(uint32_t s0, uint32_t x, const uint4 &a,
+                                          const uint32_t (&P)[4]) const {
+    uint64_t s = (uint64_t)upd(s0, x, a.x, P[0]) + upd(a.y, P[1], a.z, P[2]) + w.mul(a.w, P[3]);
+    if (s >= p) s -= p;
+    return (uint32_t)(s >= p ? s - p : s);
+  }
+  __device__ __forceinline__ uint32_t mul(uint32_t a, uint32_t b) const { return w.mul(a, b); }
+  __device__ __forceinline__ uint32_t plain(uint32_t a, uint32_t b) const { return w.mul(a, b); }
+  __device__ __forceinline__ uint32_t neg(uint32_t a) const { return a ? p - a : 0u; }
+  __device__ __forceinline__ uint32_t one() const { return 1u % p; }
+  __device__ __forceinline__ uint32_t canon(uint32_t v) const { return v; }
+};
+
+// 2. The reference's pivot choice on the panel (see the file comment).
+// The window: the first wcap <= PW_R rows at or below i0, by position, with a
+// nonzero in the panel, kept in shared memory.  With NORM arithmetic a window
+// row holds its row reduced by the pivots so far; otherwise the elimination is
+// division-free: when pivot row P (pivot value y) is chosen, every window row
+// W becomes k (y W - W[col] P), so a window row holds S_t times its row
+// reduced by the t pivots so far (S_0 = 1, S_{t+1} = k S_t y_t), and at the end
+// S_t is inverted and the S_k^-1, the pivots x_k and their inverses follow
+// from scans of products.  Pivot rows move to PV (U_k, or S_k U_k).  Rows
+// between window
+// rows are zero in the panel and can never hold a pivot.  The pivot of a
+// column is the first window row, by position, with a nonzero there; rows
+// past the last window position are reached only when no window row has one
+// and the head histogram says one of them may: they are then reduced by the
+// same recurrence, in position order.
+// Outputs: PanelOut; U (t x EW, row stride EW: the pivot rows' final panel
+// values) and the pivot inverses; the host's copy of the result as words of
+// a value and the call's sequence number (hout), so that no fence orders
+// them.  Resets *last_act to -1 and hist[] to zero for the next panel.
+//
+// Blocks of PB = 4 columns.  Warp 0 alone chooses the pivots of a block: the
+// live rows in position order, entry e in register group e / 32 of lane e %
+// 32, the block's columns in registers; a column's pivot is the first lane of
+// a ballot, its entries come by shuffles, and the elimination runs on the
+// block's columns and keeps each row's coefficients of the block's pivot rows
+// (its multipliers l; or, division-free, the row's current value as sc times
+// its value before the block plus cf[j] times that of the pivot row of the
+// block's column j).  No barrier is on that chain.  The pivot row reduces to
+// zero by itself and so leaves.  Then all warps form the remaining columns of
+// the window rows and of the block's pivot rows from those coefficients (rows
+// on warps, columns on lanes).
+//
+// Bound: the instructions on warp 0's dependent chain.  Forms with one
+// barrier per column and all 16 warps on it (window in shared memory, lanes
+// on rows; or rows in registers, a warp per row) took 1640 cycles a column
+// (p = 65521, 64 x 64 window: the search of a panel of a dense 4096^2 matrix
+// 80 us, at 2^31 - 1 102 us), and blocks with a 96-bit rank mask, division-free
+// coefficients for every p and bookkeeping in lane 0, 965 + 520.
+//
+// Bookkeeping (warp 0): s_ent[e] / s_epos[e] are the slot and the position
+// of live entry e, rewritten per block.  A transposition (i, q) moves the row
+// at position i to q: if it is a window row, it is the first entry and takes
+// the pivot's entry; a row outside the window (zero in the panel) is recorded
+// in p2r / stamp.  wrow[slot] is the row index in D.  Rows past the window
+// carry in head[] a lower bound of the first nonzero column of their reduced
+// panel part; cnt[h] counts them by that bound.
+constexpr int PW_R = 80;               // window rows
+constexpr int PW_RPW = PW_R / PS_FAST; // window rows per warp
+constexpr int PW_G = (PW_R + 31) / 32; // most window rows per lane of warp 0
+constexpr int PB = 4;                  // columns per block
+static_assert(PW_R % PS_FAST == 0, "whole rows per warp");
+// window rows padded to EW + 1 words: a column read across rows touches
+// every bank once
 constexpr int PW_LD = EW + 1;
-constexpr size_t PW_SMEM = (size_t)PW_R * PW_LD * 4;  // dynamic shared memory: the window rows
-constexpr int PW_EU = (PW_R + 31) / 32;  // window list entries per lane
+// dynamic shared memory: the window rows, later the inverse and its scratch;
+// then the table of inverses (NORM)
+constexpr int PW_INV = EW * PW_LD + 32 * EW / 2;
+constexpr size_t PW_SMEM = (((size_t)(PW_R * PW_LD > PW_INV ? PW_R * PW_LD : PW_INV) * 4) + 15) / 16 * 16;
+constexpr size_t PW_TABLE = 65536 * 2;
+// positions a thread looks at per pass of the window's compaction
+constexpr int PW_U = 4;
 // rows to solve from which the panel's multipliers come from U_P^-1
 constexpr int SOLVE_INV_ROWS = 768;
 
-template <class A>
+template <class SA, class A>
 __global__ void __launch_bounds__(PS_THREADS, 1)
     panel_search_kernel(const uint32_t *__restrict__ D, size_t ld, int i0, int m, int c0, int w,
-                        A ar, uint8_t *__restrict__ head, const uint8_t *__restrict__ act,
+                        SA sa, A ar, uint8_t *__restrict__ head, const uint8_t *__restrict__ act,
                         int *__restrict__ hist, int *__restrict__ last_act, int *__restrict__ p2r,
                         int *__restrict__ stamp, int epoch, uint32_t *__restrict__ Uout,
                         uint32_t *__restrict__ xinv_out, uint32_t *__restrict__ Uinv_out,
-                        PanelOut *out, PanelOut *hout, volatile uint32_t *hflag, uint32_t seq,
-                        int wcap) {
+                        PanelOut *out, volatile uint64_t *hout, uint32_t seq, int wcap) {
+  using V = typename SA::V;
+  using V4 = typename SA::V4;
   extern __shared__ __align__(16) uint32_t dyn_w[];
-  uint32_t(*Wv)[PW_LD] = reinterpret_cast<uint32_t(*)[PW_LD]>(dyn_w);  // PW_R rows
-  __shared__ uint32_t PV[EW][EW];
-  __shared__ int perm[2][PW_R], ppos[2][PW_R];
-  __shared__ int wrow[PW_R];
-  __shared__ uint32_t s_red[PS_FAST][EW];  // rows past the window, reduced (one per warp)
-  __shared__ int s_pcol[EW];
-  __shared__ uint32_t s_y[EW], s_S[EW], s_x[EW], s_sinv[EW], s_yinv[EW], s_xi[EW];
+  V(*Wv)[PW_LD] = reinterpret_cast<V(*)[PW_LD]>(dyn_w);  // PW_R rows
+  const uint16_t *s_inv = reinterpret_cast<const uint16_t *>(dyn_w + PW_SMEM / 4);
+  __shared__ V PV[EW][EW];
+  __shared__ V4 s_coef[PW_R];         // per slot: its coefficients of the block's pivot rows
+  __shared__ V4 s_pcoef[PB];          // division-free: the same for the block's pivot rows,
+  __shared__ V s_psc[PB], s_sc;       // their scales, and the other rows'
+  __shared__ int s_pslot[PB];         // slot of the pivot of the block's column j (-1: none)
+  __shared__ int s_pt[PB];            // its index among the panel's pivots
+  __shared__ V s_red[PS_FAST][EW];    // rows past the window, reduced (one per warp)
+  __shared__ int s_ent[PW_R], s_epos[PW_R], wrow[PW_R];
+  __shared__ int s_pcol[EW], s_tq[EW];
+  __shared__ V s_y[EW], s_sinv[EW];   // pivot values (in window rows' scale), 1 / S_k
+  __shared__ uint32_t s_xi[EW], s_det;
   __shared__ int s_cnt[EW + 1];
-  __shared__ int s_first[PS_FAST], s_wcnt[PS_FAST];
+  __shared__ int s_first[PS_FAST], s_wcnt[PW_U * PS_FAST];
   __shared__ int s_list[PS_THREADS], s_lrow[PS_THREADS], s_lhead[PS_THREADS];
   __shared__ int s_err, s_last, s_hi, s_wlast, s_uinv;
-  const uint32_t p = ar.p;
+  __shared__ int s_next, s_rare, s_t, s_nl;  // block's end, its stop, pivots, live entries
+  const uint32_t p = (uint32_t)sa.p;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  constexpr unsigned FULL = 0xffffffffu;
 
+  if constexpr (SA::NORM) {
+    // the table of inverses, on its way while the window is formed
+    char *dst = reinterpret_cast<char *>(dyn_w) + PW_SMEM;
+    for (int e = tid; e < (int)(2 * p + 15) / 16; e += PS_THREADS)
+      cp_async16(dst + 16 * e, reinterpret_cast<const char *>(sa.table) + 16 * e);
+  }
   // the window: ordered compaction of the rows with a nonzero panel
   int nl = 0;
-  if (tid == 0) s_wlast = m - 1;
+  if (tid == 0) {
+    s_wlast = m - 1;
+    s_err = 0;
+    s_last = -1;
+  }
   if (tid <= EW) {
     s_cnt[tid] = hist[tid];
     hist[tid] = 0;
   }
-  for (int base = i0; base < m && nl < wcap; base += PS_THREADS) {
-    const int pos = base + tid;
-    const bool a = pos < m && act[pos];
-    const unsigned bal = __ballot_sync(0xffffffffu, a);
-    if (lane == 0) s_wcnt[wid] = __popc(bal);
-    __syncthreads();
-    int off = 0, cnt = 0;
-    for (int k = 0; k < PS_FAST; ++k) {
-      const int v = s_wcnt[k];
-      off += k < wid ? v : 0;
-      cnt += v;
+  for (int base = i0; base < m && nl < wcap; base += PW_U * PS_THREADS) {
+    int hd[PW_U];
+#pragma unroll
+    for (int u = 0; u < PW_U; ++u) {
+      const int pos = base + u * PS_THREADS + tid;
+      hd[u] = pos < m ? (int)head[pos] : (int)HEAD_NONE;
     }
-    off += __popc(bal & ((1u << lane) - 1u));
+    unsigned bal[PW_U];
+#pragma unroll
+    for (int u = 0; u < PW_U; ++u) {
+      bal[u] = __ballot_sync(FULL, hd[u] < HEAD_NONE);
+      if (lane == 0) s_wcnt[u * PS_FAST + wid] = __popc(bal[u]);
+    }
+    __syncthreads();
+    static_assert(PW_U * PS_FAST == 64, "two counts per lane");
+    int a = s_wcnt[lane], b = s_wcnt[lane + 32];  // inclusive scan of the 64 counts
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(FULL, a, o), y = __shfl_up_sync(FULL, b, o);
+      if (lane >= o) {
+        a += x;
+        b += y;
+      }
+    }
+    b += __shfl_sync(FULL, a, 31);
+    const int cnt = __shfl_sync(FULL, b, 31);
     const int take = min(cnt, wcap - nl);
-    if (a && off < take) {
-      const int slot = nl + off;
-      perm[0][slot] = slot;
-      ppos[0][slot] = pos;
-      wrow[slot] = pos;
-      atomicSub(&s_cnt[head[pos]], 1);  // the window's rows leave the counts
-      if (off == wcap - 1 - nl) s_wlast = pos;
+#pragma unroll
+    for (int u = 0; u < PW_U; ++u) {
+      const int gp = u * PS_FAST + wid - 1;  // the count before this warp's
+      const int before = gp < 0 ? 0 : __shfl_sync(FULL, gp < 32 ? a : b, gp & 31);
+      const int off = before + __popc(bal[u] & ((1u << lane) - 1u));
+      if (hd[u] < HEAD_NONE && off < take) {
+        const int slot = nl + off, pos = base + u * PS_THREADS + tid;
+        s_ent[slot] = slot;
+        s_epos[slot] = pos;
+        wrow[slot] = pos;
+        atomicSub(&s_cnt[hd[u]], 1);  // the window's rows leave the counts
+        if (off == wcap - 1 - nl) s_wlast = pos;
+      }
     }
     nl += take;
     __syncthreads();  // s_wcnt is rewritten by the next pass
   }
-  // the window rows' panel values: all threads, consecutive lanes on
-  // consecutive columns of a row (coalesced reads)
-  for (int e = tid; e < nl * EW; e += PS_THREADS) {
-    const int slot = e / EW, c = e % EW;
-    cp_async4(&Wv[slot][c], D + (size_t)wrow[slot] * ld + c0 + (c < w ? c : 0), c < w);
+  // the window rows' panel values: rows on warps, columns on lanes
+  {
+    uint32_t a0[PW_RPW], a1[PW_RPW];
+#pragma unroll
+    for (int r = 0; r < PW_RPW; ++r) {
+      const int slot = wid + r * PS_FAST;
+      const uint32_t *row = D + (size_t)(slot < nl ? wrow[slot] : i0) * ld + c0;
+      a0[r] = lane < w ? row[lane] : 0u;
+      a1[r] = lane + 32 < w ? row[lane + 32] : 0u;
+    }
+#pragma unroll
+    for (int r = 0; r < PW_RPW; ++r) {
+      const int slot = wid + r * PS_FAST;
+      Wv[slot][lane] = sa.load(a0[r]);
+      Wv[slot][lane + 32] = sa.load(a1[r]);
+    }
   }
-  cp_async_wait_all();
+  if constexpr (SA::NORM) cp_async_wait_all();
   __syncthreads();
   const int wlast = s_wlast;  // rows past it are outside the window
 
-  int cur = 0, off = 0, i = i0, t = 0;  // the entry list: perm[cur] / ppos[cur] from off
-  uint32_t S = 1u % p;
-  for (int col = 0; col < w && i < m; ++col) {
-    const int *pm = perm[cur] + off, *pp = ppos[cur] + off;
-    int *pn = perm[cur ^ 1], *ppn = ppos[cur ^ 1];
-    // A. first window entry (by position) with a nonzero in col.  Every warp
-    // finds it by itself: column col of the window and the entry list were
-    // last written before the previous column's closing barrier, and the
-    // work of this column (phase B) writes only columns right of col and the
-    // other list buffer, so no barrier is needed here
-    int qs = 0x7fffffff;
-    for (int base = 0; base < nl; base += 32) {
-      const int e = base + lane;
-      const bool nz = e < nl && Wv[pm[e]][col] != 0u;
-      const unsigned b = __ballot_sync(0xffffffffu, nz);
-      if (b) {
-        qs = base + __ffs(b) - 1;
-        break;
+  int t = 0, col0 = 0;  // pivots so far; the current row is i0 + t
+
+  // A. warp 0: the pivots of the block's columns, with NG groups of entries
+  auto choose = [&](auto ng_c) {
+    constexpr int NG = decltype(ng_c)::value;
+    V x[NG][PB], cf[NG][PB];
+    int ent[NG], pos[NG];
+    unsigned alive[NG];  // the same in every lane
+#pragma unroll
+    for (int g = 0; g < NG; ++g) {
+      const int e = lane + 32 * g;
+      const bool in = e < nl;
+      alive[g] = __ballot_sync(FULL, in);
+      ent[g] = in ? s_ent[e] : 0;
+      pos[g] = in ? s_epos[e] : 0;
+#pragma unroll
+      for (int j = 0; j < PB; ++j) {
+        x[g][j] = (in && col0 + j < w) ? Wv[ent[g]][col0 + j] : 0;
+        cf[g][j] = 0;
       }
     }
-    const bool z = nl > 0 && pp[0] == i;  // the row at position i is window entry 0
-    const uint32_t *P;                    // the pivot row (S_t times reduced)
-    int q, drop;                          // pivot position; window entry leaving (-1: none)
-    bool relocate0 = false;               // entry 0 moves to position q, in place of qs
-    if (qs == 0x7fffffff) {
-      // none in the window: rows past it whose bound allows a pivot here
-      // (a warp-wide sum; every warp computes the same count)
-      int cand = 0;
-      if (wlast < m - 1) {
-        const int v = (lane <= col ? s_cnt[lane] : 0) + (lane + 32 <= col ? s_cnt[lane + 32] : 0);
-        cand = __reduce_add_sync(0xffffffffu, v);
+    V sc = 0;
+    if constexpr (!SA::NORM) sc = sa.one();
+    int next = min(col0 + PB, w), rare = -1;
+#pragma unroll
+    for (int j = 0; j < PB; ++j) {
+      const int col = col0 + j, i = i0 + t;
+      if (lane == 0) s_pslot[j] = -1;
+      if (col >= next || i >= m) continue;
+      unsigned nz[NG], any = 0;
+#pragma unroll
+      for (int g = 0; g < NG; ++g) {
+        nz[g] = __ballot_sync(FULL, x[g][j] != 0);
+        any |= nz[g];
       }
-      // no barrier when there is no candidate: nothing shared changes
-      if (cand == 0) continue;
-      __syncthreads();  // every thread has its count before s_cnt changes
-      // per pass the CTA lists the candidates among PS_THREADS positions
-      // (ordered compaction), then each warp reduces one of them by the t
-      // pivots, W <- y_k W - W[pcol_k] (S_k U_k), and records its exact head
-      int found = -1, fw = 0;
-      for (int base = wlast + 1; base < m && cand > 0 && found < 0; base += PS_THREADS) {
-        const int pos = base + tid;
-        int r = -1, hr = HEAD_NONE;
-        if (pos < m) {
-          r = row_at(pos, p2r, stamp, epoch);
-          hr = head[r];
-        }
-        const bool isc = hr <= col;
-        const unsigned bal = __ballot_sync(0xffffffffu, isc);
-        if (lane == 0) s_wcnt[wid] = __popc(bal);
-        __syncthreads();
-        int off = 0, ncand = 0;
-        for (int k = 0; k < PS_FAST; ++k) {
-          const int v = s_wcnt[k];
-          off += k < wid ? v : 0;
-          ncand += v;
-        }
-        if (isc) {
-          const int o = off + __popc(bal & ((1u << lane) - 1u));
-          s_list[o] = pos;
-          s_lrow[o] = r;
-          s_lhead[o] = hr;
-        }
-        __syncthreads();
-        for (int j0 = 0; j0 < ncand && found < 0; j0 += PS_FAST) {
-          const int j = j0 + wid;
-          int hit_pos = 0x7fffffff;
-          if (j < ncand) {
-            const int rj = s_lrow[j], hrj = s_lhead[j];
-            const uint32_t *v = D + (size_t)rj * ld + c0;
-            uint32_t a0 = lane < w ? v[lane] : 0u, a1 = lane + 32 < w ? v[lane + 32] : 0u;
-            for (int k = 0; k < t; ++k) {
-              const int pc = s_pcol[k];
-              const uint32_t f = __shfl_sync(0xffffffffu, pc < 32 ? a0 : a1, pc & 31);
-              const uint32_t nf = f ? p - f : 0u;
-              a0 = ar.dot2(s_y[k], a0, nf, PV[k][lane]);
-              a1 = ar.dot2(s_y[k], a1, nf, PV[k][lane + 32]);
-            }
-            s_red[wid][lane] = a0;
-            s_red[wid][lane + 32] = a1;
-            const unsigned b0 = __ballot_sync(0xffffffffu, a0 != 0u && lane >= col);
-            const unsigned b1 = __ballot_sync(0xffffffffu, a1 != 0u && lane + 32 >= col);
-            const int hn = b0 ? __ffs(b0) - 1 : (b1 ? 32 + __ffs(b1) - 1 : HEAD_NONE);
-            if (hn == col) hit_pos = s_list[j];
-            if (lane == 0 && hn != hrj) {
-              head[rj] = (uint8_t)hn;
-              atomicSub(&s_cnt[hrj], 1);
-              atomicAdd(&s_cnt[hn], 1);
-            }
+      if (any == 0) {
+        // none in the window: rows past it whose bound allows a pivot here
+        // end the block (all warps look for it)
+        if (wlast < m - 1) {
+          const int v = (lane <= col ? s_cnt[lane] : 0) + (lane + 32 <= col ? s_cnt[lane + 32] : 0);
+          if (__reduce_add_sync(FULL, v) > 0) {
+            rare = col;
+            next = col;
           }
-          if (lane == 0) s_first[wid] = hit_pos;
-          __syncthreads();
-          for (int k = 0; k < PS_FAST; ++k)
-            if (s_first[k] < (found < 0 ? 0x7fffffff : found)) {
-              found = s_first[k];
-              fw = k;
-            }
-          __syncthreads();  // s_first and s_red are rewritten by the next round
         }
-        cand -= ncand;
-      }
-      if (found < 0) {
-        __syncthreads();
         continue;
       }
-      // the pivot comes from past the window; the row at position i goes to
-      // position `found`: window entry 0 leaves the window (with the bound
-      // of its values), a row outside it is recorded in p2r
-      q = found;
-      P = s_red[fw];
-      drop = z ? 0 : -1;
-      if (wid == 0) {
-        int hd = HEAD_NONE;
-        if (z) {
-          const uint32_t *E = Wv[pm[0]];
-          const unsigned b0 = __ballot_sync(0xffffffffu, E[lane] != 0u && lane > col);
-          const unsigned b1 = __ballot_sync(0xffffffffu, E[lane + 32] != 0u && lane + 32 > col);
-          hd = b0 ? __ffs(b0) - 1 : (b1 ? 32 + __ffs(b1) - 1 : HEAD_NONE);
+      // the pivot's entry (pg, pl) and the first live entry (fg, fl)
+      int pg = 0, fg = 0;
+      unsigned pm = nz[0], fm = alive[0];
+#pragma unroll
+      for (int g = 1; g < NG; ++g) {
+        if (pm == 0) {
+          pm = nz[g];
+          pg = g;
+        }
+        if (fm == 0) {
+          fm = alive[g];
+          fg = g;
+        }
+      }
+      const int pl = __ffs((int)pm) - 1;
+      auto sel = [&](const V(&r)[NG][PB], int k, int g) {
+        V v = r[0][k];
+#pragma unroll
+        for (int u = 1; u < NG; ++u)
+          if (g == u) v = r[u][k];
+        return v;
+      };
+      V pv[PB], pc[PB];  // the pivot row's entries; division-free, its coefficients
+#pragma unroll
+      for (int k = 0; k < PB; ++k) {
+        pv[k] = 0;
+        pc[k] = 0;
+        if (k >= j) pv[k] = __shfl_sync(FULL, sel(x, k, pg), pl);
+        else if (!SA::NORM) pc[k] = __shfl_sync(FULL, sel(cf, k, pg), pl);
+      }
+      const V y = pv[j];
+      if constexpr (SA::NORM) {
+        const int iv = s_inv[sa.index(y)];
+#pragma unroll
+        for (int g = 0; g < NG; ++g) {
+          const V l = sa.plain(x[g][j], iv);
+          cf[g][j] = l;  // 1 for the pivot row
+#pragma unroll
+          for (int k = j + 1; k < PB; ++k) x[g][k] = sa.step(x[g][k], l, pv[k]);
+        }
+        if (iv == 0) {  // no inverse: the call will fail, the row leaves all the same
+          if (lane == 0) s_err = 1;
+#pragma unroll
+          for (int g = 0; g < NG; ++g)
+#pragma unroll
+            for (int k = j + 1; k < PB; ++k)
+              if (lane == pl && g == pg) x[g][k] = 0;
+        }
+        if (lane == 0) s_xi[t] = (uint32_t)iv;
+      } else {
+#pragma unroll
+        for (int g = 0; g < NG; ++g) {
+          const V na = sa.neg(x[g][j]);
+#pragma unroll
+          for (int k = 0; k < PB; ++k) {
+            if (k > j) x[g][k] = sa.upd(y, x[g][k], na, pv[k]);
+            else if (k < j) cf[g][k] = sa.upd(y, cf[g][k], na, pc[k]);
+            else cf[g][k] = sa.mul(na, sc);
+          }
         }
         if (lane == 0) {
-          const int rq = row_at(q, p2r, stamp, epoch);
-          atomicSub(&s_cnt[head[rq]], 1);
-          int ri;
-          if (z) {
-            ri = wrow[pm[0]];
-            head[ri] = (uint8_t)hd;
-            atomicAdd(&s_cnt[hd], 1);
-          } else {
-            ri = row_at(i, p2r, stamp, epoch);
+          V4 c4;
+          c4.x = pc[0];
+          c4.y = pc[1];
+          c4.z = pc[2];
+          c4.w = 0;
+          s_pcoef[j] = c4;
+          s_psc[j] = sc;
+        }
+        sc = sa.mul(y, sc);
+      }
+      if (lane == pl) {
+        int en = ent[0], po = pos[0];
+#pragma unroll
+        for (int g = 1; g < NG; ++g)
+          if (pg == g) {
+            en = ent[g];
+            po = pos[g];
           }
-          p2r[q] = ri;
+        s_pslot[j] = en;
+        s_pt[j] = t;
+        s_pcol[t] = col;
+        s_y[t] = y;
+        s_tq[t] = po;
+        if constexpr (SA::NORM) {
+          V4 c4;
+          c4.x = j > 0 ? sel(cf, 0, pg) : 0;
+          c4.y = j > 1 ? sel(cf, 1, pg) : 0;
+          c4.z = j > 2 ? sel(cf, 2, pg) : 0;
+          c4.w = 0;
+          s_pcoef[j] = c4;
+        }
+      }
+      // position i: the first entry's row, or a row outside the window
+      int f = pos[0], q = pos[0];
+#pragma unroll
+      for (int g = 1; g < NG; ++g) {
+        if (fg == g) f = pos[g];
+        if (pg == g) q = pos[g];
+      }
+      const int fl = __ffs((int)fm) - 1;
+      f = __shfl_sync(FULL, f, fl);
+      q = __shfl_sync(FULL, q, pl);
+      unsigned gone = 1u << pl;  // the entry that goes, in group gg
+      int gg = pg;
+      if (f != i) {
+        if (q != i && lane == 0) {  // the row at i is outside the window
+          p2r[q] = row_at(i, p2r, stamp, epoch);
           stamp[q] = epoch;
         }
-      }
-    } else {
-      q = pp[qs];
-      P = Wv[pm[qs]];
-      drop = qs;
-      relocate0 = z && qs > 0;
-      if (!z && q != i && tid == 0) {  // the row at i is outside the window
-        p2r[q] = row_at(i, p2r, stamp, epoch);
-        stamp[q] = epoch;
-      }
-    }
-    // B. eliminate the window rows that stay, keep the pivot row in PV, and
-    // write the new entry list
-    const uint32_t y = P[col];
-    {
-      // Warp wid takes the columns col + 1 + wid, col + 17 + wid, ..; lane
-      // takes the list entries lane, lane + 32, lane + 64.  An entry's
-      // multiplier W[col] is loaded once for all of the warp's columns, and
-      // two columns are in flight at a time (their loads issued before
-      // their stores).
-      // NU groups of 32 entries, NU fixed per instantiation (the window
-      // shrinks by one entry per pivot, so most columns need one or two)
-      auto elim = [&](auto nu_c) {
-        constexpr int NU = decltype(nu_c)::value;
-        int pr[NU];
-        uint32_t na[NU];
+      } else if (q != i) {
+        // the first entry's row moves to the pivot's entry (and position)
+        gone = 1u << fl;
+        gg = fg;
 #pragma unroll
-        for (int u = 0; u < NU; ++u) {
-          const int s = lane + 32 * u;
-          pr[u] = (s < nl && s != drop) ? pm[s] : -1;
-          const uint32_t a = pr[u] >= 0 ? Wv[pr[u]][col] : 0u;
-          na[u] = a ? p - a : 0u;
-        }
-        for (int c = col + 1 + wid; c < w; c += 2 * PS_FAST) {
-          const int c2 = c + PS_FAST;
-          const bool two = c2 < w;
-          const uint32_t pc = P[c], pc2 = two ? P[c2] : 0u;
-          uint32_t wv[NU], wv2[NU];
+        for (int k = 0; k < PB; ++k) {
+          const V vx = k > j ? __shfl_sync(FULL, sel(x, k, fg), fl) : 0;
+          const V vc = k <= j ? __shfl_sync(FULL, sel(cf, k, fg), fl) : 0;
 #pragma unroll
-          for (int u = 0; u < NU; ++u) {
-            wv[u] = pr[u] >= 0 ? Wv[pr[u]][c] : 0u;
-            wv2[u] = (pr[u] >= 0 && two) ? Wv[pr[u]][c2] : 0u;
-          }
-#pragma unroll
-          for (int u = 0; u < NU; ++u)
-            if (pr[u] >= 0) {
-              Wv[pr[u]][c] = ar.dot2(y, wv[u], na[u], pc);
-              if (two) Wv[pr[u]][c2] = ar.dot2(y, wv2[u], na[u], pc2);
+          for (int g = 0; g < NG; ++g) {
+            if (g == pg && lane == pl) {
+              x[g][k] = vx;
+              cf[g][k] = vc;
             }
+            if (g == fg && lane == fl) x[g][k] = 0;
+          }
         }
-      };
-      static_assert(PW_EU == 3, "the dispatch below covers three groups");
-      const int nu = (nl + 31) >> 5;
-      if (nu <= 1)
-        elim(std::integral_constant<int, 1>{});
-      else if (nu == 2)
-        elim(std::integral_constant<int, 2>{});
-      else
-        elim(std::integral_constant<int, 3>{});
-    }
-    if (tid < EW) PV[t][tid] = P[tid];
-    const int nn = drop >= 0 ? nl - 1 : nl;
-    // the new entry list; when entry 0 leaves and nothing moves (a pivot at
-    // the row at position i, the usual case) it is the old list from its
-    // second entry, and nothing is copied
-    const bool shift = drop == 0 && !relocate0;
-    for (int s = tid; s < nn && !shift; s += PS_THREADS) {
-      int src, pos;
-      if (relocate0) {
-        src = s < drop - 1 ? s + 1 : (s == drop - 1 ? 0 : s + 1);
-        pos = s == drop - 1 ? q : pp[src];
-      } else {
-        src = (drop >= 0 && s >= drop) ? s + 1 : s;
-        pos = pp[src];
+        int en = ent[0];
+#pragma unroll
+        for (int g = 1; g < NG; ++g)
+          if (fg == g) en = ent[g];
+        en = __shfl_sync(FULL, en, fl);
+#pragma unroll
+        for (int g = 0; g < NG; ++g)
+          if (g == pg && lane == pl) ent[g] = en;
       }
-      pn[s] = pm[src];
-      ppn[s] = pos;
+#pragma unroll
+      for (int g = 0; g < NG; ++g)
+        if (g == gg) alive[g] &= ~gone;
+      ++t;
     }
-    if (tid == 0) {
-      s_pcol[t] = col;
-      s_y[t] = y;
-      s_S[t] = S;
-      out->pcol[t] = (uint32_t)col;
-      out->ti[t] = (uint32_t)i;
-      out->tq[t] = (uint32_t)q;
+    // the live entries closed up, with their coefficients
+    int base = 0;
+#pragma unroll
+    for (int g = 0; g < NG; ++g) {
+      if (alive[g] >> lane & 1u) {
+        const int e = base + __popc(alive[g] & ((1u << lane) - 1u));
+        s_ent[e] = ent[g];
+        s_epos[e] = pos[g];
+        V4 c4;
+        c4.x = cf[g][0];
+        c4.y = cf[g][1];
+        c4.z = cf[g][2];
+        c4.w = cf[g][3];
+        s_coef[e] = c4;
+      }
+      base += __popc(alive[g]);
+    }
+    if (lane == 0) {
+      s_sc = sc;
+      s_next = next;
+      s_rare = rare;
+      s_t = t;
+      s_nl = base;
+    }
+  };
+
+  while (col0 < w && i0 + t < m) {
+    if (wid == 0) {
+      if (nl <= 32) choose(std::integral_constant<int, 1>{});
+      else if (nl <= 64) choose(std::integral_constant<int, 2>{});
+      else choose(std::integral_constant<int, PW_G>{});
     }
     __syncthreads();
-    if (shift) {
-      ++off;
-    } else {
-      cur ^= 1;
-      off = 0;
-    }
-    nl = nn;
-    S = ar.mul(S, y);
-    ++i;
-    ++t;
-  }
-
-  // inverses in parallel: S_k^-1 (exact), the pivots x_k = y_k / S_k, and
-  // the reference's inverse of each pivot (its failure is the reference's
-  // error)
-  if (tid == 0) {
-    s_err = 0;
-    s_last = -1;
-    s_hi = i - 1;
-  }
-  __syncthreads();
-  // For p < 2^31 the reference's inverse is the exact one, so x_k^-1 =
-  // S_k y_k^-1, and the two inversions of pivot k run side by side (threads
-  // k and 64 + k); for larger p the reference's inverse of x_k itself.
-  const bool exact_inv = p < 0x80000000u;
-  if (tid < t) {
-    s_sinv[tid] = inv_exact_u32(p, s_S[tid]);
-    atomicMax(&s_hi, (int)out->tq[tid]);
-  } else if (exact_inv && tid >= EW && tid < EW + t) {
-    s_yinv[tid - EW] = inv_exact_u32(p, s_y[tid - EW]);
-  }
-  __syncthreads();
-  if (tid < t) {
-    const uint32_t si = s_sinv[tid];
-    const uint32_t x = ar.mul(s_y[tid], si);
-    const uint32_t xi = exact_inv ? ar.mul(s_S[tid], s_yinv[tid]) : lela_inv_u32(p, x);
-    s_x[tid] = x;
-    s_xi[tid] = xi;
-    xinv_out[tid] = xi;
-    if (si == 0u || xi == 0u) atomicOr(&s_err, 1);
-  }
-  __syncthreads();
-  // U_k = (S_k U_k) / S_k; entries left of the pivot column are not kept up
-  // to date, and U_k is zero there
-  for (int e = tid; e < t * EW; e += PS_THREADS) {
-    const int k = e / EW, c = e % EW;
-    Uout[e] = c < s_pcol[k] ? 0u : ar.mul(PV[k][c], s_sinv[k]);
-  }
-  // last final position of a non-pivot row with a nonzero panel: the window
-  // entries, positions past the window up to the largest transposition target
-  // through p2r; beyond that rows have not moved
-  const int hi = s_hi;
-  for (int s = tid; s < nl; s += PS_THREADS)
-    if (act[wrow[perm[cur][off + s]]]) atomicMax(&s_last, ppos[cur][off + s]);
-  for (int pos = max(wlast + 1, i) + tid; pos <= hi && pos < m; pos += PS_THREADS)
-    if (act[row_at(pos, p2r, stamp, epoch)]) atomicMax(&s_last, pos);
-  __syncthreads();
-  // the panel's determinant factor: product of the x_k, by warp 0
-  uint32_t det = 1u % p;
-  if (wid == 0) {
-    uint32_t v = lane < t ? s_x[lane] : 1u % p;
-    if (lane + 32 < t) v = ar.mul(v, s_x[lane + 32]);
+    // B. the columns right of the block, from the rows' values before it
+    const int next = s_next, rare = s_rare;
+    const bool found_any = s_t > (wid == 0 ? -1 : t);  // (warp 0's t is s_t already)
+    t = s_t;
+    nl = s_nl;
+    if (found_any) {
+      const V sc = s_sc;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = ar.mul(v, __shfl_xor_sync(0xffffffffu, v, o));
-    det = v;
+      for (int h = 0; h < 2; ++h) {
+        const int c = lane + 32 * h;
+        if (h == 0 && col0 >= 32) continue;  // no column of the half is left
+        const bool right = c >= next;
+        V P[PB];  // the block's pivot rows, before it
+#pragma unroll
+        for (int k = 0; k < PB; ++k) {
+          const int ps = s_pslot[k];
+          P[k] = ps >= 0 && c >= col0 ? Wv[ps][c] : 0;
+        }
+        // the pivot rows' final values
+        V U[PB];
+        if constexpr (SA::NORM) {
+#pragma unroll
+          for (int k = 0; k < PB; ++k) U[k] = 0;
+          U[0] = P[0];
+          U[1] = sa.lin(P[1], s_pcoef[1], U);
+          U[2] = sa.lin(P[2], s_pcoef[2], U);
+          U[3] = sa.lin(P[3], s_pcoef[3], U);
+        }
+#pragma unroll
+        for (int k = 0; k < PB; ++k)
+          if (wid == k && s_pslot[k] >= 0 && c >= col0) {
+            if constexpr (SA::NORM) PV[s_pt[k]][c] = U[k];
+            else PV[s_pt[k]][c] = sa.lin(s_psc[k], P[k], s_pcoef[k], P);
+          }
+        if (right)
+          for (int e = wid; e < nl; e += PS_FAST) {
+            const V4 cf = s_coef[e];
+            V *row = Wv[s_ent[e]];
+            if constexpr (SA::NORM) row[c] = sa.lin(row[c], cf, U);
+            else row[c] = sa.lin(sc, row[c], cf, P);
+          }
+      }
+    }
+    col0 = next;
+    __syncthreads();  // the window and PV are complete; s_* may be rewritten
+    if (rare < 0) continue;
+
+    // C. column `rare`: no window row has a pivot, rows past the window may
+    const int col = rare, i = i0 + t;
+    const bool z = nl > 0 && s_epos[0] == i;  // the row at position i is the first entry's
+    int cand;
+    {
+      const int v = (lane <= col ? s_cnt[lane] : 0) + (lane + 32 <= col ? s_cnt[lane + 32] : 0);
+      cand = __reduce_add_sync(FULL, v);
+    }
+    col0 = col + 1;
+    __syncthreads();  // every thread has its count before s_cnt changes
+    // per pass the CTA lists the candidates among PS_THREADS positions
+    // (ordered compaction), then each warp reduces one of them by the t
+    // pivots and records its exact head
+    int found = -1, fw = 0;
+    for (int base = wlast + 1; base < m && cand > 0 && found < 0; base += PS_THREADS) {
+      const int pos = base + tid;
+      int r = -1, hr = HEAD_NONE;
+      if (pos < m) {
+        r = row_at(pos, p2r, stamp, epoch);
+        hr = head[r];
+      }
+      const bool isc = hr <= col;
+      const unsigned bal = __ballot_sync(FULL, isc);
+      if (lane == 0) s_wcnt[wid] = __popc(bal);
+      __syncthreads();
+      int off = 0, ncand = 0;
+      for (int k = 0; k < PS_FAST; ++k) {
+        const int v = s_wcnt[k];
+        off += k < wid ? v : 0;
+        ncand += v;
+      }
+      if (isc) {
+        const int o = off + __popc(bal & ((1u << lane) - 1u));
+        s_list[o] = pos;
+        s_lrow[o] = r;
+        s_lhead[o] = hr;
+      }
+      __syncthreads();
+      for (int j0 = 0; j0 < ncand && found < 0; j0 += PS_FAST) {
+        const int j = j0 + wid;
+        int hit_pos = 0x7fffffff;
+        if (j < ncand) {
+          const int rj = s_lrow[j], hrj = s_lhead[j];
+          const uint32_t *v = D + (size_t)rj * ld + c0;
+          V a0 = sa.load(lane < w ? v[lane] : 0u), a1 = sa.load(lane + 32 < w ? v[lane + 32] : 0u);
+          for (int k = 0; k < t; ++k) {
+            const int pc = s_pcol[k];
+            const V f = __shfl_sync(FULL, pc < 32 ? a0 : a1, pc & 31);
+            const V u0 = lane >= pc ? PV[k][lane] : 0, u1 = lane + 32 >= pc ? PV[k][lane + 32] : 0;
+            if constexpr (SA::NORM) {
+              const V l = sa.plain(f, (int)s_xi[k]);
+              a0 = sa.step(a0, l, u0);
+              a1 = sa.step(a1, l, u1);
+            } else {
+              const V nf = sa.neg(f);
+              a0 = sa.upd(s_y[k], a0, nf, u0);
+              a1 = sa.upd(s_y[k], a1, nf, u1);
+            }
+          }
+          s_red[wid][lane] = a0;
+          s_red[wid][lane + 32] = a1;
+          const unsigned b0 = __ballot_sync(FULL, a0 != 0 && lane >= col);
+          const unsigned b1 = __ballot_sync(FULL, a1 != 0 && lane + 32 >= col);
+          const int hn = b0 ? __ffs(b0) - 1 : (b1 ? 32 + __ffs(b1) - 1 : HEAD_NONE);
+          if (hn == col) hit_pos = s_list[j];
+          if (lane == 0 && hn != hrj) {
+            head[rj] = (uint8_t)hn;
+            atomicSub(&s_cnt[hrj], 1);
+            atomicAdd(&s_cnt[hn], 1);
+          }
+        }
+        if (lane == 0) s_first[wid] = hit_pos;
+        __syncthreads();
+        for (int k = 0; k < PS_FAST; ++k)
+          if (s_first[k] < (found < 0 ? 0x7fffffff : found)) {
+            found = s_first[k];
+            fw = k;
+          }
+        __syncthreads();  // s_first and s_red are rewritten by the next round
+      }
+      cand -= ncand;
+    }
+    if (found < 0) {
+      __syncthreads();
+      continue;
+    }
+    // the pivot comes from past the window; the row at position i goes to
+    // position `found`: the first entry leaves the window (with the bound of
+    // its values), a row outside it is recorded in p2r
+    const V y = s_red[fw][col];
+    if (wid == 0) {
+      int ri = -1;
+      if (z) {
+        const int slot = s_ent[0];
+        const unsigned b0 = __ballot_sync(FULL, lane > col && Wv[slot][lane] != 0);
+        const unsigned b1 = __ballot_sync(FULL, lane + 32 > col && Wv[slot][lane + 32] != 0);
+        const int hd = b0 ? __ffs(b0) - 1 : (b1 ? 32 + __ffs(b1) - 1 : HEAD_NONE);
+        ri = wrow[slot];
+        if (lane == 0) {
+          head[ri] = (uint8_t)hd;
+          atomicAdd(&s_cnt[hd], 1);
+        }
+        // the other entries close up
+        int en[PW_G], po[PW_G];
+#pragma unroll
+        for (int g = 0; g < PW_G; ++g) {
+          const int e = lane + 32 * g + 1;
+          en[g] = e < nl ? s_ent[e] : 0;
+          po[g] = e < nl ? s_epos[e] : 0;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int g = 0; g < PW_G; ++g) {
+          const int e = lane + 32 * g + 1;
+          if (e < nl) {
+            s_ent[e - 1] = en[g];
+            s_epos[e - 1] = po[g];
+          }
+        }
+      }
+      if (lane == 0) {
+        const int rq = row_at(found, p2r, stamp, epoch);
+        atomicSub(&s_cnt[head[rq]], 1);
+        if (!z) ri = row_at(i, p2r, stamp, epoch);
+        p2r[found] = ri;
+        stamp[found] = epoch;
+        s_pcol[t] = col;
+        s_y[t] = y;
+        s_tq[t] = found;
+        if constexpr (SA::NORM) {
+          s_xi[t] = s_inv[sa.index(y)];
+          if (s_xi[t] == 0u) s_err = 1;
+        }
+      }
+      PV[t][lane] = s_red[fw][lane];
+      PV[t][lane + 32] = s_red[fw][lane + 32];
+    }
+    if (z) --nl;
+    __syncthreads();
+    if constexpr (!SA::NORM) {
+      // the window rows are zero in the column: they are scaled by y
+      for (int e = wid; e < nl; e += PS_FAST) {
+        V *row = Wv[s_ent[e]];
+        row[lane] = sa.mul(y, row[lane]);
+        row[lane + 32] = sa.mul(y, row[lane + 32]);
+      }
+    }
+    ++t;
+    __syncthreads();
   }
+  __syncthreads();
+
+  // Division-free: the S_k, their inverses, the pivots x_k = y_k / S_k and the
+  // pivots' inverses, by warp 0 (lane l: k = l and l + 32) from prefix and
+  // suffix products: S_k is 1 times the product (mul) of y_0 .. y_{k-1}; with the
+  // one inverse I = 1 / S_t, 1 / S_k is I times the product of y_k ..
+  // y_{t-1}, and 1 / y_k = mul (S_k, 1 / S_{k+1}).  For p < 2^31 the
+  // reference's inverse is the exact one, so it fails for some pivot
+  // exactly when S_t, a product of all y_k, has no inverse.  For larger p
+  // the reference's inverse of each x_k itself.
+  const bool exact_inv = p < 0x80000000u;
+  const auto word = [seq](uint32_t v) { return (uint64_t)seq << 32 | v; };
+  if (wid == 0) {
+    // last final position of a non-pivot row with a nonzero panel, here of
+    // the window rows left
+    for (int e = lane; e < nl; e += 32) atomicMax(&s_last, s_epos[e]);
+    const V unit = sa.load(1u % p);
+    V x0 = unit, x1 = unit;
+    if constexpr (SA::NORM) {
+      if (lane < t) {
+        x0 = s_y[lane];
+        xinv_out[lane] = s_xi[lane];
+      }
+      if (lane + 32 < t) {
+        x1 = s_y[lane + 32];
+        xinv_out[lane + 32] = s_xi[lane + 32];
+      }
+    } else {
+      const V e = sa.one();
+      V y0 = lane < t ? s_y[lane] : e, y1 = lane + 32 < t ? s_y[lane + 32] : e;
+      V f0 = y0, f1 = y1, b0 = y0, b1 = y1;  // prefix, suffix products
+#pragma unroll 1
+      for (int o = 1; o < 32; o <<= 1) {
+        const V u0 = __shfl_up_sync(FULL, f0, o), u1 = __shfl_up_sync(FULL, f1, o);
+        const V d0 = __shfl_down_sync(FULL, b0, o), d1 = __shfl_down_sync(FULL, b1, o);
+        if (lane >= o) {
+          f0 = sa.mul(u0, f0);
+          f1 = sa.mul(u1, f1);
+        }
+        if (lane + o < 32) {
+          b0 = sa.mul(b0, d0);
+          b1 = sa.mul(b1, d1);
+        }
+      }
+      f1 = sa.mul(__shfl_sync(FULL, f0, 31), f1);
+      b0 = sa.mul(b0, __shfl_sync(FULL, b1, 0));
+      V S0 = __shfl_up_sync(FULL, f0, 1), S1 = __shfl_up_sync(FULL, f1, 1);
+      const V f31 = __shfl_sync(FULL, f0, 31);
+      if (lane == 0) S1 = f31;
+      S0 = lane == 0 ? unit : sa.mul(unit, S0);
+      S1 = sa.mul(unit, S1);
+      const V St = sa.mul(unit, __shfl_sync(FULL, f1, 31));
+      uint32_t err = 0;
+      V si0, si1;
+      uint32_t xi0, xi1;
+      if (exact_inv) {
+        const uint32_t I = t > 0 ? inv_exact_u32(p, sa.canon(St)) : 1u % p;
+        if (t > 0 && I == 0u) err = 1;
+        const V vI = sa.load(I);
+        si0 = sa.mul(vI, b0);
+        si1 = sa.mul(vI, b1);
+        V n0 = __shfl_down_sync(FULL, si0, 1), n1 = __shfl_down_sync(FULL, si1, 1);
+        const V s32 = __shfl_sync(FULL, si1, 0);
+        if (lane == 31) {
+          n0 = s32;
+          n1 = vI;
+        }
+        x0 = sa.plain(y0, si0);
+        x1 = sa.plain(y1, si1);
+        xi0 = sa.canon(sa.plain(S0, sa.mul(S0, n0)));
+        xi1 = sa.canon(sa.plain(S1, sa.mul(S1, n1)));
+      } else {
+        si0 = sa.load(inv_exact_u32(p, sa.canon(S0)));
+        si1 = sa.load(inv_exact_u32(p, sa.canon(S1)));
+        x0 = sa.plain(y0, si0);
+        x1 = sa.plain(y1, si1);
+        xi0 = lela_inv_u32(p, sa.canon(x0));
+        xi1 = lela_inv_u32(p, sa.canon(x1));
+        if (lane < t && (sa.canon(si0) == 0u || xi0 == 0u)) err = 1;
+        if (lane + 32 < t && (sa.canon(si1) == 0u || xi1 == 0u)) err = 1;
+      }
+      if (lane < t) {
+        s_sinv[lane] = si0;
+        s_xi[lane] = xi0;
+        xinv_out[lane] = xi0;
+      }
+      if (lane + 32 < t) {
+        s_sinv[lane + 32] = si1;
+        s_xi[lane + 32] = xi1;
+        xinv_out[lane + 32] = xi1;
+      }
+      if (__any_sync(FULL, err != 0u) && lane == 0) s_err = 1;
+    }
+    // the panel's determinant factor: product of the x_k
+    V dv = lane < t ? x0 : unit;
+    if (lane + 32 < t) dv = sa.plain(dv, x1);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) dv = sa.plain(dv, __shfl_xor_sync(FULL, dv, o));
+    if (lane == 0) s_det = sa.canon(dv);
+  } else if (wid == 2 || wid == 3) {
+    const int k = tid - 64;
+    if (k < t) {
+      out->pcol[k] = (uint32_t)s_pcol[k];
+      out->ti[k] = (uint32_t)(i0 + k);
+      out->tq[k] = (uint32_t)s_tq[k];
+      hout[PANEL_W_PIV + 2 * k] = word((uint32_t)s_pcol[k]);
+      hout[PANEL_W_PIV + 2 * k + 1] = word((uint32_t)s_tq[k]);
+    }
+  } else if (wid == 1) {
+    // the largest transposition target; the positions past the window up to
+    // it, through p2r (beyond it rows have not moved)
+    const int i = i0 + t;
+    int hi = i - 1;
+    if (lane < t) hi = max(hi, s_tq[lane]);
+    if (lane + 32 < t) hi = max(hi, s_tq[lane + 32]);
+    hi = __reduce_max_sync(FULL, hi);
+    int last = -1;
+    for (int pos = max(wlast + 1, i) + lane; pos <= hi && pos < m; pos += 32)
+      if (act[row_at(pos, p2r, stamp, epoch)]) last = pos;
+    atomicMax(&s_last, last);
+    if (lane == 0) s_hi = hi;
+  }
+  __syncthreads();
   if (tid == 0) {
     const int la = *last_act;
     int last = s_last;
-    if (la > hi) last = max(last, la);
+    if (la > s_hi) last = max(last, la);
     // the rows the panel's solve takes: i0 .. max(last, i0 + t - 1)
     const int rows = max(last, i0 + t - 1) - i0 + 1;
-    s_uinv = exact_inv && t > 0 && rows >= SOLVE_INV_ROWS;
-    out->uinv = hout->uinv = (uint32_t)s_uinv;
+    const uint32_t uinv = exact_inv && t > 0 && rows >= SOLVE_INV_ROWS;
+    last = max(last, 0);
+    hout[PANEL_W_T] = word((uint32_t)t | uinv << 8 | (uint32_t)s_err << 9);
+    hout[PANEL_W_LAST] = word((uint32_t)last);
+    hout[PANEL_W_DET] = word(s_det);
+    s_uinv = (int)uinv;
+    out->uinv = uinv;
     out->t = (uint32_t)t;
     out->err = (uint32_t)s_err;
-    out->last_pos = (uint32_t)(last >= 0 ? last : 0);
-    out->det = det;
+    out->last_pos = (uint32_t)last;
+    out->det = s_det;
     *last_act = -1;
-    hout->t = (uint32_t)t;
-    hout->err = (uint32_t)s_err;
-    hout->last_pos = (uint32_t)(last >= 0 ? last : 0);
-    hout->det = det;
   }
-  // the result also goes to mapped host memory, then a sequence flag: the
-  // host waits on the flag instead of a copy and a stream synchronisation
-  __syncthreads();
-  for (int k = tid; k < t; k += PS_THREADS) {
-    hout->pcol[k] = out->pcol[k];
-    hout->ti[k] = out->ti[k];
-    hout->tq[k] = out->tq[k];
+  // U_k (division-free: (S_k U_k) / S_k); entries left of the pivot column are
+  // not kept up to date, and U_k is zero there
+  auto u_at = [&](int k, int c) {
+    if constexpr (SA::NORM) return sa.canon(PV[k][c]);
+    else return sa.canon(sa.plain(PV[k][c], s_sinv[k]));
+  };
+  for (int e = tid; e < t * EW; e += PS_THREADS) {
+    const int k = e / EW, c = e % EW;
+    Uout[e] = c < s_pcol[k] ? 0u : u_at(k, c);
   }
-  __threadfence_system();
   __syncthreads();
-  if (tid == 0) *hflag = seq;
-  // After the flag, so that it overlaps the host's handling of the result
-  // (its only reader is the next kernel on the stream): for p < 2^31 (exact
+  // After the result is on its way to the host: for p < 2^31 (exact
   // pivot inverses), when at least SOLVE_INV_ROWS rows are to be solved (it
   // costs a few microseconds), the inverse of U_P, the t x t upper triangular matrix of
   // the pivot rows at the pivot columns (U_P[k][j] = U_k[pcol_j], diagonal
@@ -695,16 +1181,15 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
   // a_P U_P^-1 (a_P: its values at the pivot columns), all at once.  In the
   // window's shared memory, now free.
   if (s_uinv) {
-    uint32_t(*X)[PW_LD] = Wv;
+    uint32_t(*X)[PW_LD] = reinterpret_cast<uint32_t(*)[PW_LD]>(dyn_w);
     uint32_t *T = dyn_w + EW * PW_LD;
-    static_assert(EW * PW_LD + 32 * EW / 2 <= PW_R * PW_LD, "inverse scratch fits the window");
     for (int e = tid; e < EW * EW; e += PS_THREADS) {
       const int k = e / EW, j = e % EW;
       uint32_t v;
       if (k >= t || j >= t) v = k == j ? 1u : 0u;
       else if (j < k) v = 0u;
       else if (j == k) v = s_xi[k];
-      else v = ar.mul(PV[k][s_pcol[j]], s_sinv[k]);
+      else v = u_at(k, s_pcol[j]);
       X[k][j] = v;
     }
     __syncthreads();
@@ -970,22 +1455,27 @@ int zp_echelon_dev(Ctx *c, int m, int n, uint32_t p, uint32_t *D, size_t ld, siz
                      &gws);
   if (st) return st;
   const bool small = p < (1u << 16);
-  if ((st = ctx_smem_attr(c, (const void *)panel_search_kernel<ArithSmall>, (int)PW_SMEM,
-                          "echelon: panel search attributes")) ||
-      (st = ctx_smem_attr(c, (const void *)panel_search_kernel<ArithWide>, (int)PW_SMEM,
-                          "echelon: panel search attributes")))
-    return st;
+  const uint16_t *inv_table = nullptr;
+  if (SearchSmall::takes(p)) {
+    void *tb = nullptr;
+    if ((st = ctx_buffer(c, BUF_INV, PW_TABLE, &tb))) return st;
+    if (c->inv_p != p) {
+      inverse_table_kernel<<<((int)p + 255) / 256, 256, 0, c->stream>>>(p, static_cast<uint16_t *>(tb));
+      ctx_launched(c);
+      const cudaError_t ei = cudaGetLastError();
+      if (ei != cudaSuccess) return ctx_cuda(c, ei, "echelon: inverses");
+      c->inv_p = p;
+    }
+    inv_table = static_cast<const uint16_t *>(tb);
+  }
   const ArithSmall ars = ArithSmall::make(p);
   const ArithWide arw = ArithWide::make(p);
-  static_assert(sizeof(PanelOut) <= PANEL_FLAG_OFF, "panel result and flag share the mapped page");
   void *mh = nullptr, *md = nullptr;
   if ((st = ctx_panel_map(c, &mh, &md))) return st;
-  const PanelOut *hmap = static_cast<const PanelOut *>(mh);
   int *hperm = reinterpret_cast<int *>(static_cast<char *>(mh) + PANEL_PERM_OFF);
-  static_assert(sizeof(PanelOut) <= PANEL_PERM_OFF && 2 * (2 * EW) <= (int)PANEL_PERM_INTS, "staging layout");
-  volatile uint32_t *hflag = reinterpret_cast<volatile uint32_t *>(static_cast<char *>(mh) + PANEL_FLAG_OFF);
-  PanelOut *hmap_dev = static_cast<PanelOut *>(md);
-  uint32_t *hflag_dev = reinterpret_cast<uint32_t *>(static_cast<char *>(md) + PANEL_FLAG_OFF);
+  static_assert(2 * (2 * EW) <= (int)PANEL_PERM_INTS, "staging layout");
+  volatile uint64_t *hwords = reinterpret_cast<volatile uint64_t *>(static_cast<char *>(mh) + PANEL_WORDS_OFF);
+  volatile uint64_t *hwords_dev = reinterpret_cast<volatile uint64_t *>(static_cast<char *>(md) + PANEL_WORDS_OFF);
   cudaError_t e = cudaMemsetAsync(d_stamp, 0xff, (size_t)m * sizeof(int), c->stream);
   if (e == cudaSuccess && keep) {
     keep->swaps.clear();
@@ -1028,6 +1518,16 @@ int zp_echelon_dev(Ctx *c, int m, int n, uint32_t p, uint32_t *D, size_t ld, siz
     prof_end(c, pi);
     return s;
   };
+  auto search = [&](auto sa, auto ar, int i, int c0, int w, uint32_t seq, int wcap) -> int {
+    auto kern = panel_search_kernel<decltype(sa), decltype(ar)>;
+    const size_t smem = PW_SMEM + (decltype(sa)::NORM ? PW_TABLE : 0);
+    int s = ctx_smem_attr(c, (const void *)kern, (int)smem, "echelon: panel search attributes");
+    if (s) return s;
+    kern<<<1, PS_THREADS, smem, c->stream>>>(D, ld, i, m, c0, w, sa, ar, d_head, d_act, d_hist,
+                                                d_last, d_p2r, d_stamp, epoch, d_U, d_xinv, d_Uinv,
+                                                d_out, hwords_dev, seq, wcap);
+    return ST_OK;
+  };
   // window rows of the search: the full PW_R, or 64 when the previous panel
   // had many rows below its pivots (dense matrices, where the first 64
   // active rows nearly always hold the panel's pivots; the rows past the
@@ -1049,27 +1549,34 @@ int zp_echelon_dev(Ctx *c, int m, int n, uint32_t p, uint32_t *D, size_t ld, siz
     prof_end(c, pi);
     const uint32_t seq = ++c->panel_seq;
     pi = prof_begin(c, "ech_search");
-    if (small)
-      panel_search_kernel<<<1, PS_THREADS, PW_SMEM, c->stream>>>(
-          D, ld, i, m, c0, w, ars, d_head, d_act, d_hist, d_last, d_p2r, d_stamp, epoch, d_U,
-          d_xinv, d_Uinv, d_out, hmap_dev, hflag_dev, seq, wcap);
+    if (SearchSmall::takes(p))
+      st = search(SearchSmall::make(p, inv_table), ars, i, c0, w, seq, wcap);
+    else if (SearchMont::takes(p))
+      st = search(SearchMont::make(p), arw, i, c0, w, seq, wcap);
     else
-      panel_search_kernel<<<1, PS_THREADS, PW_SMEM, c->stream>>>(
-          D, ld, i, m, c0, w, arw, d_head, d_act, d_hist, d_last, d_p2r, d_stamp, epoch, d_U,
-          d_xinv, d_Uinv, d_out, hmap_dev, hflag_dev, seq, wcap);
+      st = search(SearchWide::make(p), arw, i, c0, w, seq, wcap);
+    if (st) return st;
     ++epoch;
     prof_end(c, pi);
     ctx_launched(c, 2);
-    if ((st = ctx_wait_flag(c, hflag, seq, "echelon: panel"))) return st;
-    h.t = hmap->t;
-    h.uinv = hmap->uinv;
-    h.err = hmap->err;
-    h.last_pos = hmap->last_pos;
-    h.det = hmap->det;
-    for (uint32_t k = 0; k < h.t && k < (uint32_t)EW; ++k) {
-      h.pcol[k] = hmap->pcol[k];
-      h.ti[k] = hmap->ti[k];
-      h.tq[k] = hmap->tq[k];
+    auto word = [&](int k, uint32_t *v) -> int {
+      int s = ctx_wait_flag(c, reinterpret_cast<volatile uint32_t *>(hwords + k) + 1, seq,
+                            "echelon: panel");
+      if (s == ST_OK) *v = (uint32_t)hwords[k];
+      return s;
+    };
+    uint32_t head_word = 0;
+    if ((st = word(PANEL_W_T, &head_word)) || (st = word(PANEL_W_LAST, &h.last_pos)) ||
+        (st = word(PANEL_W_DET, &h.det)))
+      return st;
+    h.t = std::min<uint32_t>(head_word & 0xffu, EW);
+    h.uinv = head_word >> 8 & 1u;
+    h.err = head_word >> 9 & 1u;
+    for (uint32_t k = 0; k < h.t; ++k) {
+      h.ti[k] = (uint32_t)i + k;
+      if ((st = word(PANEL_W_PIV + 2 * (int)k, &h.pcol[k])) ||
+          (st = word(PANEL_W_PIV + 2 * (int)k + 1, &h.tq[k])))
+        return st;
     }
     if (h.err) return ctx_fail(c, ST_PIVOT, "Could not invert pivot-element in the ring");
     const int t = (int)h.t;
