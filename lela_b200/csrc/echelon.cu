@@ -288,15 +288,17 @@ __global__ void __launch_bounds__(HEADS_THREADS)
 // Field arithmetic of the panel search, in three forms chosen by the host.
 //
 // SearchSmall, 32 <= p <= 65521 (the largest prime below 2^16): signed
-// residues |v| <= p/2 + 5 and pivots inverted from a table of all inverses
-// (u16, 0: none), which the CTA holds in shared memory, so a row is reduced
-// with its true multiplier l: w - l P (NORM below).  Two products and one more
-// term are below 2 (p/2 + 5)^2 + p/2 + 5 <= 2147123215 < 2^31, and q =
-// (floor(x mu / 2^32) + 2^(s-1)) >> s with mu =
-// round(2^(32+s) / p) in [2^30, 2^31) is x / p rounded up to an error of
-// 1.25 / 2^s (s = 14 for p > 2^15, one less per halving of p), so |x - q p|
-// <= p/2 + 1.25 p / 2^s <= p/2 + 5, and x = 0 mod p gives q = x / p exactly:
-// a zero is stored as 0.  Below 32 s would be 1 or less.
+// residues |v| <= p/2 + 4 and pivots inverted from a table of the inverses
+// of 0 .. p/2 (u16, 0: none), which the CTA holds in shared memory, so a row is reduced
+// with its true multiplier l: w - l P (NORM below).  Reduction: q = (x mu +
+// 2^(31+s)) >> (32 + s) with mu = round (2^(32+s) / p) in [2^30, 2^31) (s = 14
+// for p > 2^15, one less per halving of p) is x / p rounded, up to an error of
+// |x| / 2^(33+s) from mu, for |x| < 2^31; so |x - q p| <= p/2 + 1, and x = 0 mod p
+// gives q = x / p exactly: a zero is stored as 0 (s >= 3 here).  The product
+// and the rounding are one 64-bit multiply-add (2.1 issue cycles a warp
+// measured, against 6.3 for a 32-bit high product).  Two products and one more
+// term fit 32 bits (2 (p/2 + 4)^2 + p/2 + 4 < 2^31); four (below 2^32.1 in
+// 64 bits) are halved for the quotient, which then is off by 2 / p more.
 //
 // SearchMont and SearchWide reduce without division (an inverse costs more
 // than a whole column there): one elimination step is upd(y, w, na, P) = k (y
@@ -309,8 +311,9 @@ struct SearchSmall {
   using V = int;
   using V4 = int4;
   static constexpr bool NORM = true;
-  int p, mu, s, half;
-  const uint16_t *table;  // inverses of 0 .. p - 1
+  int p, mu, s;
+  long long half;
+  const uint16_t *table;  // inverses of 0 .. p / 2
   __host__ static bool takes(uint32_t p) { return p >= 32 && p <= 65521; }
   __host__ static SearchSmall make(uint32_t p, const uint16_t *table) {
     SearchSmall a;
@@ -318,32 +321,49 @@ struct SearchSmall {
     a.s = 0;
     while (((1ull << (33 + a.s)) + p) / (2ull * p) < (1ull << 30)) ++a.s;
     a.mu = (int)(((1ull << (33 + a.s)) + p) / (2ull * p));
-    a.half = 1 << (a.s - 1);
+    a.half = 1ll << (31 + a.s);
     a.table = table;
     return a;
   }
-  __device__ __forceinline__ int red(int x) const {
-    return x - ((__mulhi(x, mu) + half) >> s) * p;
+  // round (x / p), sh = s; of x / 2, sh = s - 1
+  __device__ __forceinline__ int quot(int x, int sh) const {
+    long long d;
+    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(x), "r"(mu), "l"(sh == s ? half : half >> 1));
+    return (int)(d >> 32) >> sh;
   }
+  __device__ __forceinline__ int red(int x) const { return x - quot(x, s) * p; }
   __device__ __forceinline__ int load(uint32_t v) const {
     return (int)v > (p >> 1) ? (int)v - p : (int)v;
   }
   // w - l P
   __device__ __forceinline__ int step(int w, int l, int P) const { return red(w - l * P); }
+  __device__ __forceinline__ int step2(int w, int l, int P, int l2, int P2) const {
+    return red(w - l * P - l2 * P2);
+  }
   // w - l[0] P[0] - .. - l[3] P[3]
   __device__ __forceinline__ int lin(int w, const int4 &l, const int (&P)[4]) const {
-    return red(red(w - l.x * P[0] - l.y * P[1]) - l.z * P[2] - l.w * P[3]);
+    const long long x = (long long)w - (long long)l.x * P[0] - (long long)l.y * P[1] -
+                        (long long)l.z * P[2] - (long long)l.w * P[3];
+    return (int)x - quot((int)(x >> 1), s - 1) * p;
   }
-  // a b, also for one factor in [0, p)
+  // a b, also for one factor in (-p, p)
   __device__ __forceinline__ int plain(int a, int b) const { return red(a * b); }
-  __device__ __forceinline__ int index(int v) const { return v < 0 ? v + p : v; }
-  __device__ __forceinline__ uint32_t canon(int v) const { return (uint32_t)index(v); }
+  // 1 / v in (-p, p), 0 if there is none (|v| <= p/2 + 5 and v is the
+  // residue of smallest magnitude: a few past p/2 are folded back)
+  __device__ __forceinline__ int inverse(const uint16_t *tab, int v) const {
+    int a = abs(v);
+    const bool past = a > (p >> 1);
+    if (past) a = p - a;
+    const int i = tab[a];
+    return (v < 0) != past ? -i : i;
+  }
+  __device__ __forceinline__ uint32_t canon(int v) const { return (uint32_t)(v < 0 ? v + p : v); }
 };
 
-// The inverses of 0 .. p - 1 modulo p < 2^16, 0 for those that have none.
+// The inverses of 0 .. p / 2 modulo p < 2^16, 0 for those that have none.
 __global__ void inverse_table_kernel(uint32_t p, uint16_t *__restrict__ table) {
   const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x < p) table[x] = (uint16_t)inv_exact_u32(p, x);
+  if (x <= p / 2) table[x] = (uint16_t)inv_exact_u32(p, x);
 }
 
 // SearchMont, other odd p < 2^31: canonical residues, Montgomery reduction
@@ -455,12 +475,16 @@ struct SearchWide {
 // the window rows and of the block's pivot rows from those coefficients (rows
 // on warps, columns on lanes).
 //
-// Bound: the instructions on warp 0's dependent chain.  Forms with one
+// Bound: the instructions on warp 0's dependent chain (about 130 a column) and
+// the issue slots of the block updates.  Measured on a 64 x 64 window (p =
+// 65521, a panel of a dense 4096^2 matrix): 520 cycles a column for the
+// pivots, 420 for the updates, of 78000 for the panel (41 us).  Forms with one
 // barrier per column and all 16 warps on it (window in shared memory, lanes
 // on rows; or rows in registers, a warp per row) took 1640 cycles a column
-// (p = 65521, 64 x 64 window: the search of a panel of a dense 4096^2 matrix
-// 80 us, at 2^31 - 1 102 us), and blocks with a 96-bit rank mask, division-free
-// coefficients for every p and bookkeeping in lane 0, 965 + 520.
+// (80 us a panel, at 2^31 - 1 102 us).  Rolled loops, the panel's inverse
+// included, were slower (44500 + 31400 cycles against 33500 + 26800).  On this
+// chip a ballot takes 26 cycles, __ffs 40, __reduce_min_sync 22, so the pivot's
+// lane comes from the reduction.
 //
 // Bookkeeping (warp 0): s_ent[e] / s_epos[e] are the slot and the position
 // of live entry e, rewritten per block.  A transposition (i, q) moves the row
@@ -481,7 +505,7 @@ constexpr int PW_LD = EW + 1;
 // then the table of inverses (NORM)
 constexpr int PW_INV = EW * PW_LD + 32 * EW / 2;
 constexpr size_t PW_SMEM = (((size_t)(PW_R * PW_LD > PW_INV ? PW_R * PW_LD : PW_INV) * 4) + 15) / 16 * 16;
-constexpr size_t PW_TABLE = 65536 * 2;
+constexpr size_t PW_TABLE = 65536;
 // positions a thread looks at per pass of the window's compaction
 constexpr int PW_U = 4;
 // rows to solve from which the panel's multipliers come from U_P^-1
@@ -502,20 +526,23 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
   const uint16_t *s_inv = reinterpret_cast<const uint16_t *>(dyn_w + PW_SMEM / 4);
   __shared__ V PV[EW][EW];
   __shared__ V4 s_coef[PW_R];         // per slot: its coefficients of the block's pivot rows
-  __shared__ V4 s_pcoef[PB];          // division-free: the same for the block's pivot rows,
+  V *s_coefv = reinterpret_cast<V *>(s_coef);
+  __shared__ V4 s_pcoef[PB];          // division-free: z of the block's pivot rows when chosen,
   __shared__ V s_psc[PB], s_sc;       // their scales, and the other rows'
-  __shared__ int s_pslot[PB];         // slot of the pivot of the block's column j (-1: none)
-  __shared__ int s_pt[PB];            // its index among the panel's pivots
+  // slot of the pivot of the block's column j (-1: none)
+  __shared__ __align__(16) int s_pslot[PB];
   __shared__ V s_red[PS_FAST][EW];    // rows past the window, reduced (one per warp)
   __shared__ int s_ent[PW_R], s_epos[PW_R], wrow[PW_R];
-  __shared__ int s_pcol[EW], s_tq[EW];
+  __shared__ int2 s_piv[EW];          // pivot column, transposition target
   __shared__ V s_y[EW], s_sinv[EW];   // pivot values (in window rows' scale), 1 / S_k
-  __shared__ uint32_t s_xi[EW], s_det;
+  __shared__ int s_xi[EW];            // pivots' inverses (NORM: in (-p, p))
+  __shared__ uint32_t s_det;
   __shared__ int s_cnt[EW + 1];
   __shared__ int s_first[PS_FAST], s_wcnt[PW_U * PS_FAST];
   __shared__ int s_list[PS_THREADS], s_lrow[PS_THREADS], s_lhead[PS_THREADS];
   __shared__ int s_err, s_last, s_hi, s_wlast, s_uinv;
-  __shared__ int s_next, s_rare, s_t, s_nl;  // block's end, its stop, pivots, live entries
+  // block's end, its stop, the pivots before and after it, live entries
+  __shared__ int s_next, s_rare, s_t0, s_t, s_nl;
   const uint32_t p = (uint32_t)sa.p;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   constexpr unsigned FULL = 0xffffffffu;
@@ -523,7 +550,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
   if constexpr (SA::NORM) {
     // the table of inverses, on its way while the window is formed
     char *dst = reinterpret_cast<char *>(dyn_w) + PW_SMEM;
-    for (int e = tid; e < (int)(2 * p + 15) / 16; e += PS_THREADS)
+    for (int e = tid; e < (int)(p / 2 + 1 + 7) / 8; e += PS_THREADS)
       cp_async16(dst + 16 * e, reinterpret_cast<const char *>(sa.table) + 16 * e);
   }
   // the window: ordered compaction of the rows with a nonzero panel
@@ -604,213 +631,198 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
 
   int t = 0, col0 = 0;  // pivots so far; the current row is i0 + t
 
-  // A. warp 0: the pivots of the block's columns, with NG groups of entries
+  // A. warp 0: the pivots of the block's columns, with NG groups of entries.
+  // z holds, per entry, the block's columns from the current one on, and
+  // behind them (division-free) the coefficients of the block's pivot rows
+  // chosen so far: each column drops z[0] and appends its own.
   auto choose = [&](auto ng_c) {
     constexpr int NG = decltype(ng_c)::value;
-    V x[NG][PB], cf[NG][PB];
+    constexpr uint32_t NONE = 255;
+    V z[PB][NG];
     int ent[NG], pos[NG];
-    unsigned alive[NG];  // the same in every lane
+    uint32_t live[NG];  // the entry's number, NONE when it is not live
+    auto sel = [&](const auto &r, int g) {  // r[g], g the same in every lane
+      auto v = r[0];
+#pragma unroll
+      for (int u = 1; u < NG; ++u)
+        if (g == u) v = r[u];
+      return v;
+    };
 #pragma unroll
     for (int g = 0; g < NG; ++g) {
       const int e = lane + 32 * g;
       const bool in = e < nl;
-      alive[g] = __ballot_sync(FULL, in);
+      live[g] = in ? (uint32_t)e : NONE;
       ent[g] = in ? s_ent[e] : 0;
       pos[g] = in ? s_epos[e] : 0;
 #pragma unroll
-      for (int j = 0; j < PB; ++j) {
-        x[g][j] = (in && col0 + j < w) ? Wv[ent[g]][col0 + j] : 0;
-        cf[g][j] = 0;
-      }
+      for (int j = 0; j < PB; ++j) z[j][g] = (in && col0 + j < w) ? Wv[ent[g]][col0 + j] : 0;
     }
-    V sc = 0;
+    const int t0 = t;
+    [[maybe_unused]] V sc = 0;
     if constexpr (!SA::NORM) sc = sa.one();
     int next = min(col0 + PB, w), rare = -1;
+    if (lane < PB) s_pslot[lane] = -1;
+    __syncwarp();
 #pragma unroll
     for (int j = 0; j < PB; ++j) {
+      constexpr int ZALL = PB;
+      const int zn = SA::NORM ? PB - j : ZALL;  // entries of z in use
       const int col = col0 + j, i = i0 + t;
-      if (lane == 0) s_pslot[j] = -1;
-      if (col >= next || i >= m) continue;
-      unsigned nz[NG], any = 0;
+      // the pivot's entry and the first live one
+      uint32_t key = NONE, fkey = NONE;
 #pragma unroll
       for (int g = 0; g < NG; ++g) {
-        nz[g] = __ballot_sync(FULL, x[g][j] != 0);
-        any |= nz[g];
+        if (z[0][g] != 0) key = min(key, (uint32_t)(lane + 32 * g));
+        fkey = min(fkey, live[g]);
       }
-      if (any == 0) {
+      key = __reduce_min_sync(FULL, col < next && i < m ? key : NONE);
+      V znew[NG];
+#pragma unroll
+      for (int g = 0; g < NG; ++g) znew[g] = 0;
+      if (key == NONE) {
         // none in the window: rows past it whose bound allows a pivot here
         // end the block (all warps look for it)
-        if (wlast < m - 1) {
+        if (col < next && i < m && wlast < m - 1) {
           const int v = (lane <= col ? s_cnt[lane] : 0) + (lane + 32 <= col ? s_cnt[lane + 32] : 0);
           if (__reduce_add_sync(FULL, v) > 0) {
             rare = col;
             next = col;
           }
         }
-        continue;
-      }
-      // the pivot's entry (pg, pl) and the first live entry (fg, fl)
-      int pg = 0, fg = 0;
-      unsigned pm = nz[0], fm = alive[0];
-#pragma unroll
-      for (int g = 1; g < NG; ++g) {
-        if (pm == 0) {
-          pm = nz[g];
-          pg = g;
-        }
-        if (fm == 0) {
-          fm = alive[g];
-          fg = g;
-        }
-      }
-      const int pl = __ffs((int)pm) - 1;
-      auto sel = [&](const V(&r)[NG][PB], int k, int g) {
-        V v = r[0][k];
-#pragma unroll
-        for (int u = 1; u < NG; ++u)
-          if (g == u) v = r[u][k];
-        return v;
-      };
-      V pv[PB], pc[PB];  // the pivot row's entries; division-free, its coefficients
-#pragma unroll
-      for (int k = 0; k < PB; ++k) {
-        pv[k] = 0;
-        pc[k] = 0;
-        if (k >= j) pv[k] = __shfl_sync(FULL, sel(x, k, pg), pl);
-        else if (!SA::NORM) pc[k] = __shfl_sync(FULL, sel(cf, k, pg), pl);
-      }
-      const V y = pv[j];
-      if constexpr (SA::NORM) {
-        const int iv = s_inv[sa.index(y)];
-#pragma unroll
-        for (int g = 0; g < NG; ++g) {
-          const V l = sa.plain(x[g][j], iv);
-          cf[g][j] = l;  // 1 for the pivot row
-#pragma unroll
-          for (int k = j + 1; k < PB; ++k) x[g][k] = sa.step(x[g][k], l, pv[k]);
-        }
-        if (iv == 0) {  // no inverse: the call will fail, the row leaves all the same
-          if (lane == 0) s_err = 1;
+        if constexpr (SA::NORM) {
 #pragma unroll
           for (int g = 0; g < NG; ++g)
-#pragma unroll
-            for (int k = j + 1; k < PB; ++k)
-              if (lane == pl && g == pg) x[g][k] = 0;
+            if (live[g] != NONE) s_coefv[PB * ent[g] + j] = 0;
         }
-        if (lane == 0) s_xi[t] = (uint32_t)iv;
       } else {
-#pragma unroll
-        for (int g = 0; g < NG; ++g) {
-          const V na = sa.neg(x[g][j]);
-#pragma unroll
-          for (int k = 0; k < PB; ++k) {
-            if (k > j) x[g][k] = sa.upd(y, x[g][k], na, pv[k]);
-            else if (k < j) cf[g][k] = sa.upd(y, cf[g][k], na, pc[k]);
-            else cf[g][k] = sa.mul(na, sc);
-          }
-        }
-        if (lane == 0) {
-          V4 c4;
-          c4.x = pc[0];
-          c4.y = pc[1];
-          c4.z = pc[2];
-          c4.w = 0;
-          s_pcoef[j] = c4;
-          s_psc[j] = sc;
-        }
-        sc = sa.mul(y, sc);
-      }
-      if (lane == pl) {
-        int en = ent[0], po = pos[0];
-#pragma unroll
-        for (int g = 1; g < NG; ++g)
-          if (pg == g) {
-            en = ent[g];
-            po = pos[g];
-          }
-        s_pslot[j] = en;
-        s_pt[j] = t;
-        s_pcol[t] = col;
-        s_y[t] = y;
-        s_tq[t] = po;
+        // each row's inverse, looked up while the pivot's lane is found
+        [[maybe_unused]] int inv[NG];
         if constexpr (SA::NORM) {
-          V4 c4;
-          c4.x = j > 0 ? sel(cf, 0, pg) : 0;
-          c4.y = j > 1 ? sel(cf, 1, pg) : 0;
-          c4.z = j > 2 ? sel(cf, 2, pg) : 0;
-          c4.w = 0;
-          s_pcoef[j] = c4;
-        }
-      }
-      // position i: the first entry's row, or a row outside the window
-      int f = pos[0], q = pos[0];
 #pragma unroll
-      for (int g = 1; g < NG; ++g) {
-        if (fg == g) f = pos[g];
-        if (pg == g) q = pos[g];
-      }
-      const int fl = __ffs((int)fm) - 1;
-      f = __shfl_sync(FULL, f, fl);
-      q = __shfl_sync(FULL, q, pl);
-      unsigned gone = 1u << pl;  // the entry that goes, in group gg
-      int gg = pg;
-      if (f != i) {
-        if (q != i && lane == 0) {  // the row at i is outside the window
-          p2r[q] = row_at(i, p2r, stamp, epoch);
-          stamp[q] = epoch;
+          for (int g = 0; g < NG; ++g) inv[g] = sa.inverse(s_inv, z[0][g]);
         }
-      } else if (q != i) {
-        // the first entry's row moves to the pivot's entry (and position)
-        gone = 1u << fl;
-        gg = fg;
+        const int pg = (int)key >> 5, pl = (int)key & 31;
+        V pv[PB];  // the pivot row's z
+        [[maybe_unused]] int iv = 0;
+        if constexpr (SA::NORM) iv = __shfl_sync(FULL, sel(inv, pg), pl);
 #pragma unroll
-        for (int k = 0; k < PB; ++k) {
-          const V vx = k > j ? __shfl_sync(FULL, sel(x, k, fg), fl) : 0;
-          const V vc = k <= j ? __shfl_sync(FULL, sel(cf, k, fg), fl) : 0;
+        for (int k = 0; k < PB; ++k)
+          pv[k] = k < zn ? __shfl_sync(FULL, sel(z[k], pg), pl) : 0;
+        const int q = __shfl_sync(FULL, sel(pos, pg), pl);
+        fkey = __reduce_min_sync(FULL, fkey);
+        if constexpr (SA::NORM) {
 #pragma unroll
           for (int g = 0; g < NG; ++g) {
-            if (g == pg && lane == pl) {
-              x[g][k] = vx;
-              cf[g][k] = vc;
-            }
-            if (g == fg && lane == fl) x[g][k] = 0;
+            const V l = sa.plain(z[0][g], iv);  // 1 for the pivot row
+            if (live[g] != NONE) s_coefv[PB * ent[g] + j] = l;  // by slot
+#pragma unroll
+            for (int k = 1; k < PB; ++k)
+              if (k < zn) z[k][g] = sa.step(z[k][g], l, pv[k]);
+          }
+          if (iv == 0) {  // no inverse: the call will fail, the row leaves all the same
+            if (lane == 0) s_err = 1;
+#pragma unroll
+            for (int g = 0; g < NG; ++g)
+#pragma unroll
+              for (int k = 1; k < PB; ++k)
+                if (lane == pl && g == pg) z[k][g] = 0;
+          }
+        } else {
+#pragma unroll
+          for (int g = 0; g < NG; ++g) {
+            const V na = sa.neg(z[0][g]);
+            znew[g] = sa.mul(na, sc);
+#pragma unroll
+            for (int k = 1; k < PB; ++k) z[k][g] = sa.upd(pv[0], z[k][g], na, pv[k]);
           }
         }
-        int en = ent[0];
+        if (lane == pl) {
+          s_pslot[j] = sel(ent, pg);
+          s_piv[t] = make_int2(col, q);
+          s_y[t] = pv[0];
+          if constexpr (SA::NORM) {
+            s_xi[t] = iv;
+          } else {
+            s_psc[j] = sc;
+            V4 c4;  // (only the coefficients of earlier columns are read)
+            c4.x = pv[0];
+            c4.y = pv[1];
+            c4.z = pv[2];
+            c4.w = pv[3];
+            s_pcoef[j] = c4;
+          }
+        }
+        if constexpr (!SA::NORM) sc = sa.mul(pv[0], sc);
+        uint32_t gone = key;  // the entry that goes
+        if (!(fkey == key && q == i)) {
+          // position i: the first entry's row, or a row outside the window
+          const int fg = (int)fkey >> 5, fl = (int)fkey & 31;
+          const int f = __shfl_sync(FULL, sel(pos, fg), fl);
+          if (f != i) {
+            if (q != i && lane == 0) {
+              p2r[q] = row_at(i, p2r, stamp, epoch);
+              stamp[q] = epoch;
+            }
+          } else {
+            // the first entry's row moves to the pivot's entry (and position)
+            gone = fkey;
+            const int en = __shfl_sync(FULL, sel(ent, fg), fl);
+            const V vn = __shfl_sync(FULL, sel(znew, fg), fl);
 #pragma unroll
-        for (int g = 1; g < NG; ++g)
-          if (fg == g) en = ent[g];
-        en = __shfl_sync(FULL, en, fl);
+            for (int k = 1; k < PB; ++k) {
+              const V vx = __shfl_sync(FULL, sel(z[k], fg), fl);
+#pragma unroll
+              for (int g = 0; g < NG; ++g) {
+                if (g == fg && lane == fl) z[k][g] = 0;
+                if (g == pg && lane == pl) z[k][g] = vx;
+              }
+            }
+#pragma unroll
+            for (int g = 0; g < NG; ++g)
+              if (g == pg && lane == pl) {
+                ent[g] = en;
+                znew[g] = vn;
+              }
+          }
+        }
 #pragma unroll
         for (int g = 0; g < NG; ++g)
-          if (g == pg && lane == pl) ent[g] = en;
+          if (live[g] == gone) live[g] = NONE;
+        ++t;
       }
 #pragma unroll
-      for (int g = 0; g < NG; ++g)
-        if (g == gg) alive[g] &= ~gone;
-      ++t;
+      for (int g = 0; g < NG; ++g) {
+#pragma unroll
+        for (int k = 0; k + 1 < PB; ++k) z[k][g] = z[k + 1][g];
+        z[PB - 1][g] = znew[g];
+      }
     }
-    // the live entries closed up, with their coefficients
+    // the live entries closed up (division-free: and their coefficients)
     int base = 0;
 #pragma unroll
     for (int g = 0; g < NG; ++g) {
-      if (alive[g] >> lane & 1u) {
-        const int e = base + __popc(alive[g] & ((1u << lane) - 1u));
+      const unsigned alive = __ballot_sync(FULL, live[g] != NONE);
+      if (live[g] != NONE) {
+        const int e = base + __popc(alive & ((1u << lane) - 1u));
         s_ent[e] = ent[g];
         s_epos[e] = pos[g];
-        V4 c4;
-        c4.x = cf[g][0];
-        c4.y = cf[g][1];
-        c4.z = cf[g][2];
-        c4.w = cf[g][3];
-        s_coef[e] = c4;
+        if constexpr (!SA::NORM) {
+          V4 c4;
+          c4.x = z[0][g];
+          c4.y = z[1][g];
+          c4.z = z[2][g];
+          c4.w = z[3][g];
+          s_coef[ent[g]] = c4;
+        }
       }
-      base += __popc(alive[g]);
+      base += __popc(alive);
     }
     if (lane == 0) {
       s_sc = sc;
       s_next = next;
       s_rare = rare;
+      s_t0 = t0;
       s_t = t;
       s_nl = base;
     }
@@ -825,45 +837,67 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
     __syncthreads();
     // B. the columns right of the block, from the rows' values before it
     const int next = s_next, rare = s_rare;
-    const bool found_any = s_t > (wid == 0 ? -1 : t);  // (warp 0's t is s_t already)
+    const int tb = s_t0;  // pivots before the block
+    const bool found_any = s_t > tb;
     t = s_t;
     nl = s_nl;
     if (found_any) {
-      const V sc = s_sc;
+      // a warp takes one half of the columns while both have some left, and
+      // every eighth row, then every sixteenth of the upper half
+      const bool both = col0 < 32;
+      const int wh = both ? wid >> 1 : wid, nw = both ? PS_FAST / 2 : PS_FAST;
+      const int c = lane + (both ? 32 * (wid & 1) : 32);
+      const int4 ps = *reinterpret_cast<const int4 *>(s_pslot);
+      const int psk[PB] = {ps.x, ps.y, ps.z, ps.w};
+      V P[PB];  // the block's pivot rows, before it
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int c = lane + 32 * h;
-        if (h == 0 && col0 >= 32) continue;  // no column of the half is left
-        const bool right = c >= next;
-        V P[PB];  // the block's pivot rows, before it
+      for (int k = 0; k < PB; ++k) P[k] = psk[k] >= 0 && c >= col0 ? Wv[psk[k]][c] : 0;
+      if constexpr (SA::NORM) {
+        // the pivot rows' final values, in place: U_k = P_k - sum l_kj U_j
+        const V4 l1 = s_coef[max(psk[1], 0)], l2 = s_coef[max(psk[2], 0)];
+        V4 l3 = s_coef[max(psk[3], 0)];
+        l3.w = 0;
+        P[1] = psk[1] >= 0 ? sa.step(P[1], l1.x, P[0]) : 0;
+        P[2] = psk[2] >= 0 ? sa.step2(P[2], l2.x, P[0], l2.y, P[1]) : 0;
+        const V u3 = sa.lin(P[3], l3, P);
+        P[3] = psk[3] >= 0 ? u3 : 0;
+      }
+      if (wh >= nw - PB) {  // the pivot rows to PV, a warp each (and half)
+        const int k = wh - (nw - PB);
+        int tk = tb, slot = -1;  // the pivot's index: pivots of earlier columns before it
+        V u = P[0];
 #pragma unroll
-        for (int k = 0; k < PB; ++k) {
-          const int ps = s_pslot[k];
-          P[k] = ps >= 0 && c >= col0 ? Wv[ps][c] : 0;
-        }
-        // the pivot rows' final values
-        V U[PB];
-        if constexpr (SA::NORM) {
-#pragma unroll
-          for (int k = 0; k < PB; ++k) U[k] = 0;
-          U[0] = P[0];
-          U[1] = sa.lin(P[1], s_pcoef[1], U);
-          U[2] = sa.lin(P[2], s_pcoef[2], U);
-          U[3] = sa.lin(P[3], s_pcoef[3], U);
-        }
-#pragma unroll
-        for (int k = 0; k < PB; ++k)
-          if (wid == k && s_pslot[k] >= 0 && c >= col0) {
-            if constexpr (SA::NORM) PV[s_pt[k]][c] = U[k];
-            else PV[s_pt[k]][c] = sa.lin(s_psc[k], P[k], s_pcoef[k], P);
+        for (int v = 0; v < PB; ++v) {
+          if (v < k) tk += psk[v] >= 0;
+          if (v == k) {
+            slot = psk[v];
+            u = P[v];
           }
-        if (right)
-          for (int e = wid; e < nl; e += PS_FAST) {
-            const V4 cf = s_coef[e];
-            V *row = Wv[s_ent[e]];
-            if constexpr (SA::NORM) row[c] = sa.lin(row[c], cf, U);
-            else row[c] = sa.lin(sc, row[c], cf, P);
+        }
+        if (slot >= 0) {
+          if constexpr (!SA::NORM) {
+            // at its choice in column k the row's coefficients of columns 0 .. k - 1
+            // stood behind the 4 - k columns left
+            const V *zz = reinterpret_cast<const V *>(&s_pcoef[k]);
+            V4 cf;
+            cf.x = k > 0 ? zz[PB - k] : 0;
+            cf.y = k > 1 ? zz[PB - k + 1] : 0;
+            cf.z = k > 2 ? zz[PB - k + 2] : 0;
+            cf.w = 0;
+            u = sa.lin(s_psc[k], u, cf, P);
           }
+          if (c >= col0) PV[tk][c] = u;
+        }
+      }
+      [[maybe_unused]] const V sc = s_sc;
+#pragma unroll 2
+      for (int e = wh; e < nl; e += nw) {
+        const int slot = s_ent[e];
+        const V4 cf = s_coef[slot];
+        V v = Wv[slot][c];
+        if constexpr (SA::NORM) v = sa.lin(v, cf, P);
+        else v = sa.lin(sc, v, cf, P);
+        if (c >= next) Wv[slot][c] = v;
       }
     }
     col0 = next;
@@ -916,11 +950,11 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
           const uint32_t *v = D + (size_t)rj * ld + c0;
           V a0 = sa.load(lane < w ? v[lane] : 0u), a1 = sa.load(lane + 32 < w ? v[lane + 32] : 0u);
           for (int k = 0; k < t; ++k) {
-            const int pc = s_pcol[k];
+            const int pc = s_piv[k].x;
             const V f = __shfl_sync(FULL, pc < 32 ? a0 : a1, pc & 31);
             const V u0 = lane >= pc ? PV[k][lane] : 0, u1 = lane + 32 >= pc ? PV[k][lane + 32] : 0;
             if constexpr (SA::NORM) {
-              const V l = sa.plain(f, (int)s_xi[k]);
+              const V l = sa.plain(f, s_xi[k]);
               a0 = sa.step(a0, l, u0);
               a1 = sa.step(a1, l, u1);
             } else {
@@ -996,12 +1030,11 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
         if (!z) ri = row_at(i, p2r, stamp, epoch);
         p2r[found] = ri;
         stamp[found] = epoch;
-        s_pcol[t] = col;
+        s_piv[t] = make_int2(col, found);
         s_y[t] = y;
-        s_tq[t] = found;
         if constexpr (SA::NORM) {
-          s_xi[t] = s_inv[sa.index(y)];
-          if (s_xi[t] == 0u) s_err = 1;
+          s_xi[t] = sa.inverse(s_inv, y);
+          if (s_xi[t] == 0) s_err = 1;
         }
       }
       PV[t][lane] = s_red[fw][lane];
@@ -1041,11 +1074,11 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
     if constexpr (SA::NORM) {
       if (lane < t) {
         x0 = s_y[lane];
-        xinv_out[lane] = s_xi[lane];
+        xinv_out[lane] = sa.canon(s_xi[lane]);
       }
       if (lane + 32 < t) {
         x1 = s_y[lane + 32];
-        xinv_out[lane + 32] = s_xi[lane + 32];
+        xinv_out[lane + 32] = sa.canon(s_xi[lane + 32]);
       }
     } else {
       const V e = sa.one();
@@ -1103,12 +1136,12 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
       }
       if (lane < t) {
         s_sinv[lane] = si0;
-        s_xi[lane] = xi0;
+        s_xi[lane] = (int)xi0;
         xinv_out[lane] = xi0;
       }
       if (lane + 32 < t) {
         s_sinv[lane + 32] = si1;
-        s_xi[lane + 32] = xi1;
+        s_xi[lane + 32] = (int)xi1;
         xinv_out[lane + 32] = xi1;
       }
       if (__any_sync(FULL, err != 0u) && lane == 0) s_err = 1;
@@ -1122,19 +1155,20 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
   } else if (wid == 2 || wid == 3) {
     const int k = tid - 64;
     if (k < t) {
-      out->pcol[k] = (uint32_t)s_pcol[k];
+      const int2 pv = s_piv[k];
+      out->pcol[k] = (uint32_t)pv.x;
       out->ti[k] = (uint32_t)(i0 + k);
-      out->tq[k] = (uint32_t)s_tq[k];
-      hout[PANEL_W_PIV + 2 * k] = word((uint32_t)s_pcol[k]);
-      hout[PANEL_W_PIV + 2 * k + 1] = word((uint32_t)s_tq[k]);
+      out->tq[k] = (uint32_t)pv.y;
+      hout[PANEL_W_PIV + 2 * k] = word((uint32_t)pv.x);
+      hout[PANEL_W_PIV + 2 * k + 1] = word((uint32_t)pv.y);
     }
   } else if (wid == 1) {
     // the largest transposition target; the positions past the window up to
     // it, through p2r (beyond it rows have not moved)
     const int i = i0 + t;
     int hi = i - 1;
-    if (lane < t) hi = max(hi, s_tq[lane]);
-    if (lane + 32 < t) hi = max(hi, s_tq[lane + 32]);
+    if (lane < t) hi = max(hi, s_piv[lane].y);
+    if (lane + 32 < t) hi = max(hi, s_piv[lane + 32].y);
     hi = __reduce_max_sync(FULL, hi);
     int last = -1;
     for (int pos = max(wlast + 1, i) + lane; pos <= hi && pos < m; pos += 32)
@@ -1170,7 +1204,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
   };
   for (int e = tid; e < t * EW; e += PS_THREADS) {
     const int k = e / EW, c = e % EW;
-    Uout[e] = c < s_pcol[k] ? 0u : u_at(k, c);
+    Uout[e] = c < s_piv[k].x ? 0u : u_at(k, c);
   }
   __syncthreads();
   // After the result is on its way to the host: for p < 2^31 (exact
@@ -1188,8 +1222,8 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
       uint32_t v;
       if (k >= t || j >= t) v = k == j ? 1u : 0u;
       else if (j < k) v = 0u;
-      else if (j == k) v = s_xi[k];
-      else v = u_at(k, s_pcol[j]);
+      else if (j == k) v = SA::NORM ? sa.canon(s_xi[k]) : (uint32_t)s_xi[k];
+      else v = u_at(k, s_piv[j].x);
       X[k][j] = v;
     }
     __syncthreads();
@@ -1460,7 +1494,7 @@ int zp_echelon_dev(Ctx *c, int m, int n, uint32_t p, uint32_t *D, size_t ld, siz
     void *tb = nullptr;
     if ((st = ctx_buffer(c, BUF_INV, PW_TABLE, &tb))) return st;
     if (c->inv_p != p) {
-      inverse_table_kernel<<<((int)p + 255) / 256, 256, 0, c->stream>>>(p, static_cast<uint16_t *>(tb));
+      inverse_table_kernel<<<((int)p / 2 + 256) / 256, 256, 0, c->stream>>>(p, static_cast<uint16_t *>(tb));
       ctx_launched(c);
       const cudaError_t ei = cudaGetLastError();
       if (ei != cudaSuccess) return ctx_cuda(c, ei, "echelon: inverses");
