@@ -151,42 +151,97 @@ int gf2_m4rm_dev(Ctx *c, int M, int N, int K, int alpha, const uint64_t *A, size
 }
 
 // ------------------------------------------------- int8 expansion for TC
-// Ab[r][k] = bit k0+k of row r of A (K-major bytes, row pitch Kp).
-__global__ void gf2_unpack_rows_kernel(const uint64_t *__restrict__ A, size_t lda, int M, int k0,
-                                       int kc, uint8_t *__restrict__ out, int Kp) {
-  const int kq = (kc + 3) >> 2;
-  const size_t total = (size_t)M * kq;
-  for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < total;
-       idx += (size_t)gridDim.x * blockDim.x) {
-    const int r = (int)(idx / kq), k = (int)(idx % kq) * 4;
-    const int gk = k0 + k;  // k0 is a multiple of 64, so 4 bits never straddle words
-    const uint64_t wv = A[(size_t)r * lda + (gk >> 6)] >> (gk & 63);
-    uint32_t v = 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if (k + i < kc) v |= (uint32_t)((wv >> i) & 1ull) << (8 * i);
-    *reinterpret_cast<uint32_t *>(out + (size_t)r * Kp + k) = v;
+// Four bits to four 0/1 bytes: the multiplier's copies at bits 0, 7, 14, 21
+// put bit i at bit 8i.
+__device__ __forceinline__ uint32_t spread4(uint32_t nibble) {
+  return ((nibble & 15u) * 0x00204081u) & 0x01010101u;
+}
+// Sixteen bits to sixteen 0/1 bytes.
+__device__ __forceinline__ uint4 spread16(uint32_t h) {
+  return make_uint4(spread4(h), spread4(h >> 4), spread4(h >> 8), spread4(h >> 12));
+}
+
+// Ab[r][k] = bit k0+k of row r of A (K-major bytes, row pitch Kp, a multiple
+// of 64; bytes past kc are never read).  Sixteen bits to a 16-byte store per
+// thread, lanes along the row.  Bound: the bytes written (16384^2: 268 MB;
+// four bytes a thread and an index division took 209 us).
+constexpr int UNPACK_ROWS = 8;  // rows (warps) per CTA
+__global__ void __launch_bounds__(32 * UNPACK_ROWS)
+    gf2_unpack_rows_kernel(const uint64_t *__restrict__ A, size_t lda, int M, int k0,
+                           uint8_t *__restrict__ out, int Kp) {
+  const int per = Kp / 16;
+  for (int r = blockIdx.y * UNPACK_ROWS + threadIdx.y; r < M; r += gridDim.y * UNPACK_ROWS) {
+    const uint16_t *src = reinterpret_cast<const uint16_t *>(A + (size_t)r * lda + (k0 >> 6));
+    uint4 *dst = reinterpret_cast<uint4 *>(out + (size_t)r * Kp);
+    for (int q = blockIdx.x * 32 + threadIdx.x; q < per; q += gridDim.x * 32)
+      dst[q] = spread16(__ldg(src + q));
   }
 }
 
-// Bb[n][k] = bit n of row k0+k of B: one CTA of 64 threads per 64 rows of B
-// and one word (64 columns).
-__global__ void gf2_unpack_cols_kernel(const uint64_t *__restrict__ B, size_t ldb, int k0, int kc,
-                                       int N, uint8_t *__restrict__ out, int Kp) {
-  __shared__ uint64_t rows[64];
-  const int w = blockIdx.x, kb = blockIdx.y * 64;
-  const int t = threadIdx.x;
-  rows[t] = (kb + t < kc) ? B[(size_t)(k0 + kb + t) * ldb + w] : 0ull;
-  __syncthreads();
-  const int n = w * 64 + t;
-  if (n >= N) return;
-  uint8_t *dst = out + (size_t)n * Kp + kb;
-  for (int q = 0; q < 64 && kb + q < Kp; q += 4) {
-    uint32_t v = 0;
+// Bb[n][k] = bit n of row k0+k of B.  A CTA takes UNPACK_W words of UNPACK_K
+// rows: a warp holds 32 rows' words, a 32 x 32 bit transposition per half word
+// (five exchanges of bit blocks between lanes) gives each column's 32 bits,
+// kept in shared memory; then a warp writes a column's UNPACK_K bytes at
+// once, 16 per lane.  Bound: the bytes written (16384^2, 268 MB: 580 us with
+// one column per thread and a 64-bit shift per byte, 162 us with 16-byte
+// stores a row pitch apart from the lanes of the transposition).
+constexpr int UNPACK_K = 512, UNPACK_W = 4, UNPACK_WARPS = 8;
+__device__ __forceinline__ uint32_t transpose32(uint32_t x, int lane) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) v |= (uint32_t)((rows[q + i] >> t) & 1ull) << (8 * i);
-    *reinterpret_cast<uint32_t *>(dst + q) = v;
+  for (int j = 16; j > 0; j >>= 1) {
+    const uint32_t low = j == 16  ? 0x0000ffffu
+                         : j == 8 ? 0x00ff00ffu
+                         : j == 4 ? 0x0f0f0f0fu
+                         : j == 2 ? 0x33333333u
+                                  : 0x55555555u;
+    const uint32_t y = __shfl_xor_sync(0xffffffffu, x, j);
+    x = (lane & j) ? (x & ~low) | ((y & ~low) >> j) : (x & low) | ((y & low) << j);
   }
+  return x;
+}
+__global__ void __launch_bounds__(32 * UNPACK_WARPS)
+    gf2_unpack_cols_kernel(const uint64_t *__restrict__ B, size_t ldb, int k0, int kc, int N,
+                           uint8_t *__restrict__ out, int Kp) {
+  __shared__ uint32_t bits[64 * UNPACK_W][UNPACK_K / 32 + 1];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int w0 = blockIdx.x * UNPACK_W, kb0 = blockIdx.y * UNPACK_K;
+  const int words = min(UNPACK_W, (N + 63) / 64 - w0);
+  for (int u = wid; u < UNPACK_K / 32; u += UNPACK_WARPS) {
+    const int k = kb0 + 32 * u + lane;
+    const uint64_t *src = B + (size_t)(k0 + k) * ldb + w0;
+    uint64_t v[UNPACK_W];
+#pragma unroll
+    for (int j = 0; j < UNPACK_W; ++j) v[j] = k < kc && j < words ? __ldg(src + j) : 0ull;
+#pragma unroll
+    for (int j = 0; j < UNPACK_W; ++j) {
+      bits[64 * j + lane][u] = transpose32((uint32_t)v[j], lane);
+      bits[64 * j + lane + 32][u] = transpose32((uint32_t)(v[j] >> 32), lane);
+    }
+  }
+  __syncthreads();
+  const int kk = 16 * lane;  // this lane's bytes of a column
+  if (kb0 + kk >= Kp) return;
+  const int cols = min(64 * UNPACK_W, N - 64 * w0);
+  for (int n = wid; n < cols; n += UNPACK_WARPS) {
+    const uint32_t h = bits[n][kk >> 5] >> (kk & 16);
+    *reinterpret_cast<uint4 *>(out + (size_t)(64 * w0 + n) * Kp + kb0 + kk) = spread16(h);
+  }
+}
+static_assert(UNPACK_K == 32 * 16, "a warp writes a column's bytes at once");
+
+static void unpack_rows(Ctx *c, const uint64_t *A, size_t lda, int M, int k0, uint8_t *out, int Kp) {
+  // one pass a warp up to 16 CTAs an SM, then more
+  const int gy = std::min((M + UNPACK_ROWS - 1) / UNPACK_ROWS, c->num_sms * 16);
+  const int gx = std::max(1, std::min((Kp / 16 + 31) / 32, c->num_sms * 16 / gy));
+  gf2_unpack_rows_kernel<<<dim3(gx, gy), dim3(32, UNPACK_ROWS), 0, c->stream>>>(A, lda, M, k0, out, Kp);
+  ctx_launched(c);
+}
+static void unpack_cols(Ctx *c, const uint64_t *B, size_t ldb, int k0, int kc, int N, uint8_t *out,
+                        int Kp) {
+  const int Nw = (N + 63) / 64;
+  gf2_unpack_cols_kernel<<<dim3((Nw + UNPACK_W - 1) / UNPACK_W, (Kp + UNPACK_K - 1) / UNPACK_K),
+                           32 * UNPACK_WARPS, 0, c->stream>>>(B, ldb, k0, kc, N, out, Kp);
+  ctx_launched(c);
 }
 
 int gf2_gemm_dev(Ctx *c, int kernel, int M, int N, int K, int alpha, const uint64_t *A,
@@ -213,14 +268,10 @@ int gf2_gemm_dev(Ctx *c, int kernel, int M, int N, int K, int alpha, const uint6
     const int kc = std::min(ZP_KCHUNK, K - k0);
     const int Kp = (kc + 63) & ~63;
     uint8_t *Bb = Ab + (size_t)M * Kp;
-    const size_t total = (size_t)M * ((kc + 3) / 4);
-    int grid = (int)std::min<size_t>((total + 255) / 256, (size_t)c->num_sms * 16);
     int pi = prof_begin(c, "gf2_unpack");
-    gf2_unpack_rows_kernel<<<grid, 256, 0, c->stream>>>(A, lda, M, k0, kc, Ab, Kp);
-    dim3 g2(Nw, Kp / 64);
-    gf2_unpack_cols_kernel<<<g2, 64, 0, c->stream>>>(B, ldb, k0, kc, N, Bb, Kp);
+    unpack_rows(c, A, lda, M, k0, Ab, Kp);
+    unpack_cols(c, B, ldb, k0, kc, N, Bb, Kp);
     prof_end(c, pi);
-    ctx_launched(c, 2);
     if ((st = gf2_gemm_tc_planes(c, M, N, kc, Ab, Bb, Kp, 1u, b, C, ldc))) return st;
     b = 1;
   }
@@ -279,9 +330,8 @@ int gf2_gemm_host_rows(Ctx *c, int M, int N, int K, const uint64_t *hA, size_t l
   if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream, ev_b, 0);
   if (e == cudaSuccess) {
     int pi = prof_begin(c, "gf2_unpack");
-    gf2_unpack_cols_kernel<<<dim3(Nw, Kp / 64), 64, 0, c->stream>>>(dB, (size_t)Nw, 0, K, N, Bb, Kp);
+    unpack_cols(c, dB, (size_t)Nw, 0, K, N, Bb, Kp);
     prof_end(c, pi);
-    ctx_launched(c);
     e = cudaGetLastError();
   }
   for (int j = 0; e == cudaSuccess && !st && j < nblk; ++j) {
@@ -289,13 +339,9 @@ int gf2_gemm_host_rows(Ctx *c, int M, int N, int K, const uint64_t *hA, size_t l
     uint8_t *Aj = Ab + (size_t)r0 * Kp;
     e = cudaStreamWaitEvent(c->stream, ready[j], 0);
     if (e != cudaSuccess) break;
-    const size_t total = (size_t)rows * ((K + 3) / 4);
-    const int grid = (int)std::min<size_t>((total + 255) / 256, (size_t)c->num_sms * 16);
     int pi = prof_begin(c, "gf2_unpack");
-    gf2_unpack_rows_kernel<<<grid, 256, 0, c->stream>>>(dA + (size_t)r0 * Kw, (size_t)Kw, rows, 0,
-                                                        K, Aj, Kp);
+    unpack_rows(c, dA + (size_t)r0 * Kw, (size_t)Kw, rows, 0, Aj, Kp);
     prof_end(c, pi);
-    ctx_launched(c);
     st = gf2_gemm_tc_planes(c, rows, N, K, Aj, Bb, Kp, 1u, (uint32_t)(beta & 1),
                             dC + (size_t)r0 * Nw, (size_t)Nw);
     if (st) break;
