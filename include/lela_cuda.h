@@ -61,7 +61,7 @@ enum {
 
 /* Kernel choice for the Z/p gemm (lela_cuda_set_gemm_kernel). */
 enum {
-	LELA_CUDA_GEMM_AUTO = 0,   /* small-K CUDA-core kernel for small problems, else tensor cores */
+	LELA_CUDA_GEMM_AUTO = 0,   /* tensor cores, in one launch for small K and few tiles */
 	LELA_CUDA_GEMM_PLAIN = 1,  /* CUDA-core delayed-reduction kernel */
 	LELA_CUDA_GEMM_TC = 2,     /* limb-split INT8 tcgen05 kernel */
 	LELA_CUDA_GEMM_SMALLK = 3  /* CUDA-core kernel for small K (unchecked sums when p < 2^28) */
@@ -82,7 +82,8 @@ void *lela_cuda_get_stream (lela_cuda_ctx *ctx);
 int lela_cuda_synchronize (lela_cuda_ctx *ctx);
 int lela_cuda_set_gemm_kernel (lela_cuda_ctx *ctx, int kernel);
 /* Tile variant of the tensor-core Z/p gemm: 0 = automatic (variant 0 for
- * two limbs at k >= 512 and for four limbs, else variant 1), 1 = variant 0 (wide tiles: 256 / 128 / 32
+ * four limbs, for two at k >= 512 and for one at k >= 1024 where it has tiles
+ * enough for the SMs, else variant 1), 1 = variant 0 (wide tiles: 256 / 128 / 32
  * columns for 1 / 2 / 4 limbs), 2 = variant 1 (128 / 64 columns for 1 / 2
  * limbs with two TMEM accumulator buffers, so the epilogue of one tile
  * overlaps the products of the next; four limbs always use variant 0).

@@ -1400,10 +1400,20 @@ static size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
 static int gemm_elem_dev(Ctx *c, int elem, size_t m, size_t n, size_t k, uint32_t p, uint32_t a,
                          const void *A, size_t lda, const void *B, size_t ldb, uint32_t b, void *C,
                          size_t ldc) {
-  const size_t ba = al256(m * k * 4), bb = al256(k * n * 4), bc = al256(m * n * 4);
   void *buf = nullptr;
-  int st = ctx_buffer(c, BUF_ELEM, ba + bb + bc, &buf);
-  if (st) return st;
+  int st;
+  if (k && a % p && zp_gemm_pick(c, (int)m, (int)n, (int)k, p) == GEMM_TC) {
+    // the tensor-core path splits A and B from type T; its product, rows
+    // padded to 16 bytes, and C combine in one pass
+    const size_t ldv = (n + 3) & ~(size_t)3;
+    if ((st = ctx_buffer(c, BUF_ELEM, m * ldv * 4, &buf))) return st;
+    uint32_t *V = static_cast<uint32_t *>(buf);
+    if ((st = zp_gemm_tc_elem_dev(c, elem, (int)m, (int)n, (int)k, p, a, A, lda, B, ldb, V, ldv)))
+      return st;
+    return elem_combine(c, elem, V, ldv, C, ldc, (int)m, (int)n, p, b % p);
+  }
+  const size_t ba = al256(m * k * 4), bb = al256(k * n * 4), bc = al256(m * n * 4);
+  if ((st = ctx_buffer(c, BUF_ELEM, ba + bb + bc, &buf))) return st;
   uint32_t *uA = static_cast<uint32_t *>(buf);
   uint32_t *uB = reinterpret_cast<uint32_t *>(static_cast<char *>(buf) + ba);
   uint32_t *uC = reinterpret_cast<uint32_t *>(static_cast<char *>(buf) + ba + bb);

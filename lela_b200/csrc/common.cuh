@@ -158,6 +158,12 @@ __device__ __forceinline__ void fence_barrier_init() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+// Shared-memory writes of this thread made visible to the asynchronous proxy
+// (operands of tcgen05.mma written by ordinary stores).
+__device__ __forceinline__ void fence_proxy_async() {
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
 __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(

@@ -18,10 +18,11 @@ namespace lela {
 
 // Kernel families a caller (or the selector) can force.
 enum GemmKernel : int {
-  GEMM_AUTO = 0,    // small-K CUDA-core kernel below its crossover, else tensor cores
+  GEMM_AUTO = 0,    // GEMM_DIRECT for short K and few tiles, else GEMM_TC (zp_gemm_pick)
   GEMM_PLAIN = 1,   // CUDA-core 64-bit delayed-reduction gemm (the plain GPU form)
   GEMM_TC = 2,      // limb-split INT8 tcgen05 gemm
   GEMM_SMALLK = 3,  // CUDA-core gemm for small K (no per-term wrap check when p < 2^28)
+  GEMM_DIRECT = 4,  // limb-split INT8 tcgen05 tile kernel that splits its own operands
 };
 
 // Tile variant of the tensor-core gemm (TcCfg in zp_gemm.cu): variant 0
@@ -29,7 +30,7 @@ enum GemmKernel : int {
 // (narrower tiles, two accumulator buffers, so that a tile's epilogue
 // overlaps the next tile's products); four limbs have variant 0 only.
 enum GemmTile : int {
-  GEMM_TILE_AUTO = 0,    // variant 0 for two limbs at K >= 512 and four limbs, else variant 1
+  GEMM_TILE_AUTO = 0,    // by limbs, K and tile count (zp_gemm_tile_pick)
   GEMM_TILE_WIDE = 1,    // variant 0
   GEMM_TILE_DOUBLE = 2,  // variant 1
 };

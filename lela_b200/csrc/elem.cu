@@ -11,8 +11,10 @@
 // Their gemm and trsm compute exact Z/p results (the float / double gemm of
 // lela/blas/level3-modular.tcc:25-122 accumulates blocks of products that
 // stay below 2^24 / 2^53, then reduces), so the result is a function of the
-// residues alone.  Here each operand is converted to residues in a uint32
-// scratch copy (one pass over HBM), the uint32 path computes, and the
+// residues alone.  The tensor-core gemm reads A and B as they are stored (its
+// limb split takes any element type) and leaves alpha A B as residues, which
+// elem_combine adds to beta C in place.  Elsewhere each operand is converted to
+// residues in a uint32 scratch copy (one pass over HBM), the uint32 path computes, and the
 // result is converted back: residue r is stored as r for the integer types
 // and as r or r - p, whichever lies in [-p/2, p/2], for float and double.
 // For an even p the residue p/2 has two representatives in the reference
@@ -26,44 +28,11 @@
 #include "common.cuh"
 #include "context.h"
 #include "elem.h"
+#include "elem_rep.cuh"
 
 namespace lela {
 
 namespace {
-
-template <class T>
-struct Rep;
-template <>
-struct Rep<uint8_t> {
-  static __device__ __forceinline__ uint32_t in(uint8_t x, uint32_t) { return x; }
-  static __device__ __forceinline__ uint8_t out(uint32_t r, uint32_t) { return (uint8_t)r; }
-};
-template <>
-struct Rep<uint16_t> {
-  static __device__ __forceinline__ uint32_t in(uint16_t x, uint32_t) { return x; }
-  static __device__ __forceinline__ uint16_t out(uint32_t r, uint32_t) { return (uint16_t)r; }
-};
-template <>
-struct Rep<float> {
-  // x is an integer of magnitude below 2^24, so the conversions are exact
-  static __device__ __forceinline__ uint32_t in(float x, uint32_t p) {
-    const int v = (int)x;
-    return v < 0 ? (uint32_t)(v + (int)p) : (uint32_t)v;
-  }
-  static __device__ __forceinline__ float out(uint32_t r, uint32_t p) {
-    return 2ull * r > p ? (float)((int)r - (int)p) : (float)r;
-  }
-};
-template <>
-struct Rep<double> {
-  static __device__ __forceinline__ uint32_t in(double x, uint32_t p) {
-    const long long v = (long long)x;
-    return v < 0 ? (uint32_t)(v + (long long)p) : (uint32_t)v;
-  }
-  static __device__ __forceinline__ double out(uint32_t r, uint32_t p) {
-    return 2ull * r > p ? (double)((long long)r - (long long)p) : (double)r;
-  }
-};
 
 constexpr int CONV_THREADS = 256;
 constexpr int CONV_COLS = 256;  // columns per CTA row pass
@@ -102,6 +71,43 @@ __global__ void __launch_bounds__(CONV_THREADS)
   }
 }
 
+// C <- out (beta in (C) + v), v the residues of alpha A B (beta = 0: C is not
+// read).  Four columns per thread a warp's width apart, so that loads and stores
+// coalesce for any alignment and several are in flight.
+constexpr int COMB_PER = 4;
+template <class T>
+__global__ void __launch_bounds__(CONV_THREADS)
+    combine_kernel(const uint32_t *__restrict__ V, size_t ldv, T *__restrict__ C, size_t ldc,
+                   int rows, int cols, Modulus mod, uint32_t beta) {
+  const uint32_t p = (uint32_t)mod.p;
+  const int c0 = blockIdx.x * CONV_COLS * COMB_PER + threadIdx.x;
+  for (int r = blockIdx.y; r < rows; r += gridDim.y) {
+    const uint32_t *v = V + (size_t)r * ldv;
+    T *d = C + (size_t)r * ldc;
+    uint32_t x[COMB_PER], y[COMB_PER];
+#pragma unroll
+    for (int u = 0; u < COMB_PER; ++u) {
+      const int cc = c0 + u * CONV_THREADS;
+      x[u] = cc < cols ? v[cc] : 0u;
+      y[u] = beta && cc < cols ? Rep<T>::in(d[cc], p) : 0u;
+    }
+#pragma unroll
+    for (int u = 0; u < COMB_PER; ++u) {
+      const int cc = c0 + u * CONV_THREADS;
+      if (cc < cols) {
+        uint32_t s = x[u];
+        if (beta) {  // (x < p; a caller's non-canonical element is reduced)
+          const uint32_t z = beta != 1u ? mod_mul(y[u], beta, mod)
+                             : y[u] >= p ? mod_reduce(y[u], mod) : y[u];
+          const uint32_t t = p - z;
+          s = s >= t ? s - t : s + z;
+        }
+        d[cc] = Rep<T>::out(s, p);
+      }
+    }
+  }
+}
+
 dim3 conv_grid(const Ctx *c, int rows, int cols) {
   const int gx = (cols + CONV_COLS - 1) / CONV_COLS;
   // enough CTAs for every SM several times over, capped by the rows
@@ -127,6 +133,18 @@ int from_u32_t(Ctx *c, const uint32_t *src, size_t lds, void *dst, size_t ldd, i
   ctx_launched(c);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? ST_OK : ctx_cuda(c, e, "element conversion");
+}
+
+template <class T>
+int combine_t(Ctx *c, const uint32_t *V, size_t ldv, void *C, size_t ldc, int rows, int cols,
+              uint32_t p, uint32_t beta) {
+  const int gx = (cols + CONV_COLS * COMB_PER - 1) / (CONV_COLS * COMB_PER);
+  const int want = std::max(1, (c->num_sms * 8 + gx - 1) / gx);
+  combine_kernel<T><<<dim3(gx, std::min(rows, std::min(want, 65535))), CONV_THREADS, 0, c->stream>>>(
+      V, ldv, static_cast<T *>(C), ldc, rows, cols, make_modulus(p), beta);
+  ctx_launched(c);
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? ST_OK : ctx_cuda(c, e, "element combine");
 }
 
 }  // namespace
@@ -185,6 +203,18 @@ int elem_from_u32(Ctx *c, int elem, const uint32_t *src, size_t lds, void *dst, 
     case LELA_CUDA_ELEM_U16: return from_u32_t<uint16_t>(c, src, lds, dst, ldd, rows, cols, p);
     case LELA_CUDA_ELEM_F32: return from_u32_t<float>(c, src, lds, dst, ldd, rows, cols, p);
     case LELA_CUDA_ELEM_F64: return from_u32_t<double>(c, src, lds, dst, ldd, rows, cols, p);
+    default: return ctx_fail(c, ST_ARG, "unknown element type");
+  }
+}
+
+int elem_combine(Ctx *c, int elem, const uint32_t *V, size_t ldv, void *C, size_t ldc, int rows,
+                 int cols, uint32_t p, uint32_t beta) {
+  if (rows <= 0 || cols <= 0) return ST_OK;
+  switch (elem) {
+    case LELA_CUDA_ELEM_U8: return combine_t<uint8_t>(c, V, ldv, C, ldc, rows, cols, p, beta);
+    case LELA_CUDA_ELEM_U16: return combine_t<uint16_t>(c, V, ldv, C, ldc, rows, cols, p, beta);
+    case LELA_CUDA_ELEM_F32: return combine_t<float>(c, V, ldv, C, ldc, rows, cols, p, beta);
+    case LELA_CUDA_ELEM_F64: return combine_t<double>(c, V, ldv, C, ldc, rows, cols, p, beta);
     default: return ctx_fail(c, ST_ARG, "unknown element type");
   }
 }

@@ -20,4 +20,9 @@ int elem_to_u32(Ctx *c, int elem, const void *src, size_t lds, uint32_t *dst, si
 int elem_from_u32(Ctx *c, int elem, const uint32_t *src, size_t lds, void *dst, size_t ldd,
                   int rows, int cols, uint32_t p);
 
+// C (type elem) <- beta C + V in place, V residues (row stride ldv), beta in
+// [0, p); with beta = 0 C is not read.
+int elem_combine(Ctx *c, int elem, const uint32_t *V, size_t ldv, void *C, size_t ldc, int rows,
+                 int cols, uint32_t p, uint32_t beta);
+
 }  // namespace lela

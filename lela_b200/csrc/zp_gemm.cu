@@ -37,9 +37,11 @@
 //    whose inner loop is exactly the reference's delayed-reduction dot
 //    (64-bit sum of 32x32-bit products, + 2^64 mod p on wrap-around, one
 //    final reduction).
-// 3. zp_gemm_smallk_kernel -- CUDA-core gemm for the small-K updates of the
-//    triangular solve and the echelon panels, where the tensor-core path's
-//    fixed cost (limb splits, tensor maps, pipeline start) dominates.  For
+// 3. zp_gemm_direct_kernel<L> -- the tensor-core tile product in one launch,
+//    for the short-K updates of the triangular solve and the echelon panels,
+//    where the first kernel's fixed cost (limb splits, tensor maps, pipeline
+//    start) dominates: each CTA splits its own operands into shared memory.
+// 4. zp_gemm_smallk_kernel -- CUDA-core gemm for small K, by request only.  For
 //    p < 2^28 a 64-bit sum of 256 products cannot wrap, so the products are
 //    summed without checks and the sums reduced every 256 terms.
 #include <cuda.h>
@@ -50,7 +52,9 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "../../include/lela_cuda.h"
 #include "context.h"
+#include "elem_rep.cuh"
 #include "zp_gemm.h"
 
 namespace lela {
@@ -649,61 +653,276 @@ __global__ void __launch_bounds__(tc_threads<L, T>(), 1)
   }
 }
 
-// ------------------------------------------------------------ limb splits
-// A (M x kc, row stride lda, u32) -> L planes of M x Kp bytes.
+// ------------------------------------------------- one-launch tile kernel
+// The same tile product without limb planes in memory, for short K and small
+// problems, where the two split launches and the tensor maps cost more than
+// the product: a CTA loads its 128 x K rows of A and K x BN columns of B
+// (u32), splits them into limbs on the way to shared memory (K-major, in the
+// 128-byte swizzle the tensor cores read), multiplies, and writes its tile.  K
+// goes in chunks of 128 through two stages, so a chunk's loads overlap the
+// MMAs of the one before.  Every CTA splits its own operands, so it pays only
+// where a tile's K is short or the tiles fill about one wave (zp_gemm_pick).
 template <int L>
-__global__ void split_rows_kernel(const uint32_t *__restrict__ A, size_t lda, int M, int kc,
-                                  uint8_t *__restrict__ out, int Kp) {
-  const int kq = (kc + 3) >> 2;
-  const size_t total = (size_t)M * kq;
-  const size_t plane = (size_t)M * Kp;
-  for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < total;
-       idx += (size_t)gridDim.x * blockDim.x) {
-    const int r = (int)(idx / kq), k = (int)(idx % kq) * 4;
-    const uint32_t *src = A + (size_t)r * lda + k;
-    uint32_t v[4];
+struct DirCfg {
+  static constexpr int BN = L == 4 ? 32 : 64, NMMA = L * BN;
+  static constexpr int TMEM = L * NMMA;  // 64, 256 or 512 columns
+  static constexpr int A_BYTES = L * BM * BK, B_BYTES = NMMA * BK;
+  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+  static constexpr int smem(int stages) { return stages * STAGE_BYTES + 64 + 1024; }
+};
+constexpr int DIR_THREADS = 256;
+
+// Byte offset of (row r, K byte k) in a K-major operand with 128-byte rows:
+// 16-byte pieces exchanged by the row's number in its group of eight.
+__device__ __forceinline__ int sw128(int r, int k) {
+  return r * 128 + ((((k >> 4) ^ r) & 7) << 4) + (k & 15);
+}
+// Limb l of four residues as four bytes.
+__device__ __forceinline__ uint32_t limb4(const uint32_t (&v)[4], int l) {
+  const uint32_t a = __byte_perm(v[0], v[1], (l | (4 + l) << 4) & 0xff);
+  const uint32_t b = __byte_perm(v[2], v[3], (l | (4 + l) << 4) & 0xff);
+  return (a & 0xffffu) | (b << 16);
+}
+
+template <int L, int MODE>
+__device__ __noinline__ void dir_epilogue(uint32_t tmem, uint64_t *done, uint32_t *err, uint32_t *C,
+                                          size_t ldc, int M, int N, const Modulus &mod,
+                                          uint32_t alpha, uint32_t beta) {
+  using Cfg = DirCfg<L>;
+  constexpr int W = Cfg::BN / 2;  // two warps per lane quadrant
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = warp & 3;
+  const int gm = blockIdx.y * BM + q * 32 + lane, cbeg = (warp >> 2) * W;
+  const int gn = blockIdx.x * Cfg::BN + cbeg;
+  const Mod32 m32 = Mod32::make(L < 4 ? (uint32_t)mod.p : 3u);
+  const bool vec = ((reinterpret_cast<uintptr_t>(C) & 15u) == 0) && ((ldc & 3u) == 0);
+  uint32_t *crow = gm < M ? C + (size_t)gm * ldc : nullptr;
+  uint32_t c[W];
+  if (MODE != EPI_SET) load_c<W>(c, crow, gn, N, vec);
+  if (!mbar_wait(done, 0, err)) return;
+  tc_fence_after();
+  const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)cbeg;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] = (k + i < kc) ? __ldg(src + i) : 0u;
+  for (int h = 0; h < W / 16; ++h) {
+    uint32_t v[16];
+    chunk_products<L, Cfg::BN, Cfg::NMMA>(tbase + 16 * h, v, mod, m32);
 #pragma unroll
-    for (int l = 0; l < L; ++l) {
-      uint32_t w = 0;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) w |= ((v[i] >> (8 * l)) & 0xFFu) << (8 * i);
-      *reinterpret_cast<uint32_t *>(out + l * plane + (size_t)r * Kp + k) = w;
+    for (int i = 0; i < 16; ++i)
+      c[16 * h + i] = epi_combine<MODE, (L < 4)>(v[i], MODE != EPI_SET ? c[16 * h + i] : 0u, mod,
+                                                 m32, alpha, beta);
+  }
+  store_c<W>(c, crow, gn, N, vec);
+}
+
+template <int L>
+__global__ void __launch_bounds__(DIR_THREADS, L == 4 ? 1 : 2)
+    zp_gemm_direct_kernel(const uint32_t *__restrict__ A, size_t lda,
+                          const uint32_t *__restrict__ B, size_t ldb, uint32_t *C, size_t ldc,
+                          int M, int N, int K, int stages, Modulus mod, uint32_t alpha,
+                          uint32_t beta, uint32_t *err) {
+  using Cfg = DirCfg<L>;
+  constexpr int BN = Cfg::BN;
+  constexpr uint32_t IDESC = idesc_u8_s32(BM, Cfg::NMMA);
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t *smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
+  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + stages * Cfg::STAGE_BYTES);
+  uint64_t *freeb = bars, *done = bars + 2;  // stage read by the MMAs; all MMAs done
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 3);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+  if (tid == 0) {
+    mbar_init(&freeb[0], 1);
+    mbar_init(&freeb[1], 1);
+    mbar_init(done, 1);
+    fence_barrier_init();
+  }
+  if (warp == 1) tmem_alloc(tmem_slot, Cfg::TMEM);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  const bool vecA = ((reinterpret_cast<uintptr_t>(A) & 15u) == 0) && ((lda & 3u) == 0);
+  bool ok = true;
+  int c = 0;
+  for (int k0 = 0; k0 < K; k0 += BK, ++c) {
+    const int kc = min(BK, K - k0), kr = (kc + 31) & ~31;  // multiplied: whole MMAs of 32
+    const int s = c & 1;
+    uint8_t *sa = smem + s * Cfg::STAGE_BYTES, *sb = sa + Cfg::A_BYTES;
+    // (two chunks before, this stage's)
+    if (c >= 2 && !mbar_wait(&freeb[s], (uint32_t)((c >> 1) - 1) & 1u, err)) ok = false;
+    if (__syncthreads_or(!ok)) {
+      ok = false;
+      break;
     }
+    // A: a warp per row, four columns per lane
+    constexpr int AU = 8;  // rows in flight per warp
+#pragma unroll 1
+    for (int r0 = warp * AU; r0 < BM; r0 += 8 * AU) {
+      uint32_t v[AU][4];
+      const int k = 4 * lane;
+#pragma unroll
+      for (int u = 0; u < AU; ++u) {
+        const int gm = m0 + r0 + u;
+        const uint32_t *src = A + (size_t)gm * lda + k0 + k;
+        if (gm < M && vecA && k + 3 < kc) {
+          const uint4 x = __ldg(reinterpret_cast<const uint4 *>(src));
+          v[u][0] = x.x;
+          v[u][1] = x.y;
+          v[u][2] = x.z;
+          v[u][3] = x.w;
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) v[u][i] = (gm < M && k + i < kc) ? __ldg(src + i) : 0u;
+        }
+      }
+      if (k < kr)
+#pragma unroll
+        for (int u = 0; u < AU; ++u)
+#pragma unroll
+          for (int l = 0; l < L; ++l)
+            *reinterpret_cast<uint32_t *>(sa + l * BM * BK + sw128(r0 + u, k)) = limb4(v[u], l);
+    }
+    // B: lanes on columns, four rows per thread and step
+    constexpr int BG = BN / 32, BU = 4;  // column groups; steps in flight
+#pragma unroll 1
+    for (int e0 = warp * BU; e0 < BG * (kr / 4); e0 += 8 * BU) {
+      uint32_t v[BU][4];
+#pragma unroll
+      for (int u = 0; u < BU; ++u) {
+        const int e = e0 + u, k = 4 * (e / BG), n = n0 + (e % BG) * 32 + lane;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          v[u][i] = (n < N && k + i < kc) ? __ldg(B + (size_t)(k0 + k + i) * ldb + n) : 0u;
+      }
+#pragma unroll
+      for (int u = 0; u < BU; ++u) {
+        const int e = e0 + u, k = 4 * (e / BG), nr = (e % BG) * 32 + lane;
+        if (k < kr)
+#pragma unroll
+          for (int l = 0; l < L; ++l)
+            *reinterpret_cast<uint32_t *>(sb + sw128(l * BN + nr, k)) = limb4(v[u], l);
+      }
+    }
+    fence_proxy_async();
+    __syncthreads();
+    if (tid == 0) {
+      tc_fence_after();
+      const uint64_t bd = smem_desc_sw128(sb);
+      for (int l = 0; l < L; ++l) {
+        const uint64_t ad = smem_desc_sw128(sa + l * BM * BK);
+        for (int kk = 0; kk < kr / 32; ++kk)
+          mma_u8(tmem + (uint32_t)(l * Cfg::NMMA), ad + 2 * kk, bd + 2 * kk, IDESC,
+                 (c != 0 || kk != 0) ? 1u : 0u);
+      }
+      mma_commit(&freeb[s]);
+    }
+  }
+  if (tid == 0) mma_commit(done);  // (also when a wait ran out: all MMAs end before TMEM goes)
+  if (ok) {
+    const int emode = beta == 0u ? EPI_SET
+                      : (beta == 1u && alpha == 1u) ? EPI_ADD
+                      : (beta == 1u && alpha == (uint32_t)mod.p - 1u) ? EPI_SUB
+                                                                     : EPI_AXPBY;
+    switch (emode) {
+      case EPI_ADD: dir_epilogue<L, EPI_ADD>(tmem, done, err, C, ldc, M, N, mod, alpha, beta); break;
+      case EPI_SUB: dir_epilogue<L, EPI_SUB>(tmem, done, err, C, ldc, M, N, mod, alpha, beta); break;
+      case EPI_SET: dir_epilogue<L, EPI_SET>(tmem, done, err, C, ldc, M, N, mod, alpha, beta); break;
+      default: dir_epilogue<L, EPI_AXPBY>(tmem, done, err, C, ldc, M, N, mod, alpha, beta); break;
+    }
+  }
+  if (tid == 0) mbar_drain(done, 0, err);
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem, Cfg::TMEM);
   }
 }
 
-// B (kc x N, row stride ldb, u32) -> L planes of N x Kp bytes (transposed),
-// through a 64 (k) x 32 (n) shared-memory tile.
-template <int L>
-__global__ void split_cols_kernel(const uint32_t *__restrict__ B, size_t ldb, int kc, int N,
-                                  uint8_t *__restrict__ out, int Kp) {
-  __shared__ uint32_t tile[64][33];
-  const int n0 = blockIdx.x * 32, k0 = blockIdx.y * 64;
+// ------------------------------------------------------------ limb splits
+// A (M x kc, row stride lda, elements T) -> L planes of M x Kp bytes.  Bound by
+// HBM (8192^2 of u32: 69 us, 402 MB); lanes on consecutive groups of four
+// columns, a row per warp, so no index division.
+constexpr int SPLIT_ROWS = 8;  // rows (warps) per CTA
+template <int L, class T>
+__global__ void __launch_bounds__(32 * SPLIT_ROWS)
+    split_rows_kernel(const T *__restrict__ A, size_t lda, int M, int kc, uint32_t p,
+                      uint8_t *__restrict__ out, int Kp) {
+  const int kq = (kc + 3) >> 2;
+  const size_t plane = (size_t)M * Kp;
+  for (int r = blockIdx.y * SPLIT_ROWS + threadIdx.y; r < M; r += gridDim.y * SPLIT_ROWS) {
+    const T *src = A + (size_t)r * lda;
+    uint8_t *dst = out + (size_t)r * Kp;
+    for (int q = blockIdx.x * 32 + threadIdx.x; q < kq; q += gridDim.x * 32) {
+      const int k = 4 * q;
+      uint32_t v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[i] = (k + i < kc) ? Rep<T>::in(__ldg(src + k + i), p) : 0u;
+#pragma unroll
+      for (int l = 0; l < L; ++l) {
+        uint32_t w = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w |= ((v[i] >> (8 * l)) & 0xFFu) << (8 * i);
+        *reinterpret_cast<uint32_t *>(dst + l * plane + k) = w;
+      }
+    }
+  }
+}
+static dim3 split_rows_grid(int num_sms, int M, int kc) {
+  // one pass a warp up to 16 CTAs an SM, then more
+  const int gy = std::min((M + SPLIT_ROWS - 1) / SPLIT_ROWS, num_sms * 16);
+  return dim3(std::max(1, std::min(((kc + 3) / 4 + 31) / 32, num_sms * 16 / gy)), gy);
+}
+
+// B (kc x N, row stride ldb, elements T) -> L planes of N x Kp bytes
+// (transposed), through a shared-memory tile of 64 k x NT columns (128 bytes
+// of a row of the narrow types, 32 elements of the others).
+template <class T>
+constexpr int split_cols_nt() {
+  return sizeof(T) < 4 ? 128 / (int)sizeof(T) : 32;
+}
+template <int L, class T>
+__global__ void __launch_bounds__(256)
+    split_cols_kernel(const T *__restrict__ B, size_t ldb, int kc, int N, uint32_t p,
+                      uint8_t *__restrict__ out, int Kp) {
+  using R = typename Rep<T>::Packed;
+  constexpr int NT = split_cols_nt<T>();
+  __shared__ R tile[64][NT + 4 / sizeof(R)];
+  const int n0 = blockIdx.x * NT, k0 = blockIdx.y * 64;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const size_t plane = (size_t)N * Kp;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    int k = k0 + ty + 8 * i, n = n0 + tx;
-    tile[ty + 8 * i][tx] = (k < kc && n < N) ? __ldg(B + (size_t)k * ldb + n) : 0u;
+    const int k = k0 + ty + 8 * i;
+#pragma unroll
+    for (int u = 0; u < NT / 32; ++u) {
+      const int n = n0 + tx + 32 * u;
+      tile[ty + 8 * i][tx + 32 * u] =
+          (k < kc && n < N) ? (R)Rep<T>::in(__ldg(B + (size_t)k * ldb + n), p) : (R)0;
+    }
   }
   __syncthreads();
 #pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    int w = threadIdx.x + 256 * j;
-    int n = w >> 4, kw = (w & 15) * 4;
-    int gn = n0 + n, gk = k0 + kw;
+  for (int j = 0; j < NT / 16; ++j) {
+    const int w = threadIdx.x + 256 * j;
+    const int n = w >> 4, kw = (w & 15) * 4;
+    const int gn = n0 + n, gk = k0 + kw;
     if (gn < N && gk < Kp) {
+      uint32_t v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[i] = tile[kw + i][n];
 #pragma unroll
       for (int l = 0; l < L; ++l) {
         uint32_t word = 0;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) word |= ((tile[kw + i][n] >> (8 * l)) & 0xFFu) << (8 * i);
+        for (int i = 0; i < 4; ++i) word |= ((v[i] >> (8 * l)) & 0xFFu) << (8 * i);
         *reinterpret_cast<uint32_t *>(out + l * plane + (size_t)gn * Kp + gk) = word;
       }
     }
   }
+}
+template <class T>
+static dim3 split_cols_grid(int N, int Kp) {
+  return dim3((N + split_cols_nt<T>() - 1) / split_cols_nt<T>(), (Kp + 63) / 64);
 }
 
 // ------------------------------------------------------------ plain gemm
@@ -888,9 +1107,9 @@ static int tc_attr(Ctx *c) {
                        "cudaFuncSetAttribute(zp_gemm_tc)");
 }
 
-template <int L, int T>
+template <int L, int T, class E = uint32_t>
 static int launch_tc(Ctx *c, int M, int N, int K, const Modulus &mod, uint32_t alpha,
-                     const uint32_t *A, size_t lda, const uint32_t *B, size_t ldb, uint32_t beta,
+                     const E *A, size_t lda, const E *B, size_t ldb, uint32_t beta,
                      uint32_t *C, size_t ldc, uint8_t *ws, const int2 *kr, int kbase) {
   using Cfg = TcCfg<L, T>;
   using Lay = TcLayout<L, T>;
@@ -903,12 +1122,12 @@ static int launch_tc(Ctx *c, int M, int N, int K, const Modulus &mod, uint32_t a
     uint8_t *Al = ws;
     uint8_t *Bl = ws + (size_t)L * M * Kp;
     {
-      const size_t total = (size_t)M * ((kc + 3) / 4);
-      int grid = (int)std::min<size_t>((total + 255) / 256, (size_t)c->num_sms * 16);
+      const uint32_t p = (uint32_t)mod.p;
       int pi = prof_begin(c, "zp_split");
-      split_rows_kernel<L><<<grid, 256, 0, c->stream>>>(A + k0, lda, M, kc, Al, Kp);
-      dim3 grid2((N + 31) / 32, (Kp + 63) / 64);
-      split_cols_kernel<L><<<grid2, 256, 0, c->stream>>>(B + (size_t)k0 * ldb, ldb, kc, N, Bl, Kp);
+      split_rows_kernel<L, E><<<split_rows_grid(c->num_sms, M, kc), dim3(32, SPLIT_ROWS), 0,
+                                c->stream>>>(A + k0, lda, M, kc, p, Al, Kp);
+      split_cols_kernel<L, E><<<split_cols_grid<E>(N, Kp), 256, 0, c->stream>>>(
+          B + (size_t)k0 * ldb, ldb, kc, N, p, Bl, Kp);
       prof_end(c, pi);
       ctx_launched(c, 2);
     }
@@ -932,6 +1151,25 @@ static int launch_tc(Ctx *c, int M, int N, int K, const Modulus &mod, uint32_t a
   return ST_OK;
 }
 
+template <int L>
+static int launch_direct(Ctx *c, int M, int N, int K, const Modulus &mod, uint32_t alpha,
+                         const uint32_t *A, size_t lda, const uint32_t *B, size_t ldb,
+                         uint32_t beta, uint32_t *C, size_t ldc) {
+  using Cfg = DirCfg<L>;
+  if (int st = ctx_smem_attr(c, (const void *)zp_gemm_direct_kernel<L>, Cfg::smem(2),
+                             "cudaFuncSetAttribute(zp_gemm_direct)"))
+    return st;
+  const int stages = K > BK ? 2 : 1;
+  const dim3 grid((N + Cfg::BN - 1) / Cfg::BN, (M + BM - 1) / BM);
+  int pi = prof_begin(c, "zp_gemm_direct");
+  zp_gemm_direct_kernel<L><<<grid, DIR_THREADS, Cfg::smem(stages), c->stream>>>(
+      A, lda, B, ldb, C, ldc, M, N, K, stages, mod, alpha, beta, c->dstatus);
+  prof_end(c, pi);
+  ctx_launched(c);
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? ST_OK : ctx_cuda(c, e, "zp_gemm_direct launch");
+}
+
 size_t zp_gemm_workspace_bytes(uint32_t p, int M, int N, int K) {
   const int L = zp_limbs_for(p);
   const int kc = std::min(ZP_KCHUNK, K);
@@ -939,35 +1177,63 @@ size_t zp_gemm_workspace_bytes(uint32_t p, int M, int N, int K) {
   return (size_t)L * ((size_t)M + N) * Kp + 256;
 }
 
-int zp_gemm_tile_pick(const Ctx *c, int K, uint32_t p) {
+int zp_gemm_tile_pick(const Ctx *c, int M, int N, int K, uint32_t p) {
   const int L = zp_limbs_for(p);
   if (L == 4) return 0;  // one variant for four limbs
-  // Measured on the B200 (kernel ms, M = N = 8192, p = 65521 / 251, the
-  // 32-bit reductions of the epilogue): two limbs, wide tiles with 8 / 16
-  // epilogue warps: 1.346 / 1.338 at K = 8192 (with the earlier 64-bit
-  // reduction 8 / 16 warps took 0.351 / 0.318 at K = 512 and 0.543 / 0.496
-  // at 2048).  One limb, double-buffered tiles with 8 / 16 warps: 0.256 /
-  // 0.256 at K = 2048, 0.284 / 0.322 at 3072, 0.596 / 0.642 at 8192 (0.316
-  // / 0.249 at 512 with the earlier reduction).
-  const bool wide = c->gemm_tile == GEMM_TILE_WIDE ||
-                    (c->gemm_tile == GEMM_TILE_AUTO && L == 2 && K >= 512);
+  bool wide = c->gemm_tile == GEMM_TILE_WIDE;
+  if (c->gemm_tile == GEMM_TILE_AUTO) {
+    // Measured on the B200 (kernel us, wide / double-buffered).  Two limbs, wide
+    // tiles of 128 columns: faster at long K (8192^3 1332 / 1922, 2000^3 54 /
+    // 64, 512 x 4096 x 4096 40 / 48), at K = 256 slower (4096^2 49 / 41); with
+    // at most half as many tiles as SMs the narrower tiles use twice the SMs
+    // (1024^3 19 / 15, 512^3 16 / 13).  One limb, wide tiles of 256 columns: a
+    // 128-column tile reads as many bytes of shared memory per cycle as there
+    // are (8192^2 x 8192 407 / 582, x 2048 168 / 273; 3072 x 2816 x 4096 43 /
+    // 57, 2000^3 25 / 27), but they need tiles for most SMs (512 x 4096 x
+    // 4096 25 / 21) and K enough to hide their epilogue (4096^2 x 256 37 / 32).
+    const long long tm = (M + BM - 1) / BM;
+    if (L == 2)
+      wide = K >= 512 && 2 * tm * ((N + 127) / 128) > c->num_sms;
+    else
+      wide = K >= 1024 && 5 * tm * ((N + 255) / 256) >= 4 * (long long)c->num_sms;
+  }
   if (L == 2) return wide ? 0 : 1;
   return wide ? 0 : (K <= 2048 ? 1 : 2);
 }
 
 int zp_gemm_pick(const Ctx *c, int M, int N, int K, uint32_t p) {
   if (c->gemm_kernel != GEMM_AUTO) return c->gemm_kernel;
-  // small K: the CUDA-core kernel below its measured crossover with the
-  // tensor-core path, which has a fixed cost of about 20 us (limb split and
-  // launch) and then runs far faster.  Measured on the B200 (us per call,
-  // small-K / tensor cores, p = 65521): 8000 x 448 x 64: 57.8 / 31.3;
-  // 8000 x 64 x 64: 14.9 / 20.6; 4000 x 200 x 40: 23.9 / 20.4; p = 2^31 - 1,
-  // 8000 x 448 x 64: 104.8 / 76.4 -- a crossover near 3e7 multiply-adds,
-  // higher for narrow C (the tensor cores' tiles are 64 or more columns wide)
-  const double work = (double)M * N * K;
-  const bool smallk = K <= 256 && (work <= 2.5e7 || (N <= 96 && work <= 6.0e7));
-  (void)p;
-  return smallk ? GEMM_SMALLK : GEMM_TC;
+  // The one-launch tile kernel for short K while its tiles are few: it saves
+  // the two split launches (about 7 us), but every tile splits its own operands
+  // and the CTAs do not overlap a tile's epilogue with the next tile's product.
+  // Measured on the B200 (us per call, one-launch / split and tensor cores, p =
+  // 65521): 64 x 960 x 64 9.6 / 16.2, 1000 x 448 x 64 11.5 / 18.1, 2000 x 2000 x
+  // 64 (512 tiles) 24.6 / 28.9, 8000 x 960 x 64 (945) 41 / 39, 1024^2 x 256 (128)
+  // 14.4 / 16.6, 512 x 4096 x 512 (256) 29.5 / 24.5, 512^3 (32) 20.5 / 17.6; four
+  // limbs: 64 x 9000 x 64 (282) 20.5 / 24.6, 4000 x 448 x 64 (448) 37 / 35.  The CUDA-core
+  // kernel for small K is slower at all of them (14.4 us and more).
+  const int L = zp_limbs_for(p), bn = L == 4 ? DirCfg<4>::BN : DirCfg<1>::BN;
+  const long long tiles = (long long)((M + BM - 1) / BM) * ((N + bn - 1) / bn);
+  const long long most = K <= 128 ? (L == 4 ? 2 : 4) * c->num_sms : K <= 256 ? c->num_sms : 0;
+  return tiles <= most ? GEMM_DIRECT : GEMM_TC;
+}
+
+// The tensor-core gemm for operands of type E (limb count and tile variant
+// by modulus and shape).
+template <class E>
+static int tc_dispatch(Ctx *c, int M, int N, int K, uint32_t p, uint32_t alpha, const E *A,
+                       size_t lda, const E *B, size_t ldb, uint32_t beta, uint32_t *C, size_t ldc,
+                       uint8_t *ws, const int2 *kr, int kbase) {
+  const Modulus mod = make_modulus(p);
+  const int tv = zp_gemm_tile_pick(c, M, N, K, p);
+#define LELA_TC(L, T) \
+  launch_tc<L, T, E>(c, M, N, K, mod, alpha, A, lda, B, ldb, beta, C, ldc, ws, kr, kbase)
+  switch (zp_limbs_for(p)) {
+    case 1: return tv == 0 ? LELA_TC(1, 0) : tv == 1 ? LELA_TC(1, 1) : LELA_TC(1, 2);
+    case 2: return tv == 0 ? LELA_TC(2, 0) : LELA_TC(2, 1);
+    default: return LELA_TC(4, 0);
+  }
+#undef LELA_TC
 }
 
 int zp_gemm_dev(Ctx *c, int kernel, int M, int N, int K, uint32_t p, uint32_t alpha,
@@ -1005,6 +1271,13 @@ int zp_gemm_dev(Ctx *c, int kernel, int M, int N, int K, uint32_t p, uint32_t al
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? ST_OK : ctx_cuda(c, e, "zp_gemm_smallk launch");
   }
+  if (kernel == GEMM_DIRECT) {
+    switch (zp_limbs_for(p)) {
+      case 1: return launch_direct<1>(c, M, N, K, mod, alpha, A, lda, B, ldb, beta, C, ldc);
+      case 2: return launch_direct<2>(c, M, N, K, mod, alpha, A, lda, B, ldb, beta, C, ldc);
+      default: return launch_direct<4>(c, M, N, K, mod, alpha, A, lda, B, ldb, beta, C, ldc);
+    }
+  }
   if (kernel == GEMM_PLAIN) {
     dim3 grid((N + PT - 1) / PT, (M + PT - 1) / PT);
     int pi = prof_begin(c, "zp_gemm_plain");
@@ -1022,17 +1295,27 @@ int zp_gemm_dev(Ctx *c, int kernel, int M, int N, int K, uint32_t p, uint32_t al
     if (st) return st;
     ws = static_cast<uint8_t *>(w);
   }
-  const int tv = zp_gemm_tile_pick(c, K, p);
-#define LELA_TC(L, T) launch_tc<L, T>(c, M, N, K, mod, alpha, A, lda, B, ldb, beta, C, ldc, ws, kr, kbase)
-  switch (zp_limbs_for(p)) {
-    case 1:
-      return tv == 0 ? LELA_TC(1, 0) : tv == 1 ? LELA_TC(1, 1) : LELA_TC(1, 2);
-    case 2:
-      return tv == 0 ? LELA_TC(2, 0) : LELA_TC(2, 1);
-#undef LELA_TC
-    default:
-      return launch_tc<4, 0>(c, M, N, K, mod, alpha, A, lda, B, ldb, beta, C, ldc, ws, kr, kbase);
+  return tc_dispatch<uint32_t>(c, M, N, K, p, alpha, A, lda, B, ldb, beta, C, ldc, ws, kr, kbase);
+}
+
+int zp_gemm_tc_elem_dev(Ctx *c, int elem, int M, int N, int K, uint32_t p, uint32_t alpha,
+                        const void *A, size_t lda, const void *B, size_t ldb, uint32_t *V,
+                        size_t ldv) {
+  void *w = nullptr;
+  if (int st = ctx_workspace(c, zp_gemm_workspace_bytes(p, M, N, K), &w)) return st;
+  uint8_t *ws = static_cast<uint8_t *>(w);
+  alpha %= p;
+#define LELA_ELEM(E)                                                                           \
+  tc_dispatch<E>(c, M, N, K, p, alpha, static_cast<const E *>(A), lda, static_cast<const E *>(B), \
+                 ldb, 0u, V, ldv, ws, nullptr, 0)
+  switch (elem) {
+    case LELA_CUDA_ELEM_U8: return LELA_ELEM(uint8_t);
+    case LELA_CUDA_ELEM_U16: return LELA_ELEM(uint16_t);
+    case LELA_CUDA_ELEM_F32: return LELA_ELEM(float);
+    case LELA_CUDA_ELEM_F64: return LELA_ELEM(double);
+    default: return ctx_fail(c, ST_ARG, "unknown element type");
   }
+#undef LELA_ELEM
 }
 
 // ============================================ pipelined host-pointer gemm
@@ -1095,8 +1378,8 @@ static int host_rows(Ctx *c, int M, int N, int K, const Modulus &mod, uint32_t a
   if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream, ev_b, 0);
   if (e == cudaSuccess) {
     int pi = prof_begin(c, "zp_split");
-    dim3 grid2((N + 31) / 32, (Kp + 63) / 64);
-    split_cols_kernel<L><<<grid2, 256, 0, c->stream>>>(dB, (size_t)N, K, N, Bl, Kp);
+    split_cols_kernel<L, uint32_t><<<split_cols_grid<uint32_t>(N, Kp), 256, 0, c->stream>>>(
+        dB, (size_t)N, K, N, (uint32_t)mod.p, Bl, Kp);
     prof_end(c, pi);
     ctx_launched(c);
     e = cudaGetLastError();
@@ -1109,11 +1392,10 @@ static int host_rows(Ctx *c, int M, int N, int K, const Modulus &mod, uint32_t a
     uint8_t *Al = ws + (size_t)L * r0 * Kp;
     e = cudaStreamWaitEvent(c->stream, ready[j], 0);
     if (e != cudaSuccess) break;
-    const size_t total = (size_t)rows * ((K + 3) / 4);
-    const int sgrid = (int)std::min<size_t>((total + 255) / 256, (size_t)c->num_sms * 16);
     int pi = prof_begin(c, "zp_split");
-    split_rows_kernel<L><<<sgrid, 256, 0, c->stream>>>(dA + (size_t)r0 * K, (size_t)K, rows, K,
-                                                       Al, Kp);
+    split_rows_kernel<L, uint32_t><<<split_rows_grid(c->num_sms, rows, K), dim3(32, SPLIT_ROWS), 0,
+                                     c->stream>>>(dA + (size_t)r0 * K, (size_t)K, rows, K,
+                                                  (uint32_t)mod.p, Al, Kp);
     prof_end(c, pi);
     CUtensorMap tmA;
     st = encode_3d(c, &tmA, Al, (uint64_t)K, (uint64_t)rows, L, (uint64_t)Kp,
@@ -1282,11 +1564,11 @@ int noalloc_launch(cudaStream_t s, const NoallocDevice &d, int M, int N, int K,
     const int Kp = (kc + 15) & ~15;
     uint8_t *Al = planes;
     uint8_t *Bl = planes + (size_t)L * M * Kp;
-    const size_t total = (size_t)M * ((kc + 3) / 4);
-    int grid = (int)std::min<size_t>((total + 255) / 256, (size_t)d.num_sms * 16);
-    split_rows_kernel<L><<<grid, 256, 0, s>>>(A + k0, lda, M, kc, Al, Kp);
-    dim3 grid2((N + 31) / 32, (Kp + 63) / 64);
-    split_cols_kernel<L><<<grid2, 256, 0, s>>>(B + (size_t)k0 * ldb, ldb, kc, N, Bl, Kp);
+    const uint32_t p = (uint32_t)mod.p;
+    split_rows_kernel<L, uint32_t><<<split_rows_grid(d.num_sms, M, kc), dim3(32, SPLIT_ROWS), 0, s>>>(
+        A + k0, lda, M, kc, p, Al, Kp);
+    split_cols_kernel<L, uint32_t><<<split_cols_grid<uint32_t>(N, Kp), 256, 0, s>>>(
+        B + (size_t)k0 * ldb, ldb, kc, N, p, Bl, Kp);
     CUtensorMap tmA, tmB;
     if (!noalloc_map(&tmA, Al, (uint64_t)kc, (uint64_t)M, L, (uint64_t)Kp, (uint64_t)M * Kp,
                      BK, BM, L) ||

@@ -16,7 +16,10 @@ int zp_limbs_for(uint32_t p);
 size_t zp_gemm_workspace_bytes(uint32_t p, int M, int N, int K);
 
 // C <- alpha*A*B + beta*C mod p on the handle's stream (asynchronous).
-// kernel: GEMM_AUTO, GEMM_PLAIN or GEMM_TC.  ws_override, when non-null,
+// kernel: a GemmKernel.  B may be C itself (same rows and columns, beta = 0)
+// for GEMM_TC with K <= ZP_KCHUNK, and for GEMM_DIRECT with M <= 128 and K <=
+// 256: every product that reads a tile's columns of B precedes its stores.
+// ws_override, when non-null,
 // is used instead of the handle workspace for the limb planes and must hold
 // zp_gemm_workspace_bytes(p, M, N, K) bytes.  kr (device, optional): per
 // row r of A, a column range [kr[r].x, kr[r].y) of the whole matrix outside
@@ -29,15 +32,21 @@ int zp_gemm_dev(Ctx *c, int kernel, int M, int N, int K, uint32_t p, uint32_t al
                 uint32_t *C, size_t ldc, uint8_t *ws_override, const int2 *kr = nullptr,
                 int kbase = 0);
 
+// V <- alpha*A*B mod p on the tensor cores, A and B of element type elem
+// (LELA_CUDA_ELEM_*, not uint32; p one of its moduli), V residues.  K > 0.
+int zp_gemm_tc_elem_dev(Ctx *c, int elem, int M, int N, int K, uint32_t p, uint32_t alpha,
+                        const void *A, size_t lda, const void *B, size_t ldb, uint32_t *V,
+                        size_t ldv);
+
 // The kernel GEMM_AUTO resolves to for this shape (the handle's forced
-// kernel, else the small-K crossover rule).
+// kernel, else the one-launch tile kernel for short K and few tiles, else the
+// limb-plane one).
 int zp_gemm_pick(const Ctx *c, int M, int N, int K, uint32_t p);
 // The tensor-core tile variant (TcCfg<L, T>'s T: 0, 1, or 2 for one limb)
-// for this K and modulus: the handle's forced shape (wide or
-// double-buffered), else wide for two limbs at K >= 512 and four limbs,
-// double-buffered otherwise; for one limb the number of epilogue warps
-// follows K.
-int zp_gemm_tile_pick(const Ctx *c, int K, uint32_t p);
+// for this shape and modulus: the handle's forced shape (wide or
+// double-buffered), else by limbs, K and the number of tiles; for one limb the
+// number of epilogue warps of the double-buffered tiles follows K.
+int zp_gemm_tile_pick(const Ctx *c, int M, int N, int K, uint32_t p);
 
 // Whether the host-pointer gemm of this shape is done in row blocks with
 // its copies overlapped (tensor-core path, one K chunk, at least two blocks
