@@ -191,61 +191,96 @@ struct ArithWide {
   __device__ __forceinline__ uint32_t red64(uint64_t s) const { return mod_reduce(s, mod); }
 };
 
-// Inverse of a 64 x 64 triangular matrix X (row stride LD, shared memory)
-// in place by doubling: the inverse of [[A, B], [0, C]] is [[A^-1, -A^-1 B
-// C^-1], [0, C^-1]] (lower: [[A^-1, 0], [-C^-1 B A^-1, C^-1]]), so the
+// Inverses of two 64 x 64 triangular matrices in shared memory (row stride
+// INV_LD), in place by doubling: the upper X by the first half of the CTA's
+// threads, the lower Y by the second.  The inverse of [[A, B], [0, C]] is
+// [[A^-1, -A^-1 B C^-1], [0, C^-1]] (lower: [[A^-1, 0], [-C^-1 B A^-1, C^-1]]),
+// so the
 // diagonal blocks of sizes 1, 2, 4, .., 32 are inverted level by level,
 // each level two products of b x b blocks (through T, 32 b entries) over
-// all pairs at once.  On entry the diagonal holds the inverses of the
-// diagonal entries and the rest of the triangle the matrix's entries, the
+// all pairs at once.  On entry the diagonals hold the inverses of the
+// diagonal entries and the rest of each triangle the matrix's entries, the
 // other triangle zero (the products run over whole blocks, zeros included).
 // Every thread of the CTA calls it (12 barriers).  A
 // triangular matrix with unit diagonal entries has one inverse over Z/p,
-// so the result is the one any substitution gives.
-template <class A, bool UPPER, int LD, int B>
-__device__ __forceinline__ void tri64_invert_level(uint32_t (*X)[LD], uint32_t *T, const A &ar,
-                                                   int tid, int nthreads) {
-  // products over whole b x b blocks (the zero triangle included): fixed
-  // trip counts, unrolled
-  constexpr int n = (EW / (2 * B)) * B * B;
+// so the result is the one any substitution gives.  A thread takes R rows of
+// a product's column and reads the left factor four entries at a time: with
+// one entry of the product per thread the two large levels were bound by
+// shared-memory reads, two per multiply-add (9300 cycles for one matrix).
+constexpr int INV_LD = EW + 4;                  // 16-byte rows
+constexpr int INV_M = EW * INV_LD;              // one matrix
+constexpr int INV_T = 32 * (EW / 2 + 4);        // its scratch (rows of b + 4)
+constexpr int INV_WORDS = 2 * (INV_M + INV_T);  // both
+template <class A, int B, int R>
+__device__ __forceinline__ void tri64_level(uint32_t *X, uint32_t *T, bool upper, const A &ar,
+                                            int tid) {
+  static_assert(PS_THREADS / 2 * R >= 32 * B, "one pass per product");
+  constexpr int TLD = B + (B >= 4 ? 4 : 0);  // keeps four-entry reads aligned
   const uint32_t p = ar.p;
-  for (int e = tid; e < n; e += nthreads) {
-    const int q = e / (B * B), ii = (e / B) % B, jj = e % B, r = 2 * B * q;
-    uint64_t acc = 0;
+  const int jj = tid % B, i0 = (tid / B) % (B / R) * R, q = tid / (B * B / R), r = 2 * B * q;
+  const bool in = q < EW / (2 * B);
+  uint32_t *Tq = T + q * B * TLD;
 #pragma unroll
-    for (int kk = 0; kk < B; ++kk) {
-      if constexpr (UPPER) ar.acc(acc, X[r + ii][r + B + kk], X[r + B + kk][r + B + jj]);  // B C^-1
-      else ar.acc(acc, X[r + B + ii][r + kk], X[r + kk][r + jj]);                          // B A^-1
-    }
-    T[e] = ar.red64(acc);
-  }
-  __syncthreads();
-  for (int e = tid; e < n; e += nthreads) {
-    const int q = e / (B * B), ii = (e / B) % B, jj = e % B, r = 2 * B * q;
-    const uint32_t *Tq = T + q * B * B;
-    uint64_t acc = 0;
+  for (int half = 0; half < 2; ++half) {
+    // T = B C^-1 (lower: B A^-1), then -A^-1 T (lower: -C^-1 T)
+    const uint32_t *left = half ? X + (upper ? r * INV_LD + r : (r + B) * INV_LD + r + B)
+                                : X + (upper ? r * INV_LD + r + B : (r + B) * INV_LD + r);
+    const uint32_t *right = half ? Tq : X + (upper ? (r + B) * INV_LD + r + B : r * INV_LD + r);
+    const int rld = half ? TLD : INV_LD;
+    uint32_t v[R];
+    if (in) {
+      uint64_t acc[R];
 #pragma unroll
-    for (int kk = 0; kk < B; ++kk) {
-      if constexpr (UPPER) ar.acc(acc, X[r + ii][r + kk], Tq[kk * B + jj]);  // -A^-1 (B C^-1)
-      else ar.acc(acc, X[r + B + ii][r + B + kk], Tq[kk * B + jj]);         // -C^-1 (B A^-1)
+      for (int u = 0; u < R; ++u) acc[u] = 0;
+      if constexpr (B >= 4) {
+#pragma unroll 4
+        for (int k = 0; k < B; k += 4) {
+          uint32_t b[4];
+#pragma unroll
+          for (int w = 0; w < 4; ++w) b[w] = right[(k + w) * rld + jj];
+#pragma unroll
+          for (int u = 0; u < R; ++u) {
+            const uint4 a = *reinterpret_cast<const uint4 *>(left + (i0 + u) * INV_LD + k);
+            ar.acc(acc[u], a.x, b[0]);
+            ar.acc(acc[u], a.y, b[1]);
+            ar.acc(acc[u], a.z, b[2]);
+            ar.acc(acc[u], a.w, b[3]);
+          }
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < B; ++k)
+#pragma unroll
+          for (int u = 0; u < R; ++u)
+            ar.acc(acc[u], left[(i0 + u) * INV_LD + k], right[k * rld + jj]);
+      }
+#pragma unroll
+      for (int u = 0; u < R; ++u) {
+        v[u] = ar.red64(acc[u]);
+        if (half) {
+          uint32_t *o = X + (upper ? (r + i0 + u) * INV_LD + r + B : (r + B + i0 + u) * INV_LD + r);
+          o[jj] = v[u] ? p - v[u] : 0u;
+        } else {
+          Tq[(i0 + u) * TLD + jj] = v[u];
+        }
+      }
     }
-    const uint32_t v = ar.red64(acc);
-    if constexpr (UPPER) X[r + ii][r + B + jj] = v ? p - v : 0u;
-    else X[r + B + ii][r + jj] = v ? p - v : 0u;
+    __syncthreads();
   }
-  __syncthreads();
 }
 
-template <class A, bool UPPER, int LD>
-__device__ void tri64_invert(uint32_t (*X)[LD], uint32_t *T, const A &ar, int tid,
-                             int nthreads) {
+template <class A>
+__device__ void tri64_invert2(uint32_t *X, uint32_t *Y, uint32_t *T, const A &ar, int tid) {
   static_assert(EW == 64, "six levels");
-  tri64_invert_level<A, UPPER, LD, 1>(X, T, ar, tid, nthreads);
-  tri64_invert_level<A, UPPER, LD, 2>(X, T, ar, tid, nthreads);
-  tri64_invert_level<A, UPPER, LD, 4>(X, T, ar, tid, nthreads);
-  tri64_invert_level<A, UPPER, LD, 8>(X, T, ar, tid, nthreads);
-  tri64_invert_level<A, UPPER, LD, 16>(X, T, ar, tid, nthreads);
-  tri64_invert_level<A, UPPER, LD, 32>(X, T, ar, tid, nthreads);
+  const bool upper = tid < PS_THREADS / 2;
+  uint32_t *M = upper ? X : Y, *Tm = upper ? T : T + INV_T;
+  const int t = tid & (PS_THREADS / 2 - 1);
+  tri64_level<A, 1, 1>(M, Tm, upper, ar, t);
+  tri64_level<A, 2, 1>(M, Tm, upper, ar, t);
+  tri64_level<A, 4, 1>(M, Tm, upper, ar, t);
+  tri64_level<A, 8, 1>(M, Tm, upper, ar, t);
+  tri64_level<A, 16, 2>(M, Tm, upper, ar, t);
+  tri64_level<A, 32, 4>(M, Tm, upper, ar, t);
 }
 
 // 1. First nonzero column of each row's panel part, rows i0..m-1 (one warp
@@ -501,15 +536,15 @@ static_assert(PW_R % PS_FAST == 0, "whole rows per warp");
 // window rows padded to EW + 1 words: a column read across rows touches
 // every bank once
 constexpr int PW_LD = EW + 1;
-// dynamic shared memory: the window rows, later the inverse and its scratch;
-// then the table of inverses (NORM)
-constexpr int PW_INV = EW * PW_LD + 32 * EW / 2;
-constexpr size_t PW_SMEM = (((size_t)(PW_R * PW_LD > PW_INV ? PW_R * PW_LD : PW_INV) * 4) + 15) / 16 * 16;
+// dynamic shared memory: the window rows, later the two inverses and their
+// scratch; the multipliers of the window's rows (by slot) and of pivots from
+// past it; then the table of inverses (NORM)
+constexpr int PW_AREA = PW_R * PW_LD > INV_WORDS ? PW_R * PW_LD : INV_WORDS;
+constexpr int PW_LROWS = PW_R + EW;
+constexpr size_t PW_SMEM = ((size_t)(PW_AREA + PW_LROWS * PW_LD) * 4 + 15) / 16 * 16;
 constexpr size_t PW_TABLE = 65536;
 // positions a thread looks at per pass of the window's compaction
 constexpr int PW_U = 4;
-// rows to solve from which the panel's multipliers come from U_P^-1
-constexpr int SOLVE_INV_ROWS = 768;
 
 template <class SA, class A>
 __global__ void __launch_bounds__(PS_THREADS, 1)
@@ -518,11 +553,12 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
                         int *__restrict__ hist, int *__restrict__ last_act, int *__restrict__ p2r,
                         int *__restrict__ stamp, int epoch, uint32_t *__restrict__ Uout,
                         uint32_t *__restrict__ xinv_out, uint32_t *__restrict__ Uinv_out,
-                        PanelOut *out, volatile uint64_t *hout, uint32_t seq, int wcap) {
+                        uint32_t *__restrict__ Linv_out, PanelOut *out, volatile uint64_t *hout, uint32_t seq, int wcap) {
   using V = typename SA::V;
   using V4 = typename SA::V4;
   extern __shared__ __align__(16) uint32_t dyn_w[];
   V(*Wv)[PW_LD] = reinterpret_cast<V(*)[PW_LD]>(dyn_w);  // PW_R rows
+  V(*Lm)[PW_LD] = reinterpret_cast<V(*)[PW_LD]>(dyn_w + PW_AREA);  // [slot][pivot] (division-free: raw)
   const uint16_t *s_inv = reinterpret_cast<const uint16_t *>(dyn_w + PW_SMEM / 4);
   __shared__ V PV[EW][EW];
   __shared__ V4 s_coef[PW_R];         // per slot: its coefficients of the block's pivot rows
@@ -531,10 +567,13 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
   __shared__ V s_psc[PB], s_sc;       // their scales, and the other rows'
   // slot of the pivot of the block's column j (-1: none)
   __shared__ __align__(16) int s_pslot[PB];
-  __shared__ V s_red[PS_FAST][EW];    // rows past the window, reduced (one per warp)
+  __shared__ V s_red[PS_FAST][EW];    // rows past the window, reduced (one per warp),
+  __shared__ V s_rl[PS_FAST][EW];     // and their multipliers (raw)
   __shared__ int s_ent[PW_R], s_epos[PW_R], wrow[PW_R];
   __shared__ int2 s_piv[EW];          // pivot column, transposition target
+  __shared__ int s_prow[EW];          // the pivot's row of Lm
   __shared__ V s_y[EW], s_sinv[EW];   // pivot values (in window rows' scale), 1 / S_k
+  __shared__ V s_yinv[EW];            // 1 / s_y (division-free, p < 2^31)
   __shared__ int s_xi[EW];            // pivots' inverses (NORM: in (-p, p))
   __shared__ uint32_t s_det;
   __shared__ int s_cnt[EW + 1];
@@ -715,7 +754,10 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
 #pragma unroll
           for (int g = 0; g < NG; ++g) {
             const V l = sa.plain(z[0][g], iv);  // 1 for the pivot row
-            if (live[g] != NONE) s_coefv[PB * ent[g] + j] = l;  // by slot
+            if (live[g] != NONE) {  // by slot
+              s_coefv[PB * ent[g] + j] = l;
+              Lm[ent[g]][t] = l;
+            }
 #pragma unroll
             for (int k = 1; k < PB; ++k)
               if (k < zn) z[k][g] = sa.step(z[k][g], l, pv[k]);
@@ -732,6 +774,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
 #pragma unroll
           for (int g = 0; g < NG; ++g) {
             const V na = sa.neg(z[0][g]);
+            if (live[g] != NONE) Lm[ent[g]][t] = z[0][g];
             znew[g] = sa.mul(na, sc);
 #pragma unroll
             for (int k = 1; k < PB; ++k) z[k][g] = sa.upd(pv[0], z[k][g], na, pv[k]);
@@ -740,6 +783,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
         if (lane == pl) {
           s_pslot[j] = sel(ent, pg);
           s_piv[t] = make_int2(col, q);
+          s_prow[t] = sel(ent, pg);
           s_y[t] = pv[0];
           if constexpr (SA::NORM) {
             s_xi[t] = iv;
@@ -955,10 +999,12 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
             const V u0 = lane >= pc ? PV[k][lane] : 0, u1 = lane + 32 >= pc ? PV[k][lane + 32] : 0;
             if constexpr (SA::NORM) {
               const V l = sa.plain(f, s_xi[k]);
+              if (lane == 0) s_rl[wid][k] = l;
               a0 = sa.step(a0, l, u0);
               a1 = sa.step(a1, l, u1);
             } else {
               const V nf = sa.neg(f);
+              if (lane == 0) s_rl[wid][k] = f;
               a0 = sa.upd(s_y[k], a0, nf, u0);
               a1 = sa.upd(s_y[k], a1, nf, u1);
             }
@@ -1031,6 +1077,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
         p2r[found] = ri;
         stamp[found] = epoch;
         s_piv[t] = make_int2(col, found);
+        s_prow[t] = PW_R + t;
         s_y[t] = y;
         if constexpr (SA::NORM) {
           s_xi[t] = sa.inverse(s_inv, y);
@@ -1039,9 +1086,12 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
       }
       PV[t][lane] = s_red[fw][lane];
       PV[t][lane + 32] = s_red[fw][lane + 32];
+      if (lane < t) Lm[PW_R + t][lane] = s_rl[fw][lane];
+      if (lane + 32 < t) Lm[PW_R + t][lane + 32] = s_rl[fw][lane + 32];
     }
     if (z) --nl;
     __syncthreads();
+    if (tid < nl) Lm[s_ent[tid]][t] = 0;  // the window rows' multipliers of this pivot
     if constexpr (!SA::NORM) {
       // the window rows are zero in the column: they are scaled by y
       for (int e = wid; e < nl; e += PS_FAST) {
@@ -1122,8 +1172,11 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
         }
         x0 = sa.plain(y0, si0);
         x1 = sa.plain(y1, si1);
-        xi0 = sa.canon(sa.plain(S0, sa.mul(S0, n0)));
-        xi1 = sa.canon(sa.plain(S1, sa.mul(S1, n1)));
+        const V yi0 = sa.mul(S0, n0), yi1 = sa.mul(S1, n1);
+        s_yinv[lane] = yi0;
+        s_yinv[lane + 32] = yi1;
+        xi0 = sa.canon(sa.plain(S0, yi0));
+        xi1 = sa.canon(sa.plain(S1, yi1));
       } else {
         si0 = sa.load(inv_exact_u32(p, sa.canon(S0)));
         si1 = sa.load(inv_exact_u32(p, sa.canon(S1)));
@@ -1181,9 +1234,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
     const int la = *last_act;
     int last = s_last;
     if (la > s_hi) last = max(last, la);
-    // the rows the panel's solve takes: i0 .. max(last, i0 + t - 1)
-    const int rows = max(last, i0 + t - 1) - i0 + 1;
-    const uint32_t uinv = exact_inv && t > 0 && rows >= SOLVE_INV_ROWS;
+    const uint32_t uinv = exact_inv && t > 0;
     last = max(last, 0);
     hout[PANEL_W_T] = word((uint32_t)t | uinv << 8 | (uint32_t)s_err << 9);
     hout[PANEL_W_LAST] = word((uint32_t)last);
@@ -1207,28 +1258,34 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
     Uout[e] = c < s_piv[k].x ? 0u : u_at(k, c);
   }
   __syncthreads();
-  // After the result is on its way to the host: for p < 2^31 (exact
-  // pivot inverses), when at least SOLVE_INV_ROWS rows are to be solved (it
-  // costs a few microseconds), the inverse of U_P, the t x t upper triangular matrix of
+  // After the result is on its way to the host, for p < 2^31 (exact
+  // pivot inverses): the inverses of U_P, the t x t upper triangular matrix of
   // the pivot rows at the pivot columns (U_P[k][j] = U_k[pcol_j], diagonal
-  // x_k), padded to 64 x 64 with the identity.  A row's multipliers are then
-  // a_P U_P^-1 (a_P: its values at the pivot columns), all at once.  In the
+  // x_k), and of L11, the unit lower triangle of the pivot rows' multipliers,
+  // padded to 64 x 64 with the identity.  A row's multipliers are then
+  // a_P U_P^-1 (a_P: its values at the pivot columns), all at once, and the pivot
+  // rows' other columns U12 = L11^-1 A12.  In the
   // window's shared memory, now free.
   if (s_uinv) {
-    uint32_t(*X)[PW_LD] = reinterpret_cast<uint32_t(*)[PW_LD]>(dyn_w);
-    uint32_t *T = dyn_w + EW * PW_LD;
+    uint32_t *X = dyn_w, *Y = X + INV_M, *T = Y + INV_M;
     for (int e = tid; e < EW * EW; e += PS_THREADS) {
       const int k = e / EW, j = e % EW;
-      uint32_t v;
-      if (k >= t || j >= t) v = k == j ? 1u : 0u;
-      else if (j < k) v = 0u;
-      else if (j == k) v = SA::NORM ? sa.canon(s_xi[k]) : (uint32_t)s_xi[k];
-      else v = u_at(k, s_piv[j].x);
-      X[k][j] = v;
+      uint32_t u = k == j ? 1u : 0u, l = u;
+      if (k < t && j < t) {
+        if (j == k) u = SA::NORM ? sa.canon(s_xi[k]) : (uint32_t)s_xi[k];
+        else if (j > k) u = u_at(k, s_piv[j].x);
+        else if constexpr (SA::NORM) l = sa.canon(Lm[s_prow[k]][j]);
+        else l = sa.canon(sa.plain(Lm[s_prow[k]][j], s_yinv[j]));
+      }
+      X[k * INV_LD + j] = u;
+      Y[k * INV_LD + j] = l;
     }
     __syncthreads();
-    tri64_invert<A, true, PW_LD>(X, T, ar, tid, PS_THREADS);
-    for (int e = tid; e < t * EW; e += PS_THREADS) Uinv_out[e] = X[e / EW][e % EW];
+    tri64_invert2<A>(X, Y, T, ar, tid);
+    for (int e = tid; e < t * EW; e += PS_THREADS) {
+      Uinv_out[e] = X[e / EW * INV_LD + e % EW];
+      Linv_out[e] = Y[e / EW * INV_LD + e % EW];
+    }
   }
 }
 
@@ -1464,7 +1521,7 @@ int zp_echelon_dev(Ctx *c, int m, int n, uint32_t p, uint32_t *D, size_t ld, siz
   const size_t l_bytes = (size_t)m * EB * 4;
   void *base = nullptr;
   int st = ctx_buffer(c, BUF_ECH_0,
-                      out_bytes + i_bytes + h_bytes + 3 * sq_bytes + l_bytes + 1024,
+                      out_bytes + i_bytes + h_bytes + 4 * sq_bytes + l_bytes + 1024,
                       &base);
   if (st) return st;
   uint8_t *b8 = static_cast<uint8_t *>(base);
@@ -1479,7 +1536,8 @@ int zp_echelon_dev(Ctx *c, int m, int n, uint32_t p, uint32_t *D, size_t ld, siz
   uint32_t *d_U = reinterpret_cast<uint32_t *>(b8 + out_bytes + i_bytes + h_bytes);
   uint32_t *d_xinv = d_U + EW * EW;  // pivot inverses (EW)
   uint32_t *d_Uinv = d_xinv + EW * EW;  // U_P^-1 (t x EW), p < 2^31
-  uint32_t *d_L = d_Uinv + EW * EW;  // the block's multipliers (m x EB)
+  uint32_t *d_Linv = d_Uinv + EW * EW;  // L11^-1 (t x EW), p < 2^31
+  uint32_t *d_L = d_Linv + EW * EW;  // the block's multipliers (m x EB)
   const uint32_t *d_pcol = reinterpret_cast<const uint32_t *>(b8 + offsetof(PanelOut, pcol));
   void *gws = nullptr;
   // one size for the panel and block updates and the block's trsm (which
@@ -1559,7 +1617,7 @@ int zp_echelon_dev(Ctx *c, int m, int n, uint32_t p, uint32_t *D, size_t ld, siz
     if (s) return s;
     kern<<<1, PS_THREADS, smem, c->stream>>>(D, ld, i, m, c0, w, sa, ar, d_head, d_act, d_hist,
                                                 d_last, d_p2r, d_stamp, epoch, d_U, d_xinv, d_Uinv,
-                                                d_out, hwords_dev, seq, wcap);
+                                                d_Linv, d_out, hwords_dev, seq, wcap);
     return ST_OK;
   };
   // window rows of the search: the full PW_R, or 64 when the previous panel
@@ -1670,17 +1728,14 @@ int zp_echelon_dev(Ctx *c, int m, int n, uint32_t p, uint32_t *D, size_t ld, siz
       const int groups = (r1 - i + 1 + SOLVE_THREADS / 32 - 1) / (SOLVE_THREADS / 32);
       pi = prof_begin(c, "ech_solve");
       const int sgrid = std::max(1, std::min(groups, c->num_sms * 8));
-      // U_P^-1 when the search wrote it (p < 2^31: exact pivot inverses, and
-      // many rows), else the elimination steps
+      // U_P^-1 when the search wrote it (p < 2^31: exact pivot inverses), else
+      // the elimination steps
       if (h.uinv && small)
         panel_solve_inv_kernel<<<sgrid, SOLVE_THREADS, 0, c->stream>>>(
             D, ld, i, r1, c0, w, t, d_pcol, d_U, d_Uinv, ars, Lp, EB);
       else if (h.uinv)
         panel_solve_inv_kernel<<<sgrid, SOLVE_THREADS, 0, c->stream>>>(
             D, ld, i, r1, c0, w, t, d_pcol, d_U, d_Uinv, arw, Lp, EB);
-      else if (small)
-        panel_solve_kernel<<<sgrid, SOLVE_THREADS, 0, c->stream>>>(D, ld, i, r1, c0, w, t, d_pcol,
-                                                                   d_U, d_xinv, ars, Lp, EB);
       else
         panel_solve_kernel<<<sgrid, SOLVE_THREADS, 0, c->stream>>>(D, ld, i, r1, c0, w, t, d_pcol,
                                                                    d_U, d_xinv, arw, Lp, EB);
@@ -1700,13 +1755,17 @@ int zp_echelon_dev(Ctx *c, int m, int n, uint32_t p, uint32_t *D, size_t ld, siz
     if (rest > 0) {
       uint32_t *U12 = D + (size_t)i * ld + c0 + w;
       pi = prof_begin(c, "ech_u12");
-      const int ugrid = (rest + U12_COLS - 1) / U12_COLS;
-      if (small)
-        panel_u12_kernel<<<ugrid, U12_THREADS, 0, c->stream>>>(Lp, EB, t, U12, ld, rest, ars);
-      else
+      if (h.uinv) {
+        // U12 = L11^-1 A12 in place: one tile of rows, each CTA on its columns
+        if ((st = zp_gemm_dev(c, GEMM_DIRECT, t, rest, t, p, 1, d_Linv, EW, U12, ld, 0, U12, ld,
+                              static_cast<uint8_t *>(gws))))
+          return st;
+      } else {
+        const int ugrid = (rest + U12_COLS - 1) / U12_COLS;
         panel_u12_kernel<<<ugrid, U12_THREADS, 0, c->stream>>>(Lp, EB, t, U12, ld, rest, arw);
+        ctx_launched(c);
+      }
       prof_end(c, pi);
-      ctx_launched(c);
       if (below > 0) {
         pi = prof_begin(c, "ech_update");
         st = zp_gemm_dev(c, GEMM_AUTO, below, rest, t, p, p - 1, Lp + (size_t)t * EB, EB, U12,
