@@ -58,6 +58,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "arith.cuh"
 #include "common.cuh"
 #include "context.h"
 #include "echelon.h"
@@ -97,190 +98,10 @@ enum : int {
 };
 static_assert(PANEL_WORDS_OFF + PANEL_WORDS * 8 <= PANEL_FLAG_OFF, "words below the flag");
 
-// Exact inverse of a unit x modulo p (any p < 2^32): extended Euclid on
-// unsigned remainders with 64-bit signed coefficients.  0 when gcd != 1.
-__device__ __forceinline__ uint32_t inv_exact_u32(uint32_t p, uint32_t x) {
-  uint32_t r0 = p, r1 = x;
-  int64_t s0 = 0, s1 = 1;
-  while (r1 != 0) {
-    const uint32_t q = r0 / r1;
-    const uint32_t r = r0 - q * r1;
-    r0 = r1;
-    r1 = r;
-    const int64_t s = s0 - (int64_t)q * s1;
-    s0 = s1;
-    s1 = s;
-  }
-  if (r0 != 1) return 0;
-  int64_t v = s0 % (int64_t)p;
-  if (v < 0) v += p;
-  return (uint32_t)v;
-}
-
 // Row index currently at position pos: positions touched by this panel's
 // transpositions carry the panel's epoch stamp.
 __device__ __forceinline__ int row_at(int pos, const int *p2r, const int *stamp, int epoch) {
   return stamp[pos] == epoch ? p2r[pos] : pos;
-}
-
-// sum of two products a*b + c*d modulo p (a, b, c, d < p < 2^32)
-__device__ __forceinline__ uint32_t mod_dot2(uint32_t a, uint32_t b, uint32_t c, uint32_t d,
-                                             const Modulus &mod, uint32_t two64) {
-  const uint64_t x = (uint64_t)a * b, y = (uint64_t)c * d;
-  uint64_t s = x + y;
-  if (s < y) s += two64;
-  return mod_reduce(s, mod);
-}
-
-// Field arithmetic for the panel kernels, in two forms chosen by the host:
-// ArithSmall for p < 2^16 (every product fits in 32 bits; Barrett reduction
-// with a 32-bit reciprocal, one correction) and ArithWide for any p < 2^32
-// (64-bit products and Barrett reduction).  Both return canonical residues.
-struct ArithSmall {
-  uint32_t p, mu;  // mu = floor(2^32 / p)
-  __host__ static ArithSmall make(uint32_t p) {
-    ArithSmall a;
-    a.p = p;
-    a.mu = (uint32_t)((1ull << 32) / p);
-    return a;
-  }
-  __device__ __forceinline__ uint32_t red(uint32_t x) const {
-    const uint32_t r = x - __umulhi(x, mu) * p;
-    return r >= p ? r - p : r;
-  }
-  __device__ __forceinline__ uint32_t mul(uint32_t a, uint32_t b) const { return red(a * b); }
-  // a*b + c*d
-  __device__ __forceinline__ uint32_t dot2(uint32_t a, uint32_t b, uint32_t c, uint32_t d) const {
-    const uint32_t r = red(a * b) + red(c * d);
-    return r >= p ? r - p : r;
-  }
-  // s += a*b for a sum of products reduced once at the end (red64): each
-  // product is below 2^32, so up to 2^16 of them fit
-  __device__ __forceinline__ void acc(uint64_t &s, uint32_t a, uint32_t b) const {
-    s += (uint64_t)a * b;
-  }
-  // s mod p for s < 2^48: (s mod 2^32 reduced) + (s / 2^32) (2^32 mod p)
-  __device__ __forceinline__ uint32_t red64(uint64_t s) const {
-    const uint32_t c32 = 0u - mu * p;
-    return red(red((uint32_t)s) + (uint32_t)(s >> 32) * c32);
-  }
-};
-struct ArithWide {
-  Modulus mod;
-  uint32_t p, two64;
-  __host__ static ArithWide make(uint32_t p) {
-    ArithWide a;
-    a.mod = make_modulus(p);
-    a.p = p;
-    a.two64 = two64_mod(p);
-    return a;
-  }
-  __device__ __forceinline__ uint32_t mul(uint32_t a, uint32_t b) const {
-    return mod_mul(a, b, mod);
-  }
-  __device__ __forceinline__ uint32_t dot2(uint32_t a, uint32_t b, uint32_t c, uint32_t d) const {
-    return mod_dot2(a, b, c, d, mod, two64);
-  }
-  // s += a*b modulo p: on a wrap past 2^64 the lost 2^64 comes back as
-  // 2^64 mod p (the sum then stays below 2^64: it is below the product)
-  __device__ __forceinline__ void acc(uint64_t &s, uint32_t a, uint32_t b) const {
-    const uint64_t x = (uint64_t)a * b;
-    s += x;
-    if (s < x) s += two64;
-  }
-  __device__ __forceinline__ uint32_t red64(uint64_t s) const { return mod_reduce(s, mod); }
-};
-
-// Inverses of two 64 x 64 triangular matrices in shared memory (row stride
-// INV_LD), in place by doubling: the upper X by the first half of the CTA's
-// threads, the lower Y by the second.  The inverse of [[A, B], [0, C]] is
-// [[A^-1, -A^-1 B C^-1], [0, C^-1]] (lower: [[A^-1, 0], [-C^-1 B A^-1, C^-1]]),
-// so the
-// diagonal blocks of sizes 1, 2, 4, .., 32 are inverted level by level,
-// each level two products of b x b blocks (through T, 32 b entries) over
-// all pairs at once.  On entry the diagonals hold the inverses of the
-// diagonal entries and the rest of each triangle the matrix's entries, the
-// other triangle zero (the products run over whole blocks, zeros included).
-// Every thread of the CTA calls it (12 barriers).  A
-// triangular matrix with unit diagonal entries has one inverse over Z/p,
-// so the result is the one any substitution gives.  A thread takes R rows of
-// a product's column and reads the left factor four entries at a time: with
-// one entry of the product per thread the two large levels were bound by
-// shared-memory reads, two per multiply-add (9300 cycles for one matrix).
-constexpr int INV_LD = EW + 4;                  // 16-byte rows
-constexpr int INV_M = EW * INV_LD;              // one matrix
-constexpr int INV_T = 32 * (EW / 2 + 4);        // its scratch (rows of b + 4)
-constexpr int INV_WORDS = 2 * (INV_M + INV_T);  // both
-template <class A, int B, int R>
-__device__ __forceinline__ void tri64_level(uint32_t *X, uint32_t *T, bool upper, const A &ar,
-                                            int tid) {
-  static_assert(PS_THREADS / 2 * R >= 32 * B, "one pass per product");
-  constexpr int TLD = B + (B >= 4 ? 4 : 0);  // keeps four-entry reads aligned
-  const uint32_t p = ar.p;
-  const int jj = tid % B, i0 = (tid / B) % (B / R) * R, q = tid / (B * B / R), r = 2 * B * q;
-  const bool in = q < EW / (2 * B);
-  uint32_t *Tq = T + q * B * TLD;
-#pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    // T = B C^-1 (lower: B A^-1), then -A^-1 T (lower: -C^-1 T)
-    const uint32_t *left = half ? X + (upper ? r * INV_LD + r : (r + B) * INV_LD + r + B)
-                                : X + (upper ? r * INV_LD + r + B : (r + B) * INV_LD + r);
-    const uint32_t *right = half ? Tq : X + (upper ? (r + B) * INV_LD + r + B : r * INV_LD + r);
-    const int rld = half ? TLD : INV_LD;
-    uint32_t v[R];
-    if (in) {
-      uint64_t acc[R];
-#pragma unroll
-      for (int u = 0; u < R; ++u) acc[u] = 0;
-      if constexpr (B >= 4) {
-#pragma unroll 4
-        for (int k = 0; k < B; k += 4) {
-          uint32_t b[4];
-#pragma unroll
-          for (int w = 0; w < 4; ++w) b[w] = right[(k + w) * rld + jj];
-#pragma unroll
-          for (int u = 0; u < R; ++u) {
-            const uint4 a = *reinterpret_cast<const uint4 *>(left + (i0 + u) * INV_LD + k);
-            ar.acc(acc[u], a.x, b[0]);
-            ar.acc(acc[u], a.y, b[1]);
-            ar.acc(acc[u], a.z, b[2]);
-            ar.acc(acc[u], a.w, b[3]);
-          }
-        }
-      } else {
-#pragma unroll
-        for (int k = 0; k < B; ++k)
-#pragma unroll
-          for (int u = 0; u < R; ++u)
-            ar.acc(acc[u], left[(i0 + u) * INV_LD + k], right[k * rld + jj]);
-      }
-#pragma unroll
-      for (int u = 0; u < R; ++u) {
-        v[u] = ar.red64(acc[u]);
-        if (half) {
-          uint32_t *o = X + (upper ? (r + i0 + u) * INV_LD + r + B : (r + B + i0 + u) * INV_LD + r);
-          o[jj] = v[u] ? p - v[u] : 0u;
-        } else {
-          Tq[(i0 + u) * TLD + jj] = v[u];
-        }
-      }
-    }
-    __syncthreads();
-  }
-}
-
-template <class A>
-__device__ void tri64_invert2(uint32_t *X, uint32_t *Y, uint32_t *T, const A &ar, int tid) {
-  static_assert(EW == 64, "six levels");
-  const bool upper = tid < PS_THREADS / 2;
-  uint32_t *M = upper ? X : Y, *Tm = upper ? T : T + INV_T;
-  const int t = tid & (PS_THREADS / 2 - 1);
-  tri64_level<A, 1, 1>(M, Tm, upper, ar, t);
-  tri64_level<A, 2, 1>(M, Tm, upper, ar, t);
-  tri64_level<A, 4, 1>(M, Tm, upper, ar, t);
-  tri64_level<A, 8, 1>(M, Tm, upper, ar, t);
-  tri64_level<A, 16, 2>(M, Tm, upper, ar, t);
-  tri64_level<A, 32, 4>(M, Tm, upper, ar, t);
 }
 
 // 1. First nonzero column of each row's panel part, rows i0..m-1 (one warp
@@ -539,6 +360,8 @@ constexpr int PW_LD = EW + 1;
 // dynamic shared memory: the window rows, later the two inverses and their
 // scratch; the multipliers of the window's rows (by slot) and of pivots from
 // past it; then the table of inverses (NORM)
+constexpr int INV_WORDS = 2 * (INV_M + INV_T);
+static_assert(PS_THREADS == 2 * INV_THREADS, "half of the CTA per inverse");
 constexpr int PW_AREA = PW_R * PW_LD > INV_WORDS ? PW_R * PW_LD : INV_WORDS;
 constexpr int PW_LROWS = PW_R + EW;
 constexpr size_t PW_SMEM = ((size_t)(PW_AREA + PW_LROWS * PW_LD) * 4 + 15) / 16 * 16;
@@ -1159,7 +982,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
       V si0, si1;
       uint32_t xi0, xi1;
       if (exact_inv) {
-        const uint32_t I = t > 0 ? inv_exact_u32(p, sa.canon(St)) : 1u % p;
+        const uint32_t I = t > 0 ? inv_exact_i31(p, sa.canon(St)) : 1u % p;
         if (t > 0 && I == 0u) err = 1;
         const V vI = sa.load(I);
         si0 = sa.mul(vI, b0);
@@ -1281,7 +1104,8 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
       Y[k * INV_LD + j] = l;
     }
     __syncthreads();
-    tri64_invert2<A>(X, Y, T, ar, tid);
+    const bool upper = tid < INV_THREADS;
+    tri64_invert<A>(upper ? X : Y, upper ? T : T + INV_T, upper, ar, tid & (INV_THREADS - 1));
     for (int e = tid; e < t * EW; e += PS_THREADS) {
       Uinv_out[e] = X[e / EW * INV_LD + e % EW];
       Linv_out[e] = Y[e / EW * INV_LD + e % EW];
@@ -1406,14 +1230,14 @@ __global__ void __launch_bounds__(SOLVE_THREADS)
     const uint32_t ap1 = lane + 32 < t ? (pc1 < 32 ? y0 : y1) : 0u;
     uint32_t l0 = 0u, l1 = 0u;  // multipliers k = lane, lane + 32
     if (__any_sync(0xffffffffu, (ap0 | ap1) != 0u)) {
-      uint64_t s0 = 0, s1 = 0;
+      typename A::Acc s0 = A::zero(), s1 = A::zero();
       for (int j = 0; j < t; ++j) {
         const uint32_t f = __shfl_sync(0xffffffffu, j < 32 ? ap0 : ap1, j & 31);
         ar.acc(s0, f, sUi[j][lane]);
         ar.acc(s1, f, sUi[j][lane + 32]);
       }
-      l0 = ar.red64(s0);
-      l1 = ar.red64(s1);
+      l0 = ar.sum(s0);
+      l1 = ar.sum(s1);
     }
     const int kk = pos - i0;
     uint32_t *lr = Lout + (size_t)kk * ldl;
@@ -1475,10 +1299,10 @@ __global__ void __launch_bounds__(U12_THREADS)
   for (int k = 1; k < EW; ++k) {
     if (k < t) {
       // entries j >= k still hold a_j, but L11[k][j] is zero there
-      uint64_t acc = 0;
+      typename A::Acc acc = A::zero();
 #pragma unroll
       for (int i = 0; i <= (k - 1) / 4; ++i) ar.acc(acc, sL[k][4 * i + l4], x[i]);
-      uint32_t v = ar.red64(acc);
+      uint32_t v = ar.sum(acc);
 #pragma unroll
       for (int o = 1; o <= 2; o <<= 1) {  // v + w mod p without overflow (any p < 2^32)
         const uint32_t nw = p - __shfl_xor_sync(0xffffffffu, v, o);

@@ -9,7 +9,7 @@
 // solve A22 with coefficient 1; upper: A22 first, then B1 <- alpha*B1 -
 // A12*B2, then A11), with the off-diagonal updates on the limb-split
 // tensor-core gemm.  The diagonal leaves are either 256-row blocks solved by
-// substitution on CUDA cores, or (from 1024 rows) 512-row blocks whose
+// substitution on CUDA cores, or (from 256 rows) 512-row blocks whose
 // inverses are built once and applied by the tensor-core gemm.
 //
 // Sparse operands.  When the caller says A may be sparse (Faugere-
@@ -33,6 +33,7 @@
 #include <mutex>
 #include <vector>
 
+#include "arith.cuh"
 #include "common.cuh"
 #include "context.h"
 #include "tri.h"
@@ -81,158 +82,53 @@ __global__ void __launch_bounds__(256)
   if (threadIdx.x == 0) occ[(size_t)bi * tn + bj] = nz ? 1 : 0;
 }
 
-// Solve T x = x in place for one column held by a quad of threads: thread q
-// holds the entries k = 4i + q (x[i]); T (nb x nb, nb <= 64, lower or upper
-// triangular) is in shared memory with its inverted diagonal sD (unitd: 1).
-// Right-looking: each thread keeps, per entry it holds, the 64-bit sum of
-// the products T[j][k] x[k] of the entries already solved (the reference's
-// wrap-around correction, +2^64 mod p, when NOWRAP is false; with p < 2^28
-// the sums cannot wrap).  Step k: the owner of k reduces its sum and
-// finishes x[k], one shuffle hands x[k] to the quad, and every thread adds
-// T[j][k] x[k] into the sums of its entries j still to solve -- sixteen
-// independent multiply-adds, so the sequential chain per step is one
-// reduction, one shuffle and one multiply-add.  The entries of the current
-// group of four (k / 4) sit in slot CUR: after each group the registers
-// rotate by one, so no step needs a dynamic register index, and after the
-// sixteen groups they are back in place.  Entries from nb on are zero and
-// never solved.
-template <bool UPPER, bool NOWRAP>
-__device__ __forceinline__ void tri_quad_solve(const uint32_t (*sT)[TRI_NB + 1],
-                                               const uint32_t *sD, bool unitd, int nb, int q,
-                                               uint32_t (&x)[TRI_NB / 4], const Modulus &mod,
-                                               uint32_t two64) {
-  constexpr int NI = TRI_NB / 4;
-  constexpr int CUR = UPPER ? NI - 1 : 0;  // slot s holds group (g + s - CUR) mod NI
-  const uint32_t p = (uint32_t)mod.p;
-  const int qbase = (threadIdx.x & 31) & ~3;
-  const int last = (nb - 1) >> 2;  // last group with an entry
-  uint64_t acc[NI];
-#pragma unroll
-  for (int i = 0; i < NI; ++i) acc[i] = 0ull;
-#pragma unroll 1
-  for (int gg = 0; gg < NI; ++gg) {
-    const int g = UPPER ? NI - 1 - gg : gg;
-    if (g <= last) {
-#pragma unroll
-      for (int rr = 0; rr < 4; ++rr) {
-        const int r = UPPER ? 3 - rr : rr;
-        const int k = 4 * g + r;
-        if (k < nb) {
-          // every lane forms its candidate; the owner's (q == r) is x[k]
-          const uint32_t red = mod_reduce(acc[CUR], mod);
-          uint32_t v = x[CUR] >= red ? x[CUR] - red : x[CUR] + (p - red);
-          if (!unitd) v = mod_mul(v, sD[k], mod);
-          if (q == r) x[CUR] = v;
-          v = __shfl_sync(0xffffffffu, v, qbase + r);
-#pragma unroll
-          for (int sl = 0; sl < NI; ++sl) {
-            const int j = 4 * ((g + sl - CUR) & (NI - 1)) + q;
-            if (UPPER ? j < k : j > k) {
-              const uint64_t t = (uint64_t)sT[j][k] * v;
-              acc[sl] += t;
-              if (!NOWRAP && acc[sl] < t) acc[sl] += two64;
-            }
-          }
-        }
-      }
-    }
-    // the next group into slot CUR
-    if (UPPER) {
-      const uint32_t xe = x[NI - 1];
-      const uint64_t ae = acc[NI - 1];
-#pragma unroll
-      for (int sl = NI - 1; sl > 0; --sl) {
-        x[sl] = x[sl - 1];
-        acc[sl] = acc[sl - 1];
-      }
-      x[0] = xe;
-      acc[0] = ae;
-    } else {
-      const uint32_t xe = x[0];
-      const uint64_t ae = acc[0];
-#pragma unroll
-      for (int sl = 0; sl < NI - 1; ++sl) {
-        x[sl] = x[sl + 1];
-        acc[sl] = acc[sl + 1];
-      }
-      x[NI - 1] = xe;
-      acc[NI - 1] = ae;
-    }
-  }
-}
-
-// Left solve of one diagonal block: for every column of B (a quad of
-// threads each), x <- alpha * T^-1 x, T = nb x nb (nb <= 64) lower or upper
-// triangular with inverted diagonal dinv (nullptr: unit diagonal).
-template <bool UPPER, bool NOWRAP>
-__global__ void __launch_bounds__(128)
-    tri_left_kernel(const uint32_t *__restrict__ T, size_t ldt, int nb,
-                    const uint32_t *__restrict__ dinv, uint32_t *__restrict__ B, size_t ldb,
-                    int ncols, Modulus mod, uint32_t two64, uint32_t alpha) {
-  __shared__ uint32_t sT[TRI_NB][TRI_NB + 1];
-  __shared__ uint32_t sD[TRI_NB];
-  // asynchronous copies, all in flight at once (entries outside nb x nb are
-  // zero-filled)
-  for (int e = threadIdx.x; e < TRI_NB * TRI_NB; e += blockDim.x) {
-    const int r = e / TRI_NB, cc = e % TRI_NB;
-    const bool in = r < nb && cc < nb;
-    cp_async4(&sT[r][cc], in ? T + (size_t)r * ldt + cc : T, in);
-  }
-  for (int e = threadIdx.x; e < TRI_NB; e += blockDim.x) sD[e] = (e < nb && dinv) ? dinv[e] : 1u;
-  cp_async_wait_all();
-  __syncthreads();
-  const int gt = blockIdx.x * blockDim.x + threadIdx.x;
-  const int col = gt >> 2, q = gt & 3;
-  const bool ok = col < ncols;  // every lane stays for the quad's shuffles
-  uint32_t x[TRI_NB / 4];
-#pragma unroll
-  for (int i = 0; i < TRI_NB / 4; ++i) {
-    const int k = 4 * i + q;
-    const uint32_t v = (ok && k < nb) ? B[(size_t)k * ldb + col] : 0u;
-    x[i] = (alpha == 1u) ? v : mod_mul(v, alpha, mod);
-  }
-  tri_quad_solve<UPPER, NOWRAP>(sT, sD, dinv == nullptr, nb, q, x, mod, two64);
-  if (ok)
-#pragma unroll
-    for (int i = 0; i < TRI_NB / 4; ++i) {
-      const int k = 4 * i + q;
-      if (k < nb) B[(size_t)k * ldb + col] = x[i];
-    }
-}
-
 // Inverses of all diagonal blocks at once: block b (rows/cols 64b ..
-// 64b+nb) of the triangular A; one CTA of 256 threads per block, a quad per
-// column j solving T x = e_j.  Out: the 64 x 64 inverse (zero padded) at
+// 64b+nb) of the triangular A, one CTA each, by doubling in shared memory
+// (tri64_invert).  dinv: the inverted diagonal (nullptr: ones).  Out: the 64 x
+// 64 inverse (zero padded) at
 // rows 64b.. of Tinv (row stride ldo), columns (64b mod cmod)..: ldo = cmod
 // = 64 stores the blocks one after the other; ldo = cmod = NB places them
-// on the diagonal of the NB-row block inverses.
-template <bool UPPER>
-__global__ void __launch_bounds__(256)
-    tri_inv_blocks_kernel(const uint32_t *__restrict__ A, size_t lda, int m,
+// on the diagonal of the NB-row block inverses.  Bound: the latency of the
+// twelve products (substitution, a quad of threads per column with 64
+// dependent steps, took 49 us a launch, 56 us for the upper).
+template <class A>
+__global__ void __launch_bounds__(INV_THREADS)
+    tri_inv_blocks_kernel(const uint32_t *__restrict__ M, size_t lda, int m, bool upper,
                           const uint32_t *__restrict__ dinv, uint32_t *__restrict__ Tinv,
-                          size_t ldo, int cmod, Modulus mod, uint32_t two64) {
-  __shared__ uint32_t sT[TRI_NB][TRI_NB + 1];
-  __shared__ uint32_t sD[TRI_NB];
-  const int b = blockIdx.x;
-  const int r0 = b * TRI_NB;
-  const int nb = min(TRI_NB, m - r0);
-  const uint32_t *T = A + (size_t)r0 * lda + r0;
-  for (int e = threadIdx.x; e < TRI_NB * TRI_NB; e += blockDim.x) {
-    const int r = e / TRI_NB, cc = e % TRI_NB;
-    const bool in = r < nb && cc < nb;
-    cp_async4(&sT[r][cc], in ? T + (size_t)r * lda + cc : T, in);
+                          size_t ldo, int cmod, A ar) {
+  __shared__ __align__(16) uint32_t X[INV_M], T[INV_T];
+  const int r0 = blockIdx.x * TRI_NB, nb = min(TRI_NB, m - r0);
+  const uint32_t *D = M + (size_t)r0 * lda + r0;
+#pragma unroll 8
+  for (int u = 0; u < TRI_NB * TRI_NB / INV_THREADS; ++u) {
+    const int e = threadIdx.x + u * INV_THREADS, i = e / TRI_NB, j = e % TRI_NB;
+    uint32_t v = i == j ? 1u : 0u;
+    if (i < nb && j < nb) {
+      if (i == j) v = dinv ? dinv[r0 + i] : v;
+      else if (upper ? j > i : j < i) v = D[(size_t)i * lda + j];
+    }
+    X[i * INV_LD + j] = v;
   }
-  for (int e = threadIdx.x; e < TRI_NB; e += blockDim.x) sD[e] = (e < nb && dinv) ? dinv[r0 + e] : 1u;
-  cp_async_wait_all();
   __syncthreads();
-  const int j = threadIdx.x >> 2, q = threadIdx.x & 3;
-  uint32_t x[TRI_NB / 4];
-#pragma unroll
-  for (int i = 0; i < TRI_NB / 4; ++i) x[i] = (4 * i + q == j && j < nb) ? 1u : 0u;
-  tri_quad_solve<UPPER, false>(sT, sD, dinv == nullptr, nb, q, x, mod, two64);
+  tri64_invert<A>(X, T, upper, ar, threadIdx.x);
   uint32_t *out = Tinv + (size_t)r0 * ldo + r0 % cmod;
-#pragma unroll
-  for (int i = 0; i < TRI_NB / 4; ++i) out[(size_t)(4 * i + q) * ldo + j] = (j < nb) ? x[i] : 0u;
+#pragma unroll 4
+  for (int u = 0; u < TRI_NB * TRI_NB / INV_THREADS; ++u) {
+    const int e = threadIdx.x + u * INV_THREADS, i = e / TRI_NB, j = e % TRI_NB;
+    out[(size_t)i * ldo + j] = i < nb && j < nb ? X[i * INV_LD + j] : 0u;
+  }
+}
+static void launch_inv_blocks(Ctx *c, bool upper, int m, const uint32_t *A, size_t lda,
+                              const uint32_t *dinv, uint32_t *Tinv, size_t ldo, int cmod,
+                              uint32_t p) {
+  const int nblk = (m + TRI_NB - 1) / TRI_NB;
+  if (p < (1u << 16))
+    tri_inv_blocks_kernel<<<nblk, INV_THREADS, 0, c->stream>>>(A, lda, m, upper, dinv, Tinv, ldo,
+                                                               cmod, ArithSmall::make(p));
+  else
+    tri_inv_blocks_kernel<<<nblk, INV_THREADS, 0, c->stream>>>(A, lda, m, upper, dinv, Tinv, ldo,
+                                                               cmod, ArithWide::make(p));
+  ctx_launched(c);
 }
 
 // ----------------------------------------------------------- inverse leaves
@@ -248,7 +144,7 @@ __global__ void __launch_bounds__(256)
 // its rows TI_NB b .., columns 0 ..; every level writes its off-diagonal
 // blocks in place.
 constexpr int TI_NB = 512;
-constexpr int MG_T = 64, MG_K = 32;
+constexpr int MG_T = 32, MG_K = 32;
 
 // One operand of a batched merge product: entry (i, j) of instance z sits at
 // ptr[(z rs + ro + i) ld + (z cs + co) mod cmod + j].
@@ -261,73 +157,87 @@ struct MergeOp {
   }
 };
 
-// C_z <- alpha X_z Y_z (M x N, inner dimension K) for the instances
-// z = zbase + blockIdx.z; 64 x 64 tiles as the small-K gemm.  NOWRAP
-// (p < 2^28): unchecked sums reduced every 256 terms.
-template <bool NOWRAP>
+// Which part of the inner dimension a tile at (m0, n0) needs, one factor
+// being triangular.
+enum MergeK : int {
+  MG_TO_N = 0,    // Y upper: k < n0 + MG_T
+  MG_FROM_M = 1,  // X upper: k >= m0
+  MG_FROM_N = 2,  // Y lower: k >= n0
+  MG_TO_M = 3     // X lower: k < m0 + MG_T
+};
+
+// C_z <- X_z Y_z, or its negative (M x N, inner dimension K, K <= 256) for the
+// instances z = zbase + blockIdx.z.  32 x 32 tiles, two rows and two columns a
+// thread, four k at a time; the next step's operands are in registers while a
+// step is multiplied.  Bound: shared-memory reads and multiply-adds about
+// equally.  The smaller tiles fill the SMs for the few instances of a
+// 1024-row solve, and half of the inner range is skipped (64 x 64 tiles, no
+// prefetch, whole range: 20 to 33 us a launch, 40 us for p = 2^31 - 1).
+template <class A>
 __global__ void __launch_bounds__(256)
-    tri_merge_kernel(MergeOp X, MergeOp Y, MergeOp Cop, int zbase, int M, int N, int K,
-                     Modulus mod, uint32_t two64, uint32_t alpha) {
-  __shared__ uint32_t Xs[MG_K][MG_T + 1];
-  __shared__ uint32_t Ys[MG_K][MG_T + 1];
+    tri_merge_kernel(MergeOp X, MergeOp Y, MergeOp Cop, int zbase, int M, int N, int K, int krange,
+                     A ar, bool negate) {
+  __shared__ __align__(16) uint32_t Xs[2][MG_T][MG_K + 4];
+  __shared__ uint32_t Ys[2][MG_K][MG_T];
   const int z = zbase + blockIdx.z;
   const uint32_t *__restrict__ Xp = X.at(z);
   const uint32_t *__restrict__ Yp = Y.at(z);
   uint32_t *Cp = const_cast<uint32_t *>(Cop.at(z));
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int lx = threadIdx.x & 31, ly = threadIdx.x >> 5;
   const int m0 = blockIdx.y * MG_T, n0 = blockIdx.x * MG_T;
-  uint64_t acc[4][4];
+  const int kb = krange == MG_FROM_M ? m0 : krange == MG_FROM_N ? n0 : 0;
+  const int ke = min(K, krange == MG_TO_N ? n0 + MG_T : krange == MG_TO_M ? m0 + MG_T : K);
+  uint32_t xr[4], yr[4];
+  auto load = [&](int k0) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0;
-  for (int k0 = 0; k0 < K; k0 += MG_K) {
-#pragma unroll
-    for (int e = 0; e < (MG_T * MG_K) / 256; ++e) {
-      const int idx = threadIdx.x + 256 * e;
-      const int r = idx / MG_K, kk = idx % MG_K;
-      const int gm = m0 + r, gk = k0 + kk;
-      Xs[kk][r] = (gm < M && gk < K) ? Xp[(size_t)gm * X.ld + gk] : 0u;
-      const int kr = idx / MG_T, cc = idx % MG_T;
-      const int gk2 = k0 + kr, gn = n0 + cc;
-      Ys[kr][cc] = (gk2 < K && gn < N) ? Yp[(size_t)gk2 * Y.ld + gn] : 0u;
+    for (int u = 0; u < 4; ++u) {
+      const int r = ly + 8 * u;
+      xr[u] = (m0 + r < M && k0 + lx < ke) ? Xp[(size_t)(m0 + r) * X.ld + k0 + lx] : 0u;
+      yr[u] = (k0 + r < ke && n0 + lx < N) ? Yp[(size_t)(k0 + r) * Y.ld + n0 + lx] : 0u;
     }
-    __syncthreads();
-#pragma unroll 8
-    for (int kk = 0; kk < MG_K; ++kk) {
-      uint32_t a[4], b[4];
+  };
+  typename A::Acc acc[2][2];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = Xs[kk][ty + 16 * i];
+  for (int i = 0; i < 2; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Ys[kk][tx + 16 * j];
+    for (int j = 0; j < 2; ++j) acc[i][j] = A::zero();
+  load(kb);
+  int s = 0;
+  for (int k0 = kb; k0 < ke; k0 += MG_K, s ^= 1) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+    for (int u = 0; u < 4; ++u) {
+      Xs[s][ly + 8 * u][lx] = xr[u];
+      Ys[s][ly + 8 * u][lx] = yr[u];
+    }
+    __syncthreads();  // (the other stage was last read before the previous barrier)
+    if (k0 + MG_K < ke) load(k0 + MG_K);
+#pragma unroll 2
+    for (int kk = 0; kk < MG_K; kk += 4) {
+      const uint4 a0 = *reinterpret_cast<const uint4 *>(&Xs[s][ty][kk]);
+      const uint4 a1 = *reinterpret_cast<const uint4 *>(&Xs[s][ty + 16][kk]);
+      const uint32_t av[2][4] = {{a0.x, a0.y, a0.z, a0.w}, {a1.x, a1.y, a1.z, a1.w}};
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const uint64_t t = (uint64_t)a[i] * b[j];
-          if (NOWRAP) {
-            acc[i][j] += t;
-          } else {
-            const uint64_t s = acc[i][j] + t;
-            acc[i][j] = (s < t) ? s + two64 : s;
-          }
+      for (int q = 0; q < 4; ++q) {
+        const uint32_t b0 = Ys[s][kk + q][tx], b1 = Ys[s][kk + q][tx + 16];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          ar.acc(acc[i][0], av[i][q], b0);
+          ar.acc(acc[i][1], av[i][q], b1);
         }
+      }
     }
-    if (NOWRAP && ((k0 / MG_K) & 7) == 7)
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = mod_reduce(acc[i][j], mod);
-    __syncthreads();
   }
+  const uint32_t p = ar.p;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < 2; ++i) {
     const int gm = m0 + ty + 16 * i;
     if (gm >= M) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < 2; ++j) {
       const int gn = n0 + tx + 16 * j;
-      if (gn < N) Cp[(size_t)gm * Cop.ld + gn] = mod_mul(mod_reduce(acc[i][j], mod), alpha, mod);
+      const uint32_t v = ar.sum(acc[i][j]);
+      if (gn < N) Cp[(size_t)gm * Cop.ld + gn] = negate && v ? p - v : v;
     }
   }
 }
@@ -344,33 +254,6 @@ __global__ void zp_scale2_kernel(uint32_t *C, size_t ldc, int M, int N, Modulus 
   }
 }
 
-int tri_left_block(Ctx *c, bool upper, int nb, const uint32_t *T, size_t ldt,
-                   const uint32_t *dinv, uint32_t *B, size_t ldb, int ncols, uint32_t p,
-                   uint32_t alpha) {
-  if (nb <= 0 || ncols <= 0) return ST_OK;
-  const Modulus mod = make_modulus(p);
-  const uint32_t t64 = two64_mod(p);
-  const int threads = 128;  // 32 columns, four threads each
-  const int grid = (ncols * 4 + threads - 1) / threads;
-  const bool nowrap = p < (1u << 28);
-  int pi = prof_begin(c, "tri_left");
-  if (upper && nowrap)
-    tri_left_kernel<true, true><<<grid, threads, 0, c->stream>>>(T, ldt, nb, dinv, B, ldb, ncols,
-                                                                 mod, t64, alpha);
-  else if (upper)
-    tri_left_kernel<true, false><<<grid, threads, 0, c->stream>>>(T, ldt, nb, dinv, B, ldb, ncols,
-                                                                  mod, t64, alpha);
-  else if (nowrap)
-    tri_left_kernel<false, true><<<grid, threads, 0, c->stream>>>(T, ldt, nb, dinv, B, ldb, ncols,
-                                                                  mod, t64, alpha);
-  else
-    tri_left_kernel<false, false><<<grid, threads, 0, c->stream>>>(T, ldt, nb, dinv, B, ldb, ncols,
-                                                                   mod, t64, alpha);
-  prof_end(c, pi);
-  ctx_launched(c);
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? ST_OK : ctx_cuda(c, e, "tri_left launch");
-}
 
 // Inverted diagonal blocks of the whole system: the leaf whose top-left
 // entry is A_base[off*(lda+1)] uses tinv + (off/64) * 64*64 (leaves start
@@ -668,10 +551,8 @@ static int trsm_rec(Ctx *c, const TriLeaves &TL, const TileMap *tm, int off, boo
 // (m / TI_NB + 1) * (TI_NB / 2)^2 entries (the largest level's need).
 static int tri_inverse_levels(Ctx *c, bool upper, int m, uint32_t p, const uint32_t *A,
                               size_t lda, uint32_t *W, uint32_t *T) {
-  const Modulus mod = make_modulus(p);
-  const uint32_t t64 = two64_mod(p);
-  const bool nowrap = p < (1u << 28);
   constexpr int NOMOD = 1 << 30;
+  static_assert(TI_NB / 2 <= 256, "inner dimension of the merge products");
   for (int s = 2 * TRI_NB; s <= TI_NB && s / 2 < m; s *= 2) {
     const int h = s / 2;
     const int nfull = m / s;
@@ -699,13 +580,14 @@ static int tri_inverse_levels(Ctx *c, bool upper, int m, uint32_t p, const uint3
       }
       const dim3 g1((N1 + MG_T - 1) / MG_T, (M1 + MG_T - 1) / MG_T, nz);
       const dim3 g2((N2 + MG_T - 1) / MG_T, (M2 + MG_T - 1) / MG_T, nz);
-      if (nowrap) {
-        tri_merge_kernel<true><<<g1, 256, 0, c->stream>>>(X1, Y1, Tz, zbase, M1, N1, K1, mod, t64, 1u);
-        tri_merge_kernel<true><<<g2, 256, 0, c->stream>>>(X2, Tz, C2, zbase, M2, N2, K2, mod, t64, p - 1);
-      } else {
-        tri_merge_kernel<false><<<g1, 256, 0, c->stream>>>(X1, Y1, Tz, zbase, M1, N1, K1, mod, t64, 1u);
-        tri_merge_kernel<false><<<g2, 256, 0, c->stream>>>(X2, Tz, C2, zbase, M2, N2, K2, mod, t64, p - 1);
-      }
+      auto merge = [&](auto ar) {
+        tri_merge_kernel<<<g1, 256, 0, c->stream>>>(X1, Y1, Tz, zbase, M1, N1, K1,
+                                                    upper ? MG_TO_N : MG_FROM_N, ar, false);
+        tri_merge_kernel<<<g2, 256, 0, c->stream>>>(X2, Tz, C2, zbase, M2, N2, K2,
+                                                    upper ? MG_FROM_M : MG_TO_M, ar, true);
+      };
+      if (p < (1u << 16)) merge(ArithSmall::make(p));
+      else merge(ArithWide::make(p));
       ctx_launched(c, 2);
     }
   }
@@ -724,7 +606,8 @@ static int trsm_rec_inv(Ctx *c, const TileMap *tm, int off, bool upper, int m, i
     // in place: the tensor-core path converts B to limbs in the workspace
     // before its first product, and with one K chunk (m <= TI_NB) each
     // output tile is written once, after every product that reads B
-    return zp_gemm_dev(c, GEMM_TC, m, n, m, p, alpha, W, TI_NB, B, ldb, 0, B, ldb, gemm_ws);
+    return zp_gemm_dev(c, m <= 128 ? GEMM_DIRECT : GEMM_TC, m, n, m, p, alpha, W, TI_NB, B, ldb, 0,
+                       B, ldb, gemm_ws);
   }
   const int l = ((m / 2 + TI_NB - 1) / TI_NB) * TI_NB;  // TI_NB <= l < m
   const uint32_t *A12 = A + l, *A21 = A + (size_t)l * lda, *A22 = A21 + l;
@@ -798,11 +681,13 @@ int zp_trsm_dev(Ctx *c, bool upper, bool unit, int m, int n, uint32_t p, uint32_
   if (n == 0) return ST_OK;
   int kind = c->trsm_kernel;
   if (kind == TRSM_AUTO) {
-    // inverse leaves from two leaves up (measured faster there for every
-    // width from 64 columns; a single leaf's set-up costs more than the
-    // substitution), and not when the caller forced a CUDA-core gemm
+    // inverse leaves from 256 rows up, 128 when products need 64-bit reduction
+    // (us, substitution / inverses, 500 columns: p = 65521 m = 128 32 / 37, 200
+    // 50 / 68, 256 63 / 59, 512 128 / 85, 1023 267 / 175; p = 2^31 - 1 m = 100 39 /
+    // 42, 128 48 / 42, 256 123 / 67, 1023 515 / 195; 64 and 4000 columns alike), and
+    // not when the caller forced a CUDA-core gemm
     const bool tc = c->gemm_kernel == GEMM_AUTO || c->gemm_kernel == GEMM_TC;
-    kind = (tc && m >= 2 * TI_NB) ? TRSM_INVERSE : TRSM_BLOCKS;
+    kind = (tc && m >= (p < (1u << 16) ? 256 : 128)) ? TRSM_INVERSE : TRSM_BLOCKS;
   }
   // occupied tiles of a possibly sparse A (bounding boxes of the updates)
   TileMap map;
@@ -827,13 +712,7 @@ int zp_trsm_dev(Ctx *c, bool upper, bool unit, int m, int n, uint32_t p, uint32_
     uint32_t *W = static_cast<uint32_t *>(wb);
     cudaError_t e = cudaMemsetAsync(W, 0, (size_t)nleaf * TI_NB * TI_NB * 4, c->stream);
     if (e != cudaSuccess) return ctx_cuda(c, e, "cudaMemsetAsync(trsm inverses)");
-    if (upper)
-      tri_inv_blocks_kernel<true><<<nblk, 256, 0, c->stream>>>(A, lda, m, dv, W, TI_NB, TI_NB,
-                                                              mod, two64_mod(p));
-    else
-      tri_inv_blocks_kernel<false><<<nblk, 256, 0, c->stream>>>(A, lda, m, dv, W, TI_NB, TI_NB,
-                                                               mod, two64_mod(p));
-    ctx_launched(c);
+    launch_inv_blocks(c, upper, m, A, lda, dv, W, TI_NB, TI_NB, p);
     if ((st = tri_inverse_levels(c, upper, m, p, A, lda, W, static_cast<uint32_t *>(tb))))
       return st;
     void *w = nullptr;
@@ -844,13 +723,7 @@ int zp_trsm_dev(Ctx *c, bool upper, bool unit, int m, int n, uint32_t p, uint32_
   void *tb = nullptr;
   if ((st = ctx_buffer(c, BUF_TINV, (size_t)nblk * TRI_NB * TRI_NB * 4, &tb))) return st;
   uint32_t *tinv = static_cast<uint32_t *>(tb);
-  if (upper)
-    tri_inv_blocks_kernel<true><<<nblk, 256, 0, c->stream>>>(A, lda, m, dv, tinv, TRI_NB, TRI_NB,
-                                                            mod, two64_mod(p));
-  else
-    tri_inv_blocks_kernel<false><<<nblk, 256, 0, c->stream>>>(A, lda, m, dv, tinv, TRI_NB, TRI_NB,
-                                                             mod, two64_mod(p));
-  ctx_launched(c);
+  launch_inv_blocks(c, upper, m, A, lda, dv, tinv, TRI_NB, TRI_NB, p);
   void *w = nullptr;
   if ((st = ctx_workspace(c, zp_trsm_workspace_bytes(p, m, n), &w))) return st;
   TriLeaves TL{A, tinv};

@@ -32,10 +32,4 @@ int zp_trsm_csr_upper_dev(Ctx *c, bool unit, int n, int ncols, uint32_t p, uint3
 // caller holding the workspace can size it once.
 size_t zp_trsm_workspace_bytes(uint32_t p, int m, int n);
 
-// One diagonal block (nb <= 64) solved on CUDA cores: B <- alpha*T^-1*B;
-// dinv = inverted diagonal (nullptr for a unit diagonal).
-int tri_left_block(Ctx *c, bool upper, int nb, const uint32_t *T, size_t ldt,
-                   const uint32_t *dinv, uint32_t *B, size_t ldb, int ncols, uint32_t p,
-                   uint32_t alpha);
-
 }  // namespace lela
