@@ -632,9 +632,66 @@ static int trsm_rec_inv(Ctx *c, const TileMap *tm, int off, bool upper, int m, i
   }
 }
 
-size_t zp_trsm_workspace_bytes(uint32_t p, int m, int n) {
+// The same solve leaf by leaf (left-looking), for wide right-hand sides: the
+// limb planes of A's triangle are made once and those of each solved leaf of X
+// once, and a leaf gets one update with K = all rows solved before it (its rows of
+// A times X), then its inverse.  The recursion splits every block of X once per
+// level (four times at 16 leaves) and its small updates leave SMs idle: 8192^2
+// x 4096 1340 us.  Each product has TI_NB rows, so it needs columns for the SMs.
+static bool trsm_left_pays(const Ctx *c, int m, int n, uint32_t p) {
+  const int bn = zp_limbs_for(p) == 4 ? 32 : 128;
+  return m > 2 * TI_NB && 3 * (TI_NB / 128) * ((n + bn - 1) / bn) >= 2 * c->num_sms;
+}
+static size_t trsm_left_pitch(int m) { return ((size_t)m + 15) & ~(size_t)15; }
+static size_t trsm_left_bytes(uint32_t p, int m, int n) {
+  return (size_t)zp_limbs_for(p) * ((size_t)m + n) * trsm_left_pitch(m) + 256 +
+         zp_gemm_workspace_bytes(p, TI_NB, n, TI_NB);
+}
+static int trsm_left(Ctx *c, const TileMap *tm, bool upper, int m, int n, uint32_t p,
+                     uint32_t alpha, const uint32_t *A, size_t lda, const uint32_t *W, uint32_t *B,
+                     size_t ldb, uint8_t *ws) {
+  const size_t pitch = trsm_left_pitch(m), L = (size_t)zp_limbs_for(p);
+  const ZpPlanes PA{ws, pitch, (size_t)m * pitch};
+  const ZpPlanes PX{ws + L * (size_t)m * pitch, pitch, (size_t)n * pitch};
+  uint8_t *leaf_ws = ws + ((L * ((size_t)m + n) * pitch + 255) & ~(size_t)255);
+  int st = zp_split_rows_dev(c, p, A, lda, m, m, PA, upper ? 2 : 1, TI_NB);
+  const int nl = (m + TI_NB - 1) / TI_NB;
+  for (int s = 0; !st && s < nl; ++s) {
+    const int r0 = (upper ? nl - 1 - s : s) * TI_NB, rows = std::min(TI_NB, m - r0);
+    uint32_t *Bi = B + (size_t)r0 * ldb;
+    int c0 = upper ? r0 + rows : 0, c1 = upper ? m : r0;  // solved rows of X
+    uint32_t a = alpha;
+    if (tm && c1 > c0) {
+      int b0, b1, x0, x1;
+      if (tm->box(r0, r0 + rows, c0, c1, b0, b1, x0, x1)) {
+        c0 = x0;
+        c1 = x1;
+      } else {
+        c1 = c0;
+      }
+    }
+    if (c1 > c0) {
+      if ((st = zp_gemm_planes_dev(c, rows, n, c1 - c0, p, p - 1, PA.at((size_t)r0, (size_t)c0),
+                                   PX.at(0, (size_t)c0), alpha, Bi, ldb,
+                                   tm && tm->kr ? tm->kr + r0 : nullptr, c0)))
+        return st;
+      a = 1;
+    }
+    st = zp_gemm_dev(c, rows <= 128 ? GEMM_DIRECT : GEMM_TC, rows, n, rows, p, a,
+                     W + (size_t)r0 * TI_NB, TI_NB, Bi, ldb, 0, Bi, ldb, leaf_ws);
+    if (!st && s + 1 < nl) st = zp_split_cols_dev(c, p, Bi, ldb, rows, n, PX.at(0, (size_t)r0));
+  }
+  return st;
+}
+
+static size_t trsm_rec_bytes(uint32_t p, int m, int n) {
   // the largest update is about (m/2 + leaf) x n x (m/2 + leaf)
   return zp_gemm_workspace_bytes(p, m, n, (m + 1) / 2 + std::max(TI_NB, TRI_NB));
+}
+
+size_t zp_trsm_workspace_bytes(uint32_t p, int m, int n) {
+  if (m > 2 * TI_NB) return std::max(trsm_rec_bytes(p, m, n), trsm_left_bytes(p, m, n));
+  return trsm_rec_bytes(p, m, n);
 }
 
 int zp_trsm_dev(Ctx *c, bool upper, bool unit, int m, int n, uint32_t p, uint32_t alpha,
@@ -716,7 +773,15 @@ int zp_trsm_dev(Ctx *c, bool upper, bool unit, int m, int n, uint32_t p, uint32_
     if ((st = tri_inverse_levels(c, upper, m, p, A, lda, W, static_cast<uint32_t *>(tb))))
       return st;
     void *w = nullptr;
-    if ((st = ctx_workspace(c, zp_trsm_workspace_bytes(p, m, n), &w))) return st;
+    // (where the planes of all of A do not fit, the recursion's smaller ones may)
+    if (trsm_left_pays(c, m, n, p)) {
+      st = ctx_workspace(c, zp_trsm_workspace_bytes(p, m, n), &w);
+      if (!st)
+        return trsm_left(c, tm, upper, m, n, p, alpha, A, lda, W, B, ldb, static_cast<uint8_t *>(w));
+      if (st != ST_NOMEM) return st;
+      cudaGetLastError();
+    }
+    if ((st = ctx_workspace(c, trsm_rec_bytes(p, m, n), &w))) return st;
     return trsm_rec_inv(c, tm, 0, upper, m, n, p, alpha, A, lda, W, B, ldb,
                         static_cast<uint8_t *>(w));
   }
@@ -725,7 +790,7 @@ int zp_trsm_dev(Ctx *c, bool upper, bool unit, int m, int n, uint32_t p, uint32_
   uint32_t *tinv = static_cast<uint32_t *>(tb);
   launch_inv_blocks(c, upper, m, A, lda, dv, tinv, TRI_NB, TRI_NB, p);
   void *w = nullptr;
-  if ((st = ctx_workspace(c, zp_trsm_workspace_bytes(p, m, n), &w))) return st;
+  if ((st = ctx_workspace(c, trsm_rec_bytes(p, m, n), &w))) return st;
   TriLeaves TL{A, tinv};
   return trsm_rec(c, TL, tm, 0, upper, m, n, p, alpha, A, lda, unit ? nullptr : dinv, B, ldb,
                   static_cast<uint8_t *>(w));

@@ -839,20 +839,21 @@ __global__ void __launch_bounds__(DIR_THREADS, L == 4 ? 1 : 2)
 }
 
 // ------------------------------------------------------------ limb splits
-// A (M x kc, row stride lda, elements T) -> L planes of M x Kp bytes.  Bound by
+// A (M x kc, row stride lda, elements T) -> L planes of bytes, row pitch Kp,
+// `plane` bytes apart.  Bound by
 // HBM (8192^2 of u32: 69 us, 402 MB); lanes on consecutive groups of four
-// columns, a row per warp, so no index division.
+// columns, a row per warp, so no index division.  part: 0 all columns; 1 (2)
+// only those left (right) of the row's diagonal block of nb rows.
 constexpr int SPLIT_ROWS = 8;  // rows (warps) per CTA
 template <int L, class T>
 __global__ void __launch_bounds__(32 * SPLIT_ROWS)
     split_rows_kernel(const T *__restrict__ A, size_t lda, int M, int kc, uint32_t p,
-                      uint8_t *__restrict__ out, int Kp) {
-  const int kq = (kc + 3) >> 2;
-  const size_t plane = (size_t)M * Kp;
+                      uint8_t *__restrict__ out, size_t Kp, size_t plane, int part, int nb) {
   for (int r = blockIdx.y * SPLIT_ROWS + threadIdx.y; r < M; r += gridDim.y * SPLIT_ROWS) {
     const T *src = A + (size_t)r * lda;
     uint8_t *dst = out + (size_t)r * Kp;
-    for (int q = blockIdx.x * 32 + threadIdx.x; q < kq; q += gridDim.x * 32) {
+    const int kb = part == 2 ? min(kc, (r / nb + 1) * nb) : 0, ke = part == 1 ? min(kc, r / nb * nb) : kc;
+    for (int q = (kb >> 2) + blockIdx.x * 32 + threadIdx.x; 4 * q < ke; q += gridDim.x * 32) {
       const int k = 4 * q;
       uint32_t v[4];
 #pragma unroll
@@ -873,8 +874,8 @@ static dim3 split_rows_grid(int num_sms, int M, int kc) {
   return dim3(std::max(1, std::min(((kc + 3) / 4 + 31) / 32, num_sms * 16 / gy)), gy);
 }
 
-// B (kc x N, row stride ldb, elements T) -> L planes of N x Kp bytes
-// (transposed), through a shared-memory tile of 64 k x NT columns (128 bytes
+// B (kc x N, row stride ldb, elements T) -> L planes of N rows of kout <= Kp
+// bytes (row pitch Kp, `plane` bytes apart; transposed), through a shared-memory tile of 64 k x NT columns (128 bytes
 // of a row of the narrow types, 32 elements of the others).
 template <class T>
 constexpr int split_cols_nt() {
@@ -883,13 +884,12 @@ constexpr int split_cols_nt() {
 template <int L, class T>
 __global__ void __launch_bounds__(256)
     split_cols_kernel(const T *__restrict__ B, size_t ldb, int kc, int N, uint32_t p,
-                      uint8_t *__restrict__ out, int Kp) {
+                      uint8_t *__restrict__ out, size_t Kp, size_t plane, int kout) {
   using R = typename Rep<T>::Packed;
   constexpr int NT = split_cols_nt<T>();
   __shared__ R tile[64][NT + 4 / sizeof(R)];
   const int n0 = blockIdx.x * NT, k0 = blockIdx.y * 64;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const size_t plane = (size_t)N * Kp;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int k = k0 + ty + 8 * i;
@@ -906,7 +906,7 @@ __global__ void __launch_bounds__(256)
     const int w = threadIdx.x + 256 * j;
     const int n = w >> 4, kw = (w & 15) * 4;
     const int gn = n0 + n, gk = k0 + kw;
-    if (gn < N && gk < Kp) {
+    if (gn < N && gk < kout) {
       uint32_t v[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) v[i] = tile[kw + i][n];
@@ -1125,9 +1125,10 @@ static int launch_tc(Ctx *c, int M, int N, int K, const Modulus &mod, uint32_t a
       const uint32_t p = (uint32_t)mod.p;
       int pi = prof_begin(c, "zp_split");
       split_rows_kernel<L, E><<<split_rows_grid(c->num_sms, M, kc), dim3(32, SPLIT_ROWS), 0,
-                                c->stream>>>(A + k0, lda, M, kc, p, Al, Kp);
+                                c->stream>>>(A + k0, lda, M, kc, p, Al, (size_t)Kp, (size_t)M * Kp,
+                                             0, 1);
       split_cols_kernel<L, E><<<split_cols_grid<E>(N, Kp), 256, 0, c->stream>>>(
-          B + (size_t)k0 * ldb, ldb, kc, N, p, Bl, Kp);
+          B + (size_t)k0 * ldb, ldb, kc, N, p, Bl, (size_t)Kp, (size_t)N * Kp, Kp);
       prof_end(c, pi);
       ctx_launched(c, 2);
     }
@@ -1318,6 +1319,81 @@ int zp_gemm_tc_elem_dev(Ctx *c, int elem, int M, int N, int K, uint32_t p, uint3
 #undef LELA_ELEM
 }
 
+// ------------------------------------------------- limb planes kept by callers
+template <int L, int T>
+static int launch_planes(Ctx *c, int M, int N, int K, const Modulus &mod, uint32_t alpha,
+                         const ZpPlanes &A, const ZpPlanes &B, uint32_t beta, uint32_t *C,
+                         size_t ldc, const int2 *kr, int kbase) {
+  using Cfg = TcCfg<L, T>;
+  if (int st = tc_attr<L, T>(c)) return st;
+  const int tiles = ((M + BM - 1) / BM) * ((N + Cfg::BN - 1) / Cfg::BN);
+  uint32_t b = beta;
+  for (int k0 = 0; k0 < K; k0 += ZP_KCHUNK) {
+    const int kc = std::min(ZP_KCHUNK, K - k0);
+    CUtensorMap tmA, tmB;
+    int st = encode_3d(c, &tmA, A.base + k0, (uint64_t)kc, (uint64_t)M, L, A.pitch, A.plane, BK, BM, L);
+    if (!st) st = encode_3d(c, &tmB, B.base + k0, (uint64_t)kc, (uint64_t)N, L, B.pitch, B.plane, BK,
+                            Cfg::BN, L);
+    if (st) return st;
+    int pi = prof_begin(c, "zp_gemm_tc");
+    zp_gemm_tc_kernel<L, 0, T><<<std::min(tiles, c->num_sms), tc_threads<L, T>(),
+                                 TcLayout<L, T>::SMEM, c->stream>>>(
+        tmA, tmB, C, ldc, M, N, kc, mod, alpha, b, c->dstatus, kr, kbase + k0);
+    prof_end(c, pi);
+    ctx_launched(c);
+    b = 1;
+  }
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? ST_OK : ctx_cuda(c, e, "zp_gemm_tc launch");
+}
+
+int zp_gemm_planes_dev(Ctx *c, int M, int N, int K, uint32_t p, uint32_t alpha, const ZpPlanes &A,
+                       const ZpPlanes &B, uint32_t beta, uint32_t *C, size_t ldc, const int2 *kr,
+                       int kbase) {
+  const Modulus mod = make_modulus(p);
+  const int tv = zp_gemm_tile_pick(c, M, N, K, p);
+#define LELA_PL(L, T) launch_planes<L, T>(c, M, N, K, mod, alpha, A, B, beta, C, ldc, kr, kbase)
+  switch (zp_limbs_for(p)) {
+    case 1: return tv == 0 ? LELA_PL(1, 0) : tv == 1 ? LELA_PL(1, 1) : LELA_PL(1, 2);
+    case 2: return tv == 0 ? LELA_PL(2, 0) : LELA_PL(2, 1);
+    default: return LELA_PL(4, 0);
+  }
+#undef LELA_PL
+}
+
+int zp_split_rows_dev(Ctx *c, uint32_t p, const uint32_t *A, size_t lda, int M, int K,
+                      const ZpPlanes &out, int part, int nb) {
+  const dim3 grid = split_rows_grid(c->num_sms, M, K), block(32, SPLIT_ROWS);
+#define LELA_SR(L) \
+  split_rows_kernel<L, uint32_t><<<grid, block, 0, c->stream>>>(A, lda, M, K, p, out.base, out.pitch, out.plane, part, nb)
+  switch (zp_limbs_for(p)) {
+    case 1: LELA_SR(1); break;
+    case 2: LELA_SR(2); break;
+    default: LELA_SR(4); break;
+  }
+#undef LELA_SR
+  ctx_launched(c);
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? ST_OK : ctx_cuda(c, e, "zp_split launch");
+}
+
+int zp_split_cols_dev(Ctx *c, uint32_t p, const uint32_t *B, size_t ldb, int K, int N,
+                      const ZpPlanes &out) {
+  const int kout = (K + 15) & ~15;
+  const dim3 grid = split_cols_grid<uint32_t>(N, kout);
+#define LELA_SC(L) \
+  split_cols_kernel<L, uint32_t><<<grid, 256, 0, c->stream>>>(B, ldb, K, N, p, out.base, out.pitch, out.plane, kout)
+  switch (zp_limbs_for(p)) {
+    case 1: LELA_SC(1); break;
+    case 2: LELA_SC(2); break;
+    default: LELA_SC(4); break;
+  }
+#undef LELA_SC
+  ctx_launched(c);
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? ST_OK : ctx_cuda(c, e, "zp_split launch");
+}
+
 // ============================================ pipelined host-pointer gemm
 //
 // The host-pointer gemm moves (M K + K N + 2 M N) * 4 bytes over the host
@@ -1379,7 +1455,7 @@ static int host_rows(Ctx *c, int M, int N, int K, const Modulus &mod, uint32_t a
   if (e == cudaSuccess) {
     int pi = prof_begin(c, "zp_split");
     split_cols_kernel<L, uint32_t><<<split_cols_grid<uint32_t>(N, Kp), 256, 0, c->stream>>>(
-        dB, (size_t)N, K, N, (uint32_t)mod.p, Bl, Kp);
+        dB, (size_t)N, K, N, (uint32_t)mod.p, Bl, (size_t)Kp, (size_t)N * Kp, Kp);
     prof_end(c, pi);
     ctx_launched(c);
     e = cudaGetLastError();
@@ -1395,7 +1471,8 @@ static int host_rows(Ctx *c, int M, int N, int K, const Modulus &mod, uint32_t a
     int pi = prof_begin(c, "zp_split");
     split_rows_kernel<L, uint32_t><<<split_rows_grid(c->num_sms, rows, K), dim3(32, SPLIT_ROWS), 0,
                                      c->stream>>>(dA + (size_t)r0 * K, (size_t)K, rows, K,
-                                                  (uint32_t)mod.p, Al, Kp);
+                                                  (uint32_t)mod.p, Al, (size_t)Kp,
+                                                  (size_t)rows * Kp, 0, 1);
     prof_end(c, pi);
     CUtensorMap tmA;
     st = encode_3d(c, &tmA, Al, (uint64_t)K, (uint64_t)rows, L, (uint64_t)Kp,
@@ -1566,9 +1643,9 @@ int noalloc_launch(cudaStream_t s, const NoallocDevice &d, int M, int N, int K,
     uint8_t *Bl = planes + (size_t)L * M * Kp;
     const uint32_t p = (uint32_t)mod.p;
     split_rows_kernel<L, uint32_t><<<split_rows_grid(d.num_sms, M, kc), dim3(32, SPLIT_ROWS), 0, s>>>(
-        A + k0, lda, M, kc, p, Al, Kp);
+        A + k0, lda, M, kc, p, Al, (size_t)Kp, (size_t)M * Kp, 0, 1);
     split_cols_kernel<L, uint32_t><<<split_cols_grid<uint32_t>(N, Kp), 256, 0, s>>>(
-        B + (size_t)k0 * ldb, ldb, kc, N, p, Bl, Kp);
+        B + (size_t)k0 * ldb, ldb, kc, N, p, Bl, (size_t)Kp, (size_t)N * Kp, Kp);
     CUtensorMap tmA, tmB;
     if (!noalloc_map(&tmA, Al, (uint64_t)kc, (uint64_t)M, L, (uint64_t)Kp, (uint64_t)M * Kp,
                      BK, BM, L) ||

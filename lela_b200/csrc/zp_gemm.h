@@ -48,6 +48,27 @@ int zp_gemm_pick(const Ctx *c, int M, int N, int K, uint32_t p);
 // number of epilogue warps of the double-buffered tiles follows K.
 int zp_gemm_tile_pick(const Ctx *c, int M, int N, int K, uint32_t p);
 
+// Limb planes a caller keeps: L = zp_limbs_for(p) planes `plane` bytes apart,
+// rows of bytes `pitch` apart (pitch and the addresses used multiples of 16),
+// K along a row: a row of A, or a column of B.
+struct ZpPlanes {
+  uint8_t *base;
+  size_t pitch, plane;
+  ZpPlanes at(size_t row, size_t k) const { return {base + row * pitch + k, pitch, plane}; }
+};
+// The planes of the M x K matrix A (part 1 / 2: only the columns left / right of each
+// row's diagonal block of nb rows), or of the K x N matrix B (its row K up to a
+// multiple of 16, zero there).
+int zp_split_rows_dev(Ctx *c, uint32_t p, const uint32_t *A, size_t lda, int M, int K,
+                      const ZpPlanes &out, int part, int nb);
+int zp_split_cols_dev(Ctx *c, uint32_t p, const uint32_t *B, size_t ldb, int K, int N,
+                      const ZpPlanes &out);
+// C <- alpha*A*B + beta*C on the tensor cores from planes (K > 0; kr, kbase
+// as zp_gemm_dev).
+int zp_gemm_planes_dev(Ctx *c, int M, int N, int K, uint32_t p, uint32_t alpha, const ZpPlanes &A,
+                       const ZpPlanes &B, uint32_t beta, uint32_t *C, size_t ldc,
+                       const int2 *kr = nullptr, int kbase = 0);
+
 // Whether the host-pointer gemm of this shape is done in row blocks with
 // its copies overlapped (tensor-core path, one K chunk, at least two blocks
 // of PIPE_MIN_ROWS rows).
