@@ -649,7 +649,7 @@ int lela_cuda_echelon_zp_u32_batch(lela_cuda_ctx *h, size_t count, uint32_t *con
     for (size_t j = next++; j < order.size() && !fatal.load(); j = next++) {
       const size_t i = order[j];
       const int k = kernel ? kernel[i] : 0;
-      wc->gemm_kernel = (k == 3) ? GEMM_PLAIN : GEMM_TC;
+      wc->gemm_kernel = (k == 3) ? GEMM_PLAIN : (k == 0 ? GEMM_AUTO : GEMM_TC);
       wc->gemm_tile = (k == 4) ? GEMM_TILE_DOUBLE : (k == 2 ? GEMM_TILE_WIDE : GEMM_TILE_AUTO);
       size_t r = 0;
       uint32_t d = 1;

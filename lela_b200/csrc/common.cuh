@@ -205,6 +205,47 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, uint32_t by
                : "memory");
 }
 
+// ------------------------------------------- programmatic dependent launch
+//
+// pdl_launch queues a kernel that may begin while the kernel before it on the
+// stream still runs; pdl_enter, which every kernel launched so calls before
+// it reads or writes global memory that another kernel writes or reads, lets
+// the next kernel begin and then waits until all kernels before this one have
+// ended and their memory is visible.  Launch latency, block start-up, barrier
+// and TMEM set-up and the first instruction fetches of a kernel then overlap
+// its predecessor's end.  A kernel that allocates TMEM calls pdl_enter after
+// the allocation: the next kernel's blocks start once all blocks of this one
+// have called it, so none of this kernel's allocations can wait for columns
+// held by a block that waits for this kernel.  Such a kernel must not read by
+// the non-coherent path what an earlier kernel on the stream may have written
+// (no __ldg, no const __restrict__ parameters): it began before that kernel
+// ended, and its SM's L1 may hold lines from before.
+__device__ __forceinline__ void pdl_enter() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// (early = false: an ordinary launch.)
+template <class... P, class... A>
+inline cudaError_t pdl_launch_if(bool early, void (*kernel)(P...), dim3 grid, dim3 block,
+                                 size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+template <class... P, class... A>
+inline cudaError_t pdl_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                              cudaStream_t stream, A... args) {
+  return pdl_launch_if(true, kernel, grid, block, smem, stream, args...);
+}
+
 // ------------------------------------------------------------------ TMA
 // 3-D tiled bulk tensor load global -> shared of this CTA only, completion
 // counted on an mbarrier.

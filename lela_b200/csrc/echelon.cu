@@ -110,9 +110,10 @@ __device__ __forceinline__ int row_at(int pos, const int *p2r, const int *stamp,
 // the caller has set to -1).
 constexpr int HEADS_THREADS = 256;
 __global__ void __launch_bounds__(HEADS_THREADS)
-    panel_heads_kernel(const uint32_t *__restrict__ D, size_t ld, int i0, int m, int c0, int w,
-                       uint8_t *__restrict__ head, uint8_t *__restrict__ act, int *hist,
+    panel_heads_kernel(const uint32_t *D, size_t ld, int i0, int m, int c0, int w,
+                       uint8_t *head, uint8_t *act, int *hist,
                        int *last) {
+  pdl_enter();
   __shared__ int s_last;
   __shared__ int s_hist[EW + 1];
   if (threadIdx.x == 0) s_last = -1;
@@ -371,12 +372,12 @@ constexpr int PW_U = 4;
 
 template <class SA, class A>
 __global__ void __launch_bounds__(PS_THREADS, 1)
-    panel_search_kernel(const uint32_t *__restrict__ D, size_t ld, int i0, int m, int c0, int w,
-                        SA sa, A ar, uint8_t *__restrict__ head, const uint8_t *__restrict__ act,
-                        int *__restrict__ hist, int *__restrict__ last_act, int *__restrict__ p2r,
-                        int *__restrict__ stamp, int epoch, uint32_t *__restrict__ Uout,
-                        uint32_t *__restrict__ xinv_out, uint32_t *__restrict__ Uinv_out,
-                        uint32_t *__restrict__ Linv_out, PanelOut *out, volatile uint64_t *hout, uint32_t seq, int wcap) {
+    panel_search_kernel(const uint32_t *D, size_t ld, int i0, int m, int c0, int w,
+                        SA sa, A ar, uint8_t *head, const uint8_t *act,
+                        int *hist, int *last_act, int *p2r,
+                        int *stamp, int epoch, uint32_t *Uout,
+                        uint32_t *xinv_out, uint32_t *Uinv_out,
+                        uint32_t *Linv_out, PanelOut *out, volatile uint64_t *hout, uint32_t seq, int wcap) {
   using V = typename SA::V;
   using V4 = typename SA::V4;
   extern __shared__ __align__(16) uint32_t dyn_w[];
@@ -415,6 +416,8 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
     for (int e = tid; e < (int)(p / 2 + 1 + 7) / 8; e += PS_THREADS)
       cp_async16(dst + 16 * e, reinterpret_cast<const char *>(sa.table) + 16 * e);
   }
+  // (the table was complete before the memsets that precede the first panel)
+  pdl_enter();
   // the window: ordered compaction of the rows with a nonzero panel
   int nl = 0;
   if (tid == 0) {
@@ -1121,8 +1124,9 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
 constexpr int PERM_THREADS = 256, PERM_COLS = 32;
 constexpr int PERM_PER = 2 * EW * PERM_COLS / PERM_THREADS;
 __global__ void __launch_bounds__(PERM_THREADS)
-    permute_rows_kernel(uint32_t *__restrict__ D, size_t ld, int n, const int *__restrict__ src,
-                        const int *__restrict__ dst, int cnt) {
+    permute_rows_kernel(uint32_t *D, size_t ld, int n, const int *src,
+                        const int *dst, int cnt) {
+  pdl_enter();
   const int c0 = blockIdx.x * PERM_COLS, total = cnt * PERM_COLS;
   uint32_t v[PERM_PER];
 #pragma unroll
@@ -1205,10 +1209,11 @@ __global__ void __launch_bounds__(SOLVE_THREADS)
 // it, or was zero at and below the pivot row when it was reached).
 template <class A>
 __global__ void __launch_bounds__(SOLVE_THREADS)
-    panel_solve_inv_kernel(uint32_t *__restrict__ D, size_t ld, int i0, int r1, int c0, int w,
-                           int t, const uint32_t *__restrict__ pcol,
-                           const uint32_t *__restrict__ Uin, const uint32_t *__restrict__ Uinv,
-                           A ar, uint32_t *__restrict__ Lout, size_t ldl) {
+    panel_solve_inv_kernel(uint32_t *D, size_t ld, int i0, int r1, int c0, int w,
+                           int t, const uint32_t *pcol,
+                           const uint32_t *Uin, const uint32_t *Uinv,
+                           A ar, uint32_t *Lout, size_t ldl) {
+  pdl_enter();
   __shared__ uint32_t sUi[EW][EW];
   __shared__ int sP[EW];
   const int tid = threadIdx.x, lane = tid & 31;
@@ -1439,7 +1444,8 @@ int zp_echelon_dev(Ctx *c, int m, int n, uint32_t p, uint32_t *D, size_t ld, siz
     const size_t smem = PW_SMEM + (decltype(sa)::NORM ? PW_TABLE : 0);
     int s = ctx_smem_attr(c, (const void *)kern, (int)smem, "echelon: panel search attributes");
     if (s) return s;
-    kern<<<1, PS_THREADS, smem, c->stream>>>(D, ld, i, m, c0, w, sa, ar, d_head, d_act, d_hist,
+    pdl_launch(kern, 1, PS_THREADS, smem, c->stream,
+      D, ld, i, m, c0, w, sa, ar, d_head, d_act, d_hist,
                                                 d_last, d_p2r, d_stamp, epoch, d_U, d_xinv, d_Uinv,
                                                 d_Linv, d_out, hwords_dev, seq, wcap);
     return ST_OK;
@@ -1460,7 +1466,8 @@ int zp_echelon_dev(Ctx *c, int m, int n, uint32_t p, uint32_t *D, size_t ld, siz
       delayed = -1;  // decided at the block's first panel with pivots
     }
     int pi = prof_begin(c, "ech_heads");
-    panel_heads_kernel<<<head_grid, HEADS_THREADS, 0, c->stream>>>(D, ld, i, m, c0, w, d_head,
+    pdl_launch(panel_heads_kernel, head_grid, HEADS_THREADS, 0, c->stream,
+      D, ld, i, m, c0, w, d_head,
                                                                     d_act, d_hist, d_last);
     prof_end(c, pi);
     const uint32_t seq = ++c->panel_seq;
@@ -1520,17 +1527,17 @@ int zp_echelon_dev(Ctx *c, int m, int n, uint32_t p, uint32_t *D, size_t ld, siz
       e = cudaMemcpyAsync(d_perm, hperm, (size_t)2 * cnt * sizeof(int), cudaMemcpyHostToDevice,
                           c->stream);
       if (e != cudaSuccess) return ctx_cuda(c, e, "echelon: permutation");
-      permute_rows_kernel<<<(n + PERM_COLS - 1) / PERM_COLS, PERM_THREADS, 0, c->stream>>>(
+      pdl_launch(permute_rows_kernel, (n + PERM_COLS - 1) / PERM_COLS, PERM_THREADS, 0, c->stream,
           D, ld, n, d_perm, d_perm + cnt, cnt);
       ctx_launched(c);
       if (Tb > 0) {  // the multipliers of the block's earlier panels move too
-        permute_rows_kernel<<<(EB + PERM_COLS - 1) / PERM_COLS, PERM_THREADS, 0, c->stream>>>(
+        pdl_launch(permute_rows_kernel, (EB + PERM_COLS - 1) / PERM_COLS, PERM_THREADS, 0, c->stream,
             d_L, EB, EB, d_perm, d_perm + cnt, cnt);
         ctx_launched(c);
       }
       if (keep && rank > 0) {  // and every earlier pivot's kept multipliers
-        permute_rows_kernel<<<((int)rank + PERM_COLS - 1) / PERM_COLS, PERM_THREADS, 0,
-                              c->stream>>>(keep->L, keep->ldL, (int)rank, d_perm, d_perm + cnt,
+        pdl_launch(permute_rows_kernel, ((int)rank + PERM_COLS - 1) / PERM_COLS, PERM_THREADS, 0, c->stream,
+      keep->L, keep->ldL, (int)rank, d_perm, d_perm + cnt,
                                            cnt);
         ctx_launched(c);
       }
@@ -1555,10 +1562,10 @@ int zp_echelon_dev(Ctx *c, int m, int n, uint32_t p, uint32_t *D, size_t ld, siz
       // U_P^-1 when the search wrote it (p < 2^31: exact pivot inverses), else
       // the elimination steps
       if (h.uinv && small)
-        panel_solve_inv_kernel<<<sgrid, SOLVE_THREADS, 0, c->stream>>>(
+        pdl_launch(panel_solve_inv_kernel<ArithSmall>, sgrid, SOLVE_THREADS, 0, c->stream,
             D, ld, i, r1, c0, w, t, d_pcol, d_U, d_Uinv, ars, Lp, EB);
       else if (h.uinv)
-        panel_solve_inv_kernel<<<sgrid, SOLVE_THREADS, 0, c->stream>>>(
+        pdl_launch(panel_solve_inv_kernel<ArithWide>, sgrid, SOLVE_THREADS, 0, c->stream,
             D, ld, i, r1, c0, w, t, d_pcol, d_U, d_Uinv, arw, Lp, EB);
       else
         panel_solve_kernel<<<sgrid, SOLVE_THREADS, 0, c->stream>>>(D, ld, i, r1, c0, w, t, d_pcol,

@@ -46,9 +46,10 @@ constexpr int M4_KC = 32;     // rows of B per table round (4 tables of 8)
 // T[g][w][s] in shared memory.
 template <int M4_ROWS, int M4_BW>
 __global__ void __launch_bounds__(M4_THREADS)
-    gf2_m4rm_kernel(const uint64_t *__restrict__ A, size_t lda, const uint64_t *__restrict__ B,
-                    size_t ldb, uint64_t *__restrict__ C, size_t ldc, int M, int Nw, int K,
+    gf2_m4rm_kernel(const uint64_t *A, size_t lda, const uint64_t *B,
+                    size_t ldb, uint64_t *C, size_t ldc, int M, int Nw, int K,
                     uint64_t tail_mask, int alpha, int beta) {
+  pdl_enter();
   extern __shared__ uint64_t m4_smem[];
   uint64_t(*T)[M4_BW][256] = reinterpret_cast<uint64_t(*)[M4_BW][256]>(m4_smem);
   uint64_t(*Bk)[M4_BW] = reinterpret_cast<uint64_t(*)[M4_BW]>(m4_smem + 4 * M4_BW * 256);
@@ -136,13 +137,13 @@ int gf2_m4rm_dev(Ctx *c, int M, int N, int K, int alpha, const uint64_t *A, size
   const int gy4 = (M + M4_THREADS * 4 - 1) / (M4_THREADS * 4), gy1 = (M + M4_THREADS - 1) / M4_THREADS;
   int pi = prof_begin(c, "gf2_m4rm");
   if ((size_t)gx8 * gy4 >= enough)
-    gf2_m4rm_kernel<4, 8><<<dim3(gx8, gy4), M4_THREADS, smem_for(8), c->stream>>>(
+    pdl_launch(gf2_m4rm_kernel<4, 8>, dim3(gx8, gy4), M4_THREADS, smem_for(8), c->stream,
         A, lda, B, ldb, C, ldc, M, Nw, K, tail, alpha, beta);
   else if ((size_t)gx8 * gy1 >= enough)
-    gf2_m4rm_kernel<1, 8><<<dim3(gx8, gy1), M4_THREADS, smem_for(8), c->stream>>>(
+    pdl_launch(gf2_m4rm_kernel<1, 8>, dim3(gx8, gy1), M4_THREADS, smem_for(8), c->stream,
         A, lda, B, ldb, C, ldc, M, Nw, K, tail, alpha, beta);
   else
-    gf2_m4rm_kernel<1, 2><<<dim3(gx2, gy1), M4_THREADS, smem_for(2), c->stream>>>(
+    pdl_launch(gf2_m4rm_kernel<1, 2>, dim3(gx2, gy1), M4_THREADS, smem_for(2), c->stream,
         A, lda, B, ldb, C, ldc, M, Nw, K, tail, alpha, beta);
   prof_end(c, pi);
   ctx_launched(c);
@@ -167,14 +168,15 @@ __device__ __forceinline__ uint4 spread16(uint32_t h) {
 // four bytes a thread and an index division took 209 us).
 constexpr int UNPACK_ROWS = 8;  // rows (warps) per CTA
 __global__ void __launch_bounds__(32 * UNPACK_ROWS)
-    gf2_unpack_rows_kernel(const uint64_t *__restrict__ A, size_t lda, int M, int k0,
-                           uint8_t *__restrict__ out, int Kp) {
+    gf2_unpack_rows_kernel(const uint64_t *A, size_t lda, int M, int k0,
+                           uint8_t *out, int Kp) {
+  pdl_enter();
   const int per = Kp / 16;
   for (int r = blockIdx.y * UNPACK_ROWS + threadIdx.y; r < M; r += gridDim.y * UNPACK_ROWS) {
     const uint16_t *src = reinterpret_cast<const uint16_t *>(A + (size_t)r * lda + (k0 >> 6));
     uint4 *dst = reinterpret_cast<uint4 *>(out + (size_t)r * Kp);
     for (int q = blockIdx.x * 32 + threadIdx.x; q < per; q += gridDim.x * 32)
-      dst[q] = spread16(__ldg(src + q));
+      dst[q] = spread16(src[q]);
   }
 }
 
@@ -200,8 +202,9 @@ __device__ __forceinline__ uint32_t transpose32(uint32_t x, int lane) {
   return x;
 }
 __global__ void __launch_bounds__(32 * UNPACK_WARPS)
-    gf2_unpack_cols_kernel(const uint64_t *__restrict__ B, size_t ldb, int k0, int kc, int N,
-                           uint8_t *__restrict__ out, int Kp) {
+    gf2_unpack_cols_kernel(const uint64_t *B, size_t ldb, int k0, int kc, int N,
+                           uint8_t *out, int Kp) {
+  pdl_enter();
   __shared__ uint32_t bits[64 * UNPACK_W][UNPACK_K / 32 + 1];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int w0 = blockIdx.x * UNPACK_W, kb0 = blockIdx.y * UNPACK_K;
@@ -211,7 +214,7 @@ __global__ void __launch_bounds__(32 * UNPACK_WARPS)
     const uint64_t *src = B + (size_t)(k0 + k) * ldb + w0;
     uint64_t v[UNPACK_W];
 #pragma unroll
-    for (int j = 0; j < UNPACK_W; ++j) v[j] = k < kc && j < words ? __ldg(src + j) : 0ull;
+    for (int j = 0; j < UNPACK_W; ++j) v[j] = k < kc && j < words ? src[j] : 0ull;
 #pragma unroll
     for (int j = 0; j < UNPACK_W; ++j) {
       bits[64 * j + lane][u] = transpose32((uint32_t)v[j], lane);
@@ -233,14 +236,15 @@ static void unpack_rows(Ctx *c, const uint64_t *A, size_t lda, int M, int k0, ui
   // one pass a warp up to 16 CTAs an SM, then more
   const int gy = std::min((M + UNPACK_ROWS - 1) / UNPACK_ROWS, c->num_sms * 16);
   const int gx = std::max(1, std::min((Kp / 16 + 31) / 32, c->num_sms * 16 / gy));
-  gf2_unpack_rows_kernel<<<dim3(gx, gy), dim3(32, UNPACK_ROWS), 0, c->stream>>>(A, lda, M, k0, out, Kp);
+  pdl_launch(gf2_unpack_rows_kernel, dim3(gx, gy), dim3(32, UNPACK_ROWS), 0, c->stream,
+      A, lda, M, k0, out, Kp);
   ctx_launched(c);
 }
 static void unpack_cols(Ctx *c, const uint64_t *B, size_t ldb, int k0, int kc, int N, uint8_t *out,
                         int Kp) {
   const int Nw = (N + 63) / 64;
-  gf2_unpack_cols_kernel<<<dim3((Nw + UNPACK_W - 1) / UNPACK_W, (Kp + UNPACK_K - 1) / UNPACK_K),
-                           32 * UNPACK_WARPS, 0, c->stream>>>(B, ldb, k0, kc, N, out, Kp);
+  pdl_launch(gf2_unpack_cols_kernel, dim3((Nw + UNPACK_W - 1) / UNPACK_W, (Kp + UNPACK_K - 1) / UNPACK_K), 32 * UNPACK_WARPS, 0, c->stream,
+      B, ldb, k0, kc, N, out, Kp);
   ctx_launched(c);
 }
 
@@ -396,9 +400,10 @@ constexpr int GF2_HEADS_THREADS = 256;
 // hist counts only the rows from position hist0 on (those the search reads
 // lazily, past its register window).
 __global__ void __launch_bounds__(GF2_HEADS_THREADS)
-    gf2_heads_kernel(const uint64_t *__restrict__ D, size_t ld, int i0, int m, int wc,
-                     uint64_t pmask, uint8_t *__restrict__ head, uint8_t *__restrict__ act,
+    gf2_heads_kernel(const uint64_t *D, size_t ld, int i0, int m, int wc,
+                     uint64_t pmask, uint8_t *head, uint8_t *act,
                      int *hist, int *last, int hist0) {
+  pdl_enter();
   __shared__ int s_last;
   __shared__ int s_hist[GW + 1];
   if (threadIdx.x == 0) s_last = -1;
@@ -438,12 +443,13 @@ __global__ void __launch_bounds__(GF2_HEADS_THREADS)
 constexpr int GF2_WR = 128;               // window positions (registers)
 constexpr int GF2_WU = GF2_WR / 32;       // per lane
 __global__ void __launch_bounds__(32)
-    gf2_search_kernel(const uint64_t *__restrict__ D, size_t ld, int i0, int m, int wc, int w,
-                      uint64_t pmask, uint8_t *__restrict__ head, const uint8_t *__restrict__ act,
-                      int *__restrict__ hist, int *__restrict__ last_act, int *__restrict__ p2r,
-                      int *__restrict__ stamp, int epoch, uint64_t *__restrict__ Uout,
+    gf2_search_kernel(const uint64_t *D, size_t ld, int i0, int m, int wc, int w,
+                      uint64_t pmask, uint8_t *head, const uint8_t *act,
+                      int *hist, int *last_act, int *p2r,
+                      int *stamp, int epoch, uint64_t *Uout,
                       Gf2PanelOut *out, Gf2PanelOut *hout, volatile uint32_t *hflag,
                       uint32_t seq) {
+  pdl_enter();
   __shared__ uint64_t G[GW], M[GW], s_U[GW];
   __shared__ int s_pcol[GW], s_ti[GW], s_tq[GW];
   __shared__ int s_cnt[GW + 1];
@@ -665,10 +671,11 @@ __global__ void __launch_bounds__(32)
 // on the panel word give the multipliers (L11 row of pivot row k over the
 // pivots before it; L21 row of the rows below over all t) and the final
 // word (U_k; zero below).  One thread per row.
-__global__ void gf2_solve_kernel(uint64_t *__restrict__ D, size_t ld, int i0, int r1, int wc,
-                                 uint64_t pmask, int t, const uint32_t *__restrict__ pcol,
-                                 const uint64_t *__restrict__ Uin, uint64_t *__restrict__ L11,
-                                 uint64_t *__restrict__ L21) {
+__global__ void gf2_solve_kernel(uint64_t *D, size_t ld, int i0, int r1, int wc,
+                                 uint64_t pmask, int t, const uint32_t *pcol,
+                                 const uint64_t *Uin, uint64_t *L11,
+                                 uint64_t *L21) {
+  pdl_enter();
   __shared__ uint64_t sU[GW];
   __shared__ int sP[GW];
   if (threadIdx.x < GW) {
@@ -704,8 +711,9 @@ __global__ void gf2_solve_kernel(uint64_t *__restrict__ D, size_t ld, int i0, in
 constexpr int GF2_PERM_THREADS = 256, GF2_PERM_WORDS = 16;
 constexpr int GF2_PERM_PER = 2 * GW * GF2_PERM_WORDS / GF2_PERM_THREADS;
 __global__ void __launch_bounds__(GF2_PERM_THREADS)
-    gf2_permute_rows_kernel(uint64_t *__restrict__ D, size_t ld, int nw,
-                            const int *__restrict__ src, const int *__restrict__ dst, int cnt) {
+    gf2_permute_rows_kernel(uint64_t *D, size_t ld, int nw,
+                            const int *src, const int *dst, int cnt) {
+  pdl_enter();
   const int w0 = blockIdx.x * GF2_PERM_WORDS, total = cnt * GF2_PERM_WORDS;
   uint64_t v[GF2_PERM_PER];
 #pragma unroll
@@ -729,8 +737,9 @@ __global__ void __launch_bounds__(GF2_PERM_THREADS)
 // instead of a thread's 2016 dependent XORs).
 constexpr int GF2_L11_THREADS = 256;
 __global__ void __launch_bounds__(GF2_L11_THREADS)
-    gf2_l11_solve_kernel(uint64_t *__restrict__ D, size_t ld, int i0, int t, int w1, int nw,
-                         const uint64_t *__restrict__ L11) {
+    gf2_l11_solve_kernel(uint64_t *D, size_t ld, int i0, int t, int w1, int nw,
+                         const uint64_t *L11) {
+  pdl_enter();
   const int lane = threadIdx.x & 31;
   const int w = w1 + (int)((blockIdx.x * (size_t)GF2_L11_THREADS + threadIdx.x) >> 5);
   if (w >= nw) return;  // whole warps
@@ -750,9 +759,10 @@ __global__ void __launch_bounds__(GF2_L11_THREADS)
 // t bits of L11 (pivot rows) or L21 (rows below) at bit offset off of the
 // row's GB words (the caller zeroed the block's rows).
 constexpr int GB = 8;  // panels (words) per block of delayed updates
-__global__ void gf2_deposit_kernel(uint64_t *__restrict__ Lb, int i0, int r1, int t, int off,
-                                   const uint64_t *__restrict__ L11,
-                                   const uint64_t *__restrict__ L21) {
+__global__ void gf2_deposit_kernel(uint64_t *Lb, int i0, int r1, int t, int off,
+                                   const uint64_t *L11,
+                                   const uint64_t *L21) {
+  pdl_enter();
   const int r0 = i0 + t;
   for (int pos = i0 + blockIdx.x * blockDim.x + threadIdx.x; pos <= r1;
        pos += gridDim.x * blockDim.x) {
@@ -842,8 +852,8 @@ int gf2_echelon_dev(Ctx *c, int m, int n, uint64_t *D, size_t ld, size_t *rank_o
                              D + (size_t)pan_i[j] * ld + bw1, ld);
         if (s) return s;
       }
-      gf2_l11_solve_kernel<<<(nw - bw1 + GF2_L11_THREADS / 32 - 1) / (GF2_L11_THREADS / 32),
-                             GF2_L11_THREADS, 0, c->stream>>>(D, ld, pan_i[j], pan_t[j], bw1, nw,
+      pdl_launch(gf2_l11_solve_kernel, (nw - bw1 + GF2_L11_THREADS / 32 - 1) / (GF2_L11_THREADS / 32), GF2_L11_THREADS, 0, c->stream,
+      D, ld, pan_i[j], pan_t[j], bw1, nw,
                                                               d_L11s + (size_t)j * GW);
       ctx_launched(c);
     }
@@ -868,12 +878,12 @@ int gf2_echelon_dev(Ctx *c, int m, int n, uint64_t *D, size_t ld, size_t *rank_o
     }
     const uint64_t pmask = (w == 64) ? ~0ull : ((1ull << w) - 1ull);
     int pi = prof_begin(c, "gf2_heads");
-    gf2_heads_kernel<<<head_grid, GF2_HEADS_THREADS, 0, c->stream>>>(
+    pdl_launch(gf2_heads_kernel, head_grid, GF2_HEADS_THREADS, 0, c->stream,
         D, ld, i, m, wc, pmask, d_head, d_act, d_hist, d_last, i + GF2_WR);
     prof_end(c, pi);
     const uint32_t seq = ++c->panel_seq;
     pi = prof_begin(c, "gf2_search");
-    gf2_search_kernel<<<1, 32, 0, c->stream>>>(
+    pdl_launch(gf2_search_kernel, 1, 32, 0, c->stream,
         D, ld, i, m, wc, w, pmask, d_head, d_act, d_hist, d_last, d_p2r, d_stamp, epoch++, d_U,
         d_out, hmap_dev, hflag_dev, seq);
     prof_end(c, pi);
@@ -910,12 +920,12 @@ int gf2_echelon_dev(Ctx *c, int m, int n, uint64_t *D, size_t ld, size_t *rank_o
       e = cudaMemcpyAsync(d_perm, hperm, (size_t)2 * cnt * sizeof(int), cudaMemcpyHostToDevice,
                           c->stream);
       if (e != cudaSuccess) return ctx_cuda(c, e, "gf2 echelon: permutation");
-      gf2_permute_rows_kernel<<<(nw + GF2_PERM_WORDS - 1) / GF2_PERM_WORDS, GF2_PERM_THREADS, 0,
-                                c->stream>>>(D, ld, nw, d_perm, d_perm + cnt, cnt);
+      pdl_launch(gf2_permute_rows_kernel, (nw + GF2_PERM_WORDS - 1) / GF2_PERM_WORDS, GF2_PERM_THREADS, 0, c->stream,
+      D, ld, nw, d_perm, d_perm + cnt, cnt);
       ctx_launched(c);
       if (Tb > 0) {  // the block's earlier multipliers move with their rows
-        gf2_permute_rows_kernel<<<(GB + GF2_PERM_WORDS - 1) / GF2_PERM_WORDS, GF2_PERM_THREADS,
-                                  0, c->stream>>>(d_Lb, GB, GB, d_perm, d_perm + cnt, cnt);
+        pdl_launch(gf2_permute_rows_kernel, (GB + GF2_PERM_WORDS - 1) / GF2_PERM_WORDS, GF2_PERM_THREADS, 0, c->stream,
+      d_Lb, GB, GB, d_perm, d_perm + cnt, cnt);
         ctx_launched(c);
       }
     }
@@ -932,15 +942,15 @@ int gf2_echelon_dev(Ctx *c, int m, int n, uint64_t *D, size_t ld, size_t *rank_o
     {
       const int rows = r1 - i + 1;
       pi = prof_begin(c, "gf2_solve");
-      gf2_solve_kernel<<<std::max(1, std::min((rows + 255) / 256, c->num_sms * 4)), 256, 0,
-                         c->stream>>>(D, ld, i, r1, wc, pmask, t, d_pcol, d_U, d_L11, d_L21);
+      pdl_launch(gf2_solve_kernel, std::max(1, std::min((rows + 255) / 256, c->num_sms * 4)), 256, 0,
+                 c->stream, D, ld, i, r1, wc, pmask, t, d_pcol, d_U, d_L11, d_L21);
       prof_end(c, pi);
       ctx_launched(c);
     }
     if (delayed) {
       const int rows = r1 - i + 1;
-      gf2_deposit_kernel<<<std::max(1, std::min((rows + 255) / 256, c->num_sms * 4)), 256, 0,
-                           c->stream>>>(d_Lb, i, r1, t, Tb, d_L11, d_L21);
+      pdl_launch(gf2_deposit_kernel, std::max(1, std::min((rows + 255) / 256, c->num_sms * 4)), 256,
+                 0, c->stream, d_Lb, i, r1, t, Tb, d_L11, d_L21);
       e = cudaMemcpyAsync(d_L11s + (size_t)np * GW, d_L11, (size_t)t * 8, cudaMemcpyDeviceToDevice,
                           c->stream);
       if (e != cudaSuccess) return ctx_cuda(c, e, "gf2 echelon: panel multipliers");
@@ -949,8 +959,8 @@ int gf2_echelon_dev(Ctx *c, int m, int n, uint64_t *D, size_t ld, size_t *rank_o
     // the rest of the block's words (delayed), or of all words
     const int w1 = wc + 1, wend = delayed ? bw1 : nw;
     if (w1 < wend) {
-      gf2_l11_solve_kernel<<<(wend - w1 + GF2_L11_THREADS / 32 - 1) / (GF2_L11_THREADS / 32),
-                             GF2_L11_THREADS, 0, c->stream>>>(D, ld, i, t, w1, wend, d_L11);
+      pdl_launch(gf2_l11_solve_kernel, (wend - w1 + GF2_L11_THREADS / 32 - 1) / (GF2_L11_THREADS / 32), GF2_L11_THREADS, 0, c->stream,
+      D, ld, i, t, w1, wend, d_L11);
       ctx_launched(c);
       if (below > 0) {
         // rows r0..r1, those words: C ^= L21 (one word of t bits per row) * U12

@@ -93,9 +93,10 @@ __global__ void __launch_bounds__(256)
 // dependent steps, took 49 us a launch, 56 us for the upper).
 template <class A>
 __global__ void __launch_bounds__(INV_THREADS)
-    tri_inv_blocks_kernel(const uint32_t *__restrict__ M, size_t lda, int m, bool upper,
-                          const uint32_t *__restrict__ dinv, uint32_t *__restrict__ Tinv,
+    tri_inv_blocks_kernel(const uint32_t *M, size_t lda, int m, bool upper,
+                          const uint32_t *dinv, uint32_t *Tinv,
                           size_t ldo, int cmod, A ar) {
+  pdl_enter();
   __shared__ __align__(16) uint32_t X[INV_M], T[INV_T];
   const int r0 = blockIdx.x * TRI_NB, nb = min(TRI_NB, m - r0);
   const uint32_t *D = M + (size_t)r0 * lda + r0;
@@ -123,10 +124,12 @@ static void launch_inv_blocks(Ctx *c, bool upper, int m, const uint32_t *A, size
                               uint32_t p) {
   const int nblk = (m + TRI_NB - 1) / TRI_NB;
   if (p < (1u << 16))
-    tri_inv_blocks_kernel<<<nblk, INV_THREADS, 0, c->stream>>>(A, lda, m, upper, dinv, Tinv, ldo,
+    pdl_launch(tri_inv_blocks_kernel<ArithSmall>, nblk, INV_THREADS, 0, c->stream,
+      A, lda, m, upper, dinv, Tinv, ldo,
                                                                cmod, ArithSmall::make(p));
   else
-    tri_inv_blocks_kernel<<<nblk, INV_THREADS, 0, c->stream>>>(A, lda, m, upper, dinv, Tinv, ldo,
+    pdl_launch(tri_inv_blocks_kernel<ArithWide>, nblk, INV_THREADS, 0, c->stream,
+      A, lda, m, upper, dinv, Tinv, ldo,
                                                                cmod, ArithWide::make(p));
   ctx_launched(c);
 }
@@ -177,11 +180,12 @@ template <class A>
 __global__ void __launch_bounds__(256)
     tri_merge_kernel(MergeOp X, MergeOp Y, MergeOp Cop, int zbase, int M, int N, int K, int krange,
                      A ar, bool negate) {
+  pdl_enter();
   __shared__ __align__(16) uint32_t Xs[2][MG_T][MG_K + 4];
   __shared__ uint32_t Ys[2][MG_K][MG_T];
   const int z = zbase + blockIdx.z;
-  const uint32_t *__restrict__ Xp = X.at(z);
-  const uint32_t *__restrict__ Yp = Y.at(z);
+  const uint32_t *Xp = X.at(z);
+  const uint32_t *Yp = Y.at(z);
   uint32_t *Cp = const_cast<uint32_t *>(Cop.at(z));
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   const int lx = threadIdx.x & 31, ly = threadIdx.x >> 5;
@@ -581,9 +585,11 @@ static int tri_inverse_levels(Ctx *c, bool upper, int m, uint32_t p, const uint3
       const dim3 g1((N1 + MG_T - 1) / MG_T, (M1 + MG_T - 1) / MG_T, nz);
       const dim3 g2((N2 + MG_T - 1) / MG_T, (M2 + MG_T - 1) / MG_T, nz);
       auto merge = [&](auto ar) {
-        tri_merge_kernel<<<g1, 256, 0, c->stream>>>(X1, Y1, Tz, zbase, M1, N1, K1,
+        pdl_launch(tri_merge_kernel<decltype(ar)>, g1, 256, 0, c->stream,
+      X1, Y1, Tz, zbase, M1, N1, K1,
                                                     upper ? MG_TO_N : MG_FROM_N, ar, false);
-        tri_merge_kernel<<<g2, 256, 0, c->stream>>>(X2, Tz, C2, zbase, M2, N2, K2,
+        pdl_launch(tri_merge_kernel<decltype(ar)>, g2, 256, 0, c->stream,
+      X2, Tz, C2, zbase, M2, N2, K2,
                                                     upper ? MG_FROM_M : MG_TO_M, ar, true);
       };
       if (p < (1u << 16)) merge(ArithSmall::make(p));

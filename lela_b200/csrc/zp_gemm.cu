@@ -387,7 +387,7 @@ __device__ __forceinline__ void epilogue_gf2(uint32_t tcol, int gm, int gn0, int
 // ranges.  A tile whose rows are zero in all of K keeps one block: its
 // product is zero either way.  Warp-collective (the warp's lanes share the
 // rows), so every lane of the calling warp runs it.
-__device__ __forceinline__ void tile_kblocks(const int2 *__restrict__ kr, int kbase, int m0, int M,
+__device__ __forceinline__ void tile_kblocks(const int2 *kr, int kbase, int m0, int M,
                                              int K, int &kb0, int &kb1) {
   const int nkb = (K + BK - 1) / BK;
   kb0 = 0;
@@ -481,9 +481,9 @@ __device__ __noinline__ void epilogue_tiles(uint32_t tmem, uint64_t *tfull, uint
 template <int L, int OUT, int T = 0>
 __global__ void __launch_bounds__(tc_threads<L, T>(), 1)
     zp_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA,
-                      const __grid_constant__ CUtensorMap tmB, void *__restrict__ Cv,
+                      const __grid_constant__ CUtensorMap tmB, void *Cv,
                       size_t ldc, int M, int N, int K, Modulus mod, uint32_t alpha, uint32_t beta,
-                      uint32_t *err, const int2 *__restrict__ kr = nullptr, int kbase = 0) {
+                      uint32_t *err, const int2 *kr = nullptr, int kbase = 0) {
   static_assert(OUT == 0 || (L == 1 && (T == 0 || T == GF2_TC_T)), "GF(2) output uses one limb");
   uint32_t *C = static_cast<uint32_t *>(Cv);
   using Cfg = TcCfg<L, T>;
@@ -524,6 +524,7 @@ __global__ void __launch_bounds__(tc_threads<L, T>(), 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  pdl_enter();  // (after the TMEM allocation, see there)
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
@@ -715,8 +716,8 @@ __device__ __noinline__ void dir_epilogue(uint32_t tmem, uint64_t *done, uint32_
 
 template <int L>
 __global__ void __launch_bounds__(DIR_THREADS, L == 4 ? 1 : 2)
-    zp_gemm_direct_kernel(const uint32_t *__restrict__ A, size_t lda,
-                          const uint32_t *__restrict__ B, size_t ldb, uint32_t *C, size_t ldc,
+    zp_gemm_direct_kernel(const uint32_t *A, size_t lda,
+                          const uint32_t *B, size_t ldb, uint32_t *C, size_t ldc,
                           int M, int N, int K, int stages, Modulus mod, uint32_t alpha,
                           uint32_t beta, uint32_t *err) {
   using Cfg = DirCfg<L>;
@@ -740,6 +741,7 @@ __global__ void __launch_bounds__(DIR_THREADS, L == 4 ? 1 : 2)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  pdl_enter();  // (after the TMEM allocation, see there)
   const bool vecA = ((reinterpret_cast<uintptr_t>(A) & 15u) == 0) && ((lda & 3u) == 0);
   bool ok = true;
   int c = 0;
@@ -764,14 +766,14 @@ __global__ void __launch_bounds__(DIR_THREADS, L == 4 ? 1 : 2)
         const int gm = m0 + r0 + u;
         const uint32_t *src = A + (size_t)gm * lda + k0 + k;
         if (gm < M && vecA && k + 3 < kc) {
-          const uint4 x = __ldg(reinterpret_cast<const uint4 *>(src));
+          const uint4 x = *reinterpret_cast<const uint4 *>(src);
           v[u][0] = x.x;
           v[u][1] = x.y;
           v[u][2] = x.z;
           v[u][3] = x.w;
         } else {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) v[u][i] = (gm < M && k + i < kc) ? __ldg(src + i) : 0u;
+          for (int i = 0; i < 4; ++i) v[u][i] = (gm < M && k + i < kc) ? src[i] : 0u;
         }
       }
       if (k < kr)
@@ -791,7 +793,7 @@ __global__ void __launch_bounds__(DIR_THREADS, L == 4 ? 1 : 2)
         const int e = e0 + u, k = 4 * (e / BG), n = n0 + (e % BG) * 32 + lane;
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-          v[u][i] = (n < N && k + i < kc) ? __ldg(B + (size_t)(k0 + k + i) * ldb + n) : 0u;
+          v[u][i] = (n < N && k + i < kc) ? *(B + (size_t)(k0 + k + i) * ldb + n) : 0u;
       }
 #pragma unroll
       for (int u = 0; u < BU; ++u) {
@@ -847,23 +849,35 @@ __global__ void __launch_bounds__(DIR_THREADS, L == 4 ? 1 : 2)
 constexpr int SPLIT_ROWS = 8;  // rows (warps) per CTA
 template <int L, class T>
 __global__ void __launch_bounds__(32 * SPLIT_ROWS)
-    split_rows_kernel(const T *__restrict__ A, size_t lda, int M, int kc, uint32_t p,
-                      uint8_t *__restrict__ out, size_t Kp, size_t plane, int part, int nb) {
+    split_rows_kernel(const T *A, size_t lda, int M, int kc, uint32_t p,
+                      uint8_t *out, size_t Kp, size_t plane, int part, int nb) {
+  pdl_enter();
   for (int r = blockIdx.y * SPLIT_ROWS + threadIdx.y; r < M; r += gridDim.y * SPLIT_ROWS) {
     const T *src = A + (size_t)r * lda;
     uint8_t *dst = out + (size_t)r * Kp;
     const int kb = part == 2 ? min(kc, (r / nb + 1) * nb) : 0, ke = part == 1 ? min(kc, r / nb * nb) : kc;
-    for (int q = (kb >> 2) + blockIdx.x * 32 + threadIdx.x; 4 * q < ke; q += gridDim.x * 32) {
-      const int k = 4 * q;
-      uint32_t v[4];
+    constexpr int U = 2;  // groups in flight
+    const int step = gridDim.x * 32;
+    for (int q = (kb >> 2) + blockIdx.x * 32 + threadIdx.x; 4 * q < ke; q += U * step) {
+      uint32_t v[U][4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) v[i] = (k + i < kc) ? Rep<T>::in(__ldg(src + k + i), p) : 0u;
+      for (int u = 0; u < U; ++u)
 #pragma unroll
-      for (int l = 0; l < L; ++l) {
-        uint32_t w = 0;
+        for (int i = 0; i < 4; ++i) {
+          const int k = 4 * (q + u * step) + i;
+          v[u][i] = 4 * (q + u * step) < ke && k < kc ? Rep<T>::in(src[k], p) : 0u;
+        }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) w |= ((v[i] >> (8 * l)) & 0xFFu) << (8 * i);
-        *reinterpret_cast<uint32_t *>(dst + l * plane + k) = w;
+      for (int u = 0; u < U; ++u) {
+        const int k = 4 * (q + u * step);
+        if (k >= ke) break;
+#pragma unroll
+        for (int l = 0; l < L; ++l) {
+          uint32_t w = 0;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) w |= ((v[u][i] >> (8 * l)) & 0xFFu) << (8 * i);
+          *reinterpret_cast<uint32_t *>(dst + l * plane + k) = w;
+        }
       }
     }
   }
@@ -883,8 +897,9 @@ constexpr int split_cols_nt() {
 }
 template <int L, class T>
 __global__ void __launch_bounds__(256)
-    split_cols_kernel(const T *__restrict__ B, size_t ldb, int kc, int N, uint32_t p,
-                      uint8_t *__restrict__ out, size_t Kp, size_t plane, int kout) {
+    split_cols_kernel(const T *B, size_t ldb, int kc, int N, uint32_t p,
+                      uint8_t *out, size_t Kp, size_t plane, int kout) {
+  pdl_enter();
   using R = typename Rep<T>::Packed;
   constexpr int NT = split_cols_nt<T>();
   __shared__ R tile[64][NT + 4 / sizeof(R)];
@@ -897,7 +912,7 @@ __global__ void __launch_bounds__(256)
     for (int u = 0; u < NT / 32; ++u) {
       const int n = n0 + tx + 32 * u;
       tile[ty + 8 * i][tx + 32 * u] =
-          (k < kc && n < N) ? (R)Rep<T>::in(__ldg(B + (size_t)k * ldb + n), p) : (R)0;
+          (k < kc && n < N) ? (R)Rep<T>::in(*(B + (size_t)k * ldb + n), p) : (R)0;
     }
   }
   __syncthreads();
@@ -1115,6 +1130,9 @@ static int launch_tc(Ctx *c, int M, int N, int K, const Modulus &mod, uint32_t a
   using Lay = TcLayout<L, T>;
   if (int st = tc_attr<L, T>(c)) return st;
   const int tiles = ((M + BM - 1) / BM) * ((N + Cfg::BN - 1) / Cfg::BN);
+  // An early launch saves a few us, which long products do not need; 8192^3
+  // under the power cap took 1845 us launched early and 1783 not.
+  const bool early = (double)M * N * K < 1e11;
   uint32_t b = beta;
   for (int k0 = 0; k0 < K; k0 += ZP_KCHUNK) {
     const int kc = std::min(ZP_KCHUNK, K - k0);
@@ -1124,11 +1142,10 @@ static int launch_tc(Ctx *c, int M, int N, int K, const Modulus &mod, uint32_t a
     {
       const uint32_t p = (uint32_t)mod.p;
       int pi = prof_begin(c, "zp_split");
-      split_rows_kernel<L, E><<<split_rows_grid(c->num_sms, M, kc), dim3(32, SPLIT_ROWS), 0,
-                                c->stream>>>(A + k0, lda, M, kc, p, Al, (size_t)Kp, (size_t)M * Kp,
-                                             0, 1);
-      split_cols_kernel<L, E><<<split_cols_grid<E>(N, Kp), 256, 0, c->stream>>>(
-          B + (size_t)k0 * ldb, ldb, kc, N, p, Bl, (size_t)Kp, (size_t)N * Kp, Kp);
+      pdl_launch_if(early, split_rows_kernel<L, E>, split_rows_grid(c->num_sms, M, kc), dim3(32, SPLIT_ROWS),
+                 0, c->stream, A + k0, lda, M, kc, p, Al, (size_t)Kp, (size_t)M * Kp, 0, 1);
+      pdl_launch_if(early, split_cols_kernel<L, E>, split_cols_grid<E>(N, Kp), 256, 0, c->stream,
+                 B + (size_t)k0 * ldb, ldb, kc, N, p, Bl, (size_t)Kp, (size_t)N * Kp, Kp);
       prof_end(c, pi);
       ctx_launched(c, 2);
     }
@@ -1141,8 +1158,8 @@ static int launch_tc(Ctx *c, int M, int N, int K, const Modulus &mod, uint32_t a
     if (st) return st;
     const int grid = std::min(tiles, c->num_sms);
     int pi = prof_begin(c, "zp_gemm_tc");
-    zp_gemm_tc_kernel<L, 0, T><<<grid, tc_threads<L, T>(), Lay::SMEM, c->stream>>>(
-        tmA, tmB, C, ldc, M, N, kc, mod, alpha, b, c->dstatus, kr, kbase + k0);
+    pdl_launch_if(early, zp_gemm_tc_kernel<L, 0, T>, grid, tc_threads<L, T>(), Lay::SMEM, c->stream,
+               tmA, tmB, C, ldc, M, N, kc, mod, alpha, b, c->dstatus, kr, kbase + k0);
     prof_end(c, pi);
     ctx_launched(c);
     b = 1;
@@ -1163,8 +1180,8 @@ static int launch_direct(Ctx *c, int M, int N, int K, const Modulus &mod, uint32
   const int stages = K > BK ? 2 : 1;
   const dim3 grid((N + Cfg::BN - 1) / Cfg::BN, (M + BM - 1) / BM);
   int pi = prof_begin(c, "zp_gemm_direct");
-  zp_gemm_direct_kernel<L><<<grid, DIR_THREADS, Cfg::smem(stages), c->stream>>>(
-      A, lda, B, ldb, C, ldc, M, N, K, stages, mod, alpha, beta, c->dstatus);
+  pdl_launch(zp_gemm_direct_kernel<L>, grid, DIR_THREADS, Cfg::smem(stages), c->stream, A,
+             lda, B, ldb, C, ldc, M, N, K, stages, mod, alpha, beta, c->dstatus);
   prof_end(c, pi);
   ctx_launched(c);
   const cudaError_t e = cudaGetLastError();
@@ -1336,9 +1353,9 @@ static int launch_planes(Ctx *c, int M, int N, int K, const Modulus &mod, uint32
                             Cfg::BN, L);
     if (st) return st;
     int pi = prof_begin(c, "zp_gemm_tc");
-    zp_gemm_tc_kernel<L, 0, T><<<std::min(tiles, c->num_sms), tc_threads<L, T>(),
-                                 TcLayout<L, T>::SMEM, c->stream>>>(
-        tmA, tmB, C, ldc, M, N, kc, mod, alpha, b, c->dstatus, kr, kbase + k0);
+    pdl_launch(zp_gemm_tc_kernel<L, 0, T>, std::min(tiles, c->num_sms), tc_threads<L, T>(),
+               TcLayout<L, T>::SMEM, c->stream,
+               tmA, tmB, C, ldc, M, N, kc, mod, alpha, b, c->dstatus, kr, kbase + k0);
     prof_end(c, pi);
     ctx_launched(c);
     b = 1;
@@ -1365,7 +1382,8 @@ int zp_split_rows_dev(Ctx *c, uint32_t p, const uint32_t *A, size_t lda, int M, 
                       const ZpPlanes &out, int part, int nb) {
   const dim3 grid = split_rows_grid(c->num_sms, M, K), block(32, SPLIT_ROWS);
 #define LELA_SR(L) \
-  split_rows_kernel<L, uint32_t><<<grid, block, 0, c->stream>>>(A, lda, M, K, p, out.base, out.pitch, out.plane, part, nb)
+  pdl_launch(split_rows_kernel<L, uint32_t>, grid, block, 0, c->stream, A, lda, M, K, p, \
+             out.base, out.pitch, out.plane, part, nb)
   switch (zp_limbs_for(p)) {
     case 1: LELA_SR(1); break;
     case 2: LELA_SR(2); break;
@@ -1382,7 +1400,8 @@ int zp_split_cols_dev(Ctx *c, uint32_t p, const uint32_t *B, size_t ldb, int K, 
   const int kout = (K + 15) & ~15;
   const dim3 grid = split_cols_grid<uint32_t>(N, kout);
 #define LELA_SC(L) \
-  split_cols_kernel<L, uint32_t><<<grid, 256, 0, c->stream>>>(B, ldb, K, N, p, out.base, out.pitch, out.plane, kout)
+  pdl_launch(split_cols_kernel<L, uint32_t>, grid, 256, 0, c->stream, B, ldb, K, N, p, out.base, \
+             out.pitch, out.plane, kout)
   switch (zp_limbs_for(p)) {
     case 1: LELA_SC(1); break;
     case 2: LELA_SC(2); break;
@@ -1454,8 +1473,8 @@ static int host_rows(Ctx *c, int M, int N, int K, const Modulus &mod, uint32_t a
   if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream, ev_b, 0);
   if (e == cudaSuccess) {
     int pi = prof_begin(c, "zp_split");
-    split_cols_kernel<L, uint32_t><<<split_cols_grid<uint32_t>(N, Kp), 256, 0, c->stream>>>(
-        dB, (size_t)N, K, N, (uint32_t)mod.p, Bl, (size_t)Kp, (size_t)N * Kp, Kp);
+    pdl_launch(split_cols_kernel<L, uint32_t>, split_cols_grid<uint32_t>(N, Kp), 256, 0, c->stream,
+               dB, (size_t)N, K, N, (uint32_t)mod.p, Bl, (size_t)Kp, (size_t)N * Kp, Kp);
     prof_end(c, pi);
     ctx_launched(c);
     e = cudaGetLastError();
@@ -1469,10 +1488,9 @@ static int host_rows(Ctx *c, int M, int N, int K, const Modulus &mod, uint32_t a
     e = cudaStreamWaitEvent(c->stream, ready[j], 0);
     if (e != cudaSuccess) break;
     int pi = prof_begin(c, "zp_split");
-    split_rows_kernel<L, uint32_t><<<split_rows_grid(c->num_sms, rows, K), dim3(32, SPLIT_ROWS), 0,
-                                     c->stream>>>(dA + (size_t)r0 * K, (size_t)K, rows, K,
-                                                  (uint32_t)mod.p, Al, (size_t)Kp,
-                                                  (size_t)rows * Kp, 0, 1);
+    pdl_launch(split_rows_kernel<L, uint32_t>, split_rows_grid(c->num_sms, rows, K),
+               dim3(32, SPLIT_ROWS), 0, c->stream, dA + (size_t)r0 * K, (size_t)K, rows, K,
+               (uint32_t)mod.p, Al, (size_t)Kp, (size_t)rows * Kp, 0, 1);
     prof_end(c, pi);
     CUtensorMap tmA;
     st = encode_3d(c, &tmA, Al, (uint64_t)K, (uint64_t)rows, L, (uint64_t)Kp,
@@ -1480,8 +1498,9 @@ static int host_rows(Ctx *c, int M, int N, int K, const Modulus &mod, uint32_t a
     if (st) break;
     const int tiles = ((rows + BM - 1) / BM) * ((N + Cfg::BN - 1) / Cfg::BN);
     pi = prof_begin(c, "zp_gemm_tc");
-    zp_gemm_tc_kernel<L, 0><<<std::min(tiles, c->num_sms), tc_threads<L, 0>(), Lay::SMEM, c->stream>>>(
-        tmA, tmB, dC + (size_t)r0 * N, (size_t)N, rows, N, K, mod, alpha, beta, c->dstatus);
+    pdl_launch(zp_gemm_tc_kernel<L, 0>, std::min(tiles, c->num_sms), tc_threads<L, 0>(), Lay::SMEM, c->stream,
+               tmA, tmB, dC + (size_t)r0 * N, (size_t)N, rows, N, K, mod, alpha, beta, c->dstatus, nullptr,
+               0);
     prof_end(c, pi);
     ctx_launched(c, 2);
     e = cudaGetLastError();
@@ -1642,18 +1661,18 @@ int noalloc_launch(cudaStream_t s, const NoallocDevice &d, int M, int N, int K,
     uint8_t *Al = planes;
     uint8_t *Bl = planes + (size_t)L * M * Kp;
     const uint32_t p = (uint32_t)mod.p;
-    split_rows_kernel<L, uint32_t><<<split_rows_grid(d.num_sms, M, kc), dim3(32, SPLIT_ROWS), 0, s>>>(
-        A + k0, lda, M, kc, p, Al, (size_t)Kp, (size_t)M * Kp, 0, 1);
-    split_cols_kernel<L, uint32_t><<<split_cols_grid<uint32_t>(N, Kp), 256, 0, s>>>(
-        B + (size_t)k0 * ldb, ldb, kc, N, p, Bl, (size_t)Kp, (size_t)N * Kp, Kp);
+    pdl_launch(split_rows_kernel<L, uint32_t>, split_rows_grid(d.num_sms, M, kc),
+               dim3(32, SPLIT_ROWS), 0, s, A + k0, lda, M, kc, p, Al, (size_t)Kp, (size_t)M * Kp, 0, 1);
+    pdl_launch(split_cols_kernel<L, uint32_t>, split_cols_grid<uint32_t>(N, Kp), 256, 0, s,
+               B + (size_t)k0 * ldb, ldb, kc, N, p, Bl, (size_t)Kp, (size_t)N * Kp, Kp);
     CUtensorMap tmA, tmB;
     if (!noalloc_map(&tmA, Al, (uint64_t)kc, (uint64_t)M, L, (uint64_t)Kp, (uint64_t)M * Kp,
                      BK, BM, L) ||
         !noalloc_map(&tmB, Bl, (uint64_t)kc, (uint64_t)N, L, (uint64_t)Kp, (uint64_t)N * Kp,
                      BK, Cfg::BN, L))
       return ST_CUDA;
-    zp_gemm_tc_kernel<L, 0><<<std::min(tiles, d.num_sms), tc_threads<L, 0>(), Lay::SMEM, s>>>(
-        tmA, tmB, C, ldc, M, N, kc, mod, alpha, b, err);
+    pdl_launch(zp_gemm_tc_kernel<L, 0>, std::min(tiles, d.num_sms), tc_threads<L, 0>(), Lay::SMEM, s,
+               tmA, tmB, C, ldc, M, N, kc, mod, alpha, b, err, nullptr, 0);
     b = 1;
   }
   return cudaGetLastError() == cudaSuccess ? ST_OK : ST_CUDA;
@@ -1733,9 +1752,9 @@ static int gf2_tc_launch(Ctx *c, int M, int N, int K, const uint8_t *Ab, const u
   if (st) return st;
   const int tiles = ((M + BM - 1) / BM) * ((N + Cfg::BN - 1) / Cfg::BN);
   int pi = prof_begin(c, "gf2_gemm_tc");
-  zp_gemm_tc_kernel<1, 1, T><<<std::min(tiles, c->num_sms), tc_threads<1, T>(), Lay::SMEM,
-                               c->stream>>>(tmA, tmB, C, ldc_words, M, N, K, make_modulus(2),
-                                            alpha, beta, c->dstatus);
+  pdl_launch(zp_gemm_tc_kernel<1, 1, T>, std::min(tiles, c->num_sms), tc_threads<1, T>(), Lay::SMEM,
+             c->stream, tmA, tmB, C, ldc_words, M, N, K, make_modulus(2), alpha, beta, c->dstatus,
+             nullptr, 0);
   prof_end(c, pi);
   ctx_launched(c);
   cudaError_t e = cudaGetLastError();
