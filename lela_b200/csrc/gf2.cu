@@ -387,11 +387,6 @@ int gf2_gemm_host_rows(Ctx *c, int M, int N, int K, const uint64_t *hA, size_t l
 constexpr int GW = 64;
 constexpr uint8_t GF2_HEAD_NONE = 64;
 
-struct Gf2PanelOut {
-  uint32_t t, pad0, last_pos, pad;
-  uint32_t ti[GW], tq[GW], pcol[GW];
-};
-
 __device__ __forceinline__ int gf2_row_at(int pos, const int *p2r, const int *stamp, int epoch) {
   return stamp[pos] == epoch ? p2r[pos] : pos;
 }
@@ -425,33 +420,47 @@ __global__ void __launch_bounds__(GF2_HEADS_THREADS)
 }
 
 // One warp.  The words of positions i0 .. i0 + GF2_WR - 1 (the window) sit
-// in registers, lane l holding positions i0 + l + 32 u, and are eliminated
+// in registers by columns: lane l holds the window's bits of columns l and l +
+// 32, position i0 + e at bit e, and they are eliminated
 // eagerly: when the pivot of column c is chosen, every other window row at
 // or below the current position with bit c set gets the pivot word XOR-ed
 // in, so the pivot of a column is the first window position at or below
-// the current one with the bit set (one ballot per 32 positions), and a
+// the current one with the bit set, and a
 // pivot row's word is its final U_k (reduced by the pivots before it, as the
-// reference's elimination leaves it).  Rows past the window are tested
+// reference's elimination leaves it).  A column step hands the column's 128 bits
+// to the warp (four exchanges); the pivot position, the bits to clear and the two
+// bits to trade follow from them alike in every lane, and each lane
+// applies them to its own columns where those hold a pivot bit.  (Rows on
+// lanes, the pivot from four ballots and __ffs, took 900 cycles a column, 30 us
+// a panel.)  Rows past the window are tested
 // lazily: the pivot rows are also kept as a reduced basis g_k (bit pcol_j of
 // g_k is delta_kj) with, per column c, the mask M[c] = (1 << c) | sum_k
 // g_k[c] << pcol_k, so bit c of a row reduced by all pivots so far is
 // parity(v & M[c]); head[] holds a lower bound of the first set bit of each
 // such row's reduced word and cnt[h] counts them by that bound, so the scan
 // past the window runs only when a row there may hold the pivot.  Outputs:
-// Gf2PanelOut, U (the pivot rows' final words).  Resets *last_act and
+// Gf2PanelOut, U (the pivot rows' final words); the host's copy as words of a
+// value and the sequence number (as the Z/p search's).  Resets *last_act and
 // hist[] for the next panel.
-constexpr int GF2_WR = 128;               // window positions (registers)
-constexpr int GF2_WU = GF2_WR / 32;       // per lane
+constexpr int GF2_WR = 128;               // window positions
+constexpr int GF2_WU = GF2_WR / 32;       // words of a column
+enum : int {
+  GF2_W_T = 0,     // pivots
+  GF2_W_LAST = 1,  // last_pos
+  GF2_W_PIV = 2,   // per pivot: transposition target
+  GF2_WORDS = GF2_W_PIV + GW
+};
+static_assert(PANEL_WORDS_OFF + GF2_WORDS * 8 <= PANEL_FLAG_OFF, "words below the flag");
 __global__ void __launch_bounds__(32)
     gf2_search_kernel(const uint64_t *D, size_t ld, int i0, int m, int wc, int w,
                       uint64_t pmask, uint8_t *head, const uint8_t *act,
                       int *hist, int *last_act, int *p2r,
-                      int *stamp, int epoch, uint64_t *Uout,
-                      Gf2PanelOut *out, Gf2PanelOut *hout, volatile uint32_t *hflag,
-                      uint32_t seq) {
+                      int *stamp, int epoch, uint64_t *Uout, uint32_t *pcol_out,
+                      volatile uint64_t *hout, uint32_t seq) {
   pdl_enter();
-  __shared__ uint64_t G[GW], M[GW], s_U[GW];
-  __shared__ int s_pcol[GW], s_ti[GW], s_tq[GW];
+  constexpr unsigned FULL = 0xffffffffu;
+  __shared__ uint64_t G[GW], M[GW];
+  __shared__ int s_pcol[GW], s_tq[GW], s_wr[GF2_WR];
   __shared__ int s_cnt[GW + 1];
   const int lane = threadIdx.x;
   const int wend = min(i0 + GF2_WR, m);  // positions past the window start here
@@ -460,31 +469,38 @@ __global__ void __launch_bounds__(32)
     s_cnt[h] = hist[h];
     hist[h] = 0;
   }
-  __syncwarp();
-  uint64_t wv[GF2_WU];
-  int wr[GF2_WU];  // row index at the position (-1: past the matrix)
+  uint32_t c0[GF2_WU], c1[GF2_WU];  // columns lane, lane + 32
+  {
+    uint64_t v[GF2_WU];
 #pragma unroll
-  for (int u = 0; u < GF2_WU; ++u) {
-    const int pos = i0 + lane + 32 * u;
-    wr[u] = pos < m ? pos : -1;  // no transposition has touched this panel yet
-    wv[u] = pos < m ? D[(size_t)pos * ld + wc] & pmask : 0ull;
+    for (int u = 0; u < GF2_WU; ++u) {
+      const int pos = i0 + lane + 32 * u;
+      s_wr[lane + 32 * u] = pos < m ? pos : -1;  // row at the position: none has moved yet
+      v[u] = pos < m ? D[(size_t)pos * ld + wc] & pmask : 0ull;
+    }
+#pragma unroll
+    for (int u = 0; u < GF2_WU; ++u) {
+      c0[u] = transpose32((uint32_t)v[u], lane);
+      c1[u] = transpose32((uint32_t)(v[u] >> 32), lane);
+    }
   }
   M[lane] = 1ull << lane;
   M[lane + 32] = 1ull << (lane + 32);
   __syncwarp();
-  auto pick64 = [&](int g) -> uint64_t {
-    uint64_t v = wv[0];
-#pragma unroll
-    for (int u = 1; u < GF2_WU; ++u)
-      if (g == u) v = wv[u];
-    return v;
+  // the word of the window row at position i0 + e, e < 64 (the same in every lane)
+  auto row_word = [&](int e) -> uint64_t {
+    const uint32_t a = e < 32 ? c0[0] : c0[1], b = e < 32 ? c1[0] : c1[1];
+    const uint32_t lo = __ballot_sync(FULL, (a >> (e & 31)) & 1u);
+    const uint32_t hi = __ballot_sync(FULL, (b >> (e & 31)) & 1u);
+    return (uint64_t)hi << 32 | lo;
   };
-  auto pickr = [&](int g) -> int {
-    int v = wr[0];
-#pragma unroll
-    for (int u = 1; u < GF2_WU; ++u)
-      if (g == u) v = wr[u];
-    return v;
+  auto set_row = [&](int e, uint64_t word) {
+    const uint32_t b0 = e < 32 ? 1u << e : 0u, b1 = e < 32 ? 0u : 1u << (e & 31);
+    const bool lo = (word >> lane) & 1ull, hi = (word >> (lane + 32)) & 1ull;
+    c0[0] = lo ? c0[0] | b0 : c0[0] & ~b0;
+    c0[1] = lo ? c0[1] | b1 : c0[1] & ~b1;
+    c1[0] = hi ? c1[0] | b0 : c1[0] & ~b0;
+    c1[1] = hi ? c1[1] | b1 : c1[1] & ~b1;
   };
   // The basis g_k and masks M: pivot U at column c makes g_k ^= U where g_k
   // has bit c, and M[c'] ^= M[c] for the columns c' > c where U has a bit.
@@ -502,60 +518,58 @@ __global__ void __launch_bounds__(32)
     __syncwarp();
   };
   bool basis = false;
-  int i = i0, t = 0;
-  for (int col = 0; col < w && i < m; ++col) {
-    const uint64_t bit = 1ull << col;
-    // first window position at or below i with bit col set
-    int qi = -1;
+  int t = 0;  // pivots so far; the current position is i0 + t, bit t
+#pragma unroll 1
+  for (int col = 0; col < w && i0 + t < m; ++col) {
+    // the column's bits, at or below the current position
+    uint32_t v[GF2_WU];
 #pragma unroll
-    for (int u = 0; u < GF2_WU; ++u) {
-      const int pos = i0 + lane + 32 * u;
-      const unsigned b = __ballot_sync(0xffffffffu, pos >= i && (wv[u] & bit) != 0ull);
-      if (qi < 0 && b) qi = 32 * u + __ffs(b) - 1;
-    }
-    int q;
-    uint64_t U;
-    if (qi >= 0) {
-      q = i0 + qi;
-      U = __shfl_sync(0xffffffffu, pick64(qi >> 5), qi & 31);
-      // eliminate the other window rows at or below i
+    for (int u = 0; u < GF2_WU; ++u) v[u] = __shfl_sync(FULL, col < 32 ? c0[u] : c1[u], col & 31);
+    static_assert(GF2_WU == 4 && GW <= 64, "four words, the current position in the first two");
+    v[0] &= t < 32 ? ~0u << t : 0u;
+    v[1] &= t < 32 ? ~0u : ~0u << (t & 31);
+    const int wq = v[0] ? 0 : v[1] ? 1 : v[2] ? 2 : 3;  // the pivot's word, its bit
+    const uint32_t x = v[0] ? v[0] : v[1] ? v[1] : v[2] ? v[2] : v[3];
+    const uint32_t pb = x & (0u - x);
+    int q = -1;  // the pivot's position - i0
+    if (x) {
+      q = 32 * wq + (31 - __clz((int)pb));
+      // rows to clear (the pivot's own bit stays); rows t and q trade places,
+      // row t having a 0 in this column when q > t
+      const uint32_t tb = 1u << (t & 31);
+      const bool swap = q != t;
+      uint32_t e[GF2_WU], sw[GF2_WU];
 #pragma unroll
       for (int u = 0; u < GF2_WU; ++u) {
-        const int e = lane + 32 * u;
-        if (i0 + e >= i && e != qi && (wv[u] & bit)) wv[u] ^= U;
+        e[u] = v[u] ^ (u == wq ? pb : 0u);
+        sw[u] = swap ? (u == wq ? pb : 0u) ^ (u == (t >> 5) ? tb : 0u) : 0u;
       }
-      // transposition (i, q) inside the window: the row at i (bit col clear,
-      // so not changed above) and the pivot row trade places
-      if (q != i) {
-        const int ei = i - i0;
-        const uint64_t vi = __shfl_sync(0xffffffffu, pick64(ei >> 5), ei & 31);
-        const int ri = __shfl_sync(0xffffffffu, pickr(ei >> 5), ei & 31);
-        const int rq = __shfl_sync(0xffffffffu, pickr(qi >> 5), qi & 31);
+      auto apply = [&](uint32_t(&cc)[GF2_WU]) {
+        const uint32_t cq = wq == 0 ? cc[0] : wq == 1 ? cc[1] : wq == 2 ? cc[2] : cc[3];
+        const uint32_t ct = t < 32 ? cc[0] : cc[1];
+        const bool bq = (cq & pb) != 0u, bt = (ct & tb) != 0u;
 #pragma unroll
-        for (int u = 0; u < GF2_WU; ++u) {
-          const int e = lane + 32 * u;
-          if (e == ei) {
-            wv[u] = U;
-            wr[u] = rq;
-          } else if (e == qi) {
-            wv[u] = vi;
-            wr[u] = ri;
-          }
-        }
+        for (int u = 0; u < GF2_WU; ++u) cc[u] ^= (bq ? e[u] : 0u) ^ (bq != bt ? sw[u] : 0u);
+      };
+      apply(c0);
+      apply(c1);
+      if (swap && lane == 0) {
+        const int r = s_wr[t];
+        s_wr[t] = s_wr[q];
+        s_wr[q] = r;
       }
     } else {
       // none in the window: rows past it whose bound allows a pivot here
+      const int i = i0 + t;
       int cand = 0;
       for (int h = lane; h <= col; h += 32) cand += s_cnt[h];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) cand += __shfl_xor_sync(0xffffffffu, cand, o);
+      cand = __reduce_add_sync(FULL, cand);
       if (cand == 0) continue;  // no pivot in this column
       if (!basis) {
-        for (int k = 0; k < t; ++k) basis_add(s_U[k], s_pcol[k], k);
+        for (int k = 0; k < t; ++k) basis_add(row_word(k), s_pcol[k], k);
         basis = true;
       }
-      q = -1;
-      uint64_t v = 0ull;
+      uint64_t pw = 0ull;
       for (int base = wend; base < m && cand > 0; base += 32) {
         const int pos = base + lane;
         int is_cand = 0, hit = 0;
@@ -577,155 +591,235 @@ __global__ void __launch_bounds__(32)
             hit = c == col;
           }
         }
-        cand -= __popc(__ballot_sync(0xffffffffu, is_cand));
-        const unsigned hb = __ballot_sync(0xffffffffu, hit);
+        cand -= __popc(__ballot_sync(FULL, is_cand));
+        const unsigned hb = __ballot_sync(FULL, hit);
         if (hb) {
           const int l = __ffs(hb) - 1;
-          q = base + l;
-          v = __shfl_sync(0xffffffffu, pv, l);
+          q = base + l - i0;
+          pw = __shfl_sync(FULL, pv, l);
           break;
         }
       }
       __syncwarp();
       if (q < 0) continue;  // no pivot in this column
       // the pivot row reduced by the pivots so far: U = v ^ sum_{k: v bit pcol_k} g_k
-      uint64_t x = 0;
-      if (lane < t && ((v >> s_pcol[lane]) & 1ull)) x ^= G[lane];
-      if (lane + 32 < t && ((v >> s_pcol[lane + 32]) & 1ull)) x ^= G[lane + 32];
+      uint64_t xg = 0;
+      if (lane < t && ((pw >> s_pcol[lane]) & 1ull)) xg ^= G[lane];
+      if (lane + 32 < t && ((pw >> s_pcol[lane + 32]) & 1ull)) xg ^= G[lane + 32];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) x ^= __shfl_xor_sync(0xffffffffu, x, o);
-      U = v ^ x;
+      for (int o = 16; o > 0; o >>= 1) xg ^= __shfl_xor_sync(FULL, xg, o);
+      const uint64_t U = pw ^ xg;
       // transposition (i, q): the pivot row takes position i; the window row
       // there (bit col clear, reduced by every pivot) goes to position q, with
       // the bound of its reduced word
-      const int ei = i - i0;
-      const uint64_t vi = __shfl_sync(0xffffffffu, pick64(ei >> 5), ei & 31);
-      const int ri = __shfl_sync(0xffffffffu, pickr(ei >> 5), ei & 31);
-      const int ap = gf2_row_at(q, p2r, stamp, epoch);  // before the maps change
+      const uint64_t vi = row_word(t);
+      const int ap = gf2_row_at(i0 + q, p2r, stamp, epoch);  // before the maps change
       __syncwarp();
       if (lane == 0) {
+        const int ri = s_wr[t];
         const int hv = vi ? __ffsll((long long)vi) - 1 : GF2_HEAD_NONE;
         atomicSub(&s_cnt[head[ap]], 1);  // the pivot row leaves the counts
         head[ri] = (uint8_t)hv;
         atomicAdd(&s_cnt[hv], 1);
-        p2r[q] = ri;
-        stamp[q] = epoch;
+        p2r[i0 + q] = ri;
+        stamp[i0 + q] = epoch;
+        s_wr[t] = ap;
       }
-#pragma unroll
-      for (int u = 0; u < GF2_WU; ++u)
-        if (lane + 32 * u == ei) {
-          wv[u] = U;
-          wr[u] = ap;
-        }
+      __syncwarp();
+      set_row(t, U);
+      (void)i;
     }
-    if (basis) basis_add(U, col, t);
+    if (basis) basis_add(row_word(t), col, t);
     if (lane == 0) {
-      s_U[t] = U;
       s_pcol[t] = col;
-      s_ti[t] = i;
-      s_tq[t] = q;
+      s_tq[t] = i0 + q;
     }
-    __syncwarp();
-    ++i;
     ++t;
+    __syncwarp();
   }
+  const int i = i0 + t;
   // last final position of a non-pivot row with a nonzero word
   int hi = i - 1;
   for (int k = lane; k < t; k += 32) hi = max(hi, s_tq[k]);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  hi = __reduce_max_sync(FULL, hi);
   int last = -1;
 #pragma unroll
   for (int u = 0; u < GF2_WU; ++u) {
-    const int pos = i0 + lane + 32 * u;
-    if (pos >= i && pos <= hi && wr[u] >= 0 && act[wr[u]]) last = max(last, pos);
+    const int pos = i0 + lane + 32 * u, r = s_wr[lane + 32 * u];
+    if (pos >= i && pos <= hi && r >= 0 && act[r]) last = max(last, pos);
   }
   for (int pos = max(i, wend) + lane; pos <= hi && pos < m; pos += 32)
     if (act[gf2_row_at(pos, p2r, stamp, epoch)]) last = max(last, pos);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) last = max(last, __shfl_xor_sync(0xffffffffu, last, o));
+  last = __reduce_max_sync(FULL, last);
+  const auto word = [seq](uint32_t v) { return (uint64_t)seq << 32 | v; };
   if (lane == 0) {
     const int la = *last_act;
     if (la > hi) last = la;
-    out->t = (uint32_t)t;
-    out->last_pos = (uint32_t)(last >= 0 ? last : 0);
     *last_act = -1;
-    hout->t = (uint32_t)t;
-    hout->last_pos = (uint32_t)(last >= 0 ? last : 0);
+    hout[GF2_W_T] = word((uint32_t)t);
+    hout[GF2_W_LAST] = word((uint32_t)max(last, 0));
   }
-  // the outputs; the result also goes to mapped host memory, then the
-  // sequence flag
-  __syncwarp();
-  for (int k = lane; k < t; k += 32) {
-    Uout[k] = s_U[k];
-    out->ti[k] = hout->ti[k] = (uint32_t)s_ti[k];
-    out->tq[k] = hout->tq[k] = (uint32_t)s_tq[k];
-    out->pcol[k] = hout->pcol[k] = (uint32_t)s_pcol[k];
+  // rows 0 .. t - 1 of the window are the pivot rows
+  uint64_t U[2];
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+    U[u] = (uint64_t)transpose32(c1[u], lane) << 32 | transpose32(c0[u], lane);
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int k = lane + 32 * u;
+    if (k < t) {
+      hout[GF2_W_PIV + k] = word((uint32_t)s_tq[k]);
+      Uout[k] = U[u];
+      pcol_out[k] = (uint32_t)s_pcol[k];
+    }
   }
-  __threadfence_system();
-  __syncwarp();
-  if (lane == 0) *hflag = seq;
 }
 
 // Rows i0..r1 at their final positions: the reference's elimination steps
 // on the panel word give the multipliers (L11 row of pivot row k over the
 // pivots before it; L21 row of the rows below over all t) and the final
-// word (U_k; zero below).  One thread per row.
-__global__ void gf2_solve_kernel(uint64_t *D, size_t ld, int i0, int r1, int wc,
-                                 uint64_t pmask, int t, const uint32_t *pcol,
-                                 const uint64_t *Uin, uint64_t *L11,
-                                 uint64_t *L21) {
+// word (U_k; zero below).  One thread per row.  With Lb the multipliers also go
+// into the block's rows of bits (GB words a row, at bit offset off; the caller
+// zeroed the block's rows) and, when the block has words right of the panel (w1
+// .. wend, at most GB), the first CTA, which holds all pivot rows, solves U12 =
+// L11^-1 A12 there in place: a warp per word as gf2_l11_solve_kernel.  (The
+// three steps as kernels of their own took 7.3, 3.2 and 5.6 us.)
+constexpr int GB = 8;  // panels (words) per block of delayed updates
+constexpr int GF2_SOLVE_THREADS = 256;
+__device__ __forceinline__ void gf2_u12_word(uint64_t *D, size_t ld, int i0, int t, int w,
+                                             uint64_t l0, uint64_t l1, int lane) {
+  uint64_t x0 = lane < t ? D[(size_t)(i0 + lane) * ld + w] : 0ull;
+  uint64_t x1 = lane + 32 < t ? D[(size_t)(i0 + lane + 32) * ld + w] : 0ull;
+  for (int k = 0; k < t - 1; ++k) {
+    const uint64_t xk = __shfl_sync(0xffffffffu, k < 32 ? x0 : x1, k & 31);
+    if (lane > k && ((l0 >> k) & 1ull)) x0 ^= xk;
+    if ((l1 >> k) & 1ull) x1 ^= xk;  // L11 is strictly lower: bit k set means k < the row
+  }
+  if (lane < t) D[(size_t)(i0 + lane) * ld + w] = x0;
+  if (lane + 32 < t) D[(size_t)(i0 + lane + 32) * ld + w] = x1;
+}
+__global__ void __launch_bounds__(GF2_SOLVE_THREADS)
+    gf2_solve_kernel(uint64_t *D, size_t ld, int i0, int r1, int wc, uint64_t pmask, int t,
+                     const uint32_t *pcol, const uint64_t *Uin, uint64_t *L11, uint64_t *L21,
+                     uint64_t *Lb, int off, int w1, int wend) {
   pdl_enter();
-  __shared__ uint64_t sU[GW];
+  __shared__ uint64_t sU[GW], sL[GW];
   __shared__ int sP[GW];
   if (threadIdx.x < GW) {
     sU[threadIdx.x] = threadIdx.x < t ? Uin[threadIdx.x] : 0ull;
     sP[threadIdx.x] = threadIdx.x < t ? (int)pcol[threadIdx.x] : 0;
+    sL[threadIdx.x] = 0ull;
   }
   __syncthreads();
+  static_assert(GF2_SOLVE_THREADS >= GW, "the first CTA's first pass holds the pivot rows");
   const int r0 = i0 + t;
   for (int pos = i0 + blockIdx.x * blockDim.x + threadIdx.x; pos <= r1;
        pos += gridDim.x * blockDim.x) {
     uint64_t *x = D + (size_t)pos * ld + wc;
-    uint64_t v = *x & pmask;
+    const uint64_t old = *x;
+    uint64_t v = old & pmask;
     const int kk = pos - i0, lim = kk < t ? kk : t;
     uint64_t l = 0;
-    for (int k = 0; k < lim; ++k)
-      if ((v >> sP[k]) & 1ull) {
-        v ^= sU[k];
-        l |= 1ull << k;
-      }
-    *x = (*x & ~pmask) | v;
-    if (kk < t)
+#pragma unroll 4
+    for (int k = 0; k < lim; ++k) {
+      const bool b = (v >> sP[k]) & 1ull;
+      v ^= b ? sU[k] : 0ull;
+      l |= (uint64_t)b << k;
+    }
+    *x = (old & ~pmask) | v;
+    if (kk < t) {
       L11[kk] = l;
-    else
+      sL[kk] = l;
+    } else {
       L21[pos - r0] = l;
+    }
+    if (Lb) {
+      uint64_t *row = Lb + (size_t)pos * GB;
+      const int wq = off >> 6, sh = off & 63;
+      row[wq] |= l << sh;
+      if (sh && sh + t > 64) row[wq + 1] |= l >> (64 - sh);
+    }
+  }
+  if (Lb == nullptr || blockIdx.x != 0 || w1 >= wend) return;
+  __syncthreads();
+  const int lane = threadIdx.x & 31, w = w1 + (threadIdx.x >> 5);
+  static_assert(GF2_SOLVE_THREADS / 32 >= GB, "a warp per word of the block");
+  if (w < wend) gf2_u12_word(D, ld, i0, t, w, sL[lane], sL[lane + 32], lane);
+}
+
+// C ^= L21 U12 on the words w1 .. w1 + nw - 1 (nw <= GB) of the rows r0 .. r1 of
+// D: the words of the panel's block right of it.  U12: rows i0 .. i0 + t - 1.
+// Sixteen tables of the XORs of four rows of U12 in shared memory, a thread
+// per row and word (a row's words on neighbouring threads), sixteen lookups.
+// The general four-Russians kernel, which builds tables of 256 entries per word
+// pair, took 14 us a panel here.
+constexpr int GF2_BW_THREADS = 256;
+__global__ void __launch_bounds__(GF2_BW_THREADS)
+    gf2_block_words_kernel(uint64_t *D, size_t ld, int n, int i0, int t, int w1, int nw, int r0,
+                           int r1, const uint64_t *L21) {
+  pdl_enter();
+  __shared__ uint64_t sU[GW][GB], T[GW / 4][16][GB];
+  for (int e = threadIdx.x; e < GW * GB; e += GF2_BW_THREADS) {
+    const int k = e / GB, w = e % GB;
+    // (bits past column n of the last word stay as they are)
+    const int cols = n - 64 * (w1 + w);
+    const uint64_t mask = cols >= 64 ? ~0ull : cols > 0 ? (1ull << cols) - 1ull : 0ull;
+    sU[k][w] = k < t && w < nw ? D[(size_t)(i0 + k) * ld + w1 + w] & mask : 0ull;
+  }
+  __syncthreads();
+  {
+    static_assert(GF2_BW_THREADS == GW / 4 * 16, "a table entry per thread");
+    const int g = threadIdx.x >> 4, e = threadIdx.x & 15;
+#pragma unroll
+    for (int w = 0; w < GB; ++w) {
+      uint64_t v = 0;
+#pragma unroll
+      for (int b = 0; b < 4; ++b) v ^= (e >> b) & 1 ? sU[4 * g + b][w] : 0ull;
+      T[g][e][w] = v;
+    }
+  }
+  __syncthreads();
+  const int w = threadIdx.x % GB;
+  for (int r = r0 + blockIdx.x * (GF2_BW_THREADS / GB) + threadIdx.x / GB; r <= r1;
+       r += gridDim.x * (GF2_BW_THREADS / GB)) {
+    const uint64_t l = L21[r - r0];
+    uint64_t *x = D + (size_t)r * ld + w1 + w;
+    uint64_t v = w < nw ? *x : 0ull;
+#pragma unroll
+    for (int g = 0; g < GW / 4; ++g) v ^= T[g][(l >> (4 * g)) & 15][w];
+    if (w < nw) *x = v;
   }
 }
 
 // Row permutation in one launch: each CTA takes GF2_PERM_WORDS words of
-// every moved row.  Its threads load all their words of the source rows at
+// every moved row of D, the last ones of the block's multipliers Lb (nwb words a
+// row; 0: none).  Its threads load all their words of the source rows at
 // once (at most GF2_PERM_PER each, into registers), wait at the barrier,
 // then store them to the destination rows; the CTAs own disjoint words, so
 // no grid-wide ordering is needed.  cnt <= 2 * GW rows.
 constexpr int GF2_PERM_THREADS = 256, GF2_PERM_WORDS = 16;
 constexpr int GF2_PERM_PER = 2 * GW * GF2_PERM_WORDS / GF2_PERM_THREADS;
 __global__ void __launch_bounds__(GF2_PERM_THREADS)
-    gf2_permute_rows_kernel(uint64_t *D, size_t ld, int nw,
+    gf2_permute_rows_kernel(uint64_t *D, size_t ld, int nw, uint64_t *Lb, int nwb,
                             const int *src, const int *dst, int cnt) {
   pdl_enter();
-  const int w0 = blockIdx.x * GF2_PERM_WORDS, total = cnt * GF2_PERM_WORDS;
+  const int own = (nw + GF2_PERM_WORDS - 1) / GF2_PERM_WORDS;
+  const bool lb = (int)blockIdx.x >= own;
+  uint64_t *X = lb ? Lb : D;
+  const size_t ldx = lb ? (size_t)nwb : ld;
+  const int nx = lb ? nwb : nw;
+  const int w0 = ((int)blockIdx.x - (lb ? own : 0)) * GF2_PERM_WORDS, total = cnt * GF2_PERM_WORDS;
   uint64_t v[GF2_PERM_PER];
 #pragma unroll
   for (int u = 0; u < GF2_PERM_PER; ++u) {
     const int e = threadIdx.x + u * GF2_PERM_THREADS, w = w0 + e % GF2_PERM_WORDS;
-    v[u] = (e < total && w < nw) ? D[(size_t)src[e / GF2_PERM_WORDS] * ld + w] : 0ull;
+    v[u] = (e < total && w < nx) ? X[(size_t)src[e / GF2_PERM_WORDS] * ldx + w] : 0ull;
   }
   __syncthreads();
 #pragma unroll
   for (int u = 0; u < GF2_PERM_PER; ++u) {
     const int e = threadIdx.x + u * GF2_PERM_THREADS, w = w0 + e % GF2_PERM_WORDS;
-    if (e < total && w < nw) D[(size_t)dst[e / GF2_PERM_WORDS] * ld + w] = v[u];
+    if (e < total && w < nx) X[(size_t)dst[e / GF2_PERM_WORDS] * ldx + w] = v[u];
   }
 }
 
@@ -744,34 +838,7 @@ __global__ void __launch_bounds__(GF2_L11_THREADS)
   const int w = w1 + (int)((blockIdx.x * (size_t)GF2_L11_THREADS + threadIdx.x) >> 5);
   if (w >= nw) return;  // whole warps
   const uint64_t l0 = lane < t ? L11[lane] : 0ull, l1 = lane + 32 < t ? L11[lane + 32] : 0ull;
-  uint64_t x0 = lane < t ? D[(size_t)(i0 + lane) * ld + w] : 0ull;
-  uint64_t x1 = lane + 32 < t ? D[(size_t)(i0 + lane + 32) * ld + w] : 0ull;
-  for (int k = 0; k < t - 1; ++k) {
-    const uint64_t xk = __shfl_sync(0xffffffffu, k < 32 ? x0 : x1, k & 31);
-    if (lane > k && ((l0 >> k) & 1ull)) x0 ^= xk;
-    if ((l1 >> k) & 1ull) x1 ^= xk;  // L11 is strictly lower: bit k set means k < the row
-  }
-  if (lane < t) D[(size_t)(i0 + lane) * ld + w] = x0;
-  if (lane + 32 < t) D[(size_t)(i0 + lane + 32) * ld + w] = x1;
-}
-
-// The panel's multipliers into the block's rows of bits: rows i0..r1, the
-// t bits of L11 (pivot rows) or L21 (rows below) at bit offset off of the
-// row's GB words (the caller zeroed the block's rows).
-constexpr int GB = 8;  // panels (words) per block of delayed updates
-__global__ void gf2_deposit_kernel(uint64_t *Lb, int i0, int r1, int t, int off,
-                                   const uint64_t *L11,
-                                   const uint64_t *L21) {
-  pdl_enter();
-  const int r0 = i0 + t;
-  for (int pos = i0 + blockIdx.x * blockDim.x + threadIdx.x; pos <= r1;
-       pos += gridDim.x * blockDim.x) {
-    const uint64_t l = pos < r0 ? L11[pos - i0] : L21[pos - r0];
-    uint64_t *row = Lb + (size_t)pos * GB;
-    const int wq = off >> 6, sh = off & 63;
-    row[wq] |= l << sh;
-    if (sh && sh + t > 64) row[wq + 1] |= l >> (64 - sh);
-  }
+  gf2_u12_word(D, ld, i0, t, w, l0, l1, lane);
 }
 
 int gf2_echelon_dev(Ctx *c, int m, int n, uint64_t *D, size_t ld, size_t *rank_out) {
@@ -783,7 +850,7 @@ int gf2_echelon_dev(Ctx *c, int m, int n, uint64_t *D, size_t ld, size_t *rank_o
     *rank_out = 0;
     return ST_OK;
   }
-  const size_t out_bytes = (sizeof(Gf2PanelOut) + 255) & ~(size_t)255;
+  const size_t out_bytes = GW * sizeof(uint32_t);  // pivot columns
   // p2r, stamp (m each); permutation lists (4 GW); last row (1); histogram (GW + 1)
   const size_t i_bytes =
       (((size_t)2 * m + 4 * GW + 1 + GW + 1) * sizeof(int) + 255) & ~(size_t)255;
@@ -795,7 +862,7 @@ int gf2_echelon_dev(Ctx *c, int m, int n, uint64_t *D, size_t ld, size_t *rank_o
                       &base);
   if (st) return st;
   uint8_t *b8 = static_cast<uint8_t *>(base);
-  Gf2PanelOut *d_out = reinterpret_cast<Gf2PanelOut *>(b8);
+  uint32_t *d_pcol = reinterpret_cast<uint32_t *>(b8);
   int *d_p2r = reinterpret_cast<int *>(b8 + out_bytes);
   int *d_stamp = d_p2r + m;
   int *d_perm = d_stamp + m;      // 4*GW ints
@@ -808,22 +875,18 @@ int gf2_echelon_dev(Ctx *c, int m, int n, uint64_t *D, size_t ld, size_t *rank_o
   uint64_t *d_U = d_L11 + GW;
   uint64_t *d_Lb = d_U + GW;                 // m x GB words
   uint64_t *d_L11s = d_Lb + (size_t)m * GB;                       // GB x GW words
-  const uint32_t *d_pcol = reinterpret_cast<const uint32_t *>(b8 + offsetof(Gf2PanelOut, pcol));
-  static_assert(sizeof(Gf2PanelOut) <= PANEL_FLAG_OFF, "panel result and flag share the mapped page");
   void *mh = nullptr, *md = nullptr;
   if ((st = ctx_panel_map(c, &mh, &md))) return st;
-  const Gf2PanelOut *hmap = static_cast<const Gf2PanelOut *>(mh);
   int *hperm = reinterpret_cast<int *>(static_cast<char *>(mh) + PANEL_PERM_OFF);
-  static_assert(sizeof(Gf2PanelOut) <= PANEL_PERM_OFF && 2 * (2 * GW) <= (int)PANEL_PERM_INTS, "staging layout");
-  volatile uint32_t *hflag = reinterpret_cast<volatile uint32_t *>(static_cast<char *>(mh) + PANEL_FLAG_OFF);
-  Gf2PanelOut *hmap_dev = static_cast<Gf2PanelOut *>(md);
-  uint32_t *hflag_dev = reinterpret_cast<uint32_t *>(static_cast<char *>(md) + PANEL_FLAG_OFF);
+  static_assert(2 * (2 * GW) <= (int)PANEL_PERM_INTS, "staging layout");
+  volatile uint64_t *hwords = reinterpret_cast<volatile uint64_t *>(static_cast<char *>(mh) + PANEL_WORDS_OFF);
+  volatile uint64_t *hwords_dev = reinterpret_cast<volatile uint64_t *>(static_cast<char *>(md) + PANEL_WORDS_OFF);
   cudaError_t e = cudaMemsetAsync(d_stamp, 0xff, (size_t)m * sizeof(int), c->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(d_last, 0xff, sizeof(int), c->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(d_hist, 0, (GW + 1) * sizeof(int), c->stream);
   if (e != cudaSuccess) return ctx_cuda(c, e, "gf2 echelon: scratch");
 
-  Gf2PanelOut h;
+  int tq[GW];
   std::vector<int> at, src, dst;
   int i = 0, epoch = 0;
   const int head_grid = std::max(1, std::min((m + GF2_HEADS_THREADS - 1) / GF2_HEADS_THREADS,
@@ -885,24 +948,27 @@ int gf2_echelon_dev(Ctx *c, int m, int n, uint64_t *D, size_t ld, size_t *rank_o
     pi = prof_begin(c, "gf2_search");
     pdl_launch(gf2_search_kernel, 1, 32, 0, c->stream,
         D, ld, i, m, wc, w, pmask, d_head, d_act, d_hist, d_last, d_p2r, d_stamp, epoch++, d_U,
-        d_out, hmap_dev, hflag_dev, seq);
+        d_pcol, hwords_dev, seq);
     prof_end(c, pi);
     ctx_launched(c, 2);
-    if ((st = ctx_wait_flag(c, hflag, seq, "gf2 echelon: panel"))) return st;
-    h.t = hmap->t;
-    h.last_pos = hmap->last_pos;
-    for (uint32_t k = 0; k < h.t && k < (uint32_t)GW; ++k) {
-      h.ti[k] = hmap->ti[k];
-      h.tq[k] = hmap->tq[k];
-      h.pcol[k] = hmap->pcol[k];
-    }
-    const int t = (int)h.t;
+    auto word = [&](int k, int *v) -> int {
+      const int s = ctx_wait_flag(c, reinterpret_cast<volatile uint32_t *>(hwords + k) + 1, seq,
+                                  "gf2 echelon: panel");
+      if (s == ST_OK) *v = (int)(uint32_t)hwords[k];
+      return s;
+    };
+    int t = 0, last_pos = 0;
+    if ((st = word(GF2_W_T, &t)) || (st = word(GF2_W_LAST, &last_pos))) return st;
+    t = std::min(t, GW);
     if (t == 0) continue;
     int hi = i;
-    for (int k = 0; k < t; ++k) hi = std::max(hi, (int)h.tq[k]);
+    for (int k = 0; k < t; ++k) {
+      if ((st = word(GF2_W_PIV + k, &tq[k]))) return st;
+      hi = std::max(hi, tq[k]);
+    }
     at.resize(hi - i + 1);
     for (int q = i; q <= hi; ++q) at[q - i] = q;
-    for (int k = 0; k < t; ++k) std::swap(at[h.ti[k] - i], at[h.tq[k] - i]);
+    for (int k = 0; k < t; ++k) std::swap(at[k], at[tq[k] - i]);
     src.clear();
     dst.clear();
     for (int q = i; q <= hi; ++q)
@@ -920,17 +986,15 @@ int gf2_echelon_dev(Ctx *c, int m, int n, uint64_t *D, size_t ld, size_t *rank_o
       e = cudaMemcpyAsync(d_perm, hperm, (size_t)2 * cnt * sizeof(int), cudaMemcpyHostToDevice,
                           c->stream);
       if (e != cudaSuccess) return ctx_cuda(c, e, "gf2 echelon: permutation");
-      pdl_launch(gf2_permute_rows_kernel, (nw + GF2_PERM_WORDS - 1) / GF2_PERM_WORDS, GF2_PERM_THREADS, 0, c->stream,
-      D, ld, nw, d_perm, d_perm + cnt, cnt);
+      // (the block's earlier multipliers move with their rows)
+      static_assert(GB <= GF2_PERM_WORDS, "one CTA for the block's multipliers");
+      pdl_launch(gf2_permute_rows_kernel,
+                 (nw + GF2_PERM_WORDS - 1) / GF2_PERM_WORDS + (Tb > 0 ? 1 : 0), GF2_PERM_THREADS, 0,
+                 c->stream, D, ld, nw, d_Lb, GB, d_perm, d_perm + cnt, cnt);
       ctx_launched(c);
-      if (Tb > 0) {  // the block's earlier multipliers move with their rows
-        pdl_launch(gf2_permute_rows_kernel, (GB + GF2_PERM_WORDS - 1) / GF2_PERM_WORDS, GF2_PERM_THREADS, 0, c->stream,
-      d_Lb, GB, GB, d_perm, d_perm + cnt, cnt);
-        ctx_launched(c);
-      }
     }
     const int r0 = i + t;
-    const int r1 = (h.last_pos >= (uint32_t)r0) ? (int)h.last_pos : r0 - 1;
+    const int r1 = last_pos >= r0 ? last_pos : r0 - 1;
     const int below = r1 - r0 + 1;
     if (delayed < 0) {
       delayed = below >= DELAY_ROWS && bw1 < nw;
@@ -939,34 +1003,37 @@ int gf2_echelon_dev(Ctx *c, int m, int n, uint64_t *D, size_t ld, size_t *rank_o
         if (e != cudaSuccess) return ctx_cuda(c, e, "gf2 echelon: multipliers");
       }
     }
+    // the rest of the block's words (delayed), or of all words
+    const int w1 = wc + 1, wend = delayed ? bw1 : nw;
+    uint64_t *L11 = delayed ? d_L11s + (size_t)np * GW : d_L11;
     {
       const int rows = r1 - i + 1;
       pi = prof_begin(c, "gf2_solve");
-      pdl_launch(gf2_solve_kernel, std::max(1, std::min((rows + 255) / 256, c->num_sms * 4)), 256, 0,
-                 c->stream, D, ld, i, r1, wc, pmask, t, d_pcol, d_U, d_L11, d_L21);
+      pdl_launch(gf2_solve_kernel,
+                 std::max(1, std::min((rows + GF2_SOLVE_THREADS - 1) / GF2_SOLVE_THREADS, c->num_sms * 4)),
+                 GF2_SOLVE_THREADS, 0, c->stream, D, ld, i, r1, wc, pmask, t, d_pcol, d_U, L11, d_L21,
+                 delayed ? d_Lb : nullptr, Tb, w1, wend);
       prof_end(c, pi);
       ctx_launched(c);
     }
-    if (delayed) {
-      const int rows = r1 - i + 1;
-      pdl_launch(gf2_deposit_kernel, std::max(1, std::min((rows + 255) / 256, c->num_sms * 4)), 256,
-                 0, c->stream, d_Lb, i, r1, t, Tb, d_L11, d_L21);
-      e = cudaMemcpyAsync(d_L11s + (size_t)np * GW, d_L11, (size_t)t * 8, cudaMemcpyDeviceToDevice,
-                          c->stream);
-      if (e != cudaSuccess) return ctx_cuda(c, e, "gf2 echelon: panel multipliers");
-      ctx_launched(c);
-    }
-    // the rest of the block's words (delayed), or of all words
-    const int w1 = wc + 1, wend = delayed ? bw1 : nw;
     if (w1 < wend) {
-      pdl_launch(gf2_l11_solve_kernel, (wend - w1 + GF2_L11_THREADS / 32 - 1) / (GF2_L11_THREADS / 32), GF2_L11_THREADS, 0, c->stream,
-      D, ld, i, t, w1, wend, d_L11);
-      ctx_launched(c);
+      if (!delayed) {
+        pdl_launch(gf2_l11_solve_kernel,
+                   (wend - w1 + GF2_L11_THREADS / 32 - 1) / (GF2_L11_THREADS / 32), GF2_L11_THREADS, 0,
+                   c->stream, D, ld, i, t, w1, wend, L11);
+        ctx_launched(c);
+      }
       if (below > 0) {
         // rows r0..r1, those words: C ^= L21 (one word of t bits per row) * U12
         pi = prof_begin(c, "gf2_update");
-        st = gf2_m4rm_dev(c, below, std::min(n, 64 * wend) - 64 * w1, t, 1, d_L21, 1,
-                          D + (size_t)i * ld + w1, ld, 1, D + (size_t)r0 * ld + w1, ld);
+        if (wend - w1 <= GB) {
+          pdl_launch(gf2_block_words_kernel, std::min((below + 31) / 32, c->num_sms * 4),
+                     GF2_BW_THREADS, 0, c->stream, D, ld, n, i, t, w1, wend - w1, r0, r1, d_L21);
+          ctx_launched(c);
+        } else {
+          st = gf2_m4rm_dev(c, below, std::min(n, 64 * wend) - 64 * w1, t, 1, d_L21, 1,
+                            D + (size_t)i * ld + w1, ld, 1, D + (size_t)r0 * ld + w1, ld);
+        }
         prof_end(c, pi);
         if (st) return st;
       }
