@@ -203,12 +203,14 @@ __device__ __forceinline__ void tri64_level(uint32_t *X, uint32_t *T, bool upper
     __syncthreads();
   }
 }
+// (n: the matrix is the identity from row n on; the same in every thread)
 template <class A>
-__device__ __forceinline__ void tri64_invert(uint32_t *X, uint32_t *T, bool upper, const A &ar, int t) {
+__device__ __forceinline__ void tri64_invert(uint32_t *X, uint32_t *T, bool upper, const A &ar, int t,
+                                             int n = 64) {
 #pragma unroll 1
-  for (int lb = 0; lb < 4; ++lb) tri64_level<A, 1>(X, T, upper, ar, t, lb);
-  tri64_level<A, 2>(X, T, upper, ar, t, 4);
-  tri64_level<A, 4>(X, T, upper, ar, t, 5);
+  for (int lb = 0; lb < 4 && n > 1 << lb; ++lb) tri64_level<A, 1>(X, T, upper, ar, t, lb);
+  if (n > 16) tri64_level<A, 2>(X, T, upper, ar, t, 4);
+  if (n > 32) tri64_level<A, 4>(X, T, upper, ar, t, 5);
 }
 
 }  // namespace lela

@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(HEADS_THREADS)
 //
 // SearchSmall, 32 <= p <= 65521 (the largest prime below 2^16): signed
 // residues |v| <= p/2 + 4 and pivots inverted from a table of the inverses
-// of 0 .. p/2 (u16, 0: none), which the CTA holds in shared memory, so a row is reduced
+// of 0 .. p/2 + 5 (u16, 0: none), which the CTA holds in shared memory, so a row is reduced
 // with its true multiplier l: w - l P (NORM below).  Reduction: q = (x mu +
 // 2^(31+s)) >> (32 + s) with mu = round (2^(32+s) / p) in [2^30, 2^31) (s = 14
 // for p > 2^15, one less per halving of p) is x / p rounded, up to an error of
@@ -170,7 +170,7 @@ struct SearchSmall {
   static constexpr bool NORM = true;
   int p, mu, s;
   long long half;
-  const uint16_t *table;  // inverses of 0 .. p / 2
+  const uint16_t *table;  // inverses of 0 .. p / 2 + 5
   __host__ static bool takes(uint32_t p) { return p >= 32 && p <= 65521; }
   __host__ static SearchSmall make(uint32_t p, const uint16_t *table) {
     SearchSmall a;
@@ -205,22 +205,15 @@ struct SearchSmall {
   }
   // a b, also for one factor in (-p, p)
   __device__ __forceinline__ int plain(int a, int b) const { return red(a * b); }
-  // 1 / v in (-p, p), 0 if there is none (|v| <= p/2 + 5 and v is the
-  // residue of smallest magnitude: a few past p/2 are folded back)
-  __device__ __forceinline__ int inverse(const uint16_t *tab, int v) const {
-    int a = abs(v);
-    const bool past = a > (p >> 1);
-    if (past) a = p - a;
-    const int i = tab[a];
-    return (v < 0) != past ? -i : i;
-  }
+  // 1 / |v| in [0, p), 0 if there is none
+  __device__ __forceinline__ int inverse_abs(const uint16_t *tab, int v) const { return tab[abs(v)]; }
   __device__ __forceinline__ uint32_t canon(int v) const { return (uint32_t)(v < 0 ? v + p : v); }
 };
 
-// The inverses of 0 .. p / 2 modulo p < 2^16, 0 for those that have none.
+// The inverses of 0 .. p / 2 + 5 modulo p < 2^16, 0 for those that have none.
 __global__ void inverse_table_kernel(uint32_t p, uint16_t *__restrict__ table) {
   const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x <= p / 2) table[x] = (uint16_t)inv_exact_u32(p, x);
+  if (x <= p / 2 + 5) table[x] = (uint16_t)inv_exact_u32(p, x);
 }
 
 // SearchMont, other odd p < 2^31: canonical residues, Montgomery reduction
@@ -332,14 +325,20 @@ struct SearchWide {
 // the window rows and of the block's pivot rows from those coefficients (rows
 // on warps, columns on lanes).
 //
-// Bound: the instructions on warp 0's dependent chain (about 130 a column) and
-// the issue slots of the block updates.  Measured on a 64 x 64 window (p =
-// 65521, a panel of a dense 4096^2 matrix): 520 cycles a column for the
-// pivots, 420 for the updates, of 78000 for the panel (41 us).  Forms with one
+// With NORM arithmetic warp 0 goes on to the next block at once: it applies the
+// block before to its four columns itself, while twelve warps on the other
+// three schedulers form the columns further right.
+//
+// Bound: the instructions on warp 0's dependent chain, four to five cycles each.
+// Measured on a 64 x 64 window (p = 65521, a panel of a dense 4096^2 matrix),
+// cycles a block of four columns: 1200 to load and bring up its columns, 1650 for
+// the pivots, 350 for lists and barrier; 56000 for the panel's sixteen.  With
+// the updates of a block between its pivots and the next block's 60800, and with
+// all fifteen other warps on them, sharing warp 0's scheduler, 58400.  Forms with one
 // barrier per column and all 16 warps on it (window in shared memory, lanes
 // on rows; or rows in registers, a warp per row) took 1640 cycles a column
 // (80 us a panel, at 2^31 - 1 102 us).  Rolled loops, the panel's inverse
-// included, were slower (44500 + 31400 cycles against 33500 + 26800).  On this
+// included, were slower.  On this
 // chip a ballot takes 26 cycles, __ffs 40, __reduce_min_sync 22, so the pivot's
 // lane comes from the reduction.
 //
@@ -366,7 +365,7 @@ static_assert(PS_THREADS == 2 * INV_THREADS, "half of the CTA per inverse");
 constexpr int PW_AREA = PW_R * PW_LD > INV_WORDS ? PW_R * PW_LD : INV_WORDS;
 constexpr int PW_LROWS = PW_R + EW;
 constexpr size_t PW_SMEM = ((size_t)(PW_AREA + PW_LROWS * PW_LD) * 4 + 15) / 16 * 16;
-constexpr size_t PW_TABLE = 65536;
+constexpr size_t PW_TABLE = 65536 + 64;
 // positions a thread looks at per pass of the window's compaction
 constexpr int PW_U = 4;
 
@@ -385,15 +384,18 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
   V(*Lm)[PW_LD] = reinterpret_cast<V(*)[PW_LD]>(dyn_w + PW_AREA);  // [slot][pivot] (division-free: raw)
   const uint16_t *s_inv = reinterpret_cast<const uint16_t *>(dyn_w + PW_SMEM / 4);
   __shared__ V PV[EW][EW];
-  __shared__ V4 s_coef[PW_R];         // per slot: its coefficients of the block's pivot rows
-  V *s_coefv = reinterpret_cast<V *>(s_coef);
-  __shared__ V4 s_pcoef[PB];          // division-free: z of the block's pivot rows when chosen,
-  __shared__ V s_psc[PB], s_sc;       // their scales, and the other rows'
-  // slot of the pivot of the block's column j (-1: none)
-  __shared__ __align__(16) int s_pslot[PB];
+  // per block, double-buffered (warp 0 is one block ahead): per slot the
+  // coefficients of the block's pivot rows, by pivot; division-free by column, and
+  // z of the block's pivot rows when chosen, their slots (-1: no pivot in the
+  // column) and scales, and the other rows' scale
+  __shared__ V4 s_coef[2][PW_R], s_pcoef[2][PB];
+  __shared__ __align__(16) int s_pj[2][PB];
+  __shared__ V s_psc[2][PB], s_sc[2];
+  // the block's end, its stop, the pivots before and after it, live entries after it
+  __shared__ int s_next[2], s_rare[2], s_t0[2], s_t[2], s_nl[2], s_col0;
   __shared__ V s_red[PS_FAST][EW];    // rows past the window, reduced (one per warp),
   __shared__ V s_rl[PS_FAST][EW];     // and their multipliers (raw)
-  __shared__ int s_ent[PW_R], s_epos[PW_R], wrow[PW_R];
+  __shared__ int s_ent[2][PW_R], s_epos[2][PW_R], wrow[PW_R];
   __shared__ int2 s_piv[EW];          // pivot column, transposition target
   __shared__ int s_prow[EW];          // the pivot's row of Lm
   __shared__ V s_y[EW], s_sinv[EW];   // pivot values (in window rows' scale), 1 / S_k
@@ -404,8 +406,6 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
   __shared__ int s_first[PS_FAST], s_wcnt[PW_U * PS_FAST];
   __shared__ int s_list[PS_THREADS], s_lrow[PS_THREADS], s_lhead[PS_THREADS];
   __shared__ int s_err, s_last, s_hi, s_wlast, s_uinv;
-  // block's end, its stop, the pivots before and after it, live entries
-  __shared__ int s_next, s_rare, s_t0, s_t, s_nl;
   const uint32_t p = (uint32_t)sa.p;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   constexpr unsigned FULL = 0xffffffffu;
@@ -413,7 +413,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
   if constexpr (SA::NORM) {
     // the table of inverses, on its way while the window is formed
     char *dst = reinterpret_cast<char *>(dyn_w) + PW_SMEM;
-    for (int e = tid; e < (int)(p / 2 + 1 + 7) / 8; e += PS_THREADS)
+    for (int e = tid; e < (int)(p / 2 + 6 + 7) / 8; e += PS_THREADS)
       cp_async16(dst + 16 * e, reinterpret_cast<const char *>(sa.table) + 16 * e);
   }
   // (the table was complete before the memsets that precede the first panel)
@@ -463,8 +463,8 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
       const int off = before + __popc(bal[u] & ((1u << lane) - 1u));
       if (hd[u] < HEAD_NONE && off < take) {
         const int slot = nl + off, pos = base + u * PS_THREADS + tid;
-        s_ent[slot] = slot;
-        s_epos[slot] = pos;
+        s_ent[0][slot] = slot;
+        s_epos[0][slot] = pos;
         wrow[slot] = pos;
         atomicSub(&s_cnt[hd[u]], 1);  // the window's rows leave the counts
         if (off == wcap - 1 - nl) s_wlast = pos;
@@ -493,14 +493,29 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
   if constexpr (SA::NORM) cp_async_wait_all();
   __syncthreads();
   const int wlast = s_wlast;  // rows past it are outside the window
-
+  // the final values of the nb pivot rows of a block (buffer b, from pivot tb) in
+  // one column, in place: U_k = P_k - sum l_kj U_j
+  [[maybe_unused]] auto finish = [&](V(&P)[PB], int b, int tb, int nb) {
+    if constexpr (SA::NORM) {
+      const V4 l1 = s_coef[b][s_prow[tb + (1 < nb ? 1 : 0)]], l2 = s_coef[b][s_prow[tb + (2 < nb ? 2 : 0)]];
+      V4 l3 = s_coef[b][s_prow[tb + (3 < nb ? 3 : 0)]];
+      l3.w = 0;
+      P[1] = 1 < nb ? sa.step(P[1], l1.x, P[0]) : 0;
+      P[2] = 2 < nb ? sa.step2(P[2], l2.x, P[0], l2.y, P[1]) : 0;
+      const V u3 = sa.lin(P[3], l3, P);
+      P[3] = 3 < nb ? u3 : 0;
+    }
+  };
   int t = 0, col0 = 0;  // pivots so far; the current row is i0 + t
+  int buf = 0;          // the block's buffer; the live entries on entry are list `buf`
 
   // A. warp 0: the pivots of the block's columns, with NG groups of entries.
   // z holds, per entry, the block's columns from the current one on, and
   // behind them (division-free) the coefficients of the block's pivot rows
-  // chosen so far: each column drops z[0] and appends its own.
-  auto choose = [&](auto ng_c) {
+  // chosen so far: each column drops z[0] and appends its own.  `ahead`: the
+  // block's columns still lack the block before, which the other warps are
+  // applying to the columns right of it (B): warp 0 applies it here.
+  auto choose = [&](auto ng_c, bool ahead) {
     constexpr int NG = decltype(ng_c)::value;
     constexpr uint32_t NONE = 255;
     V z[PB][NG];
@@ -518,83 +533,91 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
       const int e = lane + 32 * g;
       const bool in = e < nl;
       live[g] = in ? (uint32_t)e : NONE;
-      ent[g] = in ? s_ent[e] : 0;
-      pos[g] = in ? s_epos[e] : 0;
+      ent[g] = in ? s_ent[buf][e] : 0;
+      pos[g] = in ? s_epos[buf][e] : 0;
 #pragma unroll
       for (int j = 0; j < PB; ++j) z[j][g] = (in && col0 + j < w) ? Wv[ent[g]][col0 + j] : 0;
     }
+    if (SA::NORM && ahead) {
+      const int pb = buf ^ 1, tb = s_t0[pb], nb = t - tb, c = col0 + (lane & (PB - 1));
+      V P[PB];
+#pragma unroll
+      for (int k = 0; k < PB; ++k) P[k] = k < nb && c < w ? Wv[s_prow[tb + k]][c] : 0;
+      if constexpr (SA::NORM) finish(P, pb, tb, nb);
+      V U[PB][PB];  // [column][pivot], from lanes 0 .. PB - 1
+#pragma unroll
+      for (int j = 0; j < PB; ++j)
+#pragma unroll
+        for (int k = 0; k < PB; ++k) U[j][k] = __shfl_sync(FULL, P[k], j);
+      [[maybe_unused]] const V psc = s_sc[pb];
+#pragma unroll
+      for (int g = 0; g < NG; ++g) {
+        const V4 cf = s_coef[pb][ent[g]];
+        if (live[g] != NONE) {
+#pragma unroll
+          for (int j = 0; j < PB; ++j) {
+            if constexpr (SA::NORM) z[j][g] = sa.lin(z[j][g], cf, U[j]);
+            else z[j][g] = sa.lin(psc, z[j][g], cf, U[j]);
+            Wv[ent[g]][min(col0 + j, PW_LD - 1)] = z[j][g];
+          }
+        }
+      }
+    }
+    if (!SA::NORM && lane < PB) s_pj[buf][lane] = -1;
+    __syncwarp();
     const int t0 = t;
     [[maybe_unused]] V sc = 0;
     if constexpr (!SA::NORM) sc = sa.one();
     int next = min(col0 + PB, w), rare = -1;
-    if (lane < PB) s_pslot[lane] = -1;
-    __syncwarp();
+    V *coef[NG];
+#pragma unroll
+    for (int g = 0; g < NG; ++g) coef[g] = reinterpret_cast<V *>(&s_coef[buf][ent[g]]);
 #pragma unroll
     for (int j = 0; j < PB; ++j) {
-      constexpr int ZALL = PB;
-      const int zn = SA::NORM ? PB - j : ZALL;  // entries of z in use
-      const int col = col0 + j, i = i0 + t;
-      // the pivot's entry and the first live one
-      uint32_t key = NONE, fkey = NONE;
+      const int zn = SA::NORM ? PB - j : PB;  // entries of z in use
+      const int col = col0 + j, nb = t - t0;
+      // the pivot's entry (columns past w are zero)
+      uint32_t key = NONE;
 #pragma unroll
-      for (int g = 0; g < NG; ++g) {
-        if (z[0][g] != 0) key = min(key, (uint32_t)(lane + 32 * g));
-        fkey = min(fkey, live[g]);
+      for (int g = 0; g < NG; ++g) key = min(key, z[0][g] != 0 ? live[g] : NONE);
+      [[maybe_unused]] int inv[NG];  // each row's inverse, looked up meanwhile
+      if constexpr (SA::NORM) {
+#pragma unroll
+        for (int g = 0; g < NG; ++g) inv[g] = sa.inverse_abs(s_inv, z[0][g]);
       }
-      key = __reduce_min_sync(FULL, col < next && i < m ? key : NONE);
+      key = __reduce_min_sync(FULL, rare < 0 ? key : NONE);
       V znew[NG];
 #pragma unroll
       for (int g = 0; g < NG; ++g) znew[g] = 0;
       if (key == NONE) {
         // none in the window: rows past it whose bound allows a pivot here
         // end the block (all warps look for it)
-        if (col < next && i < m && wlast < m - 1) {
+        if (wlast < m - 1 && col < next && i0 + t < m) {
           const int v = (lane <= col ? s_cnt[lane] : 0) + (lane + 32 <= col ? s_cnt[lane + 32] : 0);
           if (__reduce_add_sync(FULL, v) > 0) {
             rare = col;
             next = col;
           }
         }
-        if constexpr (SA::NORM) {
-#pragma unroll
-          for (int g = 0; g < NG; ++g)
-            if (live[g] != NONE) s_coefv[PB * ent[g] + j] = 0;
-        }
       } else {
-        // each row's inverse, looked up while the pivot's lane is found
-        [[maybe_unused]] int inv[NG];
-        if constexpr (SA::NORM) {
-#pragma unroll
-          for (int g = 0; g < NG; ++g) inv[g] = sa.inverse(s_inv, z[0][g]);
-        }
         const int pg = (int)key >> 5, pl = (int)key & 31;
         V pv[PB];  // the pivot row's z
         [[maybe_unused]] int iv = 0;
-        if constexpr (SA::NORM) iv = __shfl_sync(FULL, sel(inv, pg), pl);
 #pragma unroll
-        for (int k = 0; k < PB; ++k)
-          pv[k] = k < zn ? __shfl_sync(FULL, sel(z[k], pg), pl) : 0;
+        for (int k = 0; k < PB; ++k) pv[k] = k < zn ? __shfl_sync(FULL, sel(z[k], pg), pl) : 0;
+        if constexpr (SA::NORM) {
+          iv = __shfl_sync(FULL, sel(inv, pg), pl);
+          iv = pv[0] < 0 ? -iv : iv;
+        }
         const int q = __shfl_sync(FULL, sel(pos, pg), pl);
-        fkey = __reduce_min_sync(FULL, fkey);
         if constexpr (SA::NORM) {
 #pragma unroll
           for (int g = 0; g < NG; ++g) {
             const V l = sa.plain(z[0][g], iv);  // 1 for the pivot row
-            if (live[g] != NONE) {  // by slot
-              s_coefv[PB * ent[g] + j] = l;
-              Lm[ent[g]][t] = l;
-            }
 #pragma unroll
             for (int k = 1; k < PB; ++k)
               if (k < zn) z[k][g] = sa.step(z[k][g], l, pv[k]);
-          }
-          if (iv == 0) {  // no inverse: the call will fail, the row leaves all the same
-            if (lane == 0) s_err = 1;
-#pragma unroll
-            for (int g = 0; g < NG; ++g)
-#pragma unroll
-              for (int k = 1; k < PB; ++k)
-                if (lane == pl && g == pg) z[k][g] = 0;
+            if (live[g] != NONE) coef[g][nb] = l;  // by slot
           }
         } else {
 #pragma unroll
@@ -607,30 +630,35 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
           }
         }
         if (lane == pl) {
-          s_pslot[j] = sel(ent, pg);
           s_piv[t] = make_int2(col, q);
           s_prow[t] = sel(ent, pg);
           s_y[t] = pv[0];
           if constexpr (SA::NORM) {
             s_xi[t] = iv;
           } else {
-            s_psc[j] = sc;
+            s_psc[buf][j] = sc;
+            s_pj[buf][j] = sel(ent, pg);
             V4 c4;  // (only the coefficients of earlier columns are read)
             c4.x = pv[0];
             c4.y = pv[1];
             c4.z = pv[2];
             c4.w = pv[3];
-            s_pcoef[j] = c4;
+            s_pcoef[buf][j] = c4;
           }
         }
         if constexpr (!SA::NORM) sc = sa.mul(pv[0], sc);
         uint32_t gone = key;  // the entry that goes
-        if (!(fkey == key && q == i)) {
+        if (q != i0 + t) {
           // position i: the first entry's row, or a row outside the window
+          const int i = i0 + t;
+          uint32_t fkey = NONE;
+#pragma unroll
+          for (int g = 0; g < NG; ++g) fkey = min(fkey, live[g]);
+          fkey = __reduce_min_sync(FULL, fkey);
           const int fg = (int)fkey >> 5, fl = (int)fkey & 31;
           const int f = __shfl_sync(FULL, sel(pos, fg), fl);
           if (f != i) {
-            if (q != i && lane == 0) {
+            if (lane == 0) {
               p2r[q] = row_at(i, p2r, stamp, epoch);
               stamp[q] = epoch;
             }
@@ -643,16 +671,15 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
             for (int k = 1; k < PB; ++k) {
               const V vx = __shfl_sync(FULL, sel(z[k], fg), fl);
 #pragma unroll
-              for (int g = 0; g < NG; ++g) {
-                if (g == fg && lane == fl) z[k][g] = 0;
+              for (int g = 0; g < NG; ++g)
                 if (g == pg && lane == pl) z[k][g] = vx;
-              }
             }
 #pragma unroll
             for (int g = 0; g < NG; ++g)
               if (g == pg && lane == pl) {
                 ent[g] = en;
                 znew[g] = vn;
+                coef[g] = reinterpret_cast<V *>(&s_coef[buf][en]);
               }
           }
         }
@@ -668,115 +695,138 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
         z[PB - 1][g] = znew[g];
       }
     }
-    // the live entries closed up (division-free: and their coefficients)
+    // the live entries closed up (division-free: and their coefficients of the
+    // block's pivot rows, which stand in z by column)
+    __syncwarp();
     int base = 0;
 #pragma unroll
     for (int g = 0; g < NG; ++g) {
       const unsigned alive = __ballot_sync(FULL, live[g] != NONE);
       if (live[g] != NONE) {
         const int e = base + __popc(alive & ((1u << lane) - 1u));
-        s_ent[e] = ent[g];
-        s_epos[e] = pos[g];
+        s_ent[buf ^ 1][e] = ent[g];
+        s_epos[buf ^ 1][e] = pos[g];
         if constexpr (!SA::NORM) {
           V4 c4;
           c4.x = z[0][g];
           c4.y = z[1][g];
           c4.z = z[2][g];
           c4.w = z[3][g];
-          s_coef[ent[g]] = c4;
+          s_coef[buf][ent[g]] = c4;
         }
       }
       base += __popc(alive);
     }
     if (lane == 0) {
-      s_sc = sc;
-      s_next = next;
-      s_rare = rare;
-      s_t0 = t0;
-      s_t = t;
-      s_nl = base;
+      s_sc[buf] = sc;
+      s_next[buf] = next;
+      s_rare[buf] = rare;
+      s_t0[buf] = t0;
+      s_t[buf] = t;
+      s_nl[buf] = base;
     }
+    nl = base;
+    if (lane == 0) s_col0 = col0;
+    col0 = next;
+    __syncwarp();
   };
 
+  bool ahead = false;
   while (col0 < w && i0 + t < m) {
     if (wid == 0) {
-      if (nl <= 32) choose(std::integral_constant<int, 1>{});
-      else if (nl <= 64) choose(std::integral_constant<int, 2>{});
-      else choose(std::integral_constant<int, PW_G>{});
+      if (nl <= 32) choose(std::integral_constant<int, 1>{}, ahead);
+      else if (nl <= 64) choose(std::integral_constant<int, 2>{}, ahead);
+      else choose(std::integral_constant<int, PW_G>{}, ahead);
     }
+    // the block's pivots are known, and the block before is applied to all
+    // columns right of this one
     __syncthreads();
-    // B. the columns right of the block, from the rows' values before it
-    const int next = s_next, rare = s_rare;
-    const int tb = s_t0;  // pivots before the block
-    const bool found_any = s_t > tb;
-    t = s_t;
-    nl = s_nl;
-    if (found_any) {
+    const int rare = s_rare[buf], tb = s_t0[buf], blk0 = wid == 0 ? s_col0 : col0;
+    col0 = s_next[buf];
+    t = s_t[buf];
+    nl = s_nl[buf];
+    // B. the other warps: the columns right of the block, from the rows'
+    // values before it; not those of the next block, which warp 0 takes
+    // itself while it chooses there (unless this one was cut short)
+    // (the twelve warps of the other three schedulers, so that warp 0 does not
+    // share its issue slots; division-free, where warp 0's own share costs more
+    // than it hides, all warps and all columns, and a barrier)
+    if ((!SA::NORM || (wid & 3) != 0) && t > tb) {
+      const int right = SA::NORM && rare < 0 ? col0 + PB : col0;
       // a warp takes one half of the columns while both have some left, and
-      // every eighth row, then every sixteenth of the upper half
-      const bool both = col0 < 32;
-      const int wh = both ? wid >> 1 : wid, nw = both ? PS_FAST / 2 : PS_FAST;
-      const int c = lane + (both ? 32 * (wid & 1) : 32);
-      const int4 ps = *reinterpret_cast<const int4 *>(s_pslot);
-      const int psk[PB] = {ps.x, ps.y, ps.z, ps.w};
-      V P[PB];  // the block's pivot rows, before it
+      // every sixth (eighth) row, then every twelfth (sixteenth) of the upper half
+      const bool both = blk0 < 32;
+      const int v0 = SA::NORM ? (wid >> 2) * 3 + (wid & 3) - 1 : wid;
+      const int warps = SA::NORM ? 12 : PS_FAST, wh = both ? v0 >> 1 : v0, nw = both ? warps / 2 : warps;
+      const int c = lane + (both ? 32 * (v0 & 1) : 32), nb = t - tb;
+      V P[PB];  // the block's pivot rows, before it (by pivot; division-free by column)
+      const int4 pj = SA::NORM ? make_int4(0, 0, 0, 0) : *reinterpret_cast<const int4 *>(s_pj[buf]);
+      const int slots[PB] = {pj.x, pj.y, pj.z, pj.w};
 #pragma unroll
-      for (int k = 0; k < PB; ++k) P[k] = psk[k] >= 0 && c >= col0 ? Wv[psk[k]][c] : 0;
-      if constexpr (SA::NORM) {
-        // the pivot rows' final values, in place: U_k = P_k - sum l_kj U_j
-        const V4 l1 = s_coef[max(psk[1], 0)], l2 = s_coef[max(psk[2], 0)];
-        V4 l3 = s_coef[max(psk[3], 0)];
-        l3.w = 0;
-        P[1] = psk[1] >= 0 ? sa.step(P[1], l1.x, P[0]) : 0;
-        P[2] = psk[2] >= 0 ? sa.step2(P[2], l2.x, P[0], l2.y, P[1]) : 0;
-        const V u3 = sa.lin(P[3], l3, P);
-        P[3] = psk[3] >= 0 ? u3 : 0;
+      for (int k = 0; k < PB; ++k) {
+        const bool there = SA::NORM ? k < nb : slots[k] >= 0;
+        P[k] = there && c >= blk0 ? Wv[SA::NORM ? s_prow[tb + k] : slots[k]][c] : 0;
       }
-      if (wh >= nw - PB) {  // the pivot rows to PV, a warp each (and half)
-        const int k = wh - (nw - PB);
-        int tk = tb, slot = -1;  // the pivot's index: pivots of earlier columns before it
-        V u = P[0];
+      if constexpr (SA::NORM) finish(P, buf, tb, nb);
+      {
+        // the pivot rows to PV, a warp each (and half)
+        int k = wh - (nw - PB), tk = tb + k;
+        bool mine = k >= 0 && k < nb;
+        if constexpr (!SA::NORM) {
+          mine = false;
+          tk = tb;
 #pragma unroll
-        for (int v = 0; v < PB; ++v) {
-          if (v < k) tk += psk[v] >= 0;
-          if (v == k) {
-            slot = psk[v];
-            u = P[v];
+          for (int x = 0; x < PB; ++x) {
+            if (x < k) tk += slots[x] >= 0;
+            if (x == k) mine = slots[x] >= 0;
           }
         }
-        if (slot >= 0) {
+        if (mine) {
+          V u = P[0];
+#pragma unroll
+          for (int x = 1; x < PB; ++x)
+            if (x == k) u = P[x];
           if constexpr (!SA::NORM) {
             // at its choice in column k the row's coefficients of columns 0 .. k - 1
             // stood behind the 4 - k columns left
-            const V *zz = reinterpret_cast<const V *>(&s_pcoef[k]);
+            const V *zz = reinterpret_cast<const V *>(&s_pcoef[buf][k]);
             V4 cf;
             cf.x = k > 0 ? zz[PB - k] : 0;
             cf.y = k > 1 ? zz[PB - k + 1] : 0;
             cf.z = k > 2 ? zz[PB - k + 2] : 0;
             cf.w = 0;
-            u = sa.lin(s_psc[k], u, cf, P);
+            u = sa.lin(s_psc[buf][k], u, cf, P);
+          } else if (c == lane + 32 && lane < k) {  // (one of the halves)
+            Lm[s_prow[tb + k]][tb + lane] = reinterpret_cast<const V *>(&s_coef[buf][s_prow[tb + k]])[lane];
           }
-          if (c >= col0) PV[tk][c] = u;
+          if (c >= blk0) PV[tk][c] = u;
+        }
+        [[maybe_unused]] const V sc = s_sc[buf];
+#pragma unroll 2
+        for (int e = wh; e < nl; e += nw) {
+          const int slot = s_ent[buf ^ 1][e];
+          const V4 cf = s_coef[buf][slot];
+          V v = Wv[slot][c];
+          if constexpr (SA::NORM) {
+            v = sa.lin(v, cf, P);
+            if (c == lane + 32 && lane < nb)
+              Lm[slot][tb + lane] = lane == 0 ? cf.x : lane == 1 ? cf.y : lane == 2 ? cf.z : cf.w;
+          } else {
+            v = sa.lin(sc, v, cf, P);
+          }
+          if (c >= right) Wv[slot][c] = v;
         }
       }
-      [[maybe_unused]] const V sc = s_sc;
-#pragma unroll 2
-      for (int e = wh; e < nl; e += nw) {
-        const int slot = s_ent[e];
-        const V4 cf = s_coef[slot];
-        V v = Wv[slot][c];
-        if constexpr (SA::NORM) v = sa.lin(v, cf, P);
-        else v = sa.lin(sc, v, cf, P);
-        if (c >= next) Wv[slot][c] = v;
-      }
     }
-    col0 = next;
-    __syncthreads();  // the window and PV are complete; s_* may be rewritten
+    ahead = SA::NORM && rare < 0 && t > tb;
+    buf ^= 1;
+    if constexpr (!SA::NORM) __syncthreads();
     if (rare < 0) continue;
 
     // C. column `rare`: no window row has a pivot, rows past the window may
+    __syncthreads();  // the window and PV are complete
     const int col = rare, i = i0 + t;
-    const bool z = nl > 0 && s_epos[0] == i;  // the row at position i is the first entry's
+    const bool z = nl > 0 && s_epos[buf][0] == i;  // the row at position i is the first entry's
     int cand;
     {
       const int v = (lane <= col ? s_cnt[lane] : 0) + (lane + 32 <= col ? s_cnt[lane + 32] : 0);
@@ -869,7 +919,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
     if (wid == 0) {
       int ri = -1;
       if (z) {
-        const int slot = s_ent[0];
+        const int slot = s_ent[buf][0];
         const unsigned b0 = __ballot_sync(FULL, lane > col && Wv[slot][lane] != 0);
         const unsigned b1 = __ballot_sync(FULL, lane + 32 > col && Wv[slot][lane + 32] != 0);
         const int hd = b0 ? __ffs(b0) - 1 : (b1 ? 32 + __ffs(b1) - 1 : HEAD_NONE);
@@ -883,16 +933,16 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
 #pragma unroll
         for (int g = 0; g < PW_G; ++g) {
           const int e = lane + 32 * g + 1;
-          en[g] = e < nl ? s_ent[e] : 0;
-          po[g] = e < nl ? s_epos[e] : 0;
+          en[g] = e < nl ? s_ent[buf][e] : 0;
+          po[g] = e < nl ? s_epos[buf][e] : 0;
         }
         __syncwarp();
 #pragma unroll
         for (int g = 0; g < PW_G; ++g) {
           const int e = lane + 32 * g + 1;
           if (e < nl) {
-            s_ent[e - 1] = en[g];
-            s_epos[e - 1] = po[g];
+            s_ent[buf][e - 1] = en[g];
+            s_epos[buf][e - 1] = po[g];
           }
         }
       }
@@ -906,8 +956,8 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
         s_prow[t] = PW_R + t;
         s_y[t] = y;
         if constexpr (SA::NORM) {
-          s_xi[t] = sa.inverse(s_inv, y);
-          if (s_xi[t] == 0) s_err = 1;
+          const int iv = sa.inverse_abs(s_inv, y);
+          s_xi[t] = y < 0 ? -iv : iv;
         }
       }
       PV[t][lane] = s_red[fw][lane];
@@ -917,11 +967,11 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
     }
     if (z) --nl;
     __syncthreads();
-    if (tid < nl) Lm[s_ent[tid]][t] = 0;  // the window rows' multipliers of this pivot
+    if (tid < nl) Lm[s_ent[buf][tid]][t] = 0;  // the window rows' multipliers of this pivot
     if constexpr (!SA::NORM) {
       // the window rows are zero in the column: they are scaled by y
       for (int e = wid; e < nl; e += PS_FAST) {
-        V *row = Wv[s_ent[e]];
+        V *row = Wv[s_ent[buf][e]];
         row[lane] = sa.mul(y, row[lane]);
         row[lane + 32] = sa.mul(y, row[lane + 32]);
       }
@@ -944,10 +994,12 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
   if (wid == 0) {
     // last final position of a non-pivot row with a nonzero panel, here of
     // the window rows left
-    for (int e = lane; e < nl; e += 32) atomicMax(&s_last, s_epos[e]);
+    for (int e = lane; e < nl; e += 32) atomicMax(&s_last, s_epos[buf][e]);
     const V unit = sa.load(1u % p);
     V x0 = unit, x1 = unit;
     if constexpr (SA::NORM) {
+      const bool none = (lane < t && s_xi[lane] == 0) || (lane + 32 < t && s_xi[lane + 32] == 0);
+      if (__any_sync(FULL, none) && lane == 0) s_err = 1;  // a pivot without an inverse
       if (lane < t) {
         x0 = s_y[lane];
         xinv_out[lane] = sa.canon(s_xi[lane]);
@@ -1108,7 +1160,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
     }
     __syncthreads();
     const bool upper = tid < INV_THREADS;
-    tri64_invert<A>(upper ? X : Y, upper ? T : T + INV_T, upper, ar, tid & (INV_THREADS - 1));
+    tri64_invert<A>(upper ? X : Y, upper ? T : T + INV_T, upper, ar, tid & (INV_THREADS - 1), t);
     for (int e = tid; e < t * EW; e += PS_THREADS) {
       Uinv_out[e] = X[e / EW * INV_LD + e % EW];
       Linv_out[e] = Y[e / EW * INV_LD + e % EW];
@@ -1381,7 +1433,7 @@ int zp_echelon_dev(Ctx *c, int m, int n, uint32_t p, uint32_t *D, size_t ld, siz
     void *tb = nullptr;
     if ((st = ctx_buffer(c, BUF_INV, PW_TABLE, &tb))) return st;
     if (c->inv_p != p) {
-      inverse_table_kernel<<<((int)p / 2 + 256) / 256, 256, 0, c->stream>>>(p, static_cast<uint16_t *>(tb));
+      inverse_table_kernel<<<((int)p / 2 + 261) / 256, 256, 0, c->stream>>>(p, static_cast<uint16_t *>(tb));
       ctx_launched(c);
       const cudaError_t ei = cudaGetLastError();
       if (ei != cudaSuccess) return ctx_cuda(c, ei, "echelon: inverses");
