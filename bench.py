@@ -436,13 +436,13 @@ def _event_ms(torch, stream, fn, reps):
 def run_dense(args, cm, stream, torch, dev, int8_peak):
     """The other dense workloads, inputs resident in HBM, CUDA events on the
     module's stream:
-    * gemm 8192^3 at p = 2^31 - 1 (four limbs: 16 limb products per output);
+    * gemm 8192^3 at p = 2^31 - 1 (by residues: 10 byte products per output);
     * trsm with the 8192 x 8192 unit-lower L (uniform off-diagonal entries)
       and an 8192 x 4096 right-hand side, at p = 65521 and 2^31 - 1;
     * the row-echelon form of a dense 8192 x 8192 matrix over Z/65521.
     Each with its roofline: algorithmic Z/p operations per second against
     the Z/p peak of its limb count (the int8 peak measured in this run /
-    limbs^2)."""
+    limbs^2; for the product by residues the byte products it does)."""
     from lela_b200 import gen
     n = 8192
     out = {}
@@ -460,12 +460,12 @@ def run_dense(args, cm, stream, torch, dev, int8_peak):
     kern = tc_ms / max(tc_n, 1)
     zp = 2.0 * n ** 3 / (ms / 1e3) / 1e12
     out["gemm_p31"] = {"workload": "gemm Z/2147483647 8192^3 C<-A*B+C", "ms": round(ms, 3),
-                       "Gop_s": round(zp * 1e3, 1), "limbs": 4,
-                       "roofline": {"bound": "tensor", "kernel": "zp_gemm_tc_kernel<4>",
+                       "Gop_s": round(zp * 1e3, 1), "byte_products": 10,
+                       "roofline": {"bound": "tensor", "kernel": "zp_gemm_tc_kernel<1, OUT_RNS>",
                                     "kernel_ms": round(kern, 3),
-                                    "achieved_int8_Tops": round(16 * 2.0 * n ** 3 / (kern / 1e3) / 1e12, 1),
+                                    "achieved_int8_Tops": round(10 * 2.0 * n ** 3 / (kern / 1e3) / 1e12, 1),
                                     "peak_int8_Tops": round(int8_peak, 1),
-                                    "frac": round(16 * 2.0 * n ** 3 / (kern / 1e3) / 1e12 / int8_peak, 4)}}
+                                    "frac": round(10 * 2.0 * n ** 3 / (kern / 1e3) / 1e12 / int8_peak, 4)}}
     del dA, dB, dC
     # trsm, both moduli
     out["trsm"] = {}

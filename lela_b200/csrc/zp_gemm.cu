@@ -17,6 +17,8 @@
 //        A*B = sum_s 2^(8s) D_s,   D_s = sum_{i+j=s} P_ij   (D_s < 4 * 2^31)
 //    reduces mod p with Barrett reduction and applies alpha and beta; the
 //    result is exact, i.e. bit-identical to LELA's.
+//    Four limbs' products of some size go by residues instead of limbs (see
+//    "residues of four limbs' work").
 //
 //    Data layout.  A is split into L planes of M x Kp bytes (K-major, i.e.
 //    row-major A), B into L planes of N x Kp bytes (K-major, i.e. B^T); Kp =
@@ -108,6 +110,15 @@ template <>
 struct TcCfg<4, 0> {
   static constexpr int BN = 32, NMMA = 128, STAGES = 2, ACC = 1, EPI = 8;
 };
+
+constexpr int RNS_MAX = 11;
+__host__ __device__ constexpr uint32_t rns_mod(int i) {
+  return i == 0 ? 256 : i == 1 ? 255 : i == 2 ? 253 : i == 3 ? 251 : i == 4 ? 247 : i == 5 ? 241
+       : i == 6 ? 239 : i == 7 ? 233 : i == 8 ? 229 : i == 9 ? 227 : 223;
+}
+// what the tensor-core kernel writes: residues modulo p, packed bits, or
+// residue bytes modulo rns_mod(i) (rns_combine_kernel)
+enum TcOut : int { OUT_ZP = 0, OUT_GF2 = 1, OUT_RNS = 2 };
 
 constexpr int BM = 128;         // rows of C per tile (UMMA M)
 constexpr int BK = 128;         // bytes (= limb elements) of K per stage
@@ -380,6 +391,41 @@ __device__ __forceinline__ void epilogue_gf2(uint32_t tcol, int gm, int gn0, int
   }
 }
 
+// Epilogue of residue product z for one thread: its row's columns [cbeg, cend)
+// of the tile modulo rns_mod(z), as bytes at plane z of C (M rows of `pitch`
+// bytes each, pitch the columns rounded up to 16; the columns past N are zero), 32 at a time
+// (one sector).
+__device__ __forceinline__ void epilogue_rns(uint32_t tcol, int gm, int gn0, int M, uint8_t *C,
+                                             size_t pitch, int z, int cbeg, int cend) {
+  const uint32_t m = rns_mod(z), mu = 0xFFFFFFFFu / m;  // (the quotient, or one less)
+  uint8_t *dst = C + ((size_t)z * M + gm) * pitch + gn0;
+#pragma unroll 1
+  for (int c0 = cbeg; c0 < cend; c0 += 32) {
+    uint32_t r[2][16];
+    tmem_ld16(tcol + c0, r[0]);
+    tmem_ld16(tcol + c0 + 16, r[1]);
+    tmem_ld_wait();
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      uint32_t w[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        w[j] = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          uint32_t v = r[h][4 * j + i];
+          v -= __umulhi(v, mu) * m;
+          v = min(v, v - m);
+          w[j] |= v << (8 * i);
+        }
+      }
+      const int c = c0 + 16 * h;
+      if (gm < M && (size_t)(gn0 + c) < pitch)
+        *reinterpret_cast<uint4 *>(dst + c) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  }
+}
+
 // K blocks [kb0, kb1) of the row tile starting at row m0: all of K, or,
 // with per-row ranges kr (row r of A is zero outside columns [kr[r].x,
 // kr[r].y) of the whole matrix; kbase = the whole matrix's column of this
@@ -484,7 +530,7 @@ __global__ void __launch_bounds__(tc_threads<L, T>(), 1)
                       const __grid_constant__ CUtensorMap tmB, void *Cv,
                       size_t ldc, int M, int N, int K, Modulus mod, uint32_t alpha, uint32_t beta,
                       uint32_t *err, const int2 *kr = nullptr, int kbase = 0) {
-  static_assert(OUT == 0 || (L == 1 && (T == 0 || T == GF2_TC_T)), "GF(2) output uses one limb");
+  static_assert(OUT == OUT_ZP || L == 1, "the byte outputs take one limb");
   uint32_t *C = static_cast<uint32_t *>(Cv);
   using Cfg = TcCfg<L, T>;
   using Lay = TcLayout<L, T>;
@@ -503,7 +549,9 @@ __global__ void __launch_bounds__(tc_threads<L, T>(), 1)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tiles_m = (M + BM - 1) / BM, tiles_n = (N + BN - 1) / BN;
-  const int num_tiles = tiles_m * tiles_n;
+  // OUT_RNS: alpha products, plane z of A times plane z of B
+  const int plane_tiles = tiles_m * tiles_n;
+  const int num_tiles = OUT == OUT_RNS ? (int)alpha * plane_tiles : plane_tiles;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) {
@@ -537,7 +585,8 @@ __global__ void __launch_bounds__(tc_threads<L, T>(), 1)
     bool ok = true;
     for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
       int mb, nb, kb0, kb1;
-      tile_coords(t, tiles_m, tiles_n, mb, nb);
+      const int z = OUT == OUT_RNS ? t / plane_tiles : 0;
+      tile_coords(t - z * plane_tiles, tiles_m, tiles_n, mb, nb);
       tile_kblocks(kr, kbase, mb * BM, M, K, kb0, kb1);
       if (lane == 0) {
         for (int kb = kb0; kb < kb1; ++kb) {
@@ -545,8 +594,8 @@ __global__ void __launch_bounds__(tc_threads<L, T>(), 1)
           uint8_t *sa = smem + s * Lay::STAGE_BYTES;
           uint8_t *sb = sa + Lay::A_BYTES;
           mbar_arrive_expect_tx(&full[s], Lay::STAGE_BYTES);
-          tma_load_3d(sa, &tmA, &full[s], kb * BK, mb * BM, 0);
-          tma_load_3d(sb, &tmB, &full[s], kb * BK, nb * BN, 0);
+          tma_load_3d(sa, &tmA, &full[s], kb * BK, mb * BM, z);
+          tma_load_3d(sb, &tmB, &full[s], kb * BK, nb * BN, z);
           issued |= 1u << s;
           last_ph[s] = ph;
           if (++s == S) { s = 0; ph ^= 1; }
@@ -567,7 +616,7 @@ __global__ void __launch_bounds__(tc_threads<L, T>(), 1)
     bool ok = true;
     for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it) {
       int mb, nb, kb0, kb1;
-      tile_coords(t, tiles_m, tiles_n, mb, nb);
+      tile_coords(OUT == OUT_RNS ? t % plane_tiles : t, tiles_m, tiles_n, mb, nb);
       tile_kblocks(kr, kbase, mb * BM, M, K, kb0, kb1);
       if (lane == 0) {
         const int a = it % ACC;
@@ -612,7 +661,7 @@ __global__ void __launch_bounds__(tc_threads<L, T>(), 1)
     const int row = q * 32 + lane;
     const int part = (warp - 2) >> 2;
     const int cbeg = part * (BN / (Cfg::EPI / 4));
-    if constexpr (OUT == 0) {
+    if constexpr (OUT == OUT_ZP) {
       const int emode = beta == 0u ? EPI_SET
                         : (beta == 1u && alpha == 1u) ? EPI_ADD
                         : (beta == 1u && alpha == (uint32_t)mod.p - 1u) ? EPI_SUB
@@ -631,15 +680,20 @@ __global__ void __launch_bounds__(tc_threads<L, T>(), 1)
       int it = 0;
       for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it) {
         int mb, nb;
-        tile_coords(t, tiles_m, tiles_n, mb, nb);
+        const int z = OUT == OUT_RNS ? t / plane_tiles : 0;
+        tile_coords(t - z * plane_tiles, tiles_m, tiles_n, mb, nb);
         const int a = it % ACC;
         const uint32_t aph = (uint32_t)(it / ACC) & 1u;
         const int gm = mb * BM + row;
         const uint32_t tbase = tmem + (uint32_t)(a * L * NMMA) + ((uint32_t)(q * 32) << 16);
         if (!mbar_wait(&tfull[a], aph, err)) break;
         tc_fence_after();
-        epilogue_gf2(tbase, gm, nb * BN, M, N, static_cast<uint64_t *>(Cv), ldc, alpha, beta,
-                     cbeg, cbeg + BN / (Cfg::EPI / 4));
+        if constexpr (OUT == OUT_RNS)
+          epilogue_rns(tbase, gm, nb * BN, M, static_cast<uint8_t *>(Cv), ldc, z, cbeg,
+                       cbeg + BN / (Cfg::EPI / 4));
+        else
+          epilogue_gf2(tbase, gm, nb * BN, M, N, static_cast<uint64_t *>(Cv), ldc, alpha, beta,
+                       cbeg, cbeg + BN / (Cfg::EPI / 4));
         tc_fence_before();
         mbar_arrive(&tempty[a]);
       }
@@ -840,6 +894,63 @@ __global__ void __launch_bounds__(DIR_THREADS, L == 4 ? 1 : 2)
   }
 }
 
+// ------------------------------------------------ residues of four limbs' work
+//
+// Four limbs take sixteen byte products per entry product.  Where the planes' extra
+// passes cost less, the product x = sum a b of the integers a, b < p, x < (p - 1)^2
+// K, is instead formed modulo n pairwise coprime moduli m_i <= 256 with P = prod
+// m_i > 2 x (n = 6 at p = 2^17, 10 at p = 2^31 and K = 4096): n one-limb products
+// of residue bytes, which the tensor-core kernel's epilogue reduces modulo m_i to
+// bytes again.  4096^3 at p = 2^31 - 1: 1015 -> 800 us a call (splits 140, products
+// 455 at 3.0 Pop/s, rns_combine_kernel 80).  Row blocks whose planes stay in L2 are no
+// faster (2048 rows 700 us, 1024 748, all 690).  A's residues carry the factor (P / m_i)^-1 mod m_i, so the
+// bytes are y_i with
+//     x = sum_i y_i (P / m_i) - t P,   t = floor(sum_i y_i / m_i),
+// and rns_combine_kernel takes that sum modulo p.  Exact: x / P < 1/2, so t is
+// floor(1/4 + sum y_i F_i / 2^15) with F_i = round(2^15 / m_i), whose error is
+// at most 11 * 255 / 2 / 2^15 < 0.05.
+// The bytes a split writes to plane l for four consecutive entries: limb l ...
+template <int L>
+struct LimbBytes {
+  static constexpr int MAX = L;
+  __device__ __forceinline__ constexpr int count() const { return L; }
+  __device__ __forceinline__ uint32_t in(uint32_t x, uint32_t) const { return x; }
+  __device__ __forceinline__ uint32_t word(const uint32_t (&v)[4], int l) const {
+    uint32_t w = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w |= ((v[i] >> (8 * l)) & 0xFFu) << (8 * i);
+    return w;
+  }
+};
+// ... or f_l x mod m_l: the bytes of x times those of coef (2^8b f_l mod m_l, at
+// byte b) sum to r < 2^18.  m = 256: its low byte.  Odd m: in floats, four
+// instructions at the full rate where the integer multiply-high and multiply go at
+// less (the splits are issue-bound: 4096^2 entries, ten moduli, A's 66 us
+// against 70, the limbs' 25).  2^23 + r is a float read from the bits; (r - (m - 1) / 2) / m rounds to floor(r / m), being at least 1 / 2m > 2^-9 from a
+// half-integer with an error below 2^-13; 2^23 + r - q m is exact.
+struct ResidueBytes {
+  static constexpr int MAX = RNS_MAX;
+  int n;
+  uint32_t coef[RNS_MAX];
+  __device__ __forceinline__ int count() const { return n; }
+  __device__ __forceinline__ uint32_t in(uint32_t x, uint32_t p) const { return x < p ? x : x % p; }
+  __device__ __forceinline__ uint32_t word(const uint32_t (&v)[4], int l) const {
+    const int m = (int)rns_mod(l);
+    uint32_t r[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      r[i] = __dp4a(v[i], coef[l], 0x4B000000u);
+      if (m != 256) {
+        const float f = __uint_as_float(r[i]);  // 2^23 + r
+        const float q = fmaf(f - (8388608.0f + (m - 1) / 2), 1.0f / m, 12582912.0f) - 12582912.0f;
+        r[i] = __float_as_uint(fmaf(q, (float)-m, f));
+      }
+    }
+    const uint32_t w = __byte_perm(__byte_perm(r[0], r[1], 0x0040), __byte_perm(r[2], r[3], 0x0040), 0x5410);
+    return w;
+  }
+};
+
 // ------------------------------------------------------------ limb splits
 // A (M x kc, row stride lda, elements T) -> L planes of bytes, row pitch Kp,
 // `plane` bytes apart.  Bound by
@@ -847,10 +958,10 @@ __global__ void __launch_bounds__(DIR_THREADS, L == 4 ? 1 : 2)
 // columns, a row per warp, so no index division.  part: 0 all columns; 1 (2)
 // only those left (right) of the row's diagonal block of nb rows.
 constexpr int SPLIT_ROWS = 8;  // rows (warps) per CTA
-template <int L, class T>
+template <class W, class T>
 __global__ void __launch_bounds__(32 * SPLIT_ROWS)
     split_rows_kernel(const T *A, size_t lda, int M, int kc, uint32_t p,
-                      uint8_t *out, size_t Kp, size_t plane, int part, int nb) {
+                      uint8_t *out, size_t Kp, size_t plane, int part, int nb, const W planes) {
   pdl_enter();
   for (int r = blockIdx.y * SPLIT_ROWS + threadIdx.y; r < M; r += gridDim.y * SPLIT_ROWS) {
     const T *src = A + (size_t)r * lda;
@@ -865,19 +976,15 @@ __global__ void __launch_bounds__(32 * SPLIT_ROWS)
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int k = 4 * (q + u * step) + i;
-          v[u][i] = 4 * (q + u * step) < ke && k < kc ? Rep<T>::in(src[k], p) : 0u;
+          v[u][i] = 4 * (q + u * step) < ke && k < kc ? planes.in(Rep<T>::in(src[k], p), p) : 0u;
         }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int k = 4 * (q + u * step);
         if (k >= ke) break;
 #pragma unroll
-        for (int l = 0; l < L; ++l) {
-          uint32_t w = 0;
-#pragma unroll
-          for (int i = 0; i < 4; ++i) w |= ((v[u][i] >> (8 * l)) & 0xFFu) << (8 * i);
-          *reinterpret_cast<uint32_t *>(dst + l * plane + k) = w;
-        }
+        for (int l = 0; l < W::MAX; ++l)
+          if (l < planes.count()) *reinterpret_cast<uint32_t *>(dst + l * plane + k) = planes.word(v[u], l);
       }
     }
   }
@@ -895,10 +1002,10 @@ template <class T>
 constexpr int split_cols_nt() {
   return sizeof(T) < 4 ? 128 / (int)sizeof(T) : 32;
 }
-template <int L, class T>
+template <class W, class T>
 __global__ void __launch_bounds__(256)
     split_cols_kernel(const T *B, size_t ldb, int kc, int N, uint32_t p,
-                      uint8_t *out, size_t Kp, size_t plane, int kout) {
+                      uint8_t *out, size_t Kp, size_t plane, int kout, const W planes) {
   pdl_enter();
   using R = typename Rep<T>::Packed;
   constexpr int NT = split_cols_nt<T>();
@@ -924,20 +1031,80 @@ __global__ void __launch_bounds__(256)
     if (gn < N && gk < kout) {
       uint32_t v[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) v[i] = tile[kw + i][n];
+      for (int i = 0; i < 4; ++i) v[i] = planes.in(tile[kw + i][n], p);
 #pragma unroll
-      for (int l = 0; l < L; ++l) {
-        uint32_t word = 0;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) word |= ((v[i] >> (8 * l)) & 0xFFu) << (8 * i);
-        *reinterpret_cast<uint32_t *>(out + l * plane + (size_t)gn * Kp + gk) = word;
-      }
+      for (int l = 0; l < W::MAX; ++l)
+        if (l < planes.count())
+          *reinterpret_cast<uint32_t *>(out + l * plane + (size_t)gn * Kp + gk) = planes.word(v, l);
     }
   }
 }
 template <class T>
 static dim3 split_cols_grid(int N, int Kp) {
   return dim3((N + split_cols_nt<T>() - 1) / split_cols_nt<T>(), (Kp + 63) / 64);
+}
+
+// ------------------------------------------------- residues back to Z/p
+// Weights of rns_combine_kernel: byte b of W[g][b] at position i is byte b of (P /
+// m_(4g+i)) mod p, F[g] the F_i, neg = -P mod p.
+struct RnsWeights {
+  int n;
+  uint32_t W[3][4], F[3], neg;
+};
+// C <- alpha x + beta C from the n residue planes Y (M rows of `pitch` bytes).
+// 4096^2 entries and n = 10 take 80 us: 300 MB, issue at 68 %.
+// Four columns a thread: the planes' words are transposed to words of one column and
+// multiplied bytewise (5 dp4a per four residues), S = sum of y_i ((P / m_i) mod p)
+// < 11 * 255 * 2^32 and t neg < 2^36 together, and one reduction.
+template <int MODE>
+__global__ void __launch_bounds__(256)
+    rns_combine_kernel(const uint8_t *Y, size_t pitch, uint32_t *C, size_t ldc, int M, int N,
+                       const RnsWeights rw, Modulus mod, uint32_t alpha, uint32_t beta) {
+  pdl_enter();
+  const int n = 4 * (blockIdx.x * 32 + threadIdx.x);
+  if (n >= N) return;
+  const bool vec = ((reinterpret_cast<uintptr_t>(C) & 15u) == 0) && ((ldc & 3u) == 0);
+  const size_t plane = (size_t)M * pitch;
+  for (int r = blockIdx.y * 8 + threadIdx.y; r < M; r += gridDim.y * 8) {
+    const uint8_t *src = Y + (size_t)r * pitch + n;
+    uint32_t y[12];
+#pragma unroll
+    for (int i = 0; i < 12; ++i)
+      y[i] = i < RNS_MAX && i < rw.n ? *reinterpret_cast<const uint32_t *>(src + i * plane) : 0u;
+    uint32_t *crow = C + (size_t)r * ldc;
+    uint32_t c[4];
+    if (MODE != EPI_SET) load_c<4>(c, crow, n, N, vec);
+    uint32_t s[4][4], t[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      t[j] = 1u << 13;
+#pragma unroll
+      for (int b = 0; b < 4; ++b) s[j][b] = 0;
+    }
+#pragma unroll
+    for (int g = 0; g < 3; ++g) {
+      const uint32_t lo01 = __byte_perm(y[4 * g], y[4 * g + 1], 0x5140);
+      const uint32_t lo23 = __byte_perm(y[4 * g + 2], y[4 * g + 3], 0x5140);
+      const uint32_t hi01 = __byte_perm(y[4 * g], y[4 * g + 1], 0x7362);
+      const uint32_t hi23 = __byte_perm(y[4 * g + 2], y[4 * g + 3], 0x7362);
+      const uint32_t col[4] = {__byte_perm(lo01, lo23, 0x5410), __byte_perm(lo01, lo23, 0x7632),
+                               __byte_perm(hi01, hi23, 0x5410), __byte_perm(hi01, hi23, 0x7632)};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        t[j] = __dp4a(col[j], rw.F[g], t[j]);
+#pragma unroll
+        for (int b = 0; b < 4; ++b) s[j][b] = __dp4a(col[j], rw.W[g][b], s[j][b]);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint64_t S = s[j][0] + ((uint64_t)s[j][1] << 8) + ((uint64_t)s[j][2] << 16) +
+                         ((uint64_t)s[j][3] << 24) + (uint64_t)(t[j] >> 15) * rw.neg;
+      c[j] = epi_combine<MODE, false>(mod_reduce(S, mod), MODE != EPI_SET ? c[j] : 0u, mod, Mod32(),
+                                      alpha, beta);
+    }
+    store_c<4>(c, crow, n, N, vec);
+  }
 }
 
 // ------------------------------------------------------------ plain gemm
@@ -1118,7 +1285,7 @@ static int encode_3d(Ctx *c, CUtensorMap *tm, void *base, uint64_t d0, uint64_t 
 
 template <int L, int T = 0>
 static int tc_attr(Ctx *c) {
-  return ctx_smem_attr(c, (const void *)zp_gemm_tc_kernel<L, 0, T>, TcLayout<L, T>::SMEM,
+  return ctx_smem_attr(c, (const void *)zp_gemm_tc_kernel<L, OUT_ZP, T>, TcLayout<L, T>::SMEM,
                        "cudaFuncSetAttribute(zp_gemm_tc)");
 }
 
@@ -1142,10 +1309,10 @@ static int launch_tc(Ctx *c, int M, int N, int K, const Modulus &mod, uint32_t a
     {
       const uint32_t p = (uint32_t)mod.p;
       int pi = prof_begin(c, "zp_split");
-      pdl_launch_if(early, split_rows_kernel<L, E>, split_rows_grid(c->num_sms, M, kc), dim3(32, SPLIT_ROWS),
-                 0, c->stream, A + k0, lda, M, kc, p, Al, (size_t)Kp, (size_t)M * Kp, 0, 1);
-      pdl_launch_if(early, split_cols_kernel<L, E>, split_cols_grid<E>(N, Kp), 256, 0, c->stream,
-                 B + (size_t)k0 * ldb, ldb, kc, N, p, Bl, (size_t)Kp, (size_t)N * Kp, Kp);
+      pdl_launch_if(early, split_rows_kernel<LimbBytes<L>, E>, split_rows_grid(c->num_sms, M, kc), dim3(32, SPLIT_ROWS),
+                 0, c->stream, A + k0, lda, M, kc, p, Al, (size_t)Kp, (size_t)M * Kp, 0, 1, LimbBytes<L>{});
+      pdl_launch_if(early, split_cols_kernel<LimbBytes<L>, E>, split_cols_grid<E>(N, Kp), 256, 0, c->stream,
+                 B + (size_t)k0 * ldb, ldb, kc, N, p, Bl, (size_t)Kp, (size_t)N * Kp, Kp, LimbBytes<L>{});
       prof_end(c, pi);
       ctx_launched(c, 2);
     }
@@ -1158,7 +1325,7 @@ static int launch_tc(Ctx *c, int M, int N, int K, const Modulus &mod, uint32_t a
     if (st) return st;
     const int grid = std::min(tiles, c->num_sms);
     int pi = prof_begin(c, "zp_gemm_tc");
-    pdl_launch_if(early, zp_gemm_tc_kernel<L, 0, T>, grid, tc_threads<L, T>(), Lay::SMEM, c->stream,
+    pdl_launch_if(early, zp_gemm_tc_kernel<L, OUT_ZP, T>, grid, tc_threads<L, T>(), Lay::SMEM, c->stream,
                tmA, tmB, C, ldc, M, N, kc, mod, alpha, b, c->dstatus, kr, kbase + k0);
     prof_end(c, pi);
     ctx_launched(c);
@@ -1167,6 +1334,148 @@ static int launch_tc(Ctx *c, int M, int N, int K, const Modulus &mod, uint32_t a
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return ctx_cuda(c, e, "zp_gemm_tc launch");
   return ST_OK;
+}
+
+// The residue split of a product of K terms modulo p: the moduli n (0: not
+// enough of them), A's and B's coefficients and the weights.
+static int rns_setup(uint32_t p, int K, ResidueBytes &ra, ResidueBytes &rb, RnsWeights &rw) {
+  const unsigned __int128 need = 2 * (unsigned __int128)((uint64_t)(p - 1) * (p - 1)) * (unsigned)K;
+  unsigned __int128 P = 1;
+  int n = 0;
+  while (n < RNS_MAX && P <= need) P *= rns_mod(n++);
+  if (P <= need) return 0;
+  ra = {};
+  rb = {};
+  rw = {};
+  ra.n = rb.n = rw.n = n;
+  for (int i = 0; i < n; ++i) {
+    const uint32_t m = rns_mod(i);
+    const unsigned __int128 q = P / m;
+    uint32_t f = 1;  // (P / m)^-1 mod m
+    while ((uint32_t)(q % m) * f % m != 1) ++f;
+    const uint32_t w = (uint32_t)(q % p);
+    for (int b = 0; b < 4; ++b) {
+      const uint32_t e = (uint32_t)((1ull << (8 * b)) % m);
+      rb.coef[i] |= e << (8 * b);
+      ra.coef[i] |= e * f % m << (8 * b);
+      rw.W[i / 4][b] |= (w >> (8 * b) & 0xFFu) << (8 * (i % 4));
+    }
+    rw.F[i / 4] |= (((1u << 15) + m / 2) / m) << (8 * (i % 4));
+  }
+  rw.neg = p - (uint32_t)(P % p);
+  return n;
+}
+
+// The product by residues in blocks of `rows` rows of A and C (B's planes are
+// made once).
+template <class E>
+static int launch_rns(Ctx *c, int M, int N, int K, int rows, const Modulus &mod, uint32_t alpha,
+                      const E *A, size_t lda, const E *B, size_t ldb, uint32_t beta, uint32_t *C,
+                      size_t ldc, uint8_t *ws, const ResidueBytes &ra, const ResidueBytes &rb,
+                      const RnsWeights &rw) {
+  using Lay = TcLayout<1, 0>;
+  constexpr int BN = TcCfg<1, 0>::BN;
+  if (int st = ctx_smem_attr(c, (const void *)zp_gemm_tc_kernel<1, OUT_RNS>, Lay::SMEM,
+                             "cudaFuncSetAttribute(zp_gemm_tc)"))
+    return st;
+  const int n = rw.n;
+  const size_t Kp = ((size_t)K + 15) & ~(size_t)15, Np = ((size_t)N + 15) & ~(size_t)15;
+  const uint32_t p = (uint32_t)mod.p;
+  uint8_t *Bl = ws, *Al = Bl + (size_t)n * N * Kp, *Y = Al + (size_t)n * rows * Kp;
+  const bool early = (double)M * N * K < 1e11;  // (as launch_tc)
+  int pi = prof_begin(c, "zp_split");
+  pdl_launch_if(early, split_cols_kernel<ResidueBytes, E>, split_cols_grid<E>(N, (int)Kp), 256, 0,
+                c->stream, B, ldb, K, N, p, Bl, Kp, (size_t)N * Kp, (int)Kp, rb);
+  prof_end(c, pi);
+  ctx_launched(c);
+  CUtensorMap tmA, tmB;
+  if (int st = encode_3d(c, &tmB, Bl, (uint64_t)K, (uint64_t)N, n, Kp, (uint64_t)N * Kp, BK, BN, 1))
+    return st;
+  for (int r0 = 0; r0 < M; r0 += rows) {
+    const int m = std::min(rows, M - r0);
+    uint32_t *Cr = C + (size_t)r0 * ldc;
+    pi = prof_begin(c, "zp_split");
+    pdl_launch_if(early, split_rows_kernel<ResidueBytes, E>, split_rows_grid(c->num_sms, m, K),
+                  dim3(32, SPLIT_ROWS), 0, c->stream, A + (size_t)r0 * lda, lda, m, K, p, Al, Kp,
+                  (size_t)m * Kp, 0, 1, ra);
+    prof_end(c, pi);
+    if (int st = encode_3d(c, &tmA, Al, (uint64_t)K, (uint64_t)m, n, Kp, (uint64_t)m * Kp, BK, BM, 1))
+      return st;
+    const long long tiles = (long long)n * ((m + BM - 1) / BM) * ((N + BN - 1) / BN);
+    pi = prof_begin(c, "zp_gemm_tc");
+    pdl_launch_if(early, zp_gemm_tc_kernel<1, OUT_RNS>, (int)std::min<long long>(tiles, c->num_sms),
+                  tc_threads<1, 0>(), Lay::SMEM, c->stream, tmA, tmB, Y, Np, m, N, K, mod,
+                  (uint32_t)n, 0u, c->dstatus, nullptr, 0);
+    prof_end(c, pi);
+    pi = prof_begin(c, "zp_combine");
+    const dim3 grid((N + 127) / 128, std::min((m + 7) / 8, 65535));
+#define LELA_RC(MODE)                                                                           \
+  pdl_launch_if(early, rns_combine_kernel<MODE>, grid, dim3(32, 8), 0, c->stream, Y, Np, Cr, ldc, \
+                m, N, rw, mod, alpha, beta)
+    if (beta == 0u) LELA_RC(EPI_SET);
+    else if (beta == 1u && alpha == 1u) LELA_RC(EPI_ADD);
+    else if (beta == 1u && alpha == p - 1u) LELA_RC(EPI_SUB);
+    else LELA_RC(EPI_AXPBY);
+#undef LELA_RC
+    prof_end(c, pi);
+    ctx_launched(c, 3);
+  }
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? ST_OK : ctx_cuda(c, e, "zp_gemm_tc launch");
+}
+
+// Whether a four-limb product goes by n residues.  They save 16 - n of 16 byte
+// products and cost planes n / 4 times as large and a pass over n bytes per entry of C.
+// Measured on the B200 (us per call from the host, limbs / residues; p = 2^16 + 1 has n =
+// 6, 2^24 - 3 8, 2^31 - 1 and 2^32 - 5 10): 4096^3 940 / 461, 576 and 693; 8192^3
+// 7062 / 2763, 7071 / 3559, 7398 / 4560; 2048^3 160 / 115, 129 and 150; 4096^2 x 512
+// 238 / 176, 201 and 226.  At n <= 8 down to 1024^2 x 2048 70 / 63 and 68, 512 x 8192 x
+// 512 89 / 84 and 87, while 1024^3 56 / 58 and 768^3 44 / 47; at n = 10 1536^3 95 / 91, 2048^2 x
+// 512 91 / 90, while 1024^2 x 8192 180 / 188, 512 x 8192 x 512 89 / 96, 1024^3 56 / 64.
+static bool rns_pays(int M, int N, int K, int n) {
+  return std::min(M, N) >= (n <= 8 ? 512 : 1536) && K >= 512 &&
+         (double)M * N * K >= 2147483648.0;
+}
+constexpr size_t RNS_MAX_BYTES = (size_t)4 << 30;
+constexpr int RNS_MIN_ROWS = 2048;
+
+// The product by residues where shape and modulus favour it and its planes can
+// be had: within RNS_MAX_BYTES in blocks of at least RNS_MIN_ROWS rows, and in the workspace as it is
+// inside a stream capture.  done says whether it was launched (else the limb
+// planes, which take less room, serve).
+template <class E>
+static int rns_try(Ctx *c, int M, int N, int K, uint32_t p, uint32_t alpha, const E *A, size_t lda,
+                   const E *B, size_t ldb, uint32_t beta, uint32_t *C, size_t ldc, bool &done) {
+  done = false;
+  if (zp_limbs_for(p) != 4 || K > ZP_KCHUNK) return ST_OK;
+  ResidueBytes ra, rb;
+  RnsWeights rw;
+  const int n = rns_setup(p, K, ra, rb, rw);
+  if (n == 0 || !rns_pays(M, N, K, n)) return ST_OK;
+  const size_t Kp = ((size_t)K + 15) & ~(size_t)15, Np = ((size_t)N + 15) & ~(size_t)15;
+  const size_t fixed = (size_t)n * N * Kp, per_row = (size_t)n * (Kp + Np);
+  if (fixed >= RNS_MAX_BYTES) return ST_OK;
+  const size_t most = (RNS_MAX_BYTES - fixed) / per_row;
+  int rows = M;
+  if ((size_t)M > most) {
+    if (most < RNS_MIN_ROWS) return ST_OK;
+    const int blocks = (int)((M + most - BM) / (most - BM + 1));
+    rows = ((M + blocks - 1) / blocks + BM - 1) / BM * BM;
+  }
+  const size_t bytes = fixed + (size_t)rows * per_row;
+  if (bytes > c->ws_bytes) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
+      return ST_OK;
+  }
+  void *w = nullptr;
+  if (ctx_workspace(c, bytes, &w)) {  // no room
+    cudaGetLastError();
+    return ST_OK;
+  }
+  done = true;
+  return launch_rns<E>(c, M, N, K, rows, make_modulus(p), alpha, A, lda, B, ldb, beta, C, ldc,
+                       static_cast<uint8_t *>(w), ra, rb, rw);
 }
 
 template <int L>
@@ -1308,6 +1617,11 @@ int zp_gemm_dev(Ctx *c, int kernel, int M, int N, int K, uint32_t p, uint32_t al
   }
   uint8_t *ws = ws_override;
   if (!ws) {
+    if (!kr) {
+      bool done;
+      const int st = rns_try<uint32_t>(c, M, N, K, p, alpha, A, lda, B, ldb, beta, C, ldc, done);
+      if (st || done) return st;
+    }
     void *w = nullptr;
     int st = ctx_workspace(c, zp_gemm_workspace_bytes(p, M, N, K), &w);
     if (st) return st;
@@ -1319,10 +1633,16 @@ int zp_gemm_dev(Ctx *c, int kernel, int M, int N, int K, uint32_t p, uint32_t al
 int zp_gemm_tc_elem_dev(Ctx *c, int elem, int M, int N, int K, uint32_t p, uint32_t alpha,
                         const void *A, size_t lda, const void *B, size_t ldb, uint32_t *V,
                         size_t ldv) {
+  alpha %= p;
+  if (elem == LELA_CUDA_ELEM_F64) {  // the only type with moduli of four limbs
+    bool done;
+    const int st = rns_try<double>(c, M, N, K, p, alpha, static_cast<const double *>(A), lda,
+                                   static_cast<const double *>(B), ldb, 0u, V, ldv, done);
+    if (st || done) return st;
+  }
   void *w = nullptr;
   if (int st = ctx_workspace(c, zp_gemm_workspace_bytes(p, M, N, K), &w)) return st;
   uint8_t *ws = static_cast<uint8_t *>(w);
-  alpha %= p;
 #define LELA_ELEM(E)                                                                           \
   tc_dispatch<E>(c, M, N, K, p, alpha, static_cast<const E *>(A), lda, static_cast<const E *>(B), \
                  ldb, 0u, V, ldv, ws, nullptr, 0)
@@ -1353,7 +1673,7 @@ static int launch_planes(Ctx *c, int M, int N, int K, const Modulus &mod, uint32
                             Cfg::BN, L);
     if (st) return st;
     int pi = prof_begin(c, "zp_gemm_tc");
-    pdl_launch(zp_gemm_tc_kernel<L, 0, T>, std::min(tiles, c->num_sms), tc_threads<L, T>(),
+    pdl_launch(zp_gemm_tc_kernel<L, OUT_ZP, T>, std::min(tiles, c->num_sms), tc_threads<L, T>(),
                TcLayout<L, T>::SMEM, c->stream,
                tmA, tmB, C, ldc, M, N, kc, mod, alpha, b, c->dstatus, kr, kbase + k0);
     prof_end(c, pi);
@@ -1382,8 +1702,8 @@ int zp_split_rows_dev(Ctx *c, uint32_t p, const uint32_t *A, size_t lda, int M, 
                       const ZpPlanes &out, int part, int nb) {
   const dim3 grid = split_rows_grid(c->num_sms, M, K), block(32, SPLIT_ROWS);
 #define LELA_SR(L) \
-  pdl_launch(split_rows_kernel<L, uint32_t>, grid, block, 0, c->stream, A, lda, M, K, p, \
-             out.base, out.pitch, out.plane, part, nb)
+  pdl_launch(split_rows_kernel<LimbBytes<L>, uint32_t>, grid, block, 0, c->stream, A, lda, M, K, p, \
+             out.base, out.pitch, out.plane, part, nb, LimbBytes<L>{})
   switch (zp_limbs_for(p)) {
     case 1: LELA_SR(1); break;
     case 2: LELA_SR(2); break;
@@ -1400,8 +1720,8 @@ int zp_split_cols_dev(Ctx *c, uint32_t p, const uint32_t *B, size_t ldb, int K, 
   const int kout = (K + 15) & ~15;
   const dim3 grid = split_cols_grid<uint32_t>(N, kout);
 #define LELA_SC(L) \
-  pdl_launch(split_cols_kernel<L, uint32_t>, grid, 256, 0, c->stream, B, ldb, K, N, p, out.base, \
-             out.pitch, out.plane, kout)
+  pdl_launch(split_cols_kernel<LimbBytes<L>, uint32_t>, grid, 256, 0, c->stream, B, ldb, K, N, p, out.base, \
+             out.pitch, out.plane, kout, LimbBytes<L>{})
   switch (zp_limbs_for(p)) {
     case 1: LELA_SC(1); break;
     case 2: LELA_SC(2); break;
@@ -1473,8 +1793,8 @@ static int host_rows(Ctx *c, int M, int N, int K, const Modulus &mod, uint32_t a
   if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream, ev_b, 0);
   if (e == cudaSuccess) {
     int pi = prof_begin(c, "zp_split");
-    pdl_launch(split_cols_kernel<L, uint32_t>, split_cols_grid<uint32_t>(N, Kp), 256, 0, c->stream,
-               dB, (size_t)N, K, N, (uint32_t)mod.p, Bl, (size_t)Kp, (size_t)N * Kp, Kp);
+    pdl_launch(split_cols_kernel<LimbBytes<L>, uint32_t>, split_cols_grid<uint32_t>(N, Kp), 256, 0, c->stream,
+               dB, (size_t)N, K, N, (uint32_t)mod.p, Bl, (size_t)Kp, (size_t)N * Kp, Kp, LimbBytes<L>{});
     prof_end(c, pi);
     ctx_launched(c);
     e = cudaGetLastError();
@@ -1488,9 +1808,9 @@ static int host_rows(Ctx *c, int M, int N, int K, const Modulus &mod, uint32_t a
     e = cudaStreamWaitEvent(c->stream, ready[j], 0);
     if (e != cudaSuccess) break;
     int pi = prof_begin(c, "zp_split");
-    pdl_launch(split_rows_kernel<L, uint32_t>, split_rows_grid(c->num_sms, rows, K),
+    pdl_launch(split_rows_kernel<LimbBytes<L>, uint32_t>, split_rows_grid(c->num_sms, rows, K),
                dim3(32, SPLIT_ROWS), 0, c->stream, dA + (size_t)r0 * K, (size_t)K, rows, K,
-               (uint32_t)mod.p, Al, (size_t)Kp, (size_t)rows * Kp, 0, 1);
+               (uint32_t)mod.p, Al, (size_t)Kp, (size_t)rows * Kp, 0, 1, LimbBytes<L>{});
     prof_end(c, pi);
     CUtensorMap tmA;
     st = encode_3d(c, &tmA, Al, (uint64_t)K, (uint64_t)rows, L, (uint64_t)Kp,
@@ -1498,7 +1818,7 @@ static int host_rows(Ctx *c, int M, int N, int K, const Modulus &mod, uint32_t a
     if (st) break;
     const int tiles = ((rows + BM - 1) / BM) * ((N + Cfg::BN - 1) / Cfg::BN);
     pi = prof_begin(c, "zp_gemm_tc");
-    pdl_launch(zp_gemm_tc_kernel<L, 0>, std::min(tiles, c->num_sms), tc_threads<L, 0>(), Lay::SMEM, c->stream,
+    pdl_launch(zp_gemm_tc_kernel<L, OUT_ZP>, std::min(tiles, c->num_sms), tc_threads<L, 0>(), Lay::SMEM, c->stream,
                tmA, tmB, dC + (size_t)r0 * N, (size_t)N, rows, N, K, mod, alpha, beta, c->dstatus, nullptr,
                0);
     prof_end(c, pi);
@@ -1661,17 +1981,17 @@ int noalloc_launch(cudaStream_t s, const NoallocDevice &d, int M, int N, int K,
     uint8_t *Al = planes;
     uint8_t *Bl = planes + (size_t)L * M * Kp;
     const uint32_t p = (uint32_t)mod.p;
-    pdl_launch(split_rows_kernel<L, uint32_t>, split_rows_grid(d.num_sms, M, kc),
-               dim3(32, SPLIT_ROWS), 0, s, A + k0, lda, M, kc, p, Al, (size_t)Kp, (size_t)M * Kp, 0, 1);
-    pdl_launch(split_cols_kernel<L, uint32_t>, split_cols_grid<uint32_t>(N, Kp), 256, 0, s,
-               B + (size_t)k0 * ldb, ldb, kc, N, p, Bl, (size_t)Kp, (size_t)N * Kp, Kp);
+    pdl_launch(split_rows_kernel<LimbBytes<L>, uint32_t>, split_rows_grid(d.num_sms, M, kc),
+               dim3(32, SPLIT_ROWS), 0, s, A + k0, lda, M, kc, p, Al, (size_t)Kp, (size_t)M * Kp, 0, 1, LimbBytes<L>{});
+    pdl_launch(split_cols_kernel<LimbBytes<L>, uint32_t>, split_cols_grid<uint32_t>(N, Kp), 256, 0, s,
+               B + (size_t)k0 * ldb, ldb, kc, N, p, Bl, (size_t)Kp, (size_t)N * Kp, Kp, LimbBytes<L>{});
     CUtensorMap tmA, tmB;
     if (!noalloc_map(&tmA, Al, (uint64_t)kc, (uint64_t)M, L, (uint64_t)Kp, (uint64_t)M * Kp,
                      BK, BM, L) ||
         !noalloc_map(&tmB, Bl, (uint64_t)kc, (uint64_t)N, L, (uint64_t)Kp, (uint64_t)N * Kp,
                      BK, Cfg::BN, L))
       return ST_CUDA;
-    pdl_launch(zp_gemm_tc_kernel<L, 0>, std::min(tiles, d.num_sms), tc_threads<L, 0>(), Lay::SMEM, s,
+    pdl_launch(zp_gemm_tc_kernel<L, OUT_ZP>, std::min(tiles, d.num_sms), tc_threads<L, 0>(), Lay::SMEM, s,
                tmA, tmB, C, ldc, M, N, kc, mod, alpha, b, err, nullptr, 0);
     b = 1;
   }
@@ -1740,7 +2060,7 @@ static int gf2_tc_launch(Ctx *c, int M, int N, int K, const uint8_t *Ab, const u
                          int Kp, uint32_t alpha, uint32_t beta, uint64_t *C, size_t ldc_words) {
   using Cfg = TcCfg<1, T>;
   using Lay = TcLayout<1, T>;
-  if (int st = ctx_smem_attr(c, (const void *)zp_gemm_tc_kernel<1, 1, T>, Lay::SMEM,
+  if (int st = ctx_smem_attr(c, (const void *)zp_gemm_tc_kernel<1, OUT_GF2, T>, Lay::SMEM,
                              "cudaFuncSetAttribute(gf2 tc)"))
     return st;
   CUtensorMap tmA, tmB;
@@ -1752,7 +2072,7 @@ static int gf2_tc_launch(Ctx *c, int M, int N, int K, const uint8_t *Ab, const u
   if (st) return st;
   const int tiles = ((M + BM - 1) / BM) * ((N + Cfg::BN - 1) / Cfg::BN);
   int pi = prof_begin(c, "gf2_gemm_tc");
-  pdl_launch(zp_gemm_tc_kernel<1, 1, T>, std::min(tiles, c->num_sms), tc_threads<1, T>(), Lay::SMEM,
+  pdl_launch(zp_gemm_tc_kernel<1, OUT_GF2, T>, std::min(tiles, c->num_sms), tc_threads<1, T>(), Lay::SMEM,
              c->stream, tmA, tmB, C, ldc_words, M, N, K, make_modulus(2), alpha, beta, c->dstatus,
              nullptr, 0);
   prof_end(c, pi);
