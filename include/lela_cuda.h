@@ -199,7 +199,7 @@ int lela_cuda_trsm_csr_upper_zp_u32_dev (lela_cuda_ctx *ctx, size_t n, size_t nc
 /* Diagonal-block solver of the trsm (and of the trsm steps inside
  * Faugere-Lachartre); every choice gives the same B. */
 enum {
-	LELA_CUDA_TRSM_AUTO = 0,    /* inverse leaves when B is wide, else block substitution */
+	LELA_CUDA_TRSM_AUTO = 0,    /* inverse leaves from 256 rows (128 for p >= 2^16), else block substitution */
 	LELA_CUDA_TRSM_BLOCKS = 1,  /* 256-row blocks by substitution on CUDA cores */
 	LELA_CUDA_TRSM_INVERSE = 2  /* 512-row blocks inverted, applied by the tensor-core gemm */
 };

@@ -44,7 +44,7 @@ enum Gf2Kernel : int {
 
 // Diagonal-block solvers of the Z/p trsm.
 enum TrsmKernel : int {
-  TRSM_AUTO = 0,     // inverse leaves for wide right-hand sides, else block substitution
+  TRSM_AUTO = 0,     // inverse leaves from 256 rows (128 for p >= 2^16), else block substitution
   TRSM_BLOCKS = 1,   // 256-row diagonal blocks by substitution on CUDA cores
   TRSM_INVERSE = 2,  // 512-row diagonal blocks inverted, applied by the tensor-core gemm
 };

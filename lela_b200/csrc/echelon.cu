@@ -27,24 +27,26 @@
 //  1. panel_heads_kernel: each row at or below the current row records the
 //     first nonzero column of its panel part (64: none), with a histogram;
 //  2. panel_search_kernel (one CTA) replays the reference's pivot choice on
-//     a window of the first rows, held in shared memory and eliminated
-//     eagerly without division (a row W becomes y W - W[c] P for pivot row
-//     P with pivot value y), so no inverse is on this sequential path; rows
-//     below the window are reduced only when the head histogram says one of
-//     them may hold a pivot the window lacks.  The pivot inverses and the
-//     pivot rows U_k come out of parallel inversions at the end, and, after
-//     the host has been signalled and when many rows are to be solved, the
-//     inverse of the pivot block U_P (the pivot rows at the pivot columns);
+//     a window of the first rows, four columns at a time: one warp chooses
+//     their pivots with the columns in registers, then all warps update the
+//     rest of the window in shared memory.  For p up to 65521 the pivots are
+//     inverted from a table; above, the elimination goes without division (a row
+//     W becomes y W - W[c] P for pivot row P with pivot value y) and the
+//     inverses come at the end.  Rows below the window are reduced only
+//     when the head histogram says one of them may hold a pivot the window
+//     lacks.  After the host has been signalled it inverts, for p < 2^31, the pivot
+//     block U_P (the pivot rows at the pivot columns) and L11;
 //  3. the host replays the recorded transpositions and moves the affected
 //     rows (at most two per pivot) with one gather;
-//  4. panel_solve_inv_kernel / panel_solve_kernel (all SMs, one warp per
-//     row): for every row from the first pivot to the last possibly nonzero
-//     row, its multipliers (the L11 row of a pivot row, the L21 row
+//  4. panel_solve_inv_kernel (p < 2^31) / panel_solve_kernel (all SMs, one
+//     warp per row): for every row from the first pivot to the last possibly
+//     nonzero row, its multipliers (the L11 row of a pivot row, the L21 row
 //     otherwise): a_P U_P^-1 from its entries a_P at the pivot columns, or
 //     the reference's elimination steps on its panel part; the panel becomes
 //     U_k in pivot row k and zero below;
-//  5. U12 = L11^-1 A12 on CUDA cores and A22 -= L21 U12 on the limb-split
-//     tensor-core gemm over the rows down to the last possibly nonzero row,
+//  5. U12 = L11^-1 A12 (a tensor-core product with the search's inverse, in place;
+//     by substitution on CUDA cores for p >= 2^31) and A22 -= L21 U12 on the
+//     tensor cores over the rows down to the last possibly nonzero row,
 //     for the columns of the panel's block of EB columns; the columns right
 //     of the block get one such update per block, with the multipliers of
 //     all its panels (K up to EB = 16 W instead of W: a sixteenth of the

@@ -25,7 +25,8 @@
 // elimination.tcc:47-139, pivot-strategy.tcc:44-66), which the dense
 // EchelonForm path (GaussJordan + move_L) reproduces.  Same exact panel
 // scheme as the Z/p version (echelon.cu) with 64-column panels = one word
-// per row; the trailing update is an M4RM product.
+// per row; the words of a panel's block are updated by tables, those right of the block
+// on the tensor cores (M4RM for few rows).
 #include <algorithm>
 #include <cstddef>
 #include <mutex>
@@ -373,17 +374,16 @@ int gf2_gemm_host_rows(Ctx *c, int M, int N, int K, const uint64_t *hA, size_t l
 // echelon.cu with GF(2) arithmetic:
 //  * gf2_heads_kernel: first set bit of each row's panel word, the head
 //    histogram and the last row with a nonzero word;
-//  * gf2_search_kernel: the reference's pivot choice, lazily.  The pivot
-//    rows are kept as a reduced basis g_k (bit pcol_j of g_k is delta_kj)
-//    and, per column c, the mask M[c] = (1 << c) | sum_k g_k[c] << pcol_k,
-//    so bit c of a row reduced by all pivots so far is parity(v & M[c]):
-//    32 positions are tested per ballot;
+//  * gf2_search_kernel: the reference's pivot choice on a window in registers,
+//    and lazily past it;
 //  * the host replays the transpositions and moves the rows;
 //  * gf2_solve_kernel: per row from the first pivot down to the last
 //    possibly nonzero row, the reference's elimination steps on the word
 //    (pivot k XOR-ed in when bit pcol_k is set) give the multipliers; pivot
-//    rows become U_k, rows below become zero;
-//  * U12 = L11^-1 A12 and the M4RM trailing update C ^= L21 U12.
+//    rows become U_k, rows below become zero; one CTA solves the block's words of
+//    U12 = L11^-1 A12 besides;
+//  * gf2_block_words_kernel: C ^= L21 U12 on the block's words; right of the block, once per
+//    block, U12 panel by panel and one tensor-core (few rows: M4RM) update.
 constexpr int GW = 64;
 constexpr uint8_t GF2_HEAD_NONE = 64;
 
