@@ -383,7 +383,7 @@ int gf2_gemm_host_rows(Ctx *c, int M, int N, int K, const uint64_t *hA, size_t l
 //    rows become U_k, rows below become zero; one CTA solves the block's words of
 //    U12 = L11^-1 A12 besides;
 //  * gf2_block_words_kernel: C ^= L21 U12 on the block's words; right of the block, once per
-//    block, U12 panel by panel and one tensor-core (few rows: M4RM) update.
+//    block, gf2_block_solve_kernel and one tensor-core (few rows: M4RM) update.
 constexpr int GW = 64;
 constexpr uint8_t GF2_HEAD_NONE = 64;
 
@@ -841,6 +841,81 @@ __global__ void __launch_bounds__(GF2_L11_THREADS)
   gf2_u12_word(D, ld, i0, t, w, l0, l1, lane);
 }
 
+// U12 = L11^-1 A12 of a whole block, on the words w1 .. nw - 1 of its T pivot rows
+// (T <= GB GW, from row i0 of D): L11 is unit lower triangular, row q's bits before
+// q in its GB words of Lb.  A CTA solves BS_WORDS words, in shared memory, 64 rows at a time: a
+// warp per word substitutes (gf2_u12_word's steps), then the rows after get
+// their sums of the 64 solved ones from sixteen tables of four rows, a thread per row
+// and word.  Bound: the 64-step chains (eight of about 2500 cycles).  Panel by panel, each panel a
+// four-Russians product for the rows before it and a substitution of its
+// own, a block of the 32768^2 form took 200 us.
+constexpr int BS_WORDS = 2, BS_THREADS = 256;
+__global__ void __launch_bounds__(BS_THREADS)
+    gf2_block_solve_kernel(uint64_t *D, size_t ld, int i0, int T, int w1, int nw,
+                           const uint64_t *Lb) {
+  pdl_enter();
+  constexpr int ROWS = GB * GW;
+  constexpr int LS = ROWS + 2;  // (the 16 words of two rows in different banks)
+  __shared__ uint64_t sL[GB * LS], X[ROWS][BS_WORDS], tab[GW / 4][16][BS_WORDS];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int wb = w1 + blockIdx.x * BS_WORDS;
+  for (int e = tid; e < ROWS * GB; e += BS_THREADS) {
+    const int r = e / GB, q = e % GB;
+    sL[q * LS + r] = r < T ? Lb[(size_t)(i0 + r) * GB + q] : 0ull;
+  }
+  for (int e = tid; e < ROWS * BS_WORDS; e += BS_THREADS) {
+    const int r = e / BS_WORDS, j = e % BS_WORDS;
+    X[r][j] = r < T && wb + j < nw ? D[(size_t)(i0 + r) * ld + wb + j] : 0ull;
+  }
+  __syncthreads();
+  for (int c = 0; GW * c < T; ++c) {
+    const uint64_t *L = sL + c * LS;
+    if (warp < BS_WORDS) {
+      const int r = GW * c + lane;
+      const uint64_t l0 = L[r] & ((1ull << lane) - 1), l1 = L[r + 32] & ((1ull << (lane + 32)) - 1);
+      uint64_t x0 = X[r][warp], x1 = X[r + 32][warp];
+#pragma unroll 4
+      for (int k = 0; k < 32; ++k) {
+        const uint64_t xk = __shfl_sync(0xffffffffu, x0, k);
+        x0 ^= (l0 >> k) & 1ull ? xk : 0ull;
+        x1 ^= (l1 >> k) & 1ull ? xk : 0ull;
+      }
+#pragma unroll 4
+      for (int k = 0; k < 31; ++k) {
+        const uint64_t xk = __shfl_sync(0xffffffffu, x1, k);
+        x1 ^= (l1 >> (k + 32)) & 1ull ? xk : 0ull;
+      }
+      X[r][warp] = x0;
+      X[r + 32][warp] = x1;
+    }
+    if (GW * (c + 1) >= T) break;
+    __syncthreads();
+    for (int e = tid; e < GW / 4 * 16 * BS_WORDS; e += BS_THREADS) {
+      const int j = e % BS_WORDS, v = (e / BS_WORDS) & 15, g = e / (16 * BS_WORDS);
+      uint64_t x = 0;
+#pragma unroll
+      for (int b = 0; b < 4; ++b)
+        if ((v >> b) & 1) x ^= X[GW * c + 4 * g + b][j];
+      tab[g][v][j] = x;
+    }
+    __syncthreads();
+    for (int e = GW * (c + 1) * BS_WORDS + tid; e < T * BS_WORDS; e += BS_THREADS) {
+      const int r = e / BS_WORDS, j = e % BS_WORDS;
+      const uint64_t l = L[r];
+      uint64_t x = X[r][j];
+#pragma unroll
+      for (int g = 0; g < GW / 4; ++g) x ^= tab[g][(l >> (4 * g)) & 15][j];
+      X[r][j] = x;
+    }
+    __syncthreads();
+  }
+  __syncthreads();
+  for (int e = tid; e < T * BS_WORDS; e += BS_THREADS) {
+    const int r = e / BS_WORDS, j = e % BS_WORDS;
+    if (wb + j < nw) D[(size_t)(i0 + r) * ld + wb + j] = X[r][j];
+  }
+}
+
 int gf2_echelon_dev(Ctx *c, int m, int n, uint64_t *D, size_t ld, size_t *rank_out) {
   if (m < 0 || n < 0) return ctx_fail(c, ST_ARG, "negative dimension");
   const int nw = (n + 63) / 64;
@@ -856,7 +931,7 @@ int gf2_echelon_dev(Ctx *c, int m, int n, uint64_t *D, size_t ld, size_t *rank_o
       (((size_t)2 * m + 4 * GW + 1 + GW + 1) * sizeof(int) + 255) & ~(size_t)255;
   const size_t h_bytes = ((size_t)2 * m + 255) & ~(size_t)255;
   void *base = nullptr;
-  const size_t lb_bytes = (size_t)m * GB * 8 + (size_t)GB * GW * 8;  // block bits, panel L11s
+  const size_t lb_bytes = (size_t)m * GB * 8;  // block bits
   int st = ctx_buffer(c, BUF_GF2_0,
                       out_bytes + i_bytes + h_bytes + (size_t)m * 8 + 2 * GW * 8 + lb_bytes + 1024,
                       &base);
@@ -873,8 +948,7 @@ int gf2_echelon_dev(Ctx *c, int m, int n, uint64_t *D, size_t ld, size_t *rank_o
   uint64_t *d_L21 = reinterpret_cast<uint64_t *>(b8 + out_bytes + i_bytes + h_bytes);
   uint64_t *d_L11 = d_L21 + m;
   uint64_t *d_U = d_L11 + GW;
-  uint64_t *d_Lb = d_U + GW;                 // m x GB words
-  uint64_t *d_L11s = d_Lb + (size_t)m * GB;                       // GB x GW words
+  uint64_t *d_Lb = d_U + GW;  // m x GB words
   void *mh = nullptr, *md = nullptr;
   if ((st = ctx_panel_map(c, &mh, &md))) return st;
   int *hperm = reinterpret_cast<int *>(static_cast<char *>(mh) + PANEL_PERM_OFF);
@@ -894,32 +968,18 @@ int gf2_echelon_dev(Ctx *c, int m, int n, uint64_t *D, size_t ld, size_t *rank_o
   // Blocks of GB words (delayed updates), as in the Z/p form: when the
   // block's first panel with pivots has at least DELAY_ROWS rows below it,
   // the block's panels update only the block's words; the words right of it
-  // get, per block, U12 = L11^-1 A12 on the block's pivot rows (panel by
-  // panel: the earlier panels' part by a gemm, then the panel's own L11) and
-  // one C ^= L21 U12 with K = the block's pivots (up to 64 GB bits) on the rows
+  // get, per block, U12 = L11^-1 A12 on the block's pivot rows and one C ^= L21 U12 with K = the block's pivots (up to 64 GB bits) on the rows
   // below.  d_Lb row q (GB words) holds the multipliers of the row at
   // position q, panel k of the block at bits Tb_k .. Tb_k + t_k - 1; later
   // panels' transpositions move d_Lb's rows with D's.
   constexpr int DELAY_ROWS = 512;
-  int ib = 0, Tb = 0, R = -1, bw1 = 0, delayed = 0, np = 0;
-  int pan_i[GB], pan_t[GB], pan_off[GB];
+  int ib = 0, Tb = 0, R = -1, bw1 = 0, delayed = 0;
   auto flush = [&]() -> int {
     if (Tb == 0 || bw1 >= nw) return ST_OK;
     const int nrest = n - 64 * bw1;  // bits right of the block
-    for (int j = 0; j < np; ++j) {
-      if (pan_off[j] > 0) {
-        // M = this panel's pivots (<= 64 rows): the four-Russians kernel,
-        // which needs no byte expansion of the wide B
-        int s = gf2_gemm_dev(c, GF2_M4RM, pan_t[j], nrest, pan_off[j], 1,
-                             d_Lb + (size_t)pan_i[j] * GB, GB, D + (size_t)ib * ld + bw1, ld, 1,
-                             D + (size_t)pan_i[j] * ld + bw1, ld);
-        if (s) return s;
-      }
-      pdl_launch(gf2_l11_solve_kernel, (nw - bw1 + GF2_L11_THREADS / 32 - 1) / (GF2_L11_THREADS / 32), GF2_L11_THREADS, 0, c->stream,
-      D, ld, pan_i[j], pan_t[j], bw1, nw,
-                                                              d_L11s + (size_t)j * GW);
-      ctx_launched(c);
-    }
+    pdl_launch(gf2_block_solve_kernel, (nw - bw1 + BS_WORDS - 1) / BS_WORDS, BS_THREADS, 0, c->stream,
+               D, ld, ib, Tb, bw1, nw, d_Lb);
+    ctx_launched(c);
     const int rb = ib + Tb;
     if (R < rb) return ST_OK;
     int pi = prof_begin(c, "gf2_block_update");
@@ -935,7 +995,6 @@ int gf2_echelon_dev(Ctx *c, int m, int n, uint64_t *D, size_t ld, size_t *rank_o
       ib = i;
       Tb = 0;
       R = -1;
-      np = 0;
       bw1 = std::min(nw, wc + GB);
       delayed = -1;  // decided at the block's first panel with pivots
     }
@@ -1005,13 +1064,12 @@ int gf2_echelon_dev(Ctx *c, int m, int n, uint64_t *D, size_t ld, size_t *rank_o
     }
     // the rest of the block's words (delayed), or of all words
     const int w1 = wc + 1, wend = delayed ? bw1 : nw;
-    uint64_t *L11 = delayed ? d_L11s + (size_t)np * GW : d_L11;
     {
       const int rows = r1 - i + 1;
       pi = prof_begin(c, "gf2_solve");
       pdl_launch(gf2_solve_kernel,
                  std::max(1, std::min((rows + GF2_SOLVE_THREADS - 1) / GF2_SOLVE_THREADS, c->num_sms * 4)),
-                 GF2_SOLVE_THREADS, 0, c->stream, D, ld, i, r1, wc, pmask, t, d_pcol, d_U, L11, d_L21,
+                 GF2_SOLVE_THREADS, 0, c->stream, D, ld, i, r1, wc, pmask, t, d_pcol, d_U, d_L11, d_L21,
                  delayed ? d_Lb : nullptr, Tb, w1, wend);
       prof_end(c, pi);
       ctx_launched(c);
@@ -1020,7 +1078,7 @@ int gf2_echelon_dev(Ctx *c, int m, int n, uint64_t *D, size_t ld, size_t *rank_o
       if (!delayed) {
         pdl_launch(gf2_l11_solve_kernel,
                    (wend - w1 + GF2_L11_THREADS / 32 - 1) / (GF2_L11_THREADS / 32), GF2_L11_THREADS, 0,
-                   c->stream, D, ld, i, t, w1, wend, L11);
+                   c->stream, D, ld, i, t, w1, wend, d_L11);
         ctx_launched(c);
       }
       if (below > 0) {
@@ -1039,10 +1097,6 @@ int gf2_echelon_dev(Ctx *c, int m, int n, uint64_t *D, size_t ld, size_t *rank_o
       }
     }
     if (delayed) {
-      pan_i[np] = i;
-      pan_t[np] = t;
-      pan_off[np] = Tb;
-      ++np;
       R = std::max(R, std::max(r1, hi));
       Tb += t;
     }

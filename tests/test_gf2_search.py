@@ -53,3 +53,16 @@ def test_bits_past_the_last_column(cuda):
     mask = np.uint64((1 << (n & 63)) - 1)
     got[:, -1] &= mask
     assert gr == wr and np.array_equal(got, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n", [(1100, 577), (1400, 1153), (1100, 1090), (2000, 1600)])
+@pytest.mark.parametrize("dependent", [0.0, 0.1, 0.6])
+def test_block_solve(cuda, m, n, dependent):
+    """Blocks of eight panels with words right of them: an even and an odd number of those, full
+    blocks and blocks whose pivots end inside a word."""
+    g = np.random.default_rng(m + n)
+    bits = gen.unpack_gf2(gen.dense_gf2(m * n, m, n), n).copy()
+    cols = np.flatnonzero(g.random(n) < dependent)
+    bits[:, cols] = bits[:, g.permutation(n)[: len(cols)]]
+    _check(cuda, gen.pack_gf2(bits), n)
