@@ -710,7 +710,7 @@ __global__ void __launch_bounds__(tc_threads<L, T>(), 1)
 
 // ------------------------------------------------- one-launch tile kernel
 // The same tile product without limb planes in memory, for short K and small
-// problems, where the two split launches and the tensor maps cost more than
+// problems, where the split launch and the tensor maps cost more than
 // the product: a CTA loads its 128 x K rows of A and K x BN columns of B
 // (u32), splits them into limbs on the way to shared memory (K-major, in the
 // 128-byte swizzle the tensor cores read), multiplies, and writes its tile.  K
@@ -959,17 +959,17 @@ struct ResidueBytes {
 // only those left (right) of the row's diagonal block of nb rows.
 constexpr int SPLIT_ROWS = 8;  // rows (warps) per CTA
 template <class W, class T>
-__global__ void __launch_bounds__(32 * SPLIT_ROWS)
-    split_rows_kernel(const T *A, size_t lda, int M, int kc, uint32_t p,
-                      uint8_t *out, size_t Kp, size_t plane, int part, int nb, const W planes) {
-  pdl_enter();
-  for (int r = blockIdx.y * SPLIT_ROWS + threadIdx.y; r < M; r += gridDim.y * SPLIT_ROWS) {
+__device__ __forceinline__ void split_rows(const T *A, size_t lda, int M, int kc, uint32_t p,
+                                           uint8_t *out, size_t Kp, size_t plane, int part, int nb,
+                                           const W &planes, int bx, int by, int gx, int gy) {
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  for (int r = by * SPLIT_ROWS + ty; r < M; r += gy * SPLIT_ROWS) {
     const T *src = A + (size_t)r * lda;
     uint8_t *dst = out + (size_t)r * Kp;
     const int kb = part == 2 ? min(kc, (r / nb + 1) * nb) : 0, ke = part == 1 ? min(kc, r / nb * nb) : kc;
     constexpr int U = 2;  // groups in flight
-    const int step = gridDim.x * 32;
-    for (int q = (kb >> 2) + blockIdx.x * 32 + threadIdx.x; 4 * q < ke; q += U * step) {
+    const int step = gx * 32;
+    for (int q = (kb >> 2) + bx * 32 + tx; 4 * q < ke; q += U * step) {
       uint32_t v[U][4];
 #pragma unroll
       for (int u = 0; u < U; ++u)
@@ -989,6 +989,14 @@ __global__ void __launch_bounds__(32 * SPLIT_ROWS)
     }
   }
 }
+template <class W, class T>
+__global__ void __launch_bounds__(32 * SPLIT_ROWS)
+    split_rows_kernel(const T *A, size_t lda, int M, int kc, uint32_t p,
+                      uint8_t *out, size_t Kp, size_t plane, int part, int nb, const W planes) {
+  pdl_enter();
+  split_rows<W, T>(A, lda, M, kc, p, out, Kp, plane, part, nb, planes, blockIdx.x, blockIdx.y,
+                   gridDim.x, gridDim.y);
+}
 static dim3 split_rows_grid(int num_sms, int M, int kc) {
   // one pass a warp up to 16 CTAs an SM, then more
   const int gy = std::min((M + SPLIT_ROWS - 1) / SPLIT_ROWS, num_sms * 16);
@@ -1003,14 +1011,13 @@ constexpr int split_cols_nt() {
   return sizeof(T) < 4 ? 128 / (int)sizeof(T) : 32;
 }
 template <class W, class T>
-__global__ void __launch_bounds__(256)
-    split_cols_kernel(const T *B, size_t ldb, int kc, int N, uint32_t p,
-                      uint8_t *out, size_t Kp, size_t plane, int kout, const W planes) {
-  pdl_enter();
+__device__ __forceinline__ void split_cols(const T *B, size_t ldb, int kc, int N, uint32_t p,
+                                           uint8_t *out, size_t Kp, size_t plane, int kout,
+                                           const W &planes, int bx, int by) {
   using R = typename Rep<T>::Packed;
   constexpr int NT = split_cols_nt<T>();
   __shared__ R tile[64][NT + 4 / sizeof(R)];
-  const int n0 = blockIdx.x * NT, k0 = blockIdx.y * 64;
+  const int n0 = bx * NT, k0 = by * 64;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
@@ -1039,9 +1046,43 @@ __global__ void __launch_bounds__(256)
     }
   }
 }
+template <class W, class T>
+__global__ void __launch_bounds__(256)
+    split_cols_kernel(const T *B, size_t ldb, int kc, int N, uint32_t p,
+                      uint8_t *out, size_t Kp, size_t plane, int kout, const W planes) {
+  pdl_enter();
+  split_cols<W, T>(B, ldb, kc, N, p, out, Kp, plane, kout, planes, blockIdx.x, blockIdx.y);
+}
 template <class T>
 static dim3 split_cols_grid(int N, int Kp) {
   return dim3((N + split_cols_nt<T>() - 1) / split_cols_nt<T>(), (Kp + 63) / 64);
+}
+
+// Both operands' planes in one launch, A's (M x kc, planes from out_a, rows Kp
+// apart) in the first gax * gay CTAs: a product of few tiles waits for each launch (512^3
+// 17.6 us a call, 20.4 with two launches).
+template <class W, class T>
+__global__ void __launch_bounds__(256)
+    split_both_kernel(const T *A, size_t lda, const T *B, size_t ldb, int M, int N, int kc,
+                      uint32_t p, uint8_t *out_a, uint8_t *out_b, int Kp, int gax, int gay, int gbx,
+                      const W wa, const W wb) {
+  static_assert(32 * SPLIT_ROWS == 256, "one block size");
+  pdl_enter();
+  const int b = blockIdx.x, na = gax * gay;
+  if (b < na)
+    split_rows<W, T>(A, lda, M, kc, p, out_a, (size_t)Kp, (size_t)M * Kp, 0, 1, wa, b % gax, b / gax,
+                     gax, gay);
+  else
+    split_cols<W, T>(B, ldb, kc, N, p, out_b, (size_t)Kp, (size_t)N * Kp, Kp, wb, (b - na) % gbx,
+                     (b - na) / gbx);
+}
+template <class W, class T>
+static void launch_split(bool early, int num_sms, cudaStream_t s, const T *A, size_t lda, const T *B,
+                         size_t ldb, int M, int N, int kc, uint32_t p, uint8_t *out_a, uint8_t *out_b,
+                         int Kp, const W &wa, const W &wb) {
+  const dim3 ga = split_rows_grid(num_sms, M, kc), gb = split_cols_grid<T>(N, Kp);
+  pdl_launch_if(early, split_both_kernel<W, T>, ga.x * ga.y + gb.x * gb.y, 256, 0, s, A, lda, B, ldb,
+                M, N, kc, p, out_a, out_b, Kp, (int)ga.x, (int)ga.y, (int)gb.x, wa, wb);
 }
 
 // ------------------------------------------------- residues back to Z/p
@@ -1309,12 +1350,10 @@ static int launch_tc(Ctx *c, int M, int N, int K, const Modulus &mod, uint32_t a
     {
       const uint32_t p = (uint32_t)mod.p;
       int pi = prof_begin(c, "zp_split");
-      pdl_launch_if(early, split_rows_kernel<LimbBytes<L>, E>, split_rows_grid(c->num_sms, M, kc), dim3(32, SPLIT_ROWS),
-                 0, c->stream, A + k0, lda, M, kc, p, Al, (size_t)Kp, (size_t)M * Kp, 0, 1, LimbBytes<L>{});
-      pdl_launch_if(early, split_cols_kernel<LimbBytes<L>, E>, split_cols_grid<E>(N, Kp), 256, 0, c->stream,
-                 B + (size_t)k0 * ldb, ldb, kc, N, p, Bl, (size_t)Kp, (size_t)N * Kp, Kp, LimbBytes<L>{});
+      launch_split(early, c->num_sms, c->stream, A + k0, lda, B + (size_t)k0 * ldb, ldb, M, N, kc, p,
+                   Al, Bl, Kp, LimbBytes<L>{}, LimbBytes<L>{});
       prof_end(c, pi);
-      ctx_launched(c, 2);
+      ctx_launched(c);
     }
     CUtensorMap tmA, tmB;
     int st = encode_3d(c, &tmA, Al, (uint64_t)kc, (uint64_t)M, L, (uint64_t)Kp,
@@ -1396,7 +1435,7 @@ static int launch_rns(Ctx *c, int M, int N, int K, int rows, const Modulus &mod,
     uint32_t *Cr = C + (size_t)r0 * ldc;
     pi = prof_begin(c, "zp_split");
     pdl_launch_if(early, split_rows_kernel<ResidueBytes, E>, split_rows_grid(c->num_sms, m, K),
-                  dim3(32, SPLIT_ROWS), 0, c->stream, A + (size_t)r0 * lda, lda, m, K, p, Al, Kp,
+                  32 * SPLIT_ROWS, 0, c->stream, A + (size_t)r0 * lda, lda, m, K, p, Al, Kp,
                   (size_t)m * Kp, 0, 1, ra);
     prof_end(c, pi);
     if (int st = encode_3d(c, &tmA, Al, (uint64_t)K, (uint64_t)m, n, Kp, (uint64_t)m * Kp, BK, BM, 1))
@@ -1531,10 +1570,10 @@ int zp_gemm_tile_pick(const Ctx *c, int M, int N, int K, uint32_t p) {
 int zp_gemm_pick(const Ctx *c, int M, int N, int K, uint32_t p) {
   if (c->gemm_kernel != GEMM_AUTO) return c->gemm_kernel;
   // The one-launch tile kernel for short K while its tiles are few: it saves
-  // the two split launches (about 7 us), but every tile splits its own operands
+  // the split launch, but every tile splits its own operands
   // and the CTAs do not overlap a tile's epilogue with the next tile's product.
-  // Measured on the B200 (us per call, one-launch / split and tensor cores, p =
-  // 65521): 64 x 960 x 64 9.6 / 16.2, 1000 x 448 x 64 11.5 / 18.1, 2000 x 2000 x
+  // Measured on the B200 (us per call, one-launch / split, then with a launch per
+  // operand, 2.7 us more, and tensor cores, p = 65521): 64 x 960 x 64 9.6 / 16.2, 1000 x 448 x 64 11.5 / 18.1, 2000 x 2000 x
   // 64 (512 tiles) 24.6 / 28.9, 8000 x 960 x 64 (945) 41 / 39, 1024^2 x 256 (128)
   // 14.4 / 16.6, 512 x 4096 x 512 (256) 29.5 / 24.5, 512^3 (32) 20.5 / 17.6; four
   // limbs: 64 x 9000 x 64 (282) 20.5 / 24.6, 4000 x 448 x 64 (448) 37 / 35.  The CUDA-core
@@ -1700,7 +1739,7 @@ int zp_gemm_planes_dev(Ctx *c, int M, int N, int K, uint32_t p, uint32_t alpha, 
 
 int zp_split_rows_dev(Ctx *c, uint32_t p, const uint32_t *A, size_t lda, int M, int K,
                       const ZpPlanes &out, int part, int nb) {
-  const dim3 grid = split_rows_grid(c->num_sms, M, K), block(32, SPLIT_ROWS);
+  const dim3 grid = split_rows_grid(c->num_sms, M, K), block(32 * SPLIT_ROWS);
 #define LELA_SR(L) \
   pdl_launch(split_rows_kernel<LimbBytes<L>, uint32_t>, grid, block, 0, c->stream, A, lda, M, K, p, \
              out.base, out.pitch, out.plane, part, nb, LimbBytes<L>{})
@@ -1809,7 +1848,7 @@ static int host_rows(Ctx *c, int M, int N, int K, const Modulus &mod, uint32_t a
     if (e != cudaSuccess) break;
     int pi = prof_begin(c, "zp_split");
     pdl_launch(split_rows_kernel<LimbBytes<L>, uint32_t>, split_rows_grid(c->num_sms, rows, K),
-               dim3(32, SPLIT_ROWS), 0, c->stream, dA + (size_t)r0 * K, (size_t)K, rows, K,
+               32 * SPLIT_ROWS, 0, c->stream, dA + (size_t)r0 * K, (size_t)K, rows, K,
                (uint32_t)mod.p, Al, (size_t)Kp, (size_t)rows * Kp, 0, 1, LimbBytes<L>{});
     prof_end(c, pi);
     CUtensorMap tmA;
@@ -1981,10 +2020,8 @@ int noalloc_launch(cudaStream_t s, const NoallocDevice &d, int M, int N, int K,
     uint8_t *Al = planes;
     uint8_t *Bl = planes + (size_t)L * M * Kp;
     const uint32_t p = (uint32_t)mod.p;
-    pdl_launch(split_rows_kernel<LimbBytes<L>, uint32_t>, split_rows_grid(d.num_sms, M, kc),
-               dim3(32, SPLIT_ROWS), 0, s, A + k0, lda, M, kc, p, Al, (size_t)Kp, (size_t)M * Kp, 0, 1, LimbBytes<L>{});
-    pdl_launch(split_cols_kernel<LimbBytes<L>, uint32_t>, split_cols_grid<uint32_t>(N, Kp), 256, 0, s,
-               B + (size_t)k0 * ldb, ldb, kc, N, p, Bl, (size_t)Kp, (size_t)N * Kp, Kp, LimbBytes<L>{});
+    launch_split(true, d.num_sms, s, A + k0, lda, B + (size_t)k0 * ldb, ldb, M, N, kc, p, Al, Bl, Kp,
+                 LimbBytes<L>{}, LimbBytes<L>{});
     CUtensorMap tmA, tmB;
     if (!noalloc_map(&tmA, Al, (uint64_t)kc, (uint64_t)M, L, (uint64_t)Kp, (uint64_t)M * Kp,
                      BK, BM, L) ||
