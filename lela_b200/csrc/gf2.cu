@@ -242,9 +242,9 @@ static void unpack_rows(Ctx *c, const uint64_t *A, size_t lda, int M, int k0, ui
   ctx_launched(c);
 }
 static void unpack_cols(Ctx *c, const uint64_t *B, size_t ldb, int k0, int kc, int N, uint8_t *out,
-                        int Kp) {
+                        int Kp, bool early) {
   const int Nw = (N + 63) / 64;
-  pdl_launch(gf2_unpack_cols_kernel, dim3((Nw + UNPACK_W - 1) / UNPACK_W, (Kp + UNPACK_K - 1) / UNPACK_K), 32 * UNPACK_WARPS, 0, c->stream,
+  pdl_launch_if(early, gf2_unpack_cols_kernel, dim3((Nw + UNPACK_W - 1) / UNPACK_W, (Kp + UNPACK_K - 1) / UNPACK_K), 32 * UNPACK_WARPS, 0, c->stream,
       B, ldb, k0, kc, N, out, Kp);
   ctx_launched(c);
 }
@@ -275,7 +275,7 @@ int gf2_gemm_dev(Ctx *c, int kernel, int M, int N, int K, int alpha, const uint6
     uint8_t *Bb = Ab + (size_t)M * Kp;
     int pi = prof_begin(c, "gf2_unpack");
     unpack_rows(c, A, lda, M, k0, Ab, Kp);
-    unpack_cols(c, B, ldb, k0, kc, N, Bb, Kp);
+    unpack_cols(c, B, ldb, k0, kc, N, Bb, Kp, gf2_early(M, N, kc));
     prof_end(c, pi);
     if ((st = gf2_gemm_tc_planes(c, M, N, kc, Ab, Bb, Kp, 1u, b, C, ldc))) return st;
     b = 1;
@@ -335,7 +335,7 @@ int gf2_gemm_host_rows(Ctx *c, int M, int N, int K, const uint64_t *hA, size_t l
   if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream, ev_b, 0);
   if (e == cudaSuccess) {
     int pi = prof_begin(c, "gf2_unpack");
-    unpack_cols(c, dB, (size_t)Nw, 0, K, N, Bb, Kp);
+    unpack_cols(c, dB, (size_t)Nw, 0, K, N, Bb, Kp, false);
     prof_end(c, pi);
     e = cudaGetLastError();
   }

@@ -2109,7 +2109,7 @@ static int gf2_tc_launch(Ctx *c, int M, int N, int K, const uint8_t *Ab, const u
   if (st) return st;
   const int tiles = ((M + BM - 1) / BM) * ((N + Cfg::BN - 1) / Cfg::BN);
   int pi = prof_begin(c, "gf2_gemm_tc");
-  pdl_launch(zp_gemm_tc_kernel<1, OUT_GF2, T>, std::min(tiles, c->num_sms), tc_threads<1, T>(), Lay::SMEM,
+  pdl_launch_if(gf2_early(M, N, K), zp_gemm_tc_kernel<1, OUT_GF2, T>, std::min(tiles, c->num_sms), tc_threads<1, T>(), Lay::SMEM,
              c->stream, tmA, tmB, C, ldc_words, M, N, K, make_modulus(2), alpha, beta, c->dstatus,
              nullptr, 0);
   prof_end(c, pi);

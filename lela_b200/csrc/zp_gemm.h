@@ -88,6 +88,11 @@ int zp_gemm_host_rows(Ctx *c, int M, int N, int K, uint32_t p, uint32_t alpha,
 }  // namespace lela
 
 namespace lela {
+// Whether a GF(2) product's kernels after the first are launched early (us per product,
+// early / in order: 1590 x 753 x 3420 21.8 / 27.3, 810 x 8264 x 523 19.9 / 23.4,
+// 2048^3 24.4 / 24.9; 13564 x 3189 x 1074 75.9 / 61.3 after a kernel that is not of
+// this chain, 4096^3 65.2 / 60.5, 16384^2 x 1024 212 / 197).
+inline bool gf2_early(int M, int N, int K) { return (double)M * N * K < 1e10; }
 // GF(2) product on the tensor cores from 0/1 byte planes (see zp_gemm.cu).
 int gf2_gemm_tc_planes(Ctx *c, int M, int N, int K, const uint8_t *Ab, const uint8_t *Bb, int Kp,
                        uint32_t alpha, uint32_t beta, uint64_t *C, size_t ldc_words);
