@@ -44,6 +44,7 @@ int ctx_cuda(Ctx *c, cudaError_t e, const char *what) {
   char buf[256];
   snprintf(buf, sizeof buf, "%s: %s", what, cudaGetErrorString(e));
   c->last_error = buf;
+  cudaGetLastError();  // reported here, and not again by the next call's launch check
   if (e == cudaErrorMemoryAllocation) return ST_NOMEM;
   return ST_CUDA;
 }

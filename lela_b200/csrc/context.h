@@ -95,8 +95,10 @@ struct Ctx {
   // search publishes its result and a sequence number; created on first use.
   void *panel_map = nullptr, *panel_map_dev = nullptr;
   uint32_t panel_seq = 0;
-  // Modulus whose inverses BUF_INV holds (0: none).  They are written on the
-  // handle's stream; a change of stream waits for the old one.
+  // Modulus whose inverses BUF_INV holds (0: none), set once a panel search
+  // that follows them on the handle's stream has signalled: a launch alone does
+  // not show that they were written (in a stream capture nothing runs).  A
+  // change of stream waits for the old one.
   uint32_t inv_p = 0;
   // Entries of the last Faugere-Lachartre CSR result kept in BUF_FL_CSR_V
   // (SIZE_MAX: none), for lela_cuda_fl_csr_fetch.

@@ -1435,11 +1435,11 @@ int zp_echelon_dev(Ctx *c, int m, int n, uint32_t p, uint32_t *D, size_t ld, siz
     void *tb = nullptr;
     if ((st = ctx_buffer(c, BUF_INV, PW_TABLE, &tb))) return st;
     if (c->inv_p != p) {
+      c->inv_p = 0;  // p only when the first panel's result shows that the table is there
       inverse_table_kernel<<<((int)p / 2 + 261) / 256, 256, 0, c->stream>>>(p, static_cast<uint16_t *>(tb));
       ctx_launched(c);
       const cudaError_t ei = cudaGetLastError();
       if (ei != cudaSuccess) return ctx_cuda(c, ei, "echelon: inverses");
-      c->inv_p = p;
     }
     inv_table = static_cast<const uint16_t *>(tb);
   }
@@ -1546,6 +1546,7 @@ int zp_echelon_dev(Ctx *c, int m, int n, uint32_t p, uint32_t *D, size_t ld, siz
     if ((st = word(PANEL_W_T, &head_word)) || (st = word(PANEL_W_LAST, &h.last_pos)) ||
         (st = word(PANEL_W_DET, &h.det)))
       return st;
+    if (inv_table) c->inv_p = p;
     h.t = std::min<uint32_t>(head_word & 0xffu, EW);
     h.uinv = head_word >> 8 & 1u;
     h.err = head_word >> 9 & 1u;
