@@ -1478,6 +1478,24 @@ static bool rns_pays(int M, int N, int K, int n) {
 constexpr size_t RNS_MAX_BYTES = (size_t)4 << 30;
 constexpr int RNS_MIN_ROWS = 2048;
 
+// Whether the matrices X (rx rows of cx entries) and C share an entry.  Views of
+// one matrix (equal strides) are compared as rectangles of it, others by their
+// whole address ranges.
+template <class E>
+static bool share_entries(const E *X, size_t ldx, int rx, int cx, const uint32_t *C, size_t ldc,
+                          int rc, int cc) {
+  const uintptr_t x0 = reinterpret_cast<uintptr_t>(X), c0 = reinterpret_cast<uintptr_t>(C);
+  const uintptr_t x1 = x0 + ((size_t)(rx - 1) * ldx + cx) * sizeof(E);
+  const uintptr_t c1 = c0 + ((size_t)(rc - 1) * ldc + cc) * sizeof(uint32_t);
+  if (x1 <= c0 || c1 <= x0) return false;
+  if (sizeof(E) != sizeof(uint32_t) || ldx != ldc || (c0 - x0) % sizeof(uint32_t)) return true;
+  // C starts q rows and s columns after X
+  const long long ld = (long long)ldx, off = (long long)(c0 - x0) / (long long)sizeof(uint32_t);
+  const long long q = off >= 0 ? off / ld : -((ld - 1 - off) / ld), s = off - q * ld;
+  if (s < cx && q < rx && q + rc > 0) return true;
+  return s + cc > ld && q + 1 < rx && q + 1 + rc > 0;  // its columns past the row's end
+}
+
 // The product by residues where shape and modulus favour it and its planes can
 // be had: within RNS_MAX_BYTES in blocks of at least RNS_MIN_ROWS rows, and in the workspace as it is
 // inside a stream capture.  done says whether it was launched (else the limb
@@ -1498,6 +1516,7 @@ static int rns_try(Ctx *c, int M, int N, int K, uint32_t p, uint32_t alpha, cons
   int rows = M;
   if ((size_t)M > most) {
     if (most < RNS_MIN_ROWS) return ST_OK;
+    if (share_entries(A, lda, M, K, C, ldc, M, N)) return ST_OK;  // a block's C may be a later one's A
     const int blocks = (int)((M + most - BM) / (most - BM + 1));
     rows = ((M + blocks - 1) / blocks + BM - 1) / BM * BM;
   }
@@ -1622,7 +1641,14 @@ int zp_gemm_dev(Ctx *c, int kernel, int M, int N, int K, uint32_t p, uint32_t al
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? ST_OK : ctx_cuda(c, e, "zp_scale launch");
   }
-  if (kernel == GEMM_AUTO) kernel = zp_gemm_pick(c, M, N, K, p);
+  if (kernel == GEMM_AUTO) {
+    kernel = zp_gemm_pick(c, M, N, K, p);
+    // C may lie over A or B where the operands are split before C is written; the
+    // one-launch kernel's CTAs read them while others already write
+    if (kernel == GEMM_DIRECT && (share_entries(A, lda, M, K, C, ldc, M, N) ||
+                                  share_entries(B, ldb, K, N, C, ldc, M, N)))
+      kernel = GEMM_TC;
+  }
   if (kernel == GEMM_SMALLK) {
     dim3 grid((N + PT - 1) / PT, (M + PT - 1) / PT);
     int pi = prof_begin(c, "zp_gemm_smallk");
