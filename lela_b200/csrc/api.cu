@@ -61,6 +61,17 @@ static int grow(Ctx *c, void **buf, size_t *have, size_t bytes, const char *what
   }
   size_t want = std::max(bytes, (size_t)1 << 20);
   cudaError_t e = cudaMalloc(buf, want);
+  if (e == cudaErrorMemoryAllocation && buf != &c->ws && c->ws && c->ws_held == 0) {
+    // The workspace may have grown for planes that a smaller one can do without:
+    // it goes back, and its next user takes what there is room for.
+    cudaGetLastError();
+    e = cudaStreamSynchronize(c->stream);
+    if (e != cudaSuccess) return ctx_cuda(c, e, "cudaStreamSynchronize");
+    cudaFree(c->ws);
+    c->ws = nullptr;
+    c->ws_bytes = 0;
+    e = cudaMalloc(buf, want);
+  }
   if (e != cudaSuccess) {
     *buf = nullptr;
     return ctx_cuda(c, e, what);

@@ -58,9 +58,12 @@ struct Ctx {
   cudaStream_t stream = nullptr;
   bool own_stream = false;
 
-  // Device workspace (grown on demand, never shrunk until destroy).
+  // Device workspace (grown on demand).  It is given back when another of the
+  // handle's allocations finds no room, unless a caller keeps a pointer to it across
+  // those (ws_held > 0, see WsHold).
   void *ws = nullptr;
   size_t ws_bytes = 0;
+  int ws_held = 0;
   // Second workspace for callers that need two live scratch regions.
   void *ws2 = nullptr;
   size_t ws2_bytes = 0;
@@ -168,6 +171,14 @@ enum BufSlot : int {
 // Grow-only allocation helpers; return ST_OK or ST_NOMEM.
 int ctx_buffer(Ctx *c, int slot, size_t bytes, void **out);
 int ctx_workspace(Ctx *c, size_t bytes, void **out);
+// Keeps the workspace where it is for the holder's life.
+struct WsHold {
+  Ctx *c;
+  explicit WsHold(Ctx *ctx) : c(ctx) { ++c->ws_held; }
+  ~WsHold() { --c->ws_held; }
+  WsHold(const WsHold &) = delete;
+  WsHold &operator=(const WsHold &) = delete;
+};
 int ctx_workspace2(Ctx *c, size_t bytes, void **out);
 int ctx_stage(Ctx *c, int slot, size_t bytes, void **out);
 // Creates the copy streams and events of the pipelined host-pointer gemm

@@ -1429,6 +1429,7 @@ int zp_echelon_dev(Ctx *c, int m, int n, uint32_t p, uint32_t *D, size_t ld, siz
                                  zp_trsm_workspace_bytes(p, EB, n)),
                      &gws);
   if (st) return st;
+  const WsHold hold(c);  // gws
   const bool small = p < (1u << 16);
   const uint16_t *inv_table = nullptr;
   if (SearchSmall::takes(p)) {
