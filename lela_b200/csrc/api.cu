@@ -86,6 +86,16 @@ int ctx_workspace(Ctx *c, size_t bytes, void **out) {
   return st;
 }
 
+bool ctx_planes_fit(const Ctx *c, size_t bytes) {
+  if (bytes <= c->ws_bytes) return true;
+  size_t fr = 0, total = 0;
+  if (cudaMemGetInfo(&fr, &total) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return fr + c->ws_bytes >= bytes + total / 16;  // (growing frees the old one first)
+}
+
 int ctx_workspace2(Ctx *c, size_t bytes, void **out) {
   int st = grow(c, &c->ws2, &c->ws2_bytes, bytes, "cudaMalloc(workspace2)");
   *out = c->ws2;

@@ -780,12 +780,12 @@ int zp_trsm_dev(Ctx *c, bool upper, bool unit, int m, int n, uint32_t p, uint32_
       return st;
     void *w = nullptr;
     // (where the planes of all of A do not fit, the recursion's smaller ones may)
-    if (trsm_left_pays(c, m, n, p)) {
-      st = ctx_workspace(c, zp_trsm_workspace_bytes(p, m, n), &w);
+    const size_t planes = zp_trsm_workspace_bytes(p, m, n);
+    if (trsm_left_pays(c, m, n, p) && ctx_planes_fit(c, planes)) {
+      st = ctx_workspace(c, planes, &w);
       if (!st)
         return trsm_left(c, tm, upper, m, n, p, alpha, A, lda, W, B, ldb, static_cast<uint8_t *>(w));
       if (st != ST_NOMEM) return st;
-      cudaGetLastError();
     }
     if ((st = ctx_workspace(c, trsm_rec_bytes(p, m, n), &w))) return st;
     return trsm_rec_inv(c, tm, 0, upper, m, n, p, alpha, A, lda, W, B, ldb,

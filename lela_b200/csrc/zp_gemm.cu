@@ -1497,7 +1497,7 @@ static bool share_entries(const E *X, size_t ldx, int rx, int cx, const uint32_t
 }
 
 // The product by residues where shape and modulus favour it and its planes can
-// be had: within RNS_MAX_BYTES in blocks of at least RNS_MIN_ROWS rows, and in the workspace as it is
+// be had: where they leave memory free (ctx_planes_fit), within RNS_MAX_BYTES in blocks of at least RNS_MIN_ROWS rows, and in the workspace as it is
 // inside a stream capture.  done says whether it was launched (else the limb
 // planes, which take less room, serve).
 template <class E>
@@ -1527,10 +1527,7 @@ static int rns_try(Ctx *c, int M, int N, int K, uint32_t p, uint32_t alpha, cons
       return ST_OK;
   }
   void *w = nullptr;
-  if (ctx_workspace(c, bytes, &w)) {  // no room
-    cudaGetLastError();
-    return ST_OK;
-  }
+  if (!ctx_planes_fit(c, bytes) || ctx_workspace(c, bytes, &w)) return ST_OK;  // no room
   done = true;
   return launch_rns<E>(c, M, N, K, rows, make_modulus(p), alpha, A, lda, B, ldb, beta, C, ldc,
                        static_cast<uint8_t *>(w), ra, rb, rw);

@@ -92,3 +92,36 @@ def test_fl_after_its_wide_solve(tidy):
     torch.cuda.empty_cache()
     assert (r, d) == (rank, det)
     assert bool((R == want).all())
+
+
+@pytest.mark.gpu
+def test_planes_leave_memory_free(tidy):
+    """With less than a sixteenth of the device free, a product modulo p > 2^16 and a wide solve take
+    the workspace of the limbs (134 MB, where the residue planes have 503) and of the recursion (42 MB and
+    the inverses, where the planes of all of A and X have 67 and their leaf's)."""
+    import torch
+    A, B = rand(1, 4096, 4096, P31), rand(2, 4096, 4096, P31)
+    T = torch.tril(rand(3, 4096, 4096, P16), -1) + torch.eye(4096, device="cuda", dtype=torch.int32)
+    Y = rand(4, 4096, 4096, P16)
+
+    def run(op):
+        C = Y.clone()
+        torch.cuda.synchronize()
+        before = free()
+        with CudaModule(0) as cm:
+            if op == "gemm":
+                cm.gemm(P31, 1, A, B, 0, C)
+            else:
+                cm.trsm(P16, 1, T, C, False, True)
+            cm.synchronize()
+            return before - free(), C
+
+    run("gemm"), run("trsm")  # the kernels
+    roomy = {op: run(op) for op in ("gemm", "trsm")}
+    filler = leave(6 << 30)
+    tight = {op: run(op) for op in ("gemm", "trsm")}
+    del filler
+    assert tight["gemm"][0] < 144 * MB < roomy["gemm"][0]
+    assert tight["trsm"][0] < roomy["trsm"][0] - 16 * MB
+    for op in tight:
+        assert bool((tight[op][1] == roomy[op][1]).all())
