@@ -88,6 +88,7 @@ int ctx_workspace(Ctx *c, size_t bytes, void **out) {
 
 bool ctx_planes_fit(const Ctx *c, size_t bytes) {
   if (bytes <= c->ws_bytes) return true;
+  if (bytes > c->planes_max) return false;
   size_t fr = 0, total = 0;
   if (cudaMemGetInfo(&fr, &total) != cudaSuccess) {
     cudaGetLastError();
@@ -1018,12 +1019,23 @@ void ctx_trim(Ctx *c) {
 }
 
 // Upper estimate of the device bytes one FL matrix needs on a handle: the
-// dense blocks A, B, C, D (4 m n), the gemm limb planes (at most 4 (m + n) m
+// dense blocks A, B, C, D (4 m n), the gemm limb planes (fl_planes: at most 4 (m + n) m
 // for the Schur complement), the triangular-solve inverses and echelon
 // bookkeeping (about 5 KB per row: the echelon's block multipliers are 4 KB),
 // and fixed scratch.
+size_t fl_planes(size_t m, size_t n) { return 4 * (m + n) * m; }
 size_t fl_bytes_estimate(size_t m, size_t n) {
-  return 4 * m * n + 4 * (m + n) * m + 5120 * m + ((size_t)256 << 20);
+  return 4 * m * n + fl_planes(m, n) + 5120 * m + ((size_t)256 << 20);
+}
+// What the planes may take beyond fl_planes where a larger workspace is faster: the
+// wide solve's leaf (L <= 4 planes of 512 columns), and for p > 2^16 the residue planes
+// of the reduced form's product, M x K by K x N with M + K <= m pivots and N <= n.
+size_t fl_planes_extra(size_t m, size_t n, uint32_t p) {
+  size_t most = fl_planes(m, n) + 2048 * (n + 512);
+  if (zp_limbs_for(p) == 4)
+    most = std::max(most, std::min(ZP_RESIDUE_MAX_BYTES,
+                                   (size_t)ZP_RESIDUE_MAX * (n + m / 4 + 32) * (m + 32)));
+  return most - fl_planes(m, n);
 }
 
 // The memory-budgeted queue of a batch: an item starts only when its
@@ -1109,9 +1121,14 @@ int lela_cuda_fl_echelonize_zp_u32_batch(lela_cuda_ctx *h, size_t count, const s
     for (int t = 0; t < nworkers; ++t) held += ctx_held_bytes(&h->workers[t]->c);
     mq.budget = fr / 10 * 9 + held;
   }
-  size_t peak = 0;
-  for (int j = 0; j < nworkers; ++j) peak += fl_bytes_estimate(m[order[j]], n[order[j]]);
+  size_t peak = 0, extra = 0;
+  for (int j = 0; j < nworkers; ++j) {
+    peak += fl_bytes_estimate(m[order[j]], n[order[j]]);
+    extra += fl_planes_extra(m[order[j]], n[order[j]], p[order[j]]);
+  }
   const bool tight = peak > mq.budget;
+  // the workspaces that the estimate does not count only where all of them fit
+  const bool capped = peak + extra > mq.budget;
   std::atomic<size_t> next(0);
   std::atomic<int> fatal(0);
   auto work = [&](lela_cuda_ctx *w) {
@@ -1127,6 +1144,7 @@ int lela_cuda_fl_echelonize_zp_u32_batch(lela_cuda_ctx *h, size_t count, const s
         if (tight) mq.release(need);
         break;
       }
+      if (capped) w->c.planes_max = fl_planes(m[i], n[i]);
       size_t rows = 0, bad = 0;
       int st = lela_cuda_fl_echelonize_zp_u32_dev(w, m[i], n[i], p[i], rowptr[i], colidx[i],
                                                   vals[i], reduced, 0, R[i], ldr[i], &rank[i],
@@ -1138,6 +1156,7 @@ int lela_cuda_fl_echelonize_zp_u32_batch(lela_cuda_ctx *h, size_t count, const s
         mq.release(need);
       }
     }
+    w->c.planes_max = SIZE_MAX;
   };
   std::vector<std::thread> th;
   for (int t = 0; t < nworkers; ++t) th.emplace_back(work, h->workers[t]);

@@ -64,6 +64,9 @@ struct Ctx {
   void *ws = nullptr;
   size_t ws_bytes = 0;
   int ws_held = 0;
+  // Most that the workspace may grow to for planes that a path with fewer could do
+  // without (ctx_planes_fit): a batch near its memory budget sets it.
+  size_t planes_max = SIZE_MAX;
   // Second workspace for callers that need two live scratch regions.
   void *ws2 = nullptr;
   size_t ws2_bytes = 0;
@@ -172,7 +175,7 @@ enum BufSlot : int {
 int ctx_buffer(Ctx *c, int slot, size_t bytes, void **out);
 int ctx_workspace(Ctx *c, size_t bytes, void **out);
 // Whether the workspace may grow to `bytes` for planes that a path with fewer could
-// do without: a sixteenth of the device's memory must stay free, for the handle's
+// do without: within planes_max, and a sixteenth of the device's memory must stay free, for the handle's
 // other buffers and for other allocators of the program (11 GB; the planes are
 // at most 4 GiB of a product and L (m + n) m bytes of a solve).
 bool ctx_planes_fit(const Ctx *c, size_t bytes);

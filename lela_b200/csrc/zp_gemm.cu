@@ -111,7 +111,7 @@ struct TcCfg<4, 0> {
   static constexpr int BN = 32, NMMA = 128, STAGES = 2, ACC = 1, EPI = 8;
 };
 
-constexpr int RNS_MAX = 11;
+constexpr int RNS_MAX = ZP_RESIDUE_MAX;
 __host__ __device__ constexpr uint32_t rns_mod(int i) {
   return i == 0 ? 256 : i == 1 ? 255 : i == 2 ? 253 : i == 3 ? 251 : i == 4 ? 247 : i == 5 ? 241
        : i == 6 ? 239 : i == 7 ? 233 : i == 8 ? 229 : i == 9 ? 227 : 223;
@@ -1475,7 +1475,7 @@ static bool rns_pays(int M, int N, int K, int n) {
   return std::min(M, N) >= (n <= 8 ? 512 : 1536) && K >= 512 &&
          (double)M * N * K >= 2147483648.0;
 }
-constexpr size_t RNS_MAX_BYTES = (size_t)4 << 30;
+constexpr size_t RNS_MAX_BYTES = ZP_RESIDUE_MAX_BYTES;
 constexpr int RNS_MIN_ROWS = 2048;
 
 // Whether the matrices X (rx rows of cx entries) and C share an entry.  Views of

@@ -15,6 +15,11 @@ constexpr int ZP_KCHUNK = 32768;
 int zp_limbs_for(uint32_t p);
 size_t zp_gemm_workspace_bytes(uint32_t p, int M, int N, int K);
 
+// A product modulo p > 2^16 by residues takes up to ZP_RESIDUE_MAX byte planes of A, B and C
+// in the workspace, at most ZP_RESIDUE_MAX_BYTES.
+constexpr int ZP_RESIDUE_MAX = 11;
+constexpr size_t ZP_RESIDUE_MAX_BYTES = (size_t)4 << 30;
+
 // C <- alpha*A*B + beta*C mod p on the handle's stream (asynchronous).
 // kernel: a GemmKernel.  B may be C itself (same rows and columns, beta = 0)
 // for GEMM_TC with K <= ZP_KCHUNK, and for GEMM_DIRECT with M <= 128 and K <=

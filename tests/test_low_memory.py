@@ -125,3 +125,32 @@ def test_planes_leave_memory_free(tidy):
     assert tight["trsm"][0] < roomy["trsm"][0] - 16 * MB
     for op in tight:
         assert bool((tight[op][1] == roomy[op][1]).all())
+
+
+@pytest.mark.gpu
+def test_fl_batch_keeps_its_budget(tidy):
+    """Two wide matrices modulo 2^31 - 1 at once, in a budget of twice the estimate that the header gives:
+    their last product's residue planes (845 MB) are not in it and must not be taken."""
+    import torch
+    import types
+    m, n = 5000, 20000
+    Xs, outs = [], []
+    for i in range(2):
+        X = gen.f4_matrix_fast(i, m, P31, n=n, density=0.002)
+        Xs.append(types.SimpleNamespace(m=m, n=n, rowptr=torch.from_numpy(X.rowptr.view(np.int64)).cuda(),
+                                        colidx=torch.from_numpy(X.colidx.view(np.int32)).cuda(),
+                                        vals=torch.from_numpy(X.vals.view(np.int32)).cuda()))
+    budget = 2 * (4 * m * n + 4 * (m + n) * m + 5120 * m + 256 * MB)
+    for limit in (0, budget):  # (the first call loads the kernels, too)
+        Rs = [torch.zeros((m, n), dtype=torch.int32, device="cuda") for _ in Xs]
+        torch.cuda.empty_cache()
+        before = free()
+        with CudaModule(0) as cm:
+            cm.set_batch_memory_budget(limit)
+            res = cm.fl_echelonize_batch(Xs, [P31, P31], Rs, True, nworkers=2)
+            cm.synchronize()
+            held = before - free()
+        outs.append((Rs, res))
+    assert outs[0][1] == outs[1][1]
+    assert all(bool((a == b).all()) for a, b in zip(outs[0][0], outs[1][0]))
+    assert held <= budget
