@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(HEADS_THREADS)
 // term fit 32 bits (2 (p/2 + 4)^2 + p/2 + 4 < 2^31); four (below 2^32.1 in
 // 64 bits) are halved for the quotient, which then is off by 2 / p more.
 //
-// SearchMont and SearchWide reduce without division (an inverse costs more
+// SearchMont and SearchPlain reduce without division (an inverse costs more
 // than a whole column there): one elimination step is upd(y, w, na, P) = k (y
 // w + na P) and a product mul(a, b) = k a b, with a unit k fixed per form;
 // lin(s, w, a, P) = k (s w + a[0] P[0] + .. + a[3] P[3]); plain(a, b) = a b. A
@@ -264,17 +264,21 @@ struct SearchMont {
   __device__ __forceinline__ uint32_t one() const { return r1; }
   __device__ __forceinline__ uint32_t canon(uint32_t v) const { return v; }
 };
-// SearchWide, any p < 2^32 (even moduli, p below 3 and p >= 2^31): canonical
-// residues, 64-bit Barrett reduction, k = 1.
-struct SearchWide {
+// SearchPlain, any p < 2^32 (even moduli, p below 3 and p >= 2^31): canonical
+// residues, Barrett reduction, k = 1.  Below 2^16 with ArithSmall's 32-bit
+// reductions, which count where rows past the window, a warp per row and all
+// its pivots, are reduced for each column without a pivot: a 3000 x 500 matrix of
+// rank 166 modulo 2 takes 2490 us, with ArithWide's 4550.
+template <class A>
+struct SearchPlain {
   using V = uint32_t;
   using V4 = uint4;
   static constexpr bool NORM = false;
-  ArithWide w;
+  A w;
   uint32_t p;
-  __host__ static SearchWide make(uint32_t p) {
-    SearchWide a;
-    a.w = ArithWide::make(p);
+  __host__ static SearchPlain make(uint32_t p) {
+    SearchPlain a;
+    a.w = A::make(p);
     a.p = p;
     return a;
   }
@@ -874,7 +878,9 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
           for (int k = 0; k < t; ++k) {
             const int pc = s_piv[k].x;
             const V f = __shfl_sync(FULL, pc < 32 ? a0 : a1, pc & 31);
-            const V u0 = lane >= pc ? PV[k][lane] : 0, u1 = lane + 32 >= pc ? PV[k][lane + 32] : 0;
+            // (left of pc PV is not kept up to date; a column there is not read again)
+            const V u0 = !SA::NORM || lane >= pc ? PV[k][lane] : 0;
+            const V u1 = !SA::NORM || lane + 32 >= pc ? PV[k][lane + 32] : 0;
             if constexpr (SA::NORM) {
               const V l = sa.plain(f, s_xi[k]);
               if (lane == 0) s_rl[wid][k] = l;
@@ -1531,8 +1537,10 @@ int zp_echelon_dev(Ctx *c, int m, int n, uint32_t p, uint32_t *D, size_t ld, siz
       st = search(SearchSmall::make(p, inv_table), ars, i, c0, w, seq, wcap);
     else if (SearchMont::takes(p))
       st = search(SearchMont::make(p), arw, i, c0, w, seq, wcap);
+    else if (small)
+      st = search(SearchPlain<ArithSmall>::make(p), ars, i, c0, w, seq, wcap);
     else
-      st = search(SearchWide::make(p), arw, i, c0, w, seq, wcap);
+      st = search(SearchPlain<ArithWide>::make(p), arw, i, c0, w, seq, wcap);
     if (st) return st;
     ++epoch;
     prof_end(c, pi);
