@@ -43,7 +43,7 @@
 //    for the short-K updates of the triangular solve and the echelon panels,
 //    where the first kernel's fixed cost (limb splits, tensor maps, pipeline
 //    start) dominates: each CTA splits its own operands into shared memory.
-// 4. zp_gemm_smallk_kernel -- CUDA-core gemm for small K, by request only.  For
+// 4. zp_gemm_smallk_kernel -- CUDA-core gemm for small K: the smallest products.  For
 //    p < 2^28 a 64-bit sum of 256 products cannot wrap, so the products are
 //    summed without checks and the sums reduced every 256 terms.
 #include <cuda.h>
@@ -1215,10 +1215,10 @@ __global__ void __launch_bounds__(256)
 // reduced modulo p after every 256 terms (256 (p-1)^2 < 2^64).
 template <bool NOWRAP>
 __global__ void __launch_bounds__(256)
-    zp_gemm_smallk_kernel(const uint32_t *__restrict__ A, size_t lda,
-                          const uint32_t *__restrict__ B, size_t ldb, uint32_t *__restrict__ C,
+    zp_gemm_smallk_kernel(const uint32_t *A, size_t lda, const uint32_t *B, size_t ldb, uint32_t *C,
                           size_t ldc, int M, int N, int K, Modulus mod, uint32_t two64,
                           uint32_t alpha, uint32_t beta) {
+  pdl_enter();
   __shared__ uint32_t As[PK][PT + 1];
   __shared__ uint32_t Bs[PK][PT + 1];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
@@ -1235,10 +1235,10 @@ __global__ void __launch_bounds__(256)
       int idx = threadIdx.x + 256 * e;
       int r = idx / PK, kk = idx % PK;
       int gm = m0 + r, gk = k0 + kk;
-      As[kk][r] = (gm < M && gk < K) ? __ldg(A + (size_t)gm * lda + gk) : 0u;
+      As[kk][r] = (gm < M && gk < K) ? A[(size_t)gm * lda + gk] : 0u;
       int kr = idx / PT, c = idx % PT;
       int gk2 = k0 + kr, gn = n0 + c;
-      Bs[kr][c] = (gk2 < K && gn < N) ? __ldg(B + (size_t)gk2 * ldb + gn) : 0u;
+      Bs[kr][c] = (gk2 < K && gn < N) ? B[(size_t)gk2 * ldb + gn] : 0u;
     }
     __syncthreads();
 #pragma unroll 8
@@ -1591,12 +1591,21 @@ int zp_gemm_pick(const Ctx *c, int M, int N, int K, uint32_t p) {
   // the split launch, but every tile splits its own operands
   // and the CTAs do not overlap a tile's epilogue with the next tile's product.
   // Measured on the B200 (us per call, one-launch / split, then with a launch per
-  // operand, 2.7 us more, and tensor cores, p = 65521): 64 x 960 x 64 9.6 / 16.2, 1000 x 448 x 64 11.5 / 18.1, 2000 x 2000 x
-  // 64 (512 tiles) 24.6 / 28.9, 8000 x 960 x 64 (945) 41 / 39, 1024^2 x 256 (128)
-  // 14.4 / 16.6, 512 x 4096 x 512 (256) 29.5 / 24.5, 512^3 (32) 20.5 / 17.6; four
-  // limbs: 64 x 9000 x 64 (282) 20.5 / 24.6, 4000 x 448 x 64 (448) 37 / 35.  The CUDA-core
-  // kernel for small K is slower at all of them (14.4 us and more).
+  // operand, 2.7 us more, and tensor cores, p = 65521): 64 x 960 x 64 9.6 / 16.2, 1000 x
+  // 448 x 64 11.5 / 18.1, 2000 x 2000 x 64 (512 tiles) 24.6 / 28.9, 8000 x 960 x 64 (945)
+  // 41 / 39, 1024^2 x 256 (128) 14.4 / 16.6, 512 x 4096 x 512 (256) 29.5 / 24.5, 512^3
+  // (32) 20.5 / 17.6; four limbs: 64 x 9000 x 64 (282) 20.5 / 24.6, 4000 x 448 x 64 (448)
+  // 37 / 35.  The CUDA-core kernel for small K is slower at all of them (14.4 us and more).
   const int L = zp_limbs_for(p), bn = L == 4 ? DirCfg<4>::BN : DirCfg<1>::BN;
+  // The smallest products, with few entries of C a thread there, go to the CUDA-core
+  // kernel for small K, which needs no barriers, TMEM or MMA (us per call alone, one-launch /
+  // CUDA cores: p = 65521 1^3 19.2 / 17.4, 16 x 16 x 32 19.1 / 17.7, 32^3 19.5 / 18.7, 16 x
+  // 64 x 32 19.6 / 18.5, 1000 x 16 x 32 19.9 / 19.2, while 64^3 20.0 / 25.3; p = 251 16^3
+  // 18.4 / 17.4, 32^3 18.5 / 18.7; four limbs alike up to 16^3; a call among others 7.0
+  // either way).
+  if (L < 4 && K <= PK && std::min(M, PT) * std::min(N, PT) <= (L == 1 ? 256 : 1024) &&
+      (long long)M * N <= 16384)
+    return GEMM_SMALLK;
   const long long tiles = (long long)((M + BM - 1) / BM) * ((N + bn - 1) / bn);
   const long long most = K <= 128 ? (L == 4 ? 2 : 4) * c->num_sms : K <= 256 ? c->num_sms : 0;
   return tiles <= most ? GEMM_DIRECT : GEMM_TC;
@@ -1643,20 +1652,21 @@ int zp_gemm_dev(Ctx *c, int kernel, int M, int N, int K, uint32_t p, uint32_t al
   if (kernel == GEMM_AUTO) {
     kernel = zp_gemm_pick(c, M, N, K, p);
     // C may lie over A or B where the operands are split before C is written; the
-    // one-launch kernel's CTAs read them while others already write
-    if (kernel == GEMM_DIRECT && (share_entries(A, lda, M, K, C, ldc, M, N) ||
-                                  share_entries(B, ldb, K, N, C, ldc, M, N)))
+    // one-launch kernels' CTAs read them while others already write
+    const bool one = kernel == GEMM_DIRECT || kernel == GEMM_SMALLK;
+    if (one && c->gemm_kernel == GEMM_AUTO &&
+        (share_entries(A, lda, M, K, C, ldc, M, N) || share_entries(B, ldb, K, N, C, ldc, M, N)))
       kernel = GEMM_TC;
   }
   if (kernel == GEMM_SMALLK) {
     dim3 grid((N + PT - 1) / PT, (M + PT - 1) / PT);
     int pi = prof_begin(c, "zp_gemm_smallk");
     if (p < (1u << 28))
-      zp_gemm_smallk_kernel<true><<<grid, 256, 0, c->stream>>>(A, lda, B, ldb, C, ldc, M, N, K,
-                                                               mod, host_two64(p), alpha, beta);
+      pdl_launch(zp_gemm_smallk_kernel<true>, grid, 256, 0, c->stream, A, lda, B, ldb, C, ldc, M, N, K,
+                 mod, host_two64(p), alpha, beta);
     else
-      zp_gemm_smallk_kernel<false><<<grid, 256, 0, c->stream>>>(A, lda, B, ldb, C, ldc, M, N, K,
-                                                                mod, host_two64(p), alpha, beta);
+      pdl_launch(zp_gemm_smallk_kernel<false>, grid, 256, 0, c->stream, A, lda, B, ldb, C, ldc, M, N, K,
+                 mod, host_two64(p), alpha, beta);
     prof_end(c, pi);
     ctx_launched(c);
     cudaError_t e = cudaGetLastError();
