@@ -642,11 +642,23 @@ static int trsm_rec_inv(Ctx *c, const TileMap *tm, int off, bool upper, int m, i
 // limb planes of A's triangle are made once and those of each solved leaf of X
 // once, and a leaf gets one update with K = all rows solved before it (its rows of
 // A times X), then its inverse.  The recursion splits every block of X once per
-// level (four times at 16 leaves) and its small updates leave SMs idle: 8192^2
-// x 4096 1340 us.  Each product has TI_NB rows, so it needs columns for the SMs.
-static bool trsm_left_pays(const Ctx *c, int m, int n, uint32_t p) {
-  const int bn = zp_limbs_for(p) == 4 ? 32 : 128;
-  return m > 2 * TI_NB && 3 * (TI_NB / 128) * ((n + bn - 1) / bn) >= 2 * c->num_sms;
+// level (four times at 16 leaves) and its small updates leave SMs idle.  Each product
+// here has TI_NB rows, so it needs columns for the SMs, and leaves enough for the splits
+// saved.  Measured (us a solve, recursion / leaf by leaf, dense lower A): p = 65521 8192
+// x 1000 598 / 684, 2500 904 / 900, 3073 1364 / 1226, 4096 1053 / 958; 4096 x 1000 292 /
+// 304, 3073 595 / 547, 8192 663 / 608; 2048 x 3073 275 / 262, 8192 291 / 278; 1537 x 3073
+// 222 / 229, 8192 248 / 245; 1025 x 3073 161 / 165.  p = 251: 8192 x 3073 1178 / 1009, 4096 x
+// 3073 542 / 480, 2048 x 3073 247 / 239, 1537 x 3073 201 / 204.  Four limbs (2^31 - 1), whose
+// tiles are 32 columns wide: 8192 x 1500 1562 / 1731, 2500 2131 / 2460, 4096 2981 / 3160;
+// 4096 x 1500 628 / 644, 8192 1822 / 1736; 1537 x 1500 244 / 261; with the sparse A of
+// Faugere-Lachartre, where a leaf's update skips its rows' empty ranges at once, 15000 x 9000
+// 8677 / 8482, 4500 x 2700 1054 / 1026, 2250 x 1350 509 / 517.
+static bool trsm_left_pays(const Ctx *c, int m, int n, uint32_t p, bool sparse) {
+  const bool wide = zp_limbs_for(p) == 4;
+  if (wide && !sparse) return false;
+  const int bn = wide ? 32 : 128;
+  return m >= (wide ? 8 : 4) * TI_NB &&
+         3 * (TI_NB / 128) * ((n + bn - 1) / bn) >= 2 * c->num_sms;
 }
 static size_t trsm_left_pitch(int m) { return ((size_t)m + 15) & ~(size_t)15; }
 static size_t trsm_left_bytes(uint32_t p, int m, int n) {
@@ -781,7 +793,7 @@ int zp_trsm_dev(Ctx *c, bool upper, bool unit, int m, int n, uint32_t p, uint32_
     void *w = nullptr;
     // (where the planes of all of A do not fit, the recursion's smaller ones may)
     const size_t planes = zp_trsm_workspace_bytes(p, m, n);
-    if (trsm_left_pays(c, m, n, p) && ctx_planes_fit(c, planes)) {
+    if (trsm_left_pays(c, m, n, p, tm != nullptr) && ctx_planes_fit(c, planes)) {
       st = ctx_workspace(c, planes, &w);
       if (!st)
         return trsm_left(c, tm, upper, m, n, p, alpha, A, lda, W, B, ldb, static_cast<uint8_t *>(w));
