@@ -89,8 +89,10 @@ int ctx_workspace(Ctx *c, size_t bytes, void **out) {
 bool ctx_planes_fit(const Ctx *c, size_t bytes) {
   if (bytes <= c->ws_bytes) return true;
   if (bytes > c->planes_max) return false;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   size_t fr = 0, total = 0;
-  if (cudaMemGetInfo(&fr, &total) != cudaSuccess) {
+  if (cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess ||
+      cap != cudaStreamCaptureStatusNone || cudaMemGetInfo(&fr, &total) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }

@@ -1496,9 +1496,10 @@ static bool share_entries(const E *X, size_t ldx, int rx, int cx, const uint32_t
   return s + cc > ld && q + 1 < rx && q + 1 + rc > 0;  // its columns past the row's end
 }
 
-// The product by residues where shape and modulus favour it and its planes can
-// be had: where they leave memory free (ctx_planes_fit), within RNS_MAX_BYTES in blocks of at least RNS_MIN_ROWS rows, and in the workspace as it is
-// inside a stream capture.  done says whether it was launched (else the limb
+// The product by residues where shape and modulus favour it and its planes can be
+// had: within RNS_MAX_BYTES in blocks of at least RNS_MIN_ROWS rows, and in a workspace
+// that may grow to hold them (ctx_planes_fit: not inside a stream capture, not
+// where little memory is left).  done says whether it was launched (else the limb
 // planes, which take less room, serve).
 template <class E>
 static int rns_try(Ctx *c, int M, int N, int K, uint32_t p, uint32_t alpha, const E *A, size_t lda,
@@ -1523,11 +1524,6 @@ static int rns_try(Ctx *c, int M, int N, int K, uint32_t p, uint32_t alpha, cons
     rows = ((M + blocks - 1) / blocks + BM - 1) / BM * BM;
   }
   const size_t bytes = fixed + (size_t)rows * per_row;
-  if (bytes > c->ws_bytes) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
-      return ST_OK;
-  }
   void *w = nullptr;
   if (!ctx_planes_fit(c, bytes) || ctx_workspace(c, bytes, &w)) return ST_OK;  // no room
   done = true;
