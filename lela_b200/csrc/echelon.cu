@@ -191,7 +191,9 @@ struct SearchSmall {
     return (int)(d >> 32) >> sh;
   }
   __device__ __forceinline__ int red(int x) const { return x - quot(x, s) * p; }
+  // (an entry that is not reduced is: the table is looked up by what comes of it)
   __device__ __forceinline__ int load(uint32_t v) const {
+    if (v >= (uint32_t)p) v %= (uint32_t)p;
     return (int)v > (p >> 1) ? (int)v - p : (int)v;
   }
   // w - l P
