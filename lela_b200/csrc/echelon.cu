@@ -109,12 +109,14 @@ __device__ __forceinline__ int row_at(int pos, const int *p2r, const int *stamp,
 // 1. First nonzero column of each row's panel part, rows i0..m-1 (one warp
 // per row); the histogram of these heads (hist[0..64], which the caller
 // has zeroed) and the largest row index with a nonzero panel (*last, which
-// the caller has set to -1).
+// the caller has set to -1).  Entries of the panel that are not reduced (a
+// caller's may not be) are, in place: the search looks inverses up by
+// their value.  (A 4096^2 form takes 5 us of 4745 more for the check; in the
+// search, at its loads, it took 15 to 45.)
 constexpr int HEADS_THREADS = 256;
 __global__ void __launch_bounds__(HEADS_THREADS)
-    panel_heads_kernel(const uint32_t *D, size_t ld, int i0, int m, int c0, int w,
-                       uint8_t *head, uint8_t *act, int *hist,
-                       int *last) {
+    panel_heads_kernel(uint32_t *D, size_t ld, int i0, int m, int c0, int w, uint32_t p,
+                       uint8_t *head, uint8_t *act, int *hist, int *last) {
   pdl_enter();
   __shared__ int s_last;
   __shared__ int s_hist[EW + 1];
@@ -125,9 +127,13 @@ __global__ void __launch_bounds__(HEADS_THREADS)
   const int warps = (gridDim.x * blockDim.x) >> 5;
   int my_last = -1;
   for (int r = i0 + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); r < m; r += warps) {
-    const uint32_t *row = D + (size_t)r * ld + c0;
-    const uint32_t a = lane < w ? row[lane] : 0u;
-    const uint32_t b = lane + 32 < w ? row[lane + 32] : 0u;
+    uint32_t *row = D + (size_t)r * ld + c0;
+    uint32_t a = lane < w ? row[lane] : 0u;
+    uint32_t b = lane + 32 < w ? row[lane + 32] : 0u;
+    if (max(a, b) >= p) {
+      if (lane < w) row[lane] = a %= p;
+      if (lane + 32 < w) row[lane + 32] = b %= p;
+    }
     const unsigned ba = __ballot_sync(0xffffffffu, a != 0u);
     const unsigned bb = __ballot_sync(0xffffffffu, b != 0u);
     const int h = ba ? __ffs(ba) - 1 : (bb ? 32 + __ffs(bb) - 1 : HEAD_NONE);
@@ -191,9 +197,8 @@ struct SearchSmall {
     return (int)(d >> 32) >> sh;
   }
   __device__ __forceinline__ int red(int x) const { return x - quot(x, s) * p; }
-  // (an entry that is not reduced is: the table is looked up by what comes of it)
+  // (reduced entries only, see panel_heads_kernel)
   __device__ __forceinline__ int load(uint32_t v) const {
-    if (v >= (uint32_t)p) v %= (uint32_t)p;
     return (int)v > (p >> 1) ? (int)v - p : (int)v;
   }
   // w - l P
@@ -1529,9 +1534,8 @@ int zp_echelon_dev(Ctx *c, int m, int n, uint32_t p, uint32_t *D, size_t ld, siz
       delayed = -1;  // decided at the block's first panel with pivots
     }
     int pi = prof_begin(c, "ech_heads");
-    pdl_launch(panel_heads_kernel, head_grid, HEADS_THREADS, 0, c->stream,
-      D, ld, i, m, c0, w, d_head,
-                                                                    d_act, d_hist, d_last);
+    pdl_launch(panel_heads_kernel, head_grid, HEADS_THREADS, 0, c->stream, D, ld, i, m, c0, w, p,
+               d_head, d_act, d_hist, d_last);
     prof_end(c, pi);
     const uint32_t seq = ++c->panel_seq;
     pi = prof_begin(c, "ech_search");

@@ -1,4 +1,4 @@
-"""Entries that are not reduced modulo p: the panel's pivot search reduces what it reads, since it looks
+"""Entries that are not reduced modulo p: a panel's entries are before its pivot search, which looks
 inverses up by value (32 <= p <= 65521).  A form of one panel is that of the reduced matrix; one of
 several ends, whatever its other kernels make of such entries, and the next form is right."""
 import numpy as np
