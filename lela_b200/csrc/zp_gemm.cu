@@ -1656,13 +1656,16 @@ int zp_gemm_dev(Ctx *c, int kernel, int M, int N, int K, uint32_t p, uint32_t al
   }
   if (kernel == GEMM_SMALLK) {
     dim3 grid((N + PT - 1) / PT, (M + PT - 1) / PT);
+    // (early only with few CTAs: more, waiting in turn beside those that still run, made a
+    // row of 1000 x 448 x 64 products, 112 CTAs each, 28.5 us a call instead of 14.4)
+    const bool early = (size_t)grid.x * grid.y <= 16;
     int pi = prof_begin(c, "zp_gemm_smallk");
     if (p < (1u << 28))
-      pdl_launch(zp_gemm_smallk_kernel<true>, grid, 256, 0, c->stream, A, lda, B, ldb, C, ldc, M, N, K,
-                 mod, host_two64(p), alpha, beta);
+      pdl_launch_if(early, zp_gemm_smallk_kernel<true>, grid, 256, 0, c->stream, A, lda, B, ldb, C, ldc, M,
+                    N, K, mod, host_two64(p), alpha, beta);
     else
-      pdl_launch(zp_gemm_smallk_kernel<false>, grid, 256, 0, c->stream, A, lda, B, ldb, C, ldc, M, N, K,
-                 mod, host_two64(p), alpha, beta);
+      pdl_launch_if(early, zp_gemm_smallk_kernel<false>, grid, 256, 0, c->stream, A, lda, B, ldb, C, ldc, M,
+                    N, K, mod, host_two64(p), alpha, beta);
     prof_end(c, pi);
     ctx_launched(c);
     cudaError_t e = cudaGetLastError();
