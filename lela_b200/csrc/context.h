@@ -175,9 +175,10 @@ enum BufSlot : int {
 int ctx_buffer(Ctx *c, int slot, size_t bytes, void **out);
 int ctx_workspace(Ctx *c, size_t bytes, void **out);
 // Whether the workspace may grow to `bytes` for planes that a path with fewer could
-// do without: not inside a stream capture, within planes_max, and a sixteenth of the device's memory must stay free, for the handle's
-// other buffers and for other allocators of the program (11 GB; the planes are
-// at most 4 GiB of a product and L (m + n) m bytes of a solve).
+// do without: not inside a stream capture, within planes_max, and while a sixteenth
+// of the device's memory (11 GB) stays free for the handle's other buffers and for
+// other allocators of the program.  The planes are at most 4 GiB of a product and
+// L (m + n) m bytes of a solve.
 bool ctx_planes_fit(const Ctx *c, size_t bytes);
 // Keeps the workspace where it is for the holder's life.
 struct WsHold {

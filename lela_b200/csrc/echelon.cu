@@ -75,18 +75,6 @@ constexpr int PS_THREADS = 512;            // panel search CTA
 constexpr int PS_FAST = PS_THREADS / 32;   // positions tested per column by whole warps
 constexpr uint8_t HEAD_NONE = 64;
 
-struct PanelOut {
-  uint32_t t;         // pivots found in the panel
-  uint32_t err;       // 1: a pivot is not invertible in Modular<uint32>
-  uint32_t uinv;      // 1: U_P^-1 written (the rows to solve take panel_solve_inv_kernel)
-  uint32_t last_pos;  // largest final position of a non-pivot row with a nonzero panel (or 0)
-  uint32_t det;       // product of the panel's pivots
-  uint32_t pad[3];
-  uint32_t pcol[EW];  // pivot columns (relative to c0)
-  uint32_t ti[EW];    // transposition k: (ti[k], tq[k])
-  uint32_t tq[EW];
-};
-
 // The host's copy of a panel's result, in mapped host memory: words of the
 // value (low half) and the search's sequence number (high half).  Each word
 // is written whole, so the host takes a word when its sequence number has
@@ -111,7 +99,7 @@ __device__ __forceinline__ int row_at(int pos, const int *p2r, const int *stamp,
 // has zeroed) and the largest row index with a nonzero panel (*last, which
 // the caller has set to -1).  Entries of the panel that are not reduced (a
 // caller's may not be) are, in place: the search looks inverses up by
-// their value.  (A 4096^2 form takes 5 us of 4745 more for the check; in the
+// their value.  (A 4096^2 form takes 5 to 15 us of 4740 more for the check; in the
 // search, at its loads, it took 15 to 45.)
 constexpr int HEADS_THREADS = 256;
 __global__ void __launch_bounds__(HEADS_THREADS)
@@ -160,10 +148,12 @@ __global__ void __launch_bounds__(HEADS_THREADS)
 // for p > 2^15, one less per halving of p) is x / p rounded, up to an error of
 // |x| / 2^(33+s) from mu, for |x| < 2^31; so |x - q p| <= p/2 + 1, and x = 0 mod p
 // gives q = x / p exactly: a zero is stored as 0 (s >= 3 here).  The product
-// and the rounding are one 64-bit multiply-add (2.1 issue cycles a warp
-// measured, against 6.3 for a 32-bit high product).  Two products and one more
-// term fit 32 bits (2 (p/2 + 4)^2 + p/2 + 4 < 2^31); four (below 2^32.1 in
-// 64 bits) are halved for the quotient, which then is off by 2 / p more.
+// and the rounding are one 64-bit multiply-add (four issue cycles a warp measured, as
+// many as a 32-bit high product, after which the rounding is an instruction more).  Two products
+// and one more term fit 32 bits (2 (p/2 + 4)^2 + p/2 + 4 < 2^31).  Four and one more are
+// halved for the quotient, which then is off by 2 / p more: half of |w| + 4 |l P|, with
+// |l| <= p/2 + 1 and |P|, |w| <= p/2 + 4, must be below 2^31, and is (4 x 32761 x 32764 +
+// 32764 < 2^32 at p = 65521, with 0.03 % to spare).
 //
 // SearchMont and SearchPlain reduce without division (an inverse costs more
 // than a whole column there): one elimination step is upd(y, w, na, P) = k (y
@@ -321,16 +311,16 @@ struct SearchPlain {
 // past the last window position are reached only when no window row has one
 // and the head histogram says one of them may: they are then reduced by the
 // same recurrence, in position order.
-// Outputs: PanelOut; U (t x EW, row stride EW: the pivot rows' final panel
-// values) and the pivot inverses; the host's copy of the result as words of
+// Outputs: the pivot columns (relative to c0); U (t x EW, row stride EW: the pivot
+// rows' final panel values) and the pivot inverses; the host's copy of the result as words of
 // a value and the call's sequence number (hout), so that no fence orders
 // them.  Resets *last_act to -1 and hist[] to zero for the next panel.
 //
 // Blocks of PB = 4 columns.  Warp 0 alone chooses the pivots of a block: the
 // live rows in position order, entry e in register group e / 32 of lane e %
-// 32, the block's columns in registers; a column's pivot is the first lane of
-// a ballot, its entries come by shuffles, and the elimination runs on the
-// block's columns and keeps each row's coefficients of the block's pivot rows
+// 32, the block's columns in registers; a column's pivot is the first live entry with
+// a nonzero there (a warp-wide minimum), its row comes by shuffles, and the elimination runs
+// on the block's columns and keeps each row's coefficients of the block's pivot rows
 // (its multipliers l; or, division-free, the row's current value as sc times
 // its value before the block plus cf[j] times that of the pivot row of the
 // block's column j).  No barrier is on that chain.  The pivot row reduces to
@@ -389,7 +379,8 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
                         int *hist, int *last_act, int *p2r,
                         int *stamp, int epoch, uint32_t *Uout,
                         uint32_t *xinv_out, uint32_t *Uinv_out,
-                        uint32_t *Linv_out, PanelOut *out, volatile uint64_t *hout, uint32_t seq, int wcap) {
+                        uint32_t *Linv_out, uint32_t *pcol_out, volatile uint64_t *hout, uint32_t seq,
+                        int wcap) {
   using V = typename SA::V;
   using V4 = typename SA::V4;
   extern __shared__ __align__(16) uint32_t dyn_w[];
@@ -551,31 +542,30 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
 #pragma unroll
       for (int j = 0; j < PB; ++j) z[j][g] = (in && col0 + j < w) ? Wv[ent[g]][col0 + j] : 0;
     }
-    if (SA::NORM && ahead) {
-      const int pb = buf ^ 1, tb = s_t0[pb], nb = t - tb, c = col0 + (lane & (PB - 1));
-      V P[PB];
+    if constexpr (SA::NORM)
+      if (ahead) {
+        const int pb = buf ^ 1, tb = s_t0[pb], nb = t - tb, c = col0 + (lane & (PB - 1));
+        V P[PB];
 #pragma unroll
-      for (int k = 0; k < PB; ++k) P[k] = k < nb && c < w ? Wv[s_prow[tb + k]][c] : 0;
-      if constexpr (SA::NORM) finish(P, pb, tb, nb);
-      V U[PB][PB];  // [column][pivot], from lanes 0 .. PB - 1
+        for (int k = 0; k < PB; ++k) P[k] = k < nb && c < w ? Wv[s_prow[tb + k]][c] : 0;
+        finish(P, pb, tb, nb);
+        V U[PB][PB];  // [column][pivot], from lanes 0 .. PB - 1
 #pragma unroll
-      for (int j = 0; j < PB; ++j)
+        for (int j = 0; j < PB; ++j)
 #pragma unroll
-        for (int k = 0; k < PB; ++k) U[j][k] = __shfl_sync(FULL, P[k], j);
-      [[maybe_unused]] const V psc = s_sc[pb];
+          for (int k = 0; k < PB; ++k) U[j][k] = __shfl_sync(FULL, P[k], j);
 #pragma unroll
-      for (int g = 0; g < NG; ++g) {
-        const V4 cf = s_coef[pb][ent[g]];
-        if (live[g] != NONE) {
+        for (int g = 0; g < NG; ++g) {
+          const V4 cf = s_coef[pb][ent[g]];
+          if (live[g] != NONE) {
 #pragma unroll
-          for (int j = 0; j < PB; ++j) {
-            if constexpr (SA::NORM) z[j][g] = sa.lin(z[j][g], cf, U[j]);
-            else z[j][g] = sa.lin(psc, z[j][g], cf, U[j]);
-            Wv[ent[g]][min(col0 + j, PW_LD - 1)] = z[j][g];
+            for (int j = 0; j < PB; ++j) {
+              z[j][g] = sa.lin(z[j][g], cf, U[j]);
+              Wv[ent[g]][min(col0 + j, PW_LD - 1)] = z[j][g];
+            }
           }
         }
       }
-    }
     if (!SA::NORM && lane < PB) s_pj[buf][lane] = -1;
     __syncwarp();
     const int t0 = t;
@@ -1102,9 +1092,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
     const int k = tid - 64;
     if (k < t) {
       const int2 pv = s_piv[k];
-      out->pcol[k] = (uint32_t)pv.x;
-      out->ti[k] = (uint32_t)(i0 + k);
-      out->tq[k] = (uint32_t)pv.y;
+      pcol_out[k] = (uint32_t)pv.x;
       hout[PANEL_W_PIV + 2 * k] = word((uint32_t)pv.x);
       hout[PANEL_W_PIV + 2 * k + 1] = word((uint32_t)pv.y);
     }
@@ -1133,11 +1121,6 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
     hout[PANEL_W_LAST] = word((uint32_t)last);
     hout[PANEL_W_DET] = word(s_det);
     s_uinv = (int)uinv;
-    out->uinv = uinv;
-    out->t = (uint32_t)t;
-    out->err = (uint32_t)s_err;
-    out->last_pos = (uint32_t)last;
-    out->det = s_det;
     *last_act = -1;
   }
   // U_k (division-free: (S_k U_k) / S_k); entries left of the pivot column are
@@ -1217,12 +1200,11 @@ __global__ void __launch_bounds__(PERM_THREADS)
 // panel becomes zero).  Row i0 + r of L = [L11; L21] goes to
 // Lout[r * ldl + 0 .. t-1].
 constexpr int SOLVE_THREADS = 256;
-template <class A>
 __global__ void __launch_bounds__(SOLVE_THREADS)
     panel_solve_kernel(uint32_t *__restrict__ D, size_t ld, int i0, int r1, int c0, int w, int t,
                        const uint32_t *__restrict__ pcol, const uint32_t *__restrict__ Uin,
-                       const uint32_t *__restrict__ xinv, A ar, uint32_t *__restrict__ Lout,
-                       size_t ldl) {
+                       const uint32_t *__restrict__ xinv, ArithWide ar,
+                       uint32_t *__restrict__ Lout, size_t ldl) {
   __shared__ uint32_t sU[EW][EW];
   __shared__ uint32_t sX[EW];
   __shared__ int sP[EW];
@@ -1337,10 +1319,9 @@ __global__ void __launch_bounds__(SOLVE_THREADS)
 // substitution with a unit diagonal.
 constexpr int U12_THREADS = 128;
 constexpr int U12_COLS = U12_THREADS / 4;
-template <class A>
 __global__ void __launch_bounds__(U12_THREADS)
     panel_u12_kernel(const uint32_t *__restrict__ L, size_t ldl, int t, uint32_t *__restrict__ B,
-                     size_t ldb, int ncols, A ar) {
+                     size_t ldb, int ncols, ArithWide ar) {
   __shared__ __align__(16) uint32_t sL[EW][EW];
   {
     constexpr int PER = EW * EW / U12_THREADS;
@@ -1371,7 +1352,7 @@ __global__ void __launch_bounds__(U12_THREADS)
   for (int k = 1; k < EW; ++k) {
     if (k < t) {
       // entries j >= k still hold a_j, but L11[k][j] is zero there
-      typename A::Acc acc = A::zero();
+      ArithWide::Acc acc = ArithWide::zero();
 #pragma unroll
       for (int i = 0; i <= (k - 1) / 4; ++i) ar.acc(acc, sL[k][4 * i + l4], x[i]);
       uint32_t v = ar.sum(acc);
@@ -1408,7 +1389,7 @@ int zp_echelon_dev(Ctx *c, int m, int n, uint32_t p, uint32_t *D, size_t ld, siz
   }
 
   // device scratch
-  const size_t out_bytes = (sizeof(PanelOut) + 255) & ~(size_t)255;
+  const size_t out_bytes = EW * sizeof(uint32_t);  // pivot columns
   // p2r, stamp (m each); permutation lists (4 EW); last row (1); histogram (EW + 1)
   const size_t i_bytes =
       (((size_t)2 * m + 4 * EW + 1 + EW + 1) * sizeof(int) + 255) & ~(size_t)255;
@@ -1421,7 +1402,7 @@ int zp_echelon_dev(Ctx *c, int m, int n, uint32_t p, uint32_t *D, size_t ld, siz
                       &base);
   if (st) return st;
   uint8_t *b8 = static_cast<uint8_t *>(base);
-  PanelOut *d_out = reinterpret_cast<PanelOut *>(b8);
+  uint32_t *d_pcol = reinterpret_cast<uint32_t *>(b8);
   int *d_p2r = reinterpret_cast<int *>(b8 + out_bytes);
   int *d_stamp = d_p2r + m;
   int *d_perm = d_stamp + m;      // 4*EW ints: src list, dst list
@@ -1434,7 +1415,6 @@ int zp_echelon_dev(Ctx *c, int m, int n, uint32_t p, uint32_t *D, size_t ld, siz
   uint32_t *d_Uinv = d_xinv + EW * EW;  // U_P^-1 (t x EW), p < 2^31
   uint32_t *d_Linv = d_Uinv + EW * EW;  // L11^-1 (t x EW), p < 2^31
   uint32_t *d_L = d_Linv + EW * EW;  // the block's multipliers (m x EB)
-  const uint32_t *d_pcol = reinterpret_cast<const uint32_t *>(b8 + offsetof(PanelOut, pcol));
   void *gws = nullptr;
   // one size for the panel and block updates and the block's trsm (which
   // takes the same workspace, so it must not grow it)
@@ -1463,8 +1443,10 @@ int zp_echelon_dev(Ctx *c, int m, int n, uint32_t p, uint32_t *D, size_t ld, siz
   if ((st = ctx_panel_map(c, &mh, &md))) return st;
   int *hperm = reinterpret_cast<int *>(static_cast<char *>(mh) + PANEL_PERM_OFF);
   static_assert(2 * (2 * EW) <= (int)PANEL_PERM_INTS, "staging layout");
-  volatile uint64_t *hwords = reinterpret_cast<volatile uint64_t *>(static_cast<char *>(mh) + PANEL_WORDS_OFF);
-  volatile uint64_t *hwords_dev = reinterpret_cast<volatile uint64_t *>(static_cast<char *>(md) + PANEL_WORDS_OFF);
+  auto words = [](void *map) {
+    return reinterpret_cast<volatile uint64_t *>(static_cast<char *>(map) + PANEL_WORDS_OFF);
+  };
+  volatile uint64_t *hwords = words(mh), *hwords_dev = words(md);
   cudaError_t e = cudaMemsetAsync(d_stamp, 0xff, (size_t)m * sizeof(int), c->stream);
   if (e == cudaSuccess && keep) {
     keep->swaps.clear();
@@ -1474,7 +1456,10 @@ int zp_echelon_dev(Ctx *c, int m, int n, uint32_t p, uint32_t *D, size_t ld, siz
   if (e == cudaSuccess) e = cudaMemsetAsync(d_hist, 0, (EW + 1) * sizeof(int), c->stream);
   if (e != cudaSuccess) return ctx_cuda(c, e, "echelon: scratch");
 
-  PanelOut h;
+  struct {
+    uint32_t t, uinv, err, last_pos, det;  // see the words' enum
+    uint32_t pcol[EW], ti[EW], tq[EW];     // pivot columns; transposition k: (ti[k], tq[k])
+  } h;
   std::vector<int> at, src, dst;
   int i = 0, epoch = 0;
   const int head_grid = std::max(1, std::min((m + 7) / 8, c->num_sms * 2));
@@ -1512,10 +1497,9 @@ int zp_echelon_dev(Ctx *c, int m, int n, uint32_t p, uint32_t *D, size_t ld, siz
     const size_t smem = PW_SMEM + (decltype(sa)::NORM ? PW_TABLE : 0);
     int s = ctx_smem_attr(c, (const void *)kern, (int)smem, "echelon: panel search attributes");
     if (s) return s;
-    pdl_launch(kern, 1, PS_THREADS, smem, c->stream,
-      D, ld, i, m, c0, w, sa, ar, d_head, d_act, d_hist,
-                                                d_last, d_p2r, d_stamp, epoch, d_U, d_xinv, d_Uinv,
-                                                d_Linv, d_out, hwords_dev, seq, wcap);
+    pdl_launch(kern, 1, PS_THREADS, smem, c->stream, D, ld, i, m, c0, w, sa, ar, d_head, d_act,
+               d_hist, d_last, d_p2r, d_stamp, epoch, d_U, d_xinv, d_Uinv, d_Linv, d_pcol,
+               hwords_dev, seq, wcap);
     return ST_OK;
   };
   // window rows of the search: the full PW_R, or 64 when the previous panel
@@ -1606,9 +1590,8 @@ int zp_echelon_dev(Ctx *c, int m, int n, uint32_t p, uint32_t *D, size_t ld, siz
         ctx_launched(c);
       }
       if (keep && rank > 0) {  // and every earlier pivot's kept multipliers
-        pdl_launch(permute_rows_kernel, ((int)rank + PERM_COLS - 1) / PERM_COLS, PERM_THREADS, 0, c->stream,
-      keep->L, keep->ldL, (int)rank, d_perm, d_perm + cnt,
-                                           cnt);
+        pdl_launch(permute_rows_kernel, ((int)rank + PERM_COLS - 1) / PERM_COLS, PERM_THREADS, 0,
+                   c->stream, keep->L, keep->ldL, (int)rank, d_perm, d_perm + cnt, cnt);
         ctx_launched(c);
       }
     }

@@ -237,15 +237,16 @@ static void unpack_rows(Ctx *c, const uint64_t *A, size_t lda, int M, int k0, ui
   // one pass a warp up to 16 CTAs an SM, then more
   const int gy = std::min((M + UNPACK_ROWS - 1) / UNPACK_ROWS, c->num_sms * 16);
   const int gx = std::max(1, std::min((Kp / 16 + 31) / 32, c->num_sms * 16 / gy));
-  pdl_launch(gf2_unpack_rows_kernel, dim3(gx, gy), dim3(32, UNPACK_ROWS), 0, c->stream,
-      A, lda, M, k0, out, Kp);
+  pdl_launch(gf2_unpack_rows_kernel, dim3(gx, gy), dim3(32, UNPACK_ROWS), 0, c->stream, A, lda, M,
+             k0, out, Kp);
   ctx_launched(c);
 }
 static void unpack_cols(Ctx *c, const uint64_t *B, size_t ldb, int k0, int kc, int N, uint8_t *out,
                         int Kp, bool early) {
   const int Nw = (N + 63) / 64;
-  pdl_launch_if(early, gf2_unpack_cols_kernel, dim3((Nw + UNPACK_W - 1) / UNPACK_W, (Kp + UNPACK_K - 1) / UNPACK_K), 32 * UNPACK_WARPS, 0, c->stream,
-      B, ldb, k0, kc, N, out, Kp);
+  const dim3 grid((Nw + UNPACK_W - 1) / UNPACK_W, (Kp + UNPACK_K - 1) / UNPACK_K);
+  pdl_launch_if(early, gf2_unpack_cols_kernel, grid, 32 * UNPACK_WARPS, 0, c->stream, B, ldb, k0, kc, N,
+                out, Kp);
   ctx_launched(c);
 }
 
@@ -560,7 +561,6 @@ __global__ void __launch_bounds__(32)
       }
     } else {
       // none in the window: rows past it whose bound allows a pivot here
-      const int i = i0 + t;
       int cand = 0;
       for (int h = lane; h <= col; h += 32) cand += s_cnt[h];
       cand = __reduce_add_sync(FULL, cand);
@@ -627,7 +627,6 @@ __global__ void __launch_bounds__(32)
       }
       __syncwarp();
       set_row(t, U);
-      (void)i;
     }
     if (basis) basis_add(row_word(t), col, t);
     if (lane == 0) {
@@ -953,8 +952,10 @@ int gf2_echelon_dev(Ctx *c, int m, int n, uint64_t *D, size_t ld, size_t *rank_o
   if ((st = ctx_panel_map(c, &mh, &md))) return st;
   int *hperm = reinterpret_cast<int *>(static_cast<char *>(mh) + PANEL_PERM_OFF);
   static_assert(2 * (2 * GW) <= (int)PANEL_PERM_INTS, "staging layout");
-  volatile uint64_t *hwords = reinterpret_cast<volatile uint64_t *>(static_cast<char *>(mh) + PANEL_WORDS_OFF);
-  volatile uint64_t *hwords_dev = reinterpret_cast<volatile uint64_t *>(static_cast<char *>(md) + PANEL_WORDS_OFF);
+  auto words = [](void *map) {
+    return reinterpret_cast<volatile uint64_t *>(static_cast<char *>(map) + PANEL_WORDS_OFF);
+  };
+  volatile uint64_t *hwords = words(mh), *hwords_dev = words(md);
   cudaError_t e = cudaMemsetAsync(d_stamp, 0xff, (size_t)m * sizeof(int), c->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(d_last, 0xff, sizeof(int), c->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(d_hist, 0, (GW + 1) * sizeof(int), c->stream);
@@ -968,7 +969,8 @@ int gf2_echelon_dev(Ctx *c, int m, int n, uint64_t *D, size_t ld, size_t *rank_o
   // Blocks of GB words (delayed updates), as in the Z/p form: when the
   // block's first panel with pivots has at least DELAY_ROWS rows below it,
   // the block's panels update only the block's words; the words right of it
-  // get, per block, U12 = L11^-1 A12 on the block's pivot rows and one C ^= L21 U12 with K = the block's pivots (up to 64 GB bits) on the rows
+  // get, per block, U12 = L11^-1 A12 on the block's pivot rows and one C ^= L21
+  // U12 with K = the block's pivots (up to 64 GB bits) on the rows
   // below.  d_Lb row q (GB words) holds the multipliers of the row at
   // position q, panel k of the block at bits Tb_k .. Tb_k + t_k - 1; later
   // panels' transpositions move d_Lb's rows with D's.

@@ -124,13 +124,11 @@ static void launch_inv_blocks(Ctx *c, bool upper, int m, const uint32_t *A, size
                               uint32_t p) {
   const int nblk = (m + TRI_NB - 1) / TRI_NB;
   if (p < (1u << 16))
-    pdl_launch(tri_inv_blocks_kernel<ArithSmall>, nblk, INV_THREADS, 0, c->stream,
-      A, lda, m, upper, dinv, Tinv, ldo,
-                                                               cmod, ArithSmall::make(p));
+    pdl_launch(tri_inv_blocks_kernel<ArithSmall>, nblk, INV_THREADS, 0, c->stream, A, lda, m, upper,
+               dinv, Tinv, ldo, cmod, ArithSmall::make(p));
   else
-    pdl_launch(tri_inv_blocks_kernel<ArithWide>, nblk, INV_THREADS, 0, c->stream,
-      A, lda, m, upper, dinv, Tinv, ldo,
-                                                               cmod, ArithWide::make(p));
+    pdl_launch(tri_inv_blocks_kernel<ArithWide>, nblk, INV_THREADS, 0, c->stream, A, lda, m, upper,
+               dinv, Tinv, ldo, cmod, ArithWide::make(p));
   ctx_launched(c);
 }
 
@@ -585,12 +583,10 @@ static int tri_inverse_levels(Ctx *c, bool upper, int m, uint32_t p, const uint3
       const dim3 g1((N1 + MG_T - 1) / MG_T, (M1 + MG_T - 1) / MG_T, nz);
       const dim3 g2((N2 + MG_T - 1) / MG_T, (M2 + MG_T - 1) / MG_T, nz);
       auto merge = [&](auto ar) {
-        pdl_launch(tri_merge_kernel<decltype(ar)>, g1, 256, 0, c->stream,
-      X1, Y1, Tz, zbase, M1, N1, K1,
-                                                    upper ? MG_TO_N : MG_FROM_N, ar, false);
-        pdl_launch(tri_merge_kernel<decltype(ar)>, g2, 256, 0, c->stream,
-      X2, Tz, C2, zbase, M2, N2, K2,
-                                                    upper ? MG_FROM_M : MG_TO_M, ar, true);
+        pdl_launch(tri_merge_kernel<decltype(ar)>, g1, 256, 0, c->stream, X1, Y1, Tz, zbase, M1, N1,
+                   K1, upper ? MG_TO_N : MG_FROM_N, ar, false);
+        pdl_launch(tri_merge_kernel<decltype(ar)>, g2, 256, 0, c->stream, X2, Tz, C2, zbase, M2, N2,
+                   K2, upper ? MG_FROM_M : MG_TO_M, ar, true);
       };
       if (p < (1u << 16)) merge(ArithSmall::make(p));
       else merge(ArithWide::make(p));

@@ -903,8 +903,8 @@ __global__ void __launch_bounds__(DIR_THREADS, L == 4 ? 1 : 2)
 // of residue bytes, which the tensor-core kernel's epilogue reduces modulo m_i to
 // bytes again.  4096^3 at p = 2^31 - 1: 1015 -> 800 us a call (splits 140, products
 // 455 at 3.0 Pop/s, rns_combine_kernel 80).  Row blocks whose planes stay in L2 are no
-// faster (2048 rows 700 us, 1024 748, all 690).  A's residues carry the factor (P / m_i)^-1 mod m_i, so the
-// bytes are y_i with
+// faster (2048 rows 700 us, 1024 748, all 690).  A's residues carry the factor (P /
+// m_i)^-1 mod m_i, so the bytes are y_i with
 //     x = sum_i y_i (P / m_i) - t P,   t = floor(sum_i y_i / m_i),
 // and rns_combine_kernel takes that sum modulo p.  Exact: x / P < 1/2, so t is
 // floor(1/4 + sum y_i F_i / 2^15) with F_i = round(2^15 / m_i), whose error is
@@ -926,8 +926,9 @@ struct LimbBytes {
 // byte b) sum to r < 2^18.  m = 256: its low byte.  Odd m: in floats, four
 // instructions at the full rate where the integer multiply-high and multiply go at
 // less (the splits are issue-bound: 4096^2 entries, ten moduli, A's 66 us
-// against 70, the limbs' 25).  2^23 + r is a float read from the bits; (r - (m - 1) / 2) / m rounds to floor(r / m), being at least 1 / 2m > 2^-9 from a
-// half-integer with an error below 2^-13; 2^23 + r - q m is exact.
+// against 70, the limbs' 25).  2^23 + r is a float read from the bits; (r - (m - 1) / 2) / m
+// rounds to floor(r / m), being at least 1 / 2m > 2^-9 from a half-integer with an error
+// below 2^-13; 2^23 + r - q m is exact.
 struct ResidueBytes {
   static constexpr int MAX = RNS_MAX;
   int n;
@@ -1004,8 +1005,8 @@ static dim3 split_rows_grid(int num_sms, int M, int kc) {
 }
 
 // B (kc x N, row stride ldb, elements T) -> L planes of N rows of kout <= Kp
-// bytes (row pitch Kp, `plane` bytes apart; transposed), through a shared-memory tile of 64 k x NT columns (128 bytes
-// of a row of the narrow types, 32 elements of the others).
+// bytes (row pitch Kp, `plane` bytes apart; transposed), through a shared-memory tile of 64 k
+// x NT columns (128 bytes of a row of the narrow types, 32 elements of the others).
 template <class T>
 constexpr int split_cols_nt() {
   return sizeof(T) < 4 ? 128 / (int)sizeof(T) : 32;
@@ -1866,8 +1867,9 @@ static int host_rows(Ctx *c, int M, int N, int K, const Modulus &mod, uint32_t a
   if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream, ev_b, 0);
   if (e == cudaSuccess) {
     int pi = prof_begin(c, "zp_split");
-    pdl_launch(split_cols_kernel<LimbBytes<L>, uint32_t>, split_cols_grid<uint32_t>(N, Kp), 256, 0, c->stream,
-               dB, (size_t)N, K, N, (uint32_t)mod.p, Bl, (size_t)Kp, (size_t)N * Kp, Kp, LimbBytes<L>{});
+    pdl_launch(split_cols_kernel<LimbBytes<L>, uint32_t>, split_cols_grid<uint32_t>(N, Kp), 256, 0,
+               c->stream, dB, (size_t)N, K, N, (uint32_t)mod.p, Bl, (size_t)Kp, (size_t)N * Kp, Kp,
+               LimbBytes<L>{});
     prof_end(c, pi);
     ctx_launched(c);
     e = cudaGetLastError();
@@ -1891,9 +1893,9 @@ static int host_rows(Ctx *c, int M, int N, int K, const Modulus &mod, uint32_t a
     if (st) break;
     const int tiles = ((rows + BM - 1) / BM) * ((N + Cfg::BN - 1) / Cfg::BN);
     pi = prof_begin(c, "zp_gemm_tc");
-    pdl_launch(zp_gemm_tc_kernel<L, OUT_ZP>, std::min(tiles, c->num_sms), tc_threads<L, 0>(), Lay::SMEM, c->stream,
-               tmA, tmB, dC + (size_t)r0 * N, (size_t)N, rows, N, K, mod, alpha, beta, c->dstatus, nullptr,
-               0);
+    pdl_launch(zp_gemm_tc_kernel<L, OUT_ZP>, std::min(tiles, c->num_sms), tc_threads<L, 0>(),
+               Lay::SMEM, c->stream, tmA, tmB, dC + (size_t)r0 * N, (size_t)N, rows, N, K, mod, alpha,
+               beta, c->dstatus, nullptr, 0);
     prof_end(c, pi);
     ctx_launched(c, 2);
     e = cudaGetLastError();
@@ -2143,9 +2145,9 @@ static int gf2_tc_launch(Ctx *c, int M, int N, int K, const uint8_t *Ab, const u
   if (st) return st;
   const int tiles = ((M + BM - 1) / BM) * ((N + Cfg::BN - 1) / Cfg::BN);
   int pi = prof_begin(c, "gf2_gemm_tc");
-  pdl_launch_if(gf2_early(M, N, K), zp_gemm_tc_kernel<1, OUT_GF2, T>, std::min(tiles, c->num_sms), tc_threads<1, T>(), Lay::SMEM,
-             c->stream, tmA, tmB, C, ldc_words, M, N, K, make_modulus(2), alpha, beta, c->dstatus,
-             nullptr, 0);
+  pdl_launch_if(gf2_early(M, N, K), zp_gemm_tc_kernel<1, OUT_GF2, T>, std::min(tiles, c->num_sms),
+                tc_threads<1, T>(), Lay::SMEM, c->stream, tmA, tmB, C, ldc_words, M, N, K,
+                make_modulus(2), alpha, beta, c->dstatus, nullptr, 0);
   prof_end(c, pi);
   ctx_launched(c);
   cudaError_t e = cudaGetLastError();
