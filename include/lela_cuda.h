@@ -117,7 +117,9 @@ int lela_cuda_profile_reset (lela_cuda_ctx *ctx);
  * copied first, then A's and C's rows block by block on a second stream of
  * the handle, and each block's rows of C are copied back on a third while
  * later blocks still arrive.  Page-locked host buffers let the copies
- * overlap. */
+ * overlap.
+ * Device form: with the automatic kernel choice and k <= 32768, C may lie
+ * over A or B; the product is that of the operands as they were. */
 int lela_cuda_gemm_zp_u32 (lela_cuda_ctx *ctx, size_t m, size_t n, size_t k, uint32_t p,
 			   uint32_t a, const uint32_t *A, size_t lda, const uint32_t *B, size_t ldb,
 			   uint32_t b, uint32_t *C, size_t ldc);
@@ -388,10 +390,12 @@ int lela_cuda_echelon_zp_u32_batch (lela_cuda_ctx *ctx, size_t count, uint32_t *
  * device output of m[i] rows, stride ldr[i]), spread over nworkers threads
  * with their own streams, largest first.  status[i] as for the single call.
  * Memory-budgeted queue: when the nworkers largest matrices may not fit in
- * the budget together (estimate per matrix: 4 m n + 4 (m + n) m + 2 KB per
+ * the budget together (estimate per matrix: 4 m n + 4 (m + n) m + 5 KB per
  * row + 256 MB), a matrix starts only when its estimate fits beside those
  * running (one that does not fit even alone runs alone), and each worker
- * frees its device buffers after a matrix.  The batch is stream-ordered on
+ * frees its device buffers after a matrix.  Larger workspaces that some
+ * products and solves are faster with are taken only where all workers'
+ * fit the budget beside the estimates.  The batch is stream-ordered on
  * the handle's stream: the workers start after the work queued there, and
  * work queued there after the call starts after the batch. */
 /* Budget of that queue in bytes; 0 (the default) = 90 % of the free device
