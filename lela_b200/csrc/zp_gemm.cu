@@ -901,8 +901,9 @@ __global__ void __launch_bounds__(DIR_THREADS, L == 4 ? 1 : 2)
 // K, is instead formed modulo n pairwise coprime moduli m_i <= 256 with P = prod
 // m_i > 2 x (n = 6 at p = 2^17, 10 at p = 2^31 and K = 4096): n one-limb products
 // of residue bytes, which the tensor-core kernel's epilogue reduces modulo m_i to
-// bytes again.  4096^3 at p = 2^31 - 1: 1015 -> 800 us a call (splits 140, products
-// 455 at 3.0 Pop/s, rns_combine_kernel 80).  Row blocks whose planes stay in L2 are no
+// bytes again.  4096^3 at p = 2^31 - 1: 1015 -> 793 us a call on new operands (splits
+// 140, products 455 at 3.0 Pop/s, rns_combine_kernel 80), 941 -> 680 for a few in a row
+// on the same ones.  Row blocks whose planes stay in L2 are no
 // faster (2048 rows 700 us, 1024 748, all 690).  A's residues carry the factor (P /
 // m_i)^-1 mod m_i, so the bytes are y_i with
 //     x = sum_i y_i (P / m_i) - t P,   t = floor(sum_i y_i / m_i),
@@ -1466,7 +1467,7 @@ static int launch_rns(Ctx *c, int M, int N, int K, int rows, const Modulus &mod,
 
 // Whether a four-limb product goes by n residues.  They save 16 - n of 16 byte
 // products and cost planes n / 4 times as large and a pass over n bytes per entry of C.
-// Measured on the B200 (us per call from the host, limbs / residues; p = 2^16 + 1 has n =
+// Measured on the B200 (us per call, a few in a row on the same operands, limbs / residues; p = 2^16 + 1 has n =
 // 6, 2^24 - 3 8, 2^31 - 1 and 2^32 - 5 10): 4096^3 940 / 461, 576 and 693; 8192^3
 // 7062 / 2763, 7071 / 3559, 7398 / 4560; 2048^3 160 / 115, 129 and 150; 4096^2 x 512
 // 238 / 176, 201 and 226.  At n <= 8 down to 1024^2 x 2048 70 / 63 and 68, 512 x 8192 x
