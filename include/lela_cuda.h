@@ -61,7 +61,8 @@ enum {
 
 /* Kernel choice for the Z/p gemm (lela_cuda_set_gemm_kernel). */
 enum {
-	LELA_CUDA_GEMM_AUTO = 0,   /* tensor cores, in one launch for small K and few tiles */
+	LELA_CUDA_GEMM_AUTO = 0,   /* tensor cores, in one launch for small K and few tiles; the
+				      smallest products on CUDA cores */
 	LELA_CUDA_GEMM_PLAIN = 1,  /* CUDA-core delayed-reduction kernel */
 	LELA_CUDA_GEMM_TC = 2,     /* limb-split INT8 tcgen05 kernel */
 	LELA_CUDA_GEMM_SMALLK = 3  /* CUDA-core kernel for small K (unchecked sums when p < 2^28) */

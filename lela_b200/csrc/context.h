@@ -18,7 +18,8 @@ namespace lela {
 
 // Kernel families a caller (or the selector) can force.
 enum GemmKernel : int {
-  GEMM_AUTO = 0,    // GEMM_DIRECT for short K and few tiles, else GEMM_TC (zp_gemm_pick)
+  GEMM_AUTO = 0,    // by shape and modulus (zp_gemm_pick): GEMM_SMALLK for the smallest products,
+                    // GEMM_DIRECT for short K and few tiles, else GEMM_TC
   GEMM_PLAIN = 1,   // CUDA-core 64-bit delayed-reduction gemm (the plain GPU form)
   GEMM_TC = 2,      // limb-split INT8 tcgen05 gemm
   GEMM_SMALLK = 3,  // CUDA-core gemm for small K (no per-term wrap check when p < 2^28)

@@ -44,7 +44,8 @@ int zp_gemm_tc_elem_dev(Ctx *c, int elem, int M, int N, int K, uint32_t p, uint3
                         size_t ldv);
 
 // The kernel GEMM_AUTO resolves to for this shape (the handle's forced
-// kernel, else the one-launch tile kernel for short K and few tiles, else the
+// kernel, else the CUDA-core kernel for the smallest products, the one-launch
+// tile kernel for short K and few tiles, and for the others the
 // limb-plane one).
 int zp_gemm_pick(const Ctx *c, int M, int N, int K, uint32_t p);
 // The tensor-core tile variant (TcCfg<L, T>'s T: 0, 1, or 2 for one limb)
