@@ -957,21 +957,33 @@ struct ResidueBytes {
 // A (M x kc, row stride lda, elements T) -> L planes of bytes, row pitch Kp,
 // `plane` bytes apart.  Bound by
 // HBM (8192^2 of u32: 69 us, 402 MB); lanes on consecutive groups of four
-// columns, a row per warp, so no index division.  part: 0 all columns; 1 (2)
-// only those left (right) of the row's diagonal block of nb rows.
-constexpr int SPLIT_ROWS = 8;  // rows (warps) per CTA
+// columns, a row per warp, so no index division; rows of at most 64 columns share a
+// warp, as many as fill it (us a product, a row per warp / shared: p = 65521 262144 x 16 x
+// 32 79 / 58, 200000 x 64 x 64 72 / 62; wider rows keep the lane count known, which
+// 2000^3 feels by 2 %).  part: 0 all
+// columns; 1 (2) only those left (right) of the row's diagonal block of nb rows.
+constexpr int SPLIT_ROWS = 8;  // warps per CTA
+// log2 of the lanes that a row of kc columns takes
+__host__ __device__ __forceinline__ int split_lanes(int kc) {
+  int l = 1;
+  while (l < 5 && (4 << l) < kc) ++l;
+  return l;
+}
 template <class W, class T>
 __device__ __forceinline__ void split_rows(const T *A, size_t lda, int M, int kc, uint32_t p,
                                            uint8_t *out, size_t Kp, size_t plane, int part, int nb,
-                                           const W &planes, int bx, int by, int gx, int gy) {
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  for (int r = by * SPLIT_ROWS + ty; r < M; r += gy * SPLIT_ROWS) {
+                                           const W &planes, int bx, int by, int gx, int gy,
+                                           const int lb) {
+  const int rows = SPLIT_ROWS * (32 >> lb);  // per CTA
+  const int tx = threadIdx.x & ((1 << lb) - 1), ty = threadIdx.x >> lb;
+  for (int r = by * rows + ty; r < M; r += gy * rows) {
     const T *src = A + (size_t)r * lda;
     uint8_t *dst = out + (size_t)r * Kp;
-    const int kb = part == 2 ? min(kc, (r / nb + 1) * nb) : 0, ke = part == 1 ? min(kc, r / nb * nb) : kc;
+    const int kb = part == 2 ? min(kc, (r / nb + 1) * nb) : 0;
+    const int ke = part == 1 ? min(kc, r / nb * nb) : kc;
     constexpr int U = 2;  // groups in flight
-    const int step = gx * 32;
-    for (int q = (kb >> 2) + bx * 32 + tx; 4 * q < ke; q += U * step) {
+    const int step = gx << lb;
+    for (int q = (kb >> 2) + (bx << lb) + tx; 4 * q < ke; q += U * step) {
       uint32_t v[U][4];
 #pragma unroll
       for (int u = 0; u < U; ++u)
@@ -986,7 +998,8 @@ __device__ __forceinline__ void split_rows(const T *A, size_t lda, int M, int kc
         if (k >= ke) break;
 #pragma unroll
         for (int l = 0; l < W::MAX; ++l)
-          if (l < planes.count()) *reinterpret_cast<uint32_t *>(dst + l * plane + k) = planes.word(v[u], l);
+          if (l < planes.count())
+            *reinterpret_cast<uint32_t *>(dst + l * plane + k) = planes.word(v[u], l);
       }
     }
   }
@@ -996,12 +1009,17 @@ __global__ void __launch_bounds__(32 * SPLIT_ROWS)
     split_rows_kernel(const T *A, size_t lda, int M, int kc, uint32_t p,
                       uint8_t *out, size_t Kp, size_t plane, int part, int nb, const W planes) {
   pdl_enter();
-  split_rows<W, T>(A, lda, M, kc, p, out, Kp, plane, part, nb, planes, blockIdx.x, blockIdx.y,
-                   gridDim.x, gridDim.y);
+  if (kc > 64)  // (the lanes of a row known)
+    split_rows<W, T>(A, lda, M, kc, p, out, Kp, plane, part, nb, planes, blockIdx.x, blockIdx.y,
+                     gridDim.x, gridDim.y, 5);
+  else
+    split_rows<W, T>(A, lda, M, kc, p, out, Kp, plane, part, nb, planes, blockIdx.x, blockIdx.y,
+                     gridDim.x, gridDim.y, split_lanes(kc));
 }
 static dim3 split_rows_grid(int num_sms, int M, int kc) {
   // one pass a warp up to 16 CTAs an SM, then more
-  const int gy = std::min((M + SPLIT_ROWS - 1) / SPLIT_ROWS, num_sms * 16);
+  const int rows = SPLIT_ROWS * (32 >> split_lanes(kc));
+  const int gy = std::min((M + rows - 1) / rows, num_sms * 16);
   return dim3(std::max(1, std::min(((kc + 3) / 4 + 31) / 32, num_sms * 16 / gy)), gy);
 }
 
@@ -1071,9 +1089,12 @@ __global__ void __launch_bounds__(256)
   static_assert(32 * SPLIT_ROWS == 256, "one block size");
   pdl_enter();
   const int b = blockIdx.x, na = gax * gay;
-  if (b < na)
+  if (b < na && kc > 64)
     split_rows<W, T>(A, lda, M, kc, p, out_a, (size_t)Kp, (size_t)M * Kp, 0, 1, wa, b % gax, b / gax,
-                     gax, gay);
+                     gax, gay, 5);
+  else if (b < na)
+    split_rows<W, T>(A, lda, M, kc, p, out_a, (size_t)Kp, (size_t)M * Kp, 0, 1, wa, b % gax, b / gax,
+                     gax, gay, split_lanes(kc));
   else
     split_cols<W, T>(B, ldb, kc, N, p, out_b, (size_t)Kp, (size_t)N * Kp, Kp, wb, (b - na) % gbx,
                      (b - na) / gbx);
