@@ -1627,7 +1627,14 @@ int zp_gemm_pick(const Ctx *c, int M, int N, int K, uint32_t p) {
     return GEMM_SMALLK;
   const long long tiles = (long long)((M + BM - 1) / BM) * ((N + bn - 1) / bn);
   const long long most = K <= 128 ? (L == 4 ? 2 : 4) * c->num_sms : K <= 256 ? c->num_sms : 0;
-  return tiles <= most ? GEMM_DIRECT : GEMM_TC;
+  if (tiles <= most) return GEMM_DIRECT;
+  // Beyond it, wide products of few rows and terms: the limb planes of B are most of the
+  // split kernels' work, and four limbs' tiles are 32 columns wide (us per call, CUDA
+  // cores / limb planes: p = 2^31 - 1 1 x 65536 x 5 55 / 99, 64 x 65536 x 5 72 / 131, x 32 72 / 85,
+  // x 48 120 / 98, 80 x 65536 x 5 121 / 129; p = 65521 1 x 65536 x 32 27 / 33, 32 x 65536 x 16 35 /
+  // 46, 64 x 65536 x 16 46 / 55, x 32 46 / 43).
+  if (M <= PT && K <= PK && (L == 4 || (L == 2 && (K <= PK / 2 || M <= 16)))) return GEMM_SMALLK;
+  return GEMM_TC;
 }
 
 // The tensor-core gemm for operands of type E (limb count and tile variant
