@@ -45,7 +45,7 @@
 //     the reference's elimination steps on its panel part; the panel becomes
 //     U_k in pivot row k and zero below;
 //  5. U12 = L11^-1 A12 (a tensor-core product with the search's inverse, in place;
-//     by substitution on CUDA cores for p >= 2^31) and A22 -= L21 U12 on the
+//     by substitution on CUDA cores for p >= 2^31 and on wide panels) and A22 -= L21 U12 on the
 //     tensor cores over the rows down to the last possibly nonzero row,
 //     for the columns of the panel's block of EB columns; the columns right
 //     of the block get one such update per block, with the multipliers of
@@ -1319,9 +1319,10 @@ __global__ void __launch_bounds__(SOLVE_THREADS)
 // substitution with a unit diagonal.
 constexpr int U12_THREADS = 128;
 constexpr int U12_COLS = U12_THREADS / 4;
+template <class A>
 __global__ void __launch_bounds__(U12_THREADS)
     panel_u12_kernel(const uint32_t *__restrict__ L, size_t ldl, int t, uint32_t *__restrict__ B,
-                     size_t ldb, int ncols, ArithWide ar) {
+                     size_t ldb, int ncols, A ar) {
   __shared__ __align__(16) uint32_t sL[EW][EW];
   {
     constexpr int PER = EW * EW / U12_THREADS;
@@ -1352,7 +1353,7 @@ __global__ void __launch_bounds__(U12_THREADS)
   for (int k = 1; k < EW; ++k) {
     if (k < t) {
       // entries j >= k still hold a_j, but L11[k][j] is zero there
-      ArithWide::Acc acc = ArithWide::zero();
+      typename A::Acc acc = A::zero();
 #pragma unroll
       for (int i = 0; i <= (k - 1) / 4; ++i) ar.acc(acc, sL[k][4 * i + l4], x[i]);
       uint32_t v = ar.sum(acc);
@@ -1372,6 +1373,19 @@ __global__ void __launch_bounds__(U12_THREADS)
     const int j = 4 * i + l4;
     if (valid && j >= 1 && j < t) B[(size_t)j * ldb + c] = x[i];
   }
+}
+
+// Whether U12 is substituted column by column for p < 2^31, too: wide panels, whose product has
+// many tiles of the same t <= 64 rows.  Measured with its launch (us, steps / product): p = 2^31
+// - 1 t = 64 4000 columns 25 / 22, 8000 27 / 33, 32000 62 / 76, 300000 437 / 573, t = 8 16000 13 /
+// 45, 300000 88 / 518; p = 65521 t = 64 32000 35 / 29, 300000 240 / 143, t = 32 32000 23 / 27, 300000
+// 123 / 121, t = 16 32000 19 / 24, 300000 89 / 119, t = 2 300000 70 / 115; p = 251 t = 24 32000 21 /
+// 22, 300000 105 / 96, t = 16 300000 88 / 94.  (Narrow panels of few pivots keep the product,
+// whose launch starts early behind the solve: a 64 x 8000 form modulo 2^31 - 1 takes 107 us with
+// it and 113 by steps, a 64 x 20000 one 130 and 121, 20 x 8000 74 and 63.)
+static bool u12_by_steps(uint32_t p, int t, int rest) {
+  if (p > 65536) return rest > (t <= 48 ? 6000 : 12000);
+  return t <= 16 && rest > 16000;
 }
 
 int zp_echelon_dev(Ctx *c, int m, int n, uint32_t p, uint32_t *D, size_t ld, size_t *rank_out,
@@ -1639,14 +1653,17 @@ int zp_echelon_dev(Ctx *c, int m, int n, uint32_t p, uint32_t *D, size_t ld, siz
     if (rest > 0) {
       uint32_t *U12 = D + (size_t)i * ld + c0 + w;
       pi = prof_begin(c, "ech_u12");
-      if (h.uinv) {
+      if (h.uinv && !u12_by_steps(p, t, rest)) {
         // U12 = L11^-1 A12 in place: one tile of rows, each CTA on its columns
         if ((st = zp_gemm_dev(c, GEMM_DIRECT, t, rest, t, p, 1, d_Linv, EW, U12, ld, 0, U12, ld,
                               static_cast<uint8_t *>(gws))))
           return st;
       } else {
         const int ugrid = (rest + U12_COLS - 1) / U12_COLS;
-        panel_u12_kernel<<<ugrid, U12_THREADS, 0, c->stream>>>(Lp, EB, t, U12, ld, rest, arw);
+        if (small)
+          panel_u12_kernel<<<ugrid, U12_THREADS, 0, c->stream>>>(Lp, EB, t, U12, ld, rest, ars);
+        else
+          panel_u12_kernel<<<ugrid, U12_THREADS, 0, c->stream>>>(Lp, EB, t, U12, ld, rest, arw);
         ctx_launched(c);
       }
       prof_end(c, pi);
