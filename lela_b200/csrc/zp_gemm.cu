@@ -959,22 +959,24 @@ struct ResidueBytes {
 // HBM (8192^2 of u32: 69 us, 402 MB); lanes on consecutive groups of four
 // columns, a row per warp, so no index division; rows of at most 64 columns share a
 // warp, as many as fill it (us a product, a row per warp / shared: p = 65521 262144 x 16 x
-// 32 79 / 58, 200000 x 64 x 64 72 / 62; wider rows keep the lane count known, which
-// 2000^3 feels by 2 %).  part: 0 all
-// columns; 1 (2) only those left (right) of the row's diagonal block of nb rows.
+// 32 79 / 58, 200000 x 64 x 64 72 / 62; kernels of their own, since both in one
+// slowed wider rows by up to 2 %).  part: 0 all columns; 1 (2) only those left
+// (right) of the row's diagonal block of nb rows.
 constexpr int SPLIT_ROWS = 8;  // warps per CTA
+// The NARROW instances below, for rows enough to fill the SMs with fewer CTAs (8192 x 8192 x
+// 64 at four limbs 605 us, narrow 610).
+static bool split_narrow(int M, int kc) { return kc <= 64 && M >= 16384; }
 // log2 of the lanes that a row of kc columns takes
 __host__ __device__ __forceinline__ int split_lanes(int kc) {
   int l = 1;
   while (l < 5 && (4 << l) < kc) ++l;
   return l;
 }
-template <class W, class T>
+template <class W, class T, bool NARROW>
 __device__ __forceinline__ void split_rows(const T *A, size_t lda, int M, int kc, uint32_t p,
                                            uint8_t *out, size_t Kp, size_t plane, int part, int nb,
-                                           const W &planes, int bx, int by, int gx, int gy,
-                                           const int lb) {
-  const int rows = SPLIT_ROWS * (32 >> lb);  // per CTA
+                                           const W &planes, int bx, int by, int gx, int gy) {
+  const int lb = NARROW ? split_lanes(kc) : 5, rows = SPLIT_ROWS * (32 >> lb);  // rows per CTA
   const int tx = threadIdx.x & ((1 << lb) - 1), ty = threadIdx.x >> lb;
   for (int r = by * rows + ty; r < M; r += gy * rows) {
     const T *src = A + (size_t)r * lda;
@@ -1004,21 +1006,17 @@ __device__ __forceinline__ void split_rows(const T *A, size_t lda, int M, int kc
     }
   }
 }
-template <class W, class T>
+template <class W, class T, bool NARROW>
 __global__ void __launch_bounds__(32 * SPLIT_ROWS)
     split_rows_kernel(const T *A, size_t lda, int M, int kc, uint32_t p,
                       uint8_t *out, size_t Kp, size_t plane, int part, int nb, const W planes) {
   pdl_enter();
-  if (kc > 64)  // (the lanes of a row known)
-    split_rows<W, T>(A, lda, M, kc, p, out, Kp, plane, part, nb, planes, blockIdx.x, blockIdx.y,
-                     gridDim.x, gridDim.y, 5);
-  else
-    split_rows<W, T>(A, lda, M, kc, p, out, Kp, plane, part, nb, planes, blockIdx.x, blockIdx.y,
-                     gridDim.x, gridDim.y, split_lanes(kc));
+  split_rows<W, T, NARROW>(A, lda, M, kc, p, out, Kp, plane, part, nb, planes, blockIdx.x,
+                           blockIdx.y, gridDim.x, gridDim.y);
 }
 static dim3 split_rows_grid(int num_sms, int M, int kc) {
   // one pass a warp up to 16 CTAs an SM, then more
-  const int rows = SPLIT_ROWS * (32 >> split_lanes(kc));
+  const int rows = SPLIT_ROWS * (split_narrow(M, kc) ? 32 >> split_lanes(kc) : 1);
   const int gy = std::min((M + rows - 1) / rows, num_sms * 16);
   return dim3(std::max(1, std::min(((kc + 3) / 4 + 31) / 32, num_sms * 16 / gy)), gy);
 }
@@ -1081,7 +1079,7 @@ static dim3 split_cols_grid(int N, int Kp) {
 // Both operands' planes in one launch, A's (M x kc, planes from out_a, rows Kp
 // apart) in the first gax * gay CTAs: a product of few tiles waits for each launch (512^3
 // 17.6 us a call, 20.4 with two launches).
-template <class W, class T>
+template <class W, class T, bool NARROW>
 __global__ void __launch_bounds__(256)
     split_both_kernel(const T *A, size_t lda, const T *B, size_t ldb, int M, int N, int kc,
                       uint32_t p, uint8_t *out_a, uint8_t *out_b, int Kp, int gax, int gay, int gbx,
@@ -1089,12 +1087,9 @@ __global__ void __launch_bounds__(256)
   static_assert(32 * SPLIT_ROWS == 256, "one block size");
   pdl_enter();
   const int b = blockIdx.x, na = gax * gay;
-  if (b < na && kc > 64)
-    split_rows<W, T>(A, lda, M, kc, p, out_a, (size_t)Kp, (size_t)M * Kp, 0, 1, wa, b % gax, b / gax,
-                     gax, gay, 5);
-  else if (b < na)
-    split_rows<W, T>(A, lda, M, kc, p, out_a, (size_t)Kp, (size_t)M * Kp, 0, 1, wa, b % gax, b / gax,
-                     gax, gay, split_lanes(kc));
+  if (b < na)
+    split_rows<W, T, NARROW>(A, lda, M, kc, p, out_a, (size_t)Kp, (size_t)M * Kp, 0, 1, wa, b % gax,
+                             b / gax, gax, gay);
   else
     split_cols<W, T>(B, ldb, kc, N, p, out_b, (size_t)Kp, (size_t)N * Kp, Kp, wb, (b - na) % gbx,
                      (b - na) / gbx);
@@ -1104,8 +1099,9 @@ static void launch_split(bool early, int num_sms, cudaStream_t s, const T *A, si
                          size_t ldb, int M, int N, int kc, uint32_t p, uint8_t *out_a, uint8_t *out_b,
                          int Kp, const W &wa, const W &wb) {
   const dim3 ga = split_rows_grid(num_sms, M, kc), gb = split_cols_grid<T>(N, Kp);
-  pdl_launch_if(early, split_both_kernel<W, T>, ga.x * ga.y + gb.x * gb.y, 256, 0, s, A, lda, B, ldb,
-                M, N, kc, p, out_a, out_b, Kp, (int)ga.x, (int)ga.y, (int)gb.x, wa, wb);
+  auto kern = split_narrow(M, kc) ? split_both_kernel<W, T, true> : split_both_kernel<W, T, false>;
+  pdl_launch_if(early, kern, ga.x * ga.y + gb.x * gb.y, 256, 0, s, A, lda, B, ldb, M, N, kc, p, out_a,
+                out_b, Kp, (int)ga.x, (int)ga.y, (int)gb.x, wa, wb);
 }
 
 // ------------------------------------------------- residues back to Z/p
@@ -1457,7 +1453,7 @@ static int launch_rns(Ctx *c, int M, int N, int K, int rows, const Modulus &mod,
     const int m = std::min(rows, M - r0);
     uint32_t *Cr = C + (size_t)r0 * ldc;
     pi = prof_begin(c, "zp_split");
-    pdl_launch_if(early, split_rows_kernel<ResidueBytes, E>, split_rows_grid(c->num_sms, m, K),
+    pdl_launch_if(early, split_rows_kernel<ResidueBytes, E, false>, split_rows_grid(c->num_sms, m, K),
                   32 * SPLIT_ROWS, 0, c->stream, A + (size_t)r0 * lda, lda, m, K, p, Al, Kp,
                   (size_t)m * Kp, 0, 1, ra);
     prof_end(c, pi);
@@ -1805,7 +1801,9 @@ int zp_split_rows_dev(Ctx *c, uint32_t p, const uint32_t *A, size_t lda, int M, 
                       const ZpPlanes &out, int part, int nb) {
   const dim3 grid = split_rows_grid(c->num_sms, M, K), block(32 * SPLIT_ROWS);
 #define LELA_SR(L) \
-  pdl_launch(split_rows_kernel<LimbBytes<L>, uint32_t>, grid, block, 0, c->stream, A, lda, M, K, p, \
+  pdl_launch(split_narrow(M, K) ? split_rows_kernel<LimbBytes<L>, uint32_t, true>         \
+                                : split_rows_kernel<LimbBytes<L>, uint32_t, false>,       \
+             grid, block, 0, c->stream, A, lda, M, K, p,                                  \
              out.base, out.pitch, out.plane, part, nb, LimbBytes<L>{})
   switch (zp_limbs_for(p)) {
     case 1: LELA_SR(1); break;
@@ -1912,7 +1910,9 @@ static int host_rows(Ctx *c, int M, int N, int K, const Modulus &mod, uint32_t a
     e = cudaStreamWaitEvent(c->stream, ready[j], 0);
     if (e != cudaSuccess) break;
     int pi = prof_begin(c, "zp_split");
-    pdl_launch(split_rows_kernel<LimbBytes<L>, uint32_t>, split_rows_grid(c->num_sms, rows, K),
+    pdl_launch(split_narrow(rows, K) ? split_rows_kernel<LimbBytes<L>, uint32_t, true>
+                                     : split_rows_kernel<LimbBytes<L>, uint32_t, false>,
+               split_rows_grid(c->num_sms, rows, K),
                32 * SPLIT_ROWS, 0, c->stream, dA + (size_t)r0 * K, (size_t)K, rows, K,
                (uint32_t)mod.p, Al, (size_t)Kp, (size_t)rows * Kp, 0, 1, LimbBytes<L>{});
     prof_end(c, pi);

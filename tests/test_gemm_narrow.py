@@ -10,8 +10,9 @@ from lela_b200 import gen
 @pytest.mark.gpu
 @pytest.mark.parametrize("p", [251, 65521, 2147483647])
 @pytest.mark.parametrize("k", [1, 3, 4, 5, 8, 9, 16, 17, 31, 32, 33, 63, 64, 65])
-def test_short_rows(cuda, p, k):
-    m, n = 1003, 70
+@pytest.mark.parametrize("m", [1003, 16383, 16389])
+def test_short_rows(cuda, p, k, m):
+    n = 70
     A, B, C = gen.dense_zp(1, m, k, p), gen.dense_zp(2, k, n, p), gen.dense_zp(3, m, n, p)
     cuda.set_gemm_kernel(2)
     try:
